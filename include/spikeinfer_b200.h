@@ -827,6 +827,33 @@ typedef struct spk_latent_prefill_args {
 } spk_latent_prefill_args;
 int spk_latent_prefill(const spk_latent_prefill_args* args, void* stream);
 
+/* Causal attention of prompt portions over the packed pools, 16-bit outputs (SPK_BF16 or SPK_F16), head_dim 64 or 128
+ * (spk_spike_prefill_form): token i of a portion sees the `context` keys before it and tokens 0 .. i of the portion, whose K and V are in
+ * the pools already.  out[t, token, head] = softmax(popc(q & k) * scale) V.  Strides are in elements (words for the pools); `portions`
+ * and `args` are host memory, `table` a device pointer.  Block ids outside the pool count as keys without spikes and set SPK_STATUS_BAD_BLOCK. */
+typedef struct spk_spike_portion {
+    const int32_t* table;       /* the sequence's block table, table_len entries */
+    int32_t start, tokens;      /* the portion's tokens in q_packed and out */
+    int32_t context;            /* keys cached before them */
+    int32_t table_len;
+} spk_spike_portion;
+typedef struct spk_spike_prefill_args {
+    const void* q_packed;       /* int32 [T, n_tok, num_q_heads, words] */
+    int64_t sq_t, sq_tok, sq_h;
+    const void* k_pool;
+    int64_t sk_t, sk_h, sk_blk, sk_slot;
+    const void* v_pool;
+    int64_t sv_t, sv_h, sv_blk, sv_slot;
+    void* out;
+    int64_t so_t, so_tok, so_h;
+    int64_t n_tok, num_blocks;
+    int32_t T, num_q_heads, num_kv_heads, head_dim, block_size, dtype;
+    float scale, _pad;
+    uint32_t* status;
+} spk_spike_prefill_args;
+int spk_spike_prefill_form(int head_dim, int out_dtype);
+int spk_spike_prefill(const spk_spike_prefill_args* args, const spk_spike_portion* portions, int n_portions, void* stream);
+
 /* Gated delta rule with one decay per head and key channel:
  *   q, k, v <- silu(causal convolution of the projections, `taps` taps per channel);  q, k <- unit vectors per head, q * dim^-1/2;
  *   S <- g * S;  u = beta (v - S^T k);  S <- S + k u^T;  o = S^T q;  g = exp(-exp(a_log) softplus(a + dt_bias)), beta = sigmoid(b);

@@ -201,6 +201,19 @@ class DeltaArgs(Structure):
                        "i n_chunks n_portions heads kv_heads dim vdim taps dtype; f eps _pad; p status")
 
 
+class SpikePortion(Structure):
+    """Mirror of ``spk_spike_portion``."""
+
+    _fields_ = _fields("p table; i start tokens context table_len")
+
+
+class SpikePrefillArgs(Structure):
+    """Mirror of ``spk_spike_prefill_args``."""
+
+    _fields_ = _fields("p q_packed; l sq_t sq_tok sq_h; p k_pool; l sk_t sk_h sk_blk sk_slot; p v_pool; l sv_t sv_h sv_blk sv_slot; p out; "
+                       "l so_t so_tok so_h n_tok num_blocks; i T num_q_heads num_kv_heads head_dim block_size dtype; f scale _pad; p status")
+
+
 # name -> (restype, argtypes); every symbol include/spikeinfer_b200.h declares
 I64P = POINTER(c_int64)
 SIGNATURES = {
@@ -285,6 +298,8 @@ SIGNATURES = {
     "spk_latent_prefill_form": (c_int, [c_int] * 5),
     "spk_latent_gather": (c_int, [POINTER(LatentGatherArgs), c_void_p]),
     "spk_latent_prefill": (c_int, [POINTER(LatentPrefillArgs), c_void_p]),
+    "spk_spike_prefill_form": (c_int, [c_int, c_int]),
+    "spk_spike_prefill": (c_int, [POINTER(SpikePrefillArgs), POINTER(SpikePortion), c_int, c_void_p]),
     "spk_delta_step": (c_int, [POINTER(DeltaArgs), c_void_p]),
     "spk_delta_chunk_tokens": (c_int, [c_int] * 3),
     "spk_delta_workspace_bytes": (c_int64, [c_int, c_int64] + [c_int] * 5),

@@ -15,7 +15,7 @@ import torch
 import torch.nn.functional as F
 
 from .kernels import (LifSiteSpec, gather_kv_unpacked, gather_kv_unpacked_batch, lif_pack_scatter, pack_spikes,
-                      paged_spike_attn_decode)
+                      paged_spike_attn_decode, paged_spike_attn_prefill, spike_prefill_form)
 from .kernels.packing import packed_width
 
 
@@ -278,7 +278,7 @@ def fused_qkv_attention(qkv: torch.Tensor, lif_q, lif_k, lif_v, k_cache, v_cache
 
     One launch runs the LIF recurrence of the q, k and v sites, packs the spikes and scatters K/V
     straight into the pools through ``meta.slot_mapping``; the decode rows then go to the popcount
-    kernel.  Dense q spikes are produced only when the batch holds prefill chunks.  ``lif_*`` are
+    kernel, prefill chunks to the tensor-core kernel (dense q spikes are produced only for chunks it does not cover).  ``lif_*`` are
     ``(beta, threshold)`` pairs.  ``rope = (cos, sin)``, each ``[n_tok, head_dim]`` in ``qkv.dtype``, applies the
     rotary embedding to the q and k currents inside the same launch; without it ``qkv`` must already be
     rotated.  Returns ``[T, n_tok, H_q * head_dim]`` in ``qkv.dtype``.
@@ -293,7 +293,9 @@ def fused_qkv_attention(qkv: torch.Tensor, lif_q, lif_k, lif_v, k_cache, v_cache
     q_packed = torch.empty((T, n_tok, hq, W), dtype=torch.int32, device=device)
     q_dense = None
     packed_prefill = meta.num_prefills and meta.prefill_row_tables is not None
-    if meta.num_prefills and not packed_prefill:
+    # 16-bit outputs attend on the tensor cores from the packed pools; fp32 keeps 32-bit probabilities (SDPA on unpacked spikes)
+    tensor_prefill = meta.num_prefills and not packed_prefill and spike_prefill_form(d, dtype)
+    if meta.num_prefills and not packed_prefill and not tensor_prefill:
         q_dense = torch.empty((T, hq, n_tok, d), dtype=dtype, device=device)
     kc, vc = _flat_pool(k_cache), _flat_pool(v_cache)
     num_slots = kc.shape[2]
@@ -321,6 +323,10 @@ def fused_qkv_attention(qkv: torch.Tensor, lif_q, lif_k, lif_v, k_cache, v_cache
         paged_spike_attn_decode(q_packed[:, n_dec:n_dec + n_pre], k_cache, v_cache, meta.prefill_row_tables,
                                 meta.prefill_row_lens, head_dim=d, block_size=meta.block_size, num_q_heads=hq,
                                 num_kv_heads=hkv, out=out[:, n_dec:n_dec + n_pre], status=meta.status)
+    elif tensor_prefill:
+        paged_spike_attn_prefill(q_packed, kc, vc, meta.prefill_block_tables, meta.prefill_query_starts, meta.prefill_query_lens,
+                                 meta.prefill_context_lens, out, head_dim=d, block_size=meta.block_size, num_q_heads=hq, num_kv_heads=hkv,
+                                 status=meta.status)
     elif meta.num_prefills:
         _prefill_chunks(q_dense, k_cache, v_cache, meta, out, hq, hkv, d)
     return out.view(T, n_tok, hq * d)

@@ -31,7 +31,7 @@ NO_FMA_CONTRACTION = {"spk_lif.cu", "spk_norm.cu"}
 # Groups of translation units a model may need; "core" (C ABI basics, batch metadata, sampling) is part of every library.
 COMPONENTS = {
     "core": ("spk_capi.cu", "spk_meta.cu", "spk_sample.cu"),
-    "spike": ("spk_attn.cu", "spk_attn_stream.cu", "spk_lif.cu", "spk_norm.cu", "spk_pack.cu"),
+    "spike": ("spk_attn.cu", "spk_attn_prefill.cu", "spk_attn_stream.cu", "spk_lif.cu", "spk_norm.cu", "spk_pack.cu"),
     "dense": ("spk_postnorm.cu", "spk_paged_attn.cu", "spk_sigmoid_prefill.cu", "spk_sigmoid_decode.cu", "spk_decay.cu",
               "spk_decay_mma.cu"),
     "latent": ("spk_prenorm.cu", "spk_experts.cu", "spk_experts_mma.cu", "spk_latent.cu", "spk_latent_decode.cu",

@@ -1,0 +1,393 @@
+// Prefill attention over the packed spike pools on the fifth-generation tensor cores (tcgen05), 16-bit outputs, head_dim 64 or 128.
+//
+// CTA = (128 query tokens of one portion, timestep, query head), two CTAs per SM.  Nine warps:
+//  * warps 4-7 read the packed K and V rows of 64 keys through the block table and expand their bits: K to bytes (e4m3 0 or 1), V to
+//    halves (0 or 1), in the swizzled operand layouts; a stage ahead of the MMAs, the next stage's words already in registers;
+//  * warp 8 issues S = Q K^T (kind::f8f6f4, exact: scores are counts) into one of two TMEM buffers and O += P V (kind::f16, P read from
+//    TMEM).  S of step t + 1 goes out before the wait for the weights of step t, so scores are ready when a step's weights are done;
+//  * warps 0-3, a thread per query row, turn scores into weights exp((score - popc(q)) * scale) * 2^14 in halves.  popc(q) bounds every
+//    score of the row: no running maximum, no rescaling of O, and 2^14 keeps the smallest possible weight a normal half.  Their 32-bit
+//    sum, also times 2^14, divides the row at the end.
+// Bits expand in an order that is cheapest for the bit tricks (byte b of word j: bit j + 8 b; half h: bit j + 16 h), the same for Q and K;
+// V's column order is undone when a row is stored.
+//
+// What bounds it: the special-function pipe, one exponential per (query, key) pair, 1024 cycles per 128 x 128 pairs; S and O take about 400 at
+// 64 channels.  Why 64 keys per step: S is double-buffered beside O of up to 128 channels within 256 TMEM columns, so that two CTAs fit an
+// SM and one's set-up and drain hide behind the other's steps.
+// Measured, whole fused_qkv_attention calls against SDPA on spikes unpacked to bf16: 16 x 512 tokens, 14/2 heads of 64, 608 -> 152 us; three
+// portions of 766 to 1531 tokens behind 700 cached, 28/4 heads of 128, 4922 -> 375 us; error against 64 bits 1.8e-3 -> 1.6e-3.
+#include <algorithm>
+
+#include "spk_tensor.cuh"
+
+namespace {
+
+using namespace spk_tc;
+
+constexpr int kRows = 128;                  // query tokens per CTA
+constexpr int kKeys = 64;                   // keys per step
+constexpr int kStages = 3;
+constexpr int kThreads = 288;
+constexpr int kQBytes = kRows * 128;        // rows of 128 bytes; 64 channels use the first half
+constexpr int kKBytes = kKeys * 128;
+constexpr int kVColTile = kKeys * 128;      // 64 channels
+constexpr uint32_t kTmemS = 0, kTmemO = 128;
+constexpr int kMaxPortions = 48, kMaxTiles = 512;
+constexpr float kLog2e = 1.4426950408889634f;
+
+struct Launch {
+    spk_spike_prefill_args a;
+    spk_spike_portion portions[kMaxPortions];
+    uint32_t tiles[kMaxTiles];  // portion << 24 | query tile of the portion
+    int vec;                    // rows of the output allow 16-byte stores
+};
+
+struct Bars {
+    uint64_t kv_full[kStages], kv_free[kStages], s_full[2], p_full[2], q_full, o_full;
+    int abort;
+    uint32_t tmem;
+};
+
+__device__ __forceinline__ void mma_f8_by(uint32_t who, uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, bool acc) {
+    asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 q, %5, 0;\n\t"
+                 "@q tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], %1, %2, %3, p;\n\t}\n"
+                 ::"r"(d), "l"(a), "l"(b), "r"(idesc), "r"(acc ? 1 : 0), "r"(who) : "memory");
+}
+__device__ __forceinline__ void mma_ts_by(uint32_t who, uint32_t d, uint32_t a, uint64_t b, uint32_t idesc, bool acc) {
+    asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 q, %5, 0;\n\t"
+                 "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}\n"
+                 ::"r"(d), "r"(a), "l"(b), "r"(idesc), "r"(acc ? 1 : 0), "r"(who) : "memory");
+}
+
+// One word's 32 channels as e4m3 bytes (0x38 is 1.0) at 16-byte groups 2 w and 2 w + 1 of a 128-byte row.
+__device__ __forceinline__ void expand_bytes(uint8_t* row, int r, int w, uint32_t bits) {
+#pragma unroll
+    for (int g = 0; g < 2; ++g) {
+        uint4 v;
+        uint32_t* p = reinterpret_cast<uint32_t*>(&v);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) p[j] = ((bits >> (4 * g + j)) & 0x01010101u) * 0x38u;
+        *reinterpret_cast<uint4*>(row + (((2 * w + g) ^ (r & 7)) << 4)) = v;
+    }
+}
+// The same as halves (0x3c00 is 1.0), four groups of a 64-channel column tile.
+__device__ __forceinline__ void expand_halves(uint8_t* row, int r, int w, uint32_t bits) {
+#pragma unroll
+    for (int g = 0; g < 4; ++g) {
+        uint4 v;
+        uint32_t* p = reinterpret_cast<uint32_t*>(&v);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) p[j] = ((bits >> (4 * g + j)) & 0x00010001u) * 0x3c00u;
+        *reinterpret_cast<uint4*>(row + (((4 * (w & 1) + g) ^ (r & 7)) << 4)) = v;
+    }
+}
+
+template <typename TO>
+__device__ __forceinline__ uint32_t pack_pair(float lo, float hi);
+template <>
+__device__ __forceinline__ uint32_t pack_pair<__nv_bfloat16>(float lo, float hi) { return pack_bf16(lo, hi); }
+template <>
+__device__ __forceinline__ uint32_t pack_pair<__half>(float lo, float hi) {
+    const __half2 v = __floats2half2_rn(lo, hi);
+    return *reinterpret_cast<const uint32_t*>(&v);
+}
+
+template <int W>
+constexpr int shared_bytes() { return kQBytes + kStages * (kKBytes + W / 2 * kVColTile) + 1024 + 256; }
+
+template <int W, typename TO>
+__global__ void __launch_bounds__(kThreads, 2)
+spike_prefill_kernel(const __grid_constant__ Launch l) {
+    constexpr int kVBytes = W / 2 * kVColTile;
+    extern __shared__ uint8_t raw[];
+    uint8_t* q_s = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(raw) + 1023) & ~uintptr_t(1023));
+    uint8_t* k_s = q_s + kQBytes;
+    uint8_t* v_s = k_s + kStages * kKBytes;
+    Bars* bars = reinterpret_cast<Bars*>(v_s + kStages * kVBytes);
+    const spk_spike_prefill_args& a = l.a;
+    const int warp = threadIdx.x >> 5;
+    const int h = blockIdx.x % a.num_q_heads, ts = blockIdx.x / a.num_q_heads;
+    const int g = h / (a.num_q_heads / a.num_kv_heads);
+    const uint32_t tile = l.tiles[blockIdx.y];
+    const spk_spike_portion& por = l.portions[tile >> 24];
+    const int first = static_cast<int>(tile & 0xffffffu) * kRows;  // query row of the portion
+    const int nq = por.tokens - first < kRows ? por.tokens - first : kRows;
+    const int pos0 = por.context + first;
+    const int keys = pos0 + nq;
+    const int steps = (keys + kKeys - 1) / kKeys;
+
+    if (threadIdx.x == 0) {
+        for (int i = 0; i < kStages; ++i) {
+            mbar_init(smem_u32(&bars->kv_full[i]), 128);
+            mbar_init(smem_u32(&bars->kv_free[i]), 1);
+        }
+        for (int i = 0; i < 2; ++i) {
+            mbar_init(smem_u32(&bars->s_full[i]), 1);
+            mbar_init(smem_u32(&bars->p_full[i]), 128);
+        }
+        mbar_init(smem_u32(&bars->q_full), 128);
+        mbar_init(smem_u32(&bars->o_full), 1);
+        bars->abort = 0;
+    }
+    if (warp == 8) tmem_alloc(smem_u32(&bars->tmem), 256);
+    fence_async_shared();
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = bars->tmem;
+    volatile int* abort = &bars->abort;
+
+    if (warp >= 4 && warp < 8) {  // ---- K and V bits to operands: thread = (key, half of the words)
+        const int e = threadIdx.x - 128, key = e & (kKeys - 1), half = e >> 6;
+        const int bs_log2 = 31 - __clz(a.block_size), bs_mask = a.block_size - 1;
+        const uint32_t* kp = static_cast<const uint32_t*>(a.k_pool) + ts * a.sk_t + g * a.sk_h + half * (W / 2);
+        const uint32_t* vp = static_cast<const uint32_t*>(a.v_pool) + ts * a.sv_t + g * a.sv_h + half * (W / 2);
+        auto entry = [&](int t) {
+            const int j = t * kKeys + key;
+            return j < keys ? por.table[j >> bs_log2] : -1;
+        };
+        uint32_t kw[W / 2], vw[W / 2];
+        auto fetch = [&](int t, int block) {
+            const int j = t * kKeys + key;
+#pragma unroll
+            for (int i = 0; i < W / 2; ++i) kw[i] = vw[i] = 0u;
+            if (j >= keys) return;
+            if (block < 0 || block >= a.num_blocks) {
+                spk_flag(a.status, SPK_STATUS_BAD_BLOCK);
+                return;
+            }
+            const int64_t ko = block * a.sk_blk + (j & bs_mask) * a.sk_slot, vo = block * a.sv_blk + (j & bs_mask) * a.sv_slot;
+#pragma unroll
+            for (int i = 0; i < W / 2; ++i) {
+                kw[i] = kp[ko + i];
+                vw[i] = vp[vo + i];
+            }
+        };
+        int block = entry(1);
+        fetch(0, entry(0));
+        for (int t = 0; t < steps; ++t) {
+            const int stage = t % kStages;
+            uint32_t kb[W / 2], vb[W / 2];
+#pragma unroll
+            for (int i = 0; i < W / 2; ++i) {
+                kb[i] = kw[i];
+                vb[i] = vw[i];
+            }
+            if (t + 1 < steps) {
+                fetch(t + 1, block);
+                block = entry(t + 2);
+            }
+            if (t >= kStages && !__all_sync(~0u, mbar_wait(smem_u32(&bars->kv_free[stage]), ((t / kStages) - 1) & 1, abort))) break;
+            uint8_t* kr = k_s + stage * kKBytes + key * 128;
+            uint8_t* vr = v_s + stage * kVBytes + key * 128;
+#pragma unroll
+            for (int i = 0; i < W / 2; ++i) {
+                const int w = half * (W / 2) + i;
+                expand_bytes(kr, key, w, kb[i]);
+                expand_halves(vr + (w >> 1) * kVColTile, key, w, vb[i]);
+            }
+            fence_async_shared();
+            mbar_arrive(smem_u32(&bars->kv_full[stage]));
+        }
+    } else if (warp == 8) {  // ---- MMAs
+        constexpr uint32_t s_desc = (1u << 4) | (static_cast<uint32_t>(kKeys >> 3) << 17) | (static_cast<uint32_t>(kRows >> 4) << 24);
+        constexpr uint32_t o_desc = (1u << 4) | (1u << 16) | (static_cast<uint32_t>(W * 32 >> 3) << 17) | (static_cast<uint32_t>(kRows >> 4) << 24);
+        const uint32_t who = elect_one();
+        auto scores = [&](int t) {
+            const int stage = t % kStages;
+            if (!mbar_wait(smem_u32(&bars->kv_full[stage]), (t / kStages) & 1, abort)) return false;
+            tc_fence_after();
+            const uint64_t qd = desc_sw128(smem_u32(q_s), 16, 1024), kd = desc_sw128(smem_u32(k_s + stage * kKBytes), 16, 1024);
+#pragma unroll
+            for (int s = 0; s < W; ++s)  // 32 channels (32 bytes of a row) per MMA
+                mma_f8_by(who, tmem + kTmemS + (t & 1) * kKeys, qd + 2 * s, kd + 2 * s, s_desc, s > 0);
+            if (who) mma_commit(smem_u32(&bars->s_full[t & 1]));
+            return true;
+        };
+        bool ok = __all_sync(~0u, mbar_wait(smem_u32(&bars->q_full), 0, abort)) && __all_sync(~0u, scores(0));
+        for (int t = 0; ok && t < steps; ++t) {
+            const int stage = t % kStages, buf = t & 1;
+            // MMAs of one thread run in order: the buffer's previous weights (step t - 1) have been read before S overwrites them
+            if (t + 1 < steps) ok = __all_sync(~0u, scores(t + 1));
+            ok = ok && __all_sync(~0u, mbar_wait(smem_u32(&bars->p_full[buf]), (t >> 1) & 1, abort));
+            if (!ok) break;
+            tc_fence_after();
+            const uint64_t vd = desc_sw128(smem_u32(v_s + stage * kVBytes), kVColTile, 1024);
+#pragma unroll
+            for (int s = 0; s < kKeys / 16; ++s)
+                mma_ts_by(who, tmem + kTmemO, tmem + kTmemS + buf * kKeys + s * 8, vd + s * (2048 >> 4), o_desc, t > 0 || s > 0);
+            if (who) mma_commit(smem_u32(&bars->kv_free[stage]));
+            __syncwarp();
+        }
+        if (who) mma_commit(smem_u32(&bars->o_full));
+        mbar_wait(smem_u32(&bars->o_full), 0);
+    } else {  // ---- scores to weights: thread = query row
+        const int r = threadIdx.x;
+        const int64_t token = por.start + first + r;
+        float sum = 0.0f;
+        uint64_t c1, c0;
+        {
+            const uint32_t* q = static_cast<const uint32_t*>(a.q_packed) + ts * a.sq_t + token * a.sq_tok + h * a.sq_h;
+            int ones = 0;
+#pragma unroll
+            for (int w = 0; w < W; ++w) {
+                const uint32_t bits = r < nq ? q[w] : 0u;
+                ones += __popc(bits);
+                expand_bytes(q_s + r * 128, r, w, bits);
+            }
+            fence_async_shared();
+            mbar_arrive(smem_u32(&bars->q_full));
+            const float c = a.scale * kLog2e, b = 14.0f - ones * c;
+            c1 = f2_pack(c, c);
+            c0 = f2_pack(b, b);
+        }
+        const uint32_t lanes = static_cast<uint32_t>(warp * 32) << 16;
+        uint64_t sums = f2_pack(0.0f, 0.0f);
+        bool ok = true;
+        for (int t = 0; t < steps; ++t) {
+            ok = __all_sync(~0u, mbar_wait(smem_u32(&bars->s_full[t & 1]), (t >> 1) & 1, abort));
+            if (!ok) break;
+            tc_fence_after();
+            const uint32_t at = tmem + lanes + kTmemS + (t & 1) * kKeys;
+            const int last = pos0 + r - t * kKeys;  // last visible column of this row
+#pragma unroll 1
+            for (int c = 0; c < 2; ++c) {
+                uint32_t sc[32];
+                tmem_ld32(at + c * 32, sc);
+                tmem_wait_ld(sc);
+                const int seen = last - c * 32;
+                const bool whole = __all_sync(~0u, seen >= 31);
+                uint32_t p[16];
+#pragma unroll
+                for (int i = 0; i < 16; ++i) {
+                    float x, y;
+                    f2_unpack(f2_fma(f2_pack(__uint_as_float(sc[2 * i]), __uint_as_float(sc[2 * i + 1])), c1, c0), x, y);
+                    x = ex2(x);
+                    y = ex2(y);
+                    if (!whole) {
+                        x = 2 * i <= seen ? x : 0.0f;
+                        y = 2 * i + 1 <= seen ? y : 0.0f;
+                    }
+                    sums = f2_add(sums, f2_pack(x, y));
+                    p[i] = pack_pair<__half>(x, y);
+                }
+                tmem_st16(at + c * 16, p);  // over columns of this half that have been read
+            }
+            tmem_wait_st();
+            tc_fence_before();
+            mbar_arrive(smem_u32(&bars->p_full[t & 1]));
+        }
+        float x, y;
+        f2_unpack(sums, x, y);
+        sum = x + y;
+        ok = __all_sync(~0u, ok && mbar_wait(smem_u32(&bars->o_full), 0, abort) && *abort == 0);
+        tc_fence_after();
+        const float inv = ok && r < nq ? 1.0f / sum : 0.0f;
+        TO* out = static_cast<TO*>(a.out) + ts * a.so_t + token * a.so_tok + h * a.so_h;
+#pragma unroll
+        for (int w = 0; w < W; ++w) {
+            uint32_t o[32];
+            tmem_ld32(tmem + lanes + kTmemO + w * 32, o);
+            tmem_wait_ld(o);
+            if (r < nq) {
+                // column 2 j is channel j of the word, column 2 j + 1 channel j + 16
+#pragma unroll
+                for (int m = 0; m < 4; ++m) {
+                    uint32_t v[4];
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) {
+                        const int j = (m & 1) * 8 + 2 * k;
+                        const float lo = __uint_as_float(o[2 * j + (m >> 1)]) * inv, hi = __uint_as_float(o[2 * j + 2 + (m >> 1)]) * inv;
+                        v[k] = ok ? pack_pair<TO>(lo, hi) : 0u;
+                    }
+                    TO* dst = out + w * 32 + m * 8;
+                    if (l.vec) {
+                        *reinterpret_cast<uint4*>(dst) = make_uint4(v[0], v[1], v[2], v[3]);
+                    } else {
+#pragma unroll
+                        for (int k = 0; k < 4; ++k) {
+                            reinterpret_cast<uint16_t*>(dst)[2 * k] = static_cast<uint16_t>(v[k]);
+                            reinterpret_cast<uint16_t*>(dst)[2 * k + 1] = static_cast<uint16_t>(v[k] >> 16);
+                        }
+                    }
+                }
+            }
+            __syncwarp();
+        }
+    }
+    __syncwarp();
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    if (threadIdx.x == 0 && *abort != 0) spk_flag(a.status, SPK_STATUS_DEVICE_WAIT_EXPIRED);
+    if (warp == 8) tmem_dealloc(tmem, 256);
+}
+
+template <int W, typename TO>
+int launch(const Launch& l, int tiles, cudaStream_t s) {
+    constexpr int bytes = shared_bytes<W>();
+    static_assert(sizeof(Bars) <= 256 && 2 * bytes <= 224 * 1024, "shared memory of two CTAs");
+    static_assert(sizeof(Launch) <= 4096, "kernel parameters");
+    const cudaError_t e = cudaFuncSetAttribute(spike_prefill_kernel<W, TO>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    if (e != cudaSuccess) return spk_set_cuda_error(e);
+    spike_prefill_kernel<W, TO><<<dim3(l.a.num_q_heads * l.a.T, tiles), kThreads, bytes, s>>>(l);
+    SPK_CHECK_LAUNCH();
+    return SPK_OK;
+}
+
+}  // namespace
+
+extern "C" int spk_spike_prefill_form(int head_dim, int out_dtype) {
+    return (head_dim == 64 || head_dim == 128) && (out_dtype == SPK_BF16 || out_dtype == SPK_F16);
+}
+
+extern "C" int spk_spike_prefill(const spk_spike_prefill_args* args, const spk_spike_portion* portions, int n_portions, void* stream) {
+    if (args == nullptr || (n_portions > 0 && portions == nullptr)) return SPK_ERR_NULL_POINTER;
+    const spk_spike_prefill_args& a = *args;
+    if (!spk_spike_prefill_form(a.head_dim, a.dtype)) return SPK_ERR_UNSUPPORTED;
+    if (a.T < 1 || a.num_q_heads < 1 || a.num_kv_heads < 1 || a.num_q_heads % a.num_kv_heads != 0 || a.num_blocks < 1 || a.block_size < 1 ||
+        (a.block_size & (a.block_size - 1)) != 0 || n_portions < 0)
+        return SPK_ERR_BAD_SHAPE;
+    if (!(a.scale > 0.0f) || a.scale * a.head_dim > 16.0f) return SPK_ERR_UNSUPPORTED;  // the smallest weight has to stay a normal half
+    if (a.q_packed == nullptr || a.k_pool == nullptr || a.v_pool == nullptr || a.out == nullptr) return SPK_ERR_NULL_POINTER;
+    const int64_t heads = static_cast<int64_t>(a.num_q_heads) * a.T;
+    if (heads > 0x7fffffff) return SPK_ERR_TOO_LARGE;
+    for (int i = 0; i < n_portions; ++i) {
+        const spk_spike_portion& p = portions[i];
+        if (p.tokens < 0 || p.context < 0 || p.start < 0 || p.start > a.n_tok || p.tokens > a.n_tok - p.start) return SPK_ERR_BAD_SHAPE;
+        const int64_t keys = static_cast<int64_t>(p.context) + p.tokens;
+        if (p.tokens > 0 && p.table == nullptr) return SPK_ERR_NULL_POINTER;
+        if (keys > 0x7fffffff - 2 * kKeys) return SPK_ERR_TOO_LARGE;
+        if (p.tokens > 0 && keys > p.table_len * a.block_size) return SPK_ERR_BAD_SHAPE;
+    }
+    Launch l;
+    l.a = a;
+    l.vec = reinterpret_cast<uintptr_t>(a.out) % 16 == 0 && a.so_t % 8 == 0 && a.so_tok % 8 == 0 && a.so_h % 8 == 0;
+    int held = 0, tiles = 0, keys_of[kMaxTiles] = {}, rc = SPK_OK;
+    auto flush = [&]() {
+        // the tiles that see the most keys start first
+        uint32_t order[kMaxTiles];
+        int by[kMaxTiles];
+        for (int i = 0; i < tiles; ++i) by[i] = i;
+        std::stable_sort(by, by + tiles, [&](int x, int y) { return keys_of[x] > keys_of[y]; });
+        for (int i = 0; i < tiles; ++i) order[i] = l.tiles[by[i]];
+        std::copy(order, order + tiles, l.tiles);
+        const cudaStream_t s = spk_stream(stream);
+        if (tiles > 0) {
+            if (a.head_dim == 64) rc = a.dtype == SPK_BF16 ? launch<2, __nv_bfloat16>(l, tiles, s) : launch<2, __half>(l, tiles, s);
+            else rc = a.dtype == SPK_BF16 ? launch<4, __nv_bfloat16>(l, tiles, s) : launch<4, __half>(l, tiles, s);
+        }
+        held = tiles = 0;
+    };
+    for (int i = 0; i < n_portions && rc == SPK_OK; ++i) {
+        const int n = (portions[i].tokens + kRows - 1) / kRows;
+        for (int t = 0; t < n && rc == SPK_OK; ++t) {
+            if (t == 0 || held == 0) l.portions[held++] = portions[i];
+            l.tiles[tiles] = static_cast<uint32_t>(held - 1) << 24 | static_cast<uint32_t>(t);
+            keys_of[tiles] = portions[i].context + std::min((t + 1) * kRows, portions[i].tokens);
+            if (++tiles == kMaxTiles || (held == kMaxPortions && t + 1 == n)) flush();
+        }
+    }
+    if (rc == SPK_OK) flush();
+    return rc;
+}

@@ -17,7 +17,9 @@ from .spike_attention import (
     gather_kv_unpacked_batch,
     paged_spike_attn_decode,
     paged_spike_attn_decode_noalloc,
+    paged_spike_attn_prefill,
     qk_scores,
+    spike_prefill_form,
 )
 
 __all__ = [
@@ -39,6 +41,8 @@ __all__ = [
     "BITS_PER_WORD",
     "paged_spike_attn_decode",
     "paged_spike_attn_decode_noalloc",
+    "paged_spike_attn_prefill",
+    "spike_prefill_form",
     "gather_kv_unpacked",
     "gather_kv_unpacked_batch",
     "qk_scores",

@@ -7,6 +7,7 @@ is :224-244.  ``qk_scores`` exposes the exact integer scores for checking.
 from __future__ import annotations
 
 import math
+from ctypes import byref
 
 import torch
 
@@ -171,6 +172,44 @@ def gather_kv_unpacked_batch(cache: torch.Tensor, block_tables: torch.Tensor, se
                                               out.data_ptr(), _lib.dtype_code(dtype), _lib.ptr(status),
                                               _lib.current_stream(cache.device))
     _lib.check(rc, "spk_gather_kv_unpacked_batch")
+    return out
+
+
+def spike_prefill_form(head_dim: int, dtype: torch.dtype) -> bool:
+    """Whether :func:`paged_spike_attn_prefill` covers this head size and output type."""
+    return dtype in (torch.bfloat16, torch.float16) and bool(_lib.load().spk_spike_prefill_form(head_dim, _lib.dtype_code(dtype)))
+
+
+def paged_spike_attn_prefill(q_packed: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, block_tables: list[torch.Tensor],
+                             starts: list[int], lens: list[int], contexts: list[int], out: torch.Tensor, *, head_dim: int,
+                             block_size: int, num_q_heads: int, num_kv_heads: int, status: torch.Tensor | None = None) -> torch.Tensor:
+    """Causal attention of prompt portions against the packed pools that already hold their K and V, one launch for all of them.
+
+    Portion i is tokens ``starts[i] .. starts[i] + lens[i] - 1`` of ``q_packed`` int32 ``[T, n_tok, H_q, W]`` and of ``out``
+    ``[T, n_tok, H_q, head_dim]`` (16-bit), behind ``contexts[i]`` cached keys; ``block_tables[i]`` is its sequence's table."""
+    T, n_tok, n_heads, words = q_packed.shape
+    if words != packed_width(head_dim) or n_heads != num_q_heads:
+        raise ValueError(f"q has {n_heads} heads of {words} words, expected {num_q_heads} of {packed_width(head_dim)}")
+    _lib.require_cuda(q_packed, "paged_spike_attn_prefill q_packed")
+    dev = q_packed.device
+    if q_packed.stride(3) != 1 or out.stride(3) != 1 or out.shape != (T, n_tok, n_heads, head_dim):
+        raise ValueError("q_packed and out must have a contiguous last axis, out [T, n_tok, H_q, head_dim]")
+    if not len(block_tables) == len(starts) == len(lens) == len(contexts):
+        raise ValueError("one table, start, length and context per portion")
+    if T == 0 or not lens:
+        return out
+    tables = [t if t.dtype == torch.int32 and t.device == dev and t.is_contiguous() else t.to(device=dev, dtype=torch.int32).contiguous()
+              for t in block_tables]
+    portions = (_lib.SpikePortion * len(lens))(*[(t.data_ptr(), s, n, c, t.numel()) for t, s, n, c in zip(tables, starts, lens, contexts)])
+    sk, sv = _pool_strides(k_cache, block_size), _pool_strides(v_cache, block_size)
+    a = _lib.SpikePrefillArgs(q_packed.data_ptr(), q_packed.stride(0), q_packed.stride(1), q_packed.stride(2), k_cache.data_ptr(), *sk[:4],
+                              v_cache.data_ptr(), *sv[:4], out.data_ptr(), out.stride(0), out.stride(1), out.stride(2), n_tok, min(sk[4], sv[4]),
+                              T, num_q_heads, num_kv_heads, head_dim, block_size, _lib.dtype_code(out.dtype), 1.0 / math.sqrt(head_dim), 0.0,
+                              _lib.ptr(status))
+    lib = _lib.load()
+    with torch.cuda.device(dev):
+        rc = lib.spk_spike_prefill(byref(a), portions, len(lens), _lib.current_stream(dev))
+    _lib.check(rc, "spk_spike_prefill")
     return out
 
 

@@ -426,3 +426,53 @@ def test_softmax_range_beyond_the_weight_format_is_refused(dev):
     assert lib.spk_attn_decode(*args, 0.125, *tail) == 0
     torch.cuda.synchronize()
     assert torch.isfinite(out).all() and not (out == 7.0).all()
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("heads, kv_heads, dim, page", [(4, 2, 64, 16), (7, 1, 128, 8), (2, 2, 128, 64)])
+@pytest.mark.parametrize("portions", [[(1, 0)], [(1, 63), (2, 64), (128, 0)], [(63, 1), (64, 0), (65, 63)], [(129, 0), (127, 129), (300, 77)],
+                                      [(3, 5)] * 70])
+def test_prefill_attention_on_the_tensor_cores(dev, portions, heads, kv_heads, dim, page, dtype):
+    """Portions at and around the kernel's tiles of 128 queries and steps of 64 keys, behind cached keys, one launch for up to 48 portions
+    and several beyond, against float64 on the unpacked bits."""
+    g = torch.Generator().manual_seed(dim + len(portions))
+    T, n_tok = 2, sum(n for n, _ in portions)
+    need = [-(-(n + c) // page) for n, c in portions]
+    blocks = sum(need) + 1
+    order = torch.randperm(blocks - 1, generator=g).to(torch.int32)
+    word = lambda *s: torch.randint(-2 ** 31, 2 ** 31, s, generator=g, dtype=torch.int64).to(torch.int32)
+    pool = lambda: word(T, kv_heads, blocks * page, dim // 32) & word(T, kv_heads, blocks * page, dim // 32)
+    k, v, q = pool(), pool(), word(T, n_tok, heads, dim // 32)
+    tables = list(order.split(need))
+    starts = [sum(n for n, _ in portions[:i]) for i in range(len(portions))]
+    out = torch.full((T, n_tok, heads, dim), float("nan"), dtype=dtype, device=dev)
+    status = torch.zeros(1, dtype=torch.int32, device=dev)
+    kernels.paged_spike_attn_prefill(q.to(dev), k.to(dev), v.to(dev), [t.to(dev) for t in tables], starts, [n for n, _ in portions],
+                                     [c for _, c in portions], out, head_dim=dim, block_size=page, num_q_heads=heads, num_kv_heads=kv_heads,
+                                     status=status)
+    assert int(status) == 0
+    bits = lambda w: orc.unpack_spikes(w, dim).to(torch.float64)
+    for (n, c), start, table in zip(portions, starts, tables):
+        kk, vv = (orc.gather_kv_unpacked(p, table, n + c, dim, page, torch.float64).repeat_interleave(heads // kv_heads, dim=1) for p in (k, v))
+        score = bits(q[:, start: start + n]).transpose(1, 2) @ kk.mT * dim ** -0.5
+        score.masked_fill_(torch.ones(n, n + c, dtype=torch.bool).triu(c + 1), float("-inf"))
+        want = (score.softmax(-1) @ vv).transpose(1, 2)
+        got = out[:, start: start + n].cpu().to(torch.float64)
+        # one rounding to the output's type, and weights of 11 bits whose sum is one against values of at most one
+        ulp = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11
+        assert bool(((got - want).abs() <= ulp * want.abs() + 2.0 ** -11).all())
+
+
+def test_prefill_attention_flags_blocks_outside_the_pool(dev):
+    q = torch.zeros(1, 20, 2, 2, dtype=torch.int32, device=dev)
+    pool = torch.full((1, 1, 32, 2), -1, dtype=torch.int32, device=dev)
+    out, status = torch.empty(1, 20, 2, 64, dtype=torch.bfloat16, device=dev), torch.zeros(1, dtype=torch.int32, device=dev)
+    run = lambda table, tokens=20: kernels.paged_spike_attn_prefill(q, pool, pool, [torch.tensor(table, dtype=torch.int32, device=dev)], [0], [tokens], [0],
+                                                                    out, head_dim=64, block_size=16, num_q_heads=2, num_kv_heads=1, status=status)
+    run([0, 1])
+    assert int(status) == 0 and torch.equal(out, torch.ones_like(out))
+    run([0, 7])
+    assert int(status) == 1 and float(out[0, 19, 0, 0]) == 0.80078125  # 16 of 20 equal weights, in bf16
+    for table, tokens in (([0], 20), ([0, 1], 21)):  # a table too short, tokens beyond the batch
+        with pytest.raises(Exception):
+            run(table, tokens)
