@@ -358,7 +358,7 @@ extern "C" int spk_spike_prefill(const spk_spike_prefill_args* args, const spk_s
         const int64_t keys = static_cast<int64_t>(p.context) + p.tokens;
         if (p.tokens > 0 && p.table == nullptr) return SPK_ERR_NULL_POINTER;
         if (keys > 0x7fffffff - 2 * kKeys) return SPK_ERR_TOO_LARGE;
-        if (p.tokens > 0 && keys > p.table_len * a.block_size) return SPK_ERR_BAD_SHAPE;
+        if (p.tokens > 0 && keys > static_cast<int64_t>(p.table_len) * a.block_size) return SPK_ERR_BAD_SHAPE;
     }
     Launch l;
     l.a = a;

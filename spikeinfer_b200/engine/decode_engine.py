@@ -353,10 +353,9 @@ class SpikeDecodeEngine(PagedDecodeEngine):
                  graph_buckets: bool = True, short_context_keys: int = 768, max_prefill_tokens: int | None = None) -> None:
         super().__init__(model, num_blocks, block_size, max_num_seqs, max_model_len, use_graph, graph_buckets,
                          short_context_keys, max_prefill_tokens)
-        # True: prompts attend through the packed popcount kernel in one batched launch per layer (3x faster at
-        # 64 prompts of 128 tokens, exact-score fp32 softmax).  False (default): one SDPA per sequence on unpacked
-        # spikes in the model dtype, as the reference does; in bf16 that rounds the probabilities to bf16, so
-        # the two differ at the 1e-2 level there, enough to flip near-tie tokens.  In fp32 they agree to 1e-5.
+        # True: prompts attend through the packed popcount kernel, one row per token, in one batched launch per layer (exact-score fp32
+        # softmax).  False (default): 16-bit models attend on the tensor cores, one launch per layer, weights of 11 bits; fp32 models one SDPA
+        # per sequence on unpacked spikes.  The two differ at the 1e-3 level in 16 bits, enough to flip near-tie tokens.  In fp32 they agree to 1e-5.
         self.packed_prefill = packed_prefill
 
     def _finish_prefill_meta(self, meta: AttentionMetadata) -> None:

@@ -200,7 +200,7 @@ def paged_spike_attn_prefill(q_packed: torch.Tensor, k_cache: torch.Tensor, v_ca
         return out
     tables = [t if t.dtype == torch.int32 and t.device == dev and t.is_contiguous() else t.to(device=dev, dtype=torch.int32).contiguous()
               for t in block_tables]
-    portions = (_lib.SpikePortion * len(lens))(*[(t.data_ptr(), s, n, c, t.numel()) for t, s, n, c in zip(tables, starts, lens, contexts)])
+    portions = (_lib.SpikePortion * len(lens))(*[(t.data_ptr(), int(s), int(n), int(c), t.numel()) for t, s, n, c in zip(tables, starts, lens, contexts)])
     sk, sv = _pool_strides(k_cache, block_size), _pool_strides(v_cache, block_size)
     a = _lib.SpikePrefillArgs(q_packed.data_ptr(), q_packed.stride(0), q_packed.stride(1), q_packed.stride(2), k_cache.data_ptr(), *sk[:4],
                               v_cache.data_ptr(), *sv[:4], out.data_ptr(), out.stride(0), out.stride(1), out.stride(2), n_tok, min(sk[4], sv[4]),
