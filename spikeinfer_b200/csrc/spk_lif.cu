@@ -285,14 +285,6 @@ __device__ __forceinline__ void chain8(const Raw8<TX> (&raw)[4], const float (&b
                                           bits[0], bits[1], bits[2], bits[3])), ...);
 }
 
-// The same with the currents supplied by `cur(t, channel)` (e.g. rotated on the fly).
-template <int MODE, typename F, int... C>
-__device__ __forceinline__ void chain8_of(F&& cur, const float (&b)[8], const float (&th)[8], float (&u)[8],
-                                          uint32_t (&bits)[4], std::integer_sequence<int, C...>) {
-    ((u[C] = lif_chain4<MODE, (1u << C)>(cur(0, C), cur(1, C), cur(2, C), cur(3, C), b[C], th[C], bits[0], bits[1],
-                                          bits[2], bits[3])), ...);
-}
-
 // One timestep of the 8 channels of a segment; bit c of `bits` = spike of channel c.
 template <int MODE, typename TX, int... C>
 __device__ __forceinline__ void step8(Lif (&st)[8], const Raw8<TX>& raw, const float (&b)[8], const float (&th)[8],
@@ -309,6 +301,40 @@ template <>
 __device__ __forceinline__ float round_to<__nv_bfloat16>(float v) { return __bfloat162float(__float2bfloat16_rn(v)); }
 template <>
 __device__ __forceinline__ float round_to<__half>(float v) { return __half2float(__float2half_rn(v)); }
+
+// Rotary embedding of a segment: x * cos + p * sin, every operation rounded to the model dtype as the eager expression
+// (x * cos) + (rotate_half(x) * sin) does; `p` is the partner segment, negated when `negate`.  The 16-bit forms work on pairs: a product of
+// two of their values is exact in 32 bits and a sum of two rounds the same directly or through 32 bits (24 >= 2 * 11 + 2 bits), so
+// one packed operation gives the bits of the 32-bit operation rounded afterwards, in 3 instead of about 20 instructions per pair.
+__device__ __forceinline__ void rotate8(Raw8<float>& x, const Raw8<float>& p, const Raw8<float>& c, const Raw8<float>& s, bool negate) {
+    const float sign = negate ? -1.0f : 1.0f;
+    auto turn = [&](float& xv, float pv, float cv, float sv) { xv = __fadd_rn(__fmul_rn(xv, cv), __fmul_rn(sign * pv, sv)); };
+    turn(x.a.x, p.a.x, c.a.x, s.a.x); turn(x.a.y, p.a.y, c.a.y, s.a.y); turn(x.a.z, p.a.z, c.a.z, s.a.z); turn(x.a.w, p.a.w, c.a.w, s.a.w);
+    turn(x.b.x, p.b.x, c.b.x, s.b.x); turn(x.b.y, p.b.y, c.b.y, s.b.y); turn(x.b.z, p.b.z, c.b.z, s.b.z); turn(x.b.w, p.b.w, c.b.w, s.b.w);
+}
+template <typename T2>
+__device__ __forceinline__ uint32_t rotate2(uint32_t x, uint32_t p, uint32_t c, uint32_t s, uint32_t flip) {
+    const T2* xv = reinterpret_cast<const T2*>(&x);
+    const T2* cv = reinterpret_cast<const T2*>(&c);
+    const T2* sv = reinterpret_cast<const T2*>(&s);
+    p ^= flip;
+    const T2* pv = reinterpret_cast<const T2*>(&p);
+    const T2 r = __hadd2_rn(__hmul2_rn(*xv, *cv), __hmul2_rn(*pv, *sv));
+    return *reinterpret_cast<const uint32_t*>(&r);
+}
+template <typename T2, typename R>
+__device__ __forceinline__ void rotate8_pairs(R& x, const R& p, const R& c, const R& s, bool negate) {
+    const uint32_t flip = negate ? 0x80008000u : 0u;
+    x.v = make_uint4(rotate2<T2>(x.v.x, p.v.x, c.v.x, s.v.x, flip), rotate2<T2>(x.v.y, p.v.y, c.v.y, s.v.y, flip),
+                     rotate2<T2>(x.v.z, p.v.z, c.v.z, s.v.z, flip), rotate2<T2>(x.v.w, p.v.w, c.v.w, s.v.w, flip));
+}
+__device__ __forceinline__ void rotate8(Raw8<__nv_bfloat16>& x, const Raw8<__nv_bfloat16>& p, const Raw8<__nv_bfloat16>& c,
+                                        const Raw8<__nv_bfloat16>& s, bool negate) {
+    rotate8_pairs<__nv_bfloat162>(x, p, c, s, negate);
+}
+__device__ __forceinline__ void rotate8(Raw8<__half>& x, const Raw8<__half>& p, const Raw8<__half>& c, const Raw8<__half>& s, bool negate) {
+    rotate8_pairs<__half2>(x, p, c, s, negate);
+}
 
 // Packs 8 fp32 values (already representable in TX) into the 16/32 bytes of a dense TX row segment.
 template <typename TX>
@@ -574,17 +600,14 @@ __device__ __forceinline__ void fused_site_vec(const spk_lif_site& s, uint32_t u
                 }
                 uint32_t bits[kStepGroup] = {0, 0, 0, 0};
                 if (ROPE && rope) {
-                    // rotary embedding on the fly (T = 4 only, checked on the host): every operation rounded to the
-                    // model dtype, as the eager expression (x * cos) + (rotate_half(x) * sin) does
+                    // rotary embedding on the fly (T = 4 only, checked on the host)
                     Raw8<TX> partner[kStepGroup];
 #pragma unroll
                     for (int i = 0; i < kStepGroup; ++i) partner[i].load(xp + i * sx_t + partner_off);
+#pragma unroll
+                    for (int i = 0; i < kStepGroup; ++i) rotate8(raw[i], partner[i], cr, sr, first_half);
                     float uf[kSeg];
-                    chain8_of<MODE>([&](int t, int c) {
-                        const float a = round_to<TX>(__fmul_rn(raw[t].get(c), cr.get(c)));
-                        const float r = round_to<TX>(__fmul_rn(partner_sign * partner[t].get(c), sr.get(c)));
-                        return round_to<TX>(__fadd_rn(a, r));
-                    }, b, th, uf, bits, std::make_integer_sequence<int, kSeg>{});
+                    chain8<MODE, TX>(raw, b, th, uf, bits, std::make_integer_sequence<int, kSeg>{});
 #pragma unroll
                     for (int c = 0; c < kSeg; ++c) st[c].init(uf[c], th[c]);
                 } else if (t0 == 0) {
@@ -697,7 +720,12 @@ __device__ __forceinline__ void fused_site_vec(const spk_lif_site& s, uint32_t u
 // product): the same copies, arithmetic and stores as fused_site_vec<.., ASYNC, PLAIN> would issue, with the
 // per-token bookkeeping reduced to running pointers and 32-bit counters.  At 11 instructions per element-step that
 // bookkeeping was 40 % of the issue slots of an issue-bound kernel.
-template <typename TX, int MODE>
+//
+// ROPE: q and k sites with the rotary embedding (N / 8 a power of two up to 32, checked on the host): the lanes of a row then share a warp,
+// and a lane reads its partner channels from the slots of the lane that copied them.  Two barriers of the warp per token order those reads
+// against the copies.  It is bound by issue (about 290 instructions per warp and token) and, below 8192 tokens of 14/2 heads, by the latency of
+// its few tokens per lane: 53.5 -> 24.6 us there (1.4 -> 3.1 TB/s of currents), 4.0 TB/s at four times that.
+template <typename TX, int MODE, bool ROPE>
 __device__ __forceinline__ void stream_plain_site(const spk_lif_site& s, uint32_t units, uint32_t per_tok,
                                                   uint32_t per_row, int toks, uint32_t unit, int lane, int64_t n_tok,
                                                   uint32_t* status, uint4* stage, int slots) {
@@ -766,19 +794,41 @@ __device__ __forceinline__ void stream_plain_site(const spk_lif_site& s, uint32_
     uint32_t* wp = wbase != nullptr && !scatter ? wbase + tok0 * so_tok : nullptr;  // running, when rows are the tokens
     const int64_t mem_step = static_cast<int64_t>(s.H) * s.N;
     float* mo = s.mem_out != nullptr ? s.mem_out + (tok0 * s.H + h) * s.N + c0 : nullptr;
+    const bool first_half = 2 * sg < per_row;
+    const int partner = (lane ^ static_cast<int>(per_row >> 1)) - lane;  // in 16-byte slots
+    const TX* cos_p = ROPE ? static_cast<const TX*>(s.rope_cos) + tok0 * s.s_rope_tok + c0 : nullptr;
+    const TX* sin_p = ROPE ? static_cast<const TX*>(s.rope_sin) + tok0 * s.s_rope_tok + c0 : nullptr;
     uint32_t drain = 0;  // byte offset of the stage the next token is read from
 
     for (int j = 0; j < toks; ++j) {
+        const bool live = j < n_mine;
+        Raw8<TX> cr, sr;
+        if (ROPE) {
+            __syncwarp();  // the partner lanes have read the stage that is filled next
+            if (live) {
+                cr.load(cos_p);
+                sr.load(sin_p);
+                cos_p += s.s_rope_tok;
+                sin_p += s.s_rope_tok;
+            }
+        }
         issue();
         cp_async_wait<kStages - 1>();  // this lane's copies for token j have landed
-        const bool live = j < n_mine;
+        if (ROPE) __syncwarp();        // and those of the other lanes
         const bool all_live = __all_sync(0xffffffffu, live);
         const uint4* mine_stage = reinterpret_cast<const uint4*>(reinterpret_cast<const uint8_t*>(stage) + drain);
         drain = drain == (kStages - 1) * stage_bytes ? 0u : drain + stage_bytes;
         if (!live) continue;
         Raw8<TX> raw[kStepGroup];
 #pragma unroll
-        for (int i = 0; i < kStepGroup; ++i) raw[i].from_smem(mine_stage + i * VECS * 32);
+        for (int i = 0; i < kStepGroup; ++i) {
+            raw[i].from_smem(mine_stage + i * VECS * 32);
+            if (ROPE) {
+                Raw8<TX> other;
+                other.from_smem(mine_stage + i * VECS * 32 + partner);
+                rotate8(raw[i], other, cr, sr, first_half);
+            }
+        }
         float uf[kSeg];
         uint32_t bits[kStepGroup] = {0, 0, 0, 0};
         chain8<MODE, TX>(raw, b, th, uf, bits, std::make_integer_sequence<int, kSeg>{});
@@ -808,7 +858,7 @@ __device__ __forceinline__ void stream_plain_site(const spk_lif_site& s, uint32_
 }
 
 template <int MODE, bool ROPE, bool FULL, bool ASYNC, bool PLAIN>
-__global__ void __launch_bounds__(kFusedThreads, (ROPE && !PLAIN) ? 1 : (ASYNC ? 4 : 2))
+__global__ void __launch_bounds__(kFusedThreads, (ROPE && !PLAIN) ? 1 : (ASYNC ? (ROPE ? 3 : 4) : 2))
 lif_pack_scatter_vec_kernel(VecArgs args, int T, int64_t n_tok, uint32_t* status) {
     // A next launch that asked to overlap this one (the attention after the q/k/v sites: it reads only lengths and
     // block tables until this grid has finished) may be placed from now on; without such a launch this does nothing.
@@ -823,9 +873,12 @@ lif_pack_scatter_vec_kernel(VecArgs args, int T, int64_t n_tok, uint32_t* status
     uint4* stage = ASYNC ? stage_smem + (threadIdx.x >> 5) * kStages * args.slots * 32 + lane : nullptr;
 #define SPK_SITE(TX_)                                                                                              \
     do {                                                                                                            \
-        if (ASYNC && PLAIN && FULL && !ROPE)                                                                        \
-            stream_plain_site<TX_, MODE>(s, args.units[site], args.per_tok[site], args.per_row[site], args.toks,    \
-                                         unit, lane, n_tok, status, stage, args.slots);                             \
+        if (ASYNC && PLAIN && FULL && ROPE && s.rope_cos != nullptr)                                                \
+            stream_plain_site<TX_, MODE, true>(s, args.units[site], args.per_tok[site], args.per_row[site],         \
+                                               args.toks, unit, lane, n_tok, status, stage, args.slots);            \
+        else if (ASYNC && PLAIN && FULL)                                                                            \
+            stream_plain_site<TX_, MODE, false>(s, args.units[site], args.per_tok[site], args.per_row[site],        \
+                                                args.toks, unit, lane, n_tok, status, stage, args.slots);           \
         else                                                                                                        \
             fused_site_vec<TX_, MODE, ROPE, FULL, ASYNC, PLAIN>(s, args.units[site], args.per_tok[site],            \
                                                                 args.per_row[site], args.toks, unit, lane, T, n_tok, \
@@ -1079,9 +1132,27 @@ extern "C" int spk_lif_pack_scatter(const spk_lif_site* sites, int n_sites, int 
         }
         int toks = 4;
         while (toks > 1 && (n_tok / toks) * widest < 148LL * 2048) toks >>= 1;
+        bool plain = true;  // packed bits, gated product, final membrane only: the other feature tests fold away
+        bool rows_in_warps = true;  // the lanes of a rotated row share a warp
+        for (int i = 0; i < n_sites; ++i) {
+            plain = plain && sites[i].mem0 == nullptr && sites[i].dense == nullptr;
+            if (sites[i].rope_cos != nullptr) {
+                const int64_t per_row = sites[i].N / kSeg;
+                rows_in_warps = rows_in_warps && per_row <= 32 && (per_row & (per_row - 1)) == 0;
+            }
+        }
+        const bool plain_rope = plain && any_rope && !any_gated && T == kStepGroup;  // the q/k/v launch of a layer
+        plain = plain && !any_rope;
         // Bandwidth-sized launches stream through shared memory (cp.async, kStages tokens in flight per lane).
-        const bool streaming = !any_rope && T <= kStepGroup && toks == 4 && (n_tok / 8) * widest >= 148LL * 2048;
-        if (streaming) toks = 8;
+        // With the rotary embedding the walks are short: 14/2 heads of 64 (112 lanes per token) in bf16, streaming walks of 2 / 4 / 8 tokens
+        // against reading global memory directly: 512 tokens 4.4 / 5.4 / 8.6 against 4.6 us, 1024 5.7 / 6.6 / 8.5 against 7.1, 4096 14.6 / 15.3 /
+        // 17.0 against 23.3, 8192 25.5 / 24.6 / 26.6 against 37.0, 32768 95 / 82 / 75 against 131.  32-bit currents fill the slots of two CTAs
+        // per SM and gain nothing (4096 tokens 33.7 / 31.0 / 29.8 against 28.0).
+        const int64_t lanes = n_tok * widest;
+        const bool rope_streaming = plain_rope && rows_in_warps && !any_f32 && lanes >= 148LL * 512;
+        const bool streaming = rope_streaming || (!any_rope && T <= kStepGroup && toks == 4 && (n_tok / 8) * widest >= 148LL * 2048);
+        if (rope_streaming) toks = lanes >= 148LL * 10240 ? 8 : lanes >= 148LL * 6144 ? 4 : 2;
+        else if (streaming) toks = 8;
         va.toks = toks;
         va.slots = kStepGroup * (any_f32 ? 2 : 1) * (any_gated ? 2 : 1);
         const size_t stage_bytes = streaming ? static_cast<size_t>(kFusedThreads / 32) * kStages * va.slots * 32 * 16 : 0;
@@ -1110,10 +1181,6 @@ extern "C" int spk_lif_pack_scatter(const spk_lif_site* sites, int n_sites, int 
             cudaStream_t vst = spk_stream(stream);
             const bool sub = reset_mode == SPK_RESET_SUBTRACT_DELAYED;
             const bool full = T % kStepGroup == 0;  // no partial group of timesteps: the per-step bounds checks drop out
-            bool plain = true;  // packed bits, gated product, final membrane only: the other feature tests fold away
-            for (int i = 0; i < n_sites; ++i) plain = plain && sites[i].mem0 == nullptr && sites[i].dense == nullptr;
-            const bool plain_rope = plain && any_rope && !any_gated && T == kStepGroup;  // the decode step's q/k/v launch
-            plain = plain && !any_rope;
 #define SPK_LAUNCH_VEC(MODE_, ROPE_, FULL_, ASYNC_, PLAIN_)                                                                \
     do {                                                                                                              \
         auto kern = lif_pack_scatter_vec_kernel<MODE_, ROPE_, FULL_, ASYNC_, PLAIN_>;                                       \
@@ -1126,7 +1193,8 @@ extern "C" int spk_lif_pack_scatter(const spk_lif_site* sites, int n_sites, int 
     } while (0)
 #define SPK_LAUNCH_MODE(MODE_)                                                          \
     do {                                                                                \
-        if (streaming && full && plain && !any_gated) SPK_LAUNCH_VEC(MODE_, false, true, true, true); \
+        if (rope_streaming) SPK_LAUNCH_VEC(MODE_, true, true, true, true); \
+        else if (streaming && full && plain && !any_gated) SPK_LAUNCH_VEC(MODE_, false, true, true, true); \
         else if (streaming) { if (full) SPK_LAUNCH_VEC(MODE_, false, true, true, false); else SPK_LAUNCH_VEC(MODE_, false, false, true, false); } \
         else if (plain_rope) SPK_LAUNCH_VEC(MODE_, true, true, false, true); \
         else if (any_rope) { if (full) SPK_LAUNCH_VEC(MODE_, true, true, false, false); else SPK_LAUNCH_VEC(MODE_, true, false, false, false); } \

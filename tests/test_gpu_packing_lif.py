@@ -396,6 +396,34 @@ def test_fused_rope_is_bit_exact_with_the_eager_expression(dtype, T, D, reset_mo
     assert torch.equal(mem.cpu(), want_u)
 
 
+@pytest.mark.parametrize("lanes, H, D, dtype", [(148 * 512 - 1, 3, 64, torch.bfloat16), (148 * 512, 3, 64, torch.bfloat16), (148 * 512, 5, 32, torch.float16),
+                                                (148 * 512, 1, 256, torch.bfloat16), (148 * 512, 3, 96, torch.bfloat16),
+                                                (148 * 6144, 7, 128, torch.float16), (148 * 10240, 14, 64, torch.bfloat16)])
+def test_fused_rope_at_streaming_sizes(lanes, H, D, dtype, dev):
+    """q and v sites of one launch around the sizes from which lanes walk 2, 4 and 8 tokens through shared memory, odd token counts (the last
+    walk is short), rows of 4 to 32 lanes and of 12 (which do not share a warp); q and its rotary factors from wider buffers, v through slots."""
+    T, W, n_tok = 4, D // 32, (lanes + H * D // 8 - 1) // (H * D // 8)
+    n_tok += 1 - n_tok % 2
+    g = torch.Generator(device=dev).manual_seed(lanes + D)
+    x = (torch.randn(T, n_tok, (H + 1) * D, generator=g, device=dev) * 1.5).to(dtype)
+    q, v = x.unflatten(-1, (H + 1, D)).split((H, 1), dim=2)
+    ang = torch.randn(n_tok, 2 * D, generator=g, device=dev)
+    cos, sin = ang.cos().to(dtype)[:, :D], ang.sin().to(dtype)[:, :D]
+    cur = (q * cos[None, :, None, :]) + (torch.cat((-q[..., D // 2:], q[..., : D // 2]), dim=-1) * sin[None, :, None, :])
+    beta, th = torch.rand(D, generator=g, device=dev), torch.rand(D, generator=g, device=dev) * 0.9 + 0.1
+    slots = torch.randperm(n_tok + 3, generator=g, device=dev)[:n_tok]
+    packed = torch.empty(T, n_tok, H, W, dtype=torch.int32, device=dev)
+    pool = torch.zeros(T, n_tok + 3, 1, W, dtype=torch.int32, device=dev)
+    mem = torch.empty(n_tok, H, D, device=dev)
+    kernels.lif_pack_scatter([
+        kernels.LifSiteSpec(x=q, beta=beta, threshold=th, packed=packed, packed_strides=(n_tok * H * W, H * W, W), mem_out=mem, rope_cos=cos, rope_sin=sin),
+        kernels.LifSiteSpec(x=v, beta=beta, threshold=th, packed=pool, packed_strides=((n_tok + 3) * W, W, W), slot_mapping=slots, num_rows=n_tok + 3)])
+    for got, src, u in ((packed, cur, mem), (pool[:, slots], v, None)):
+        want_s, want_u = orc.lif_multistep(src.cpu(), beta.cpu(), th.cpu(), out_dtype=torch.uint8)
+        assert torch.equal(got.cpu(), orc.pack_spikes(want_s))
+        assert u is None or torch.equal(u.cpu(), want_u)
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 def test_gated_product_on_strided_gemm_output(dtype, dev):
     T, n_tok, N = 4, 21, 4864
