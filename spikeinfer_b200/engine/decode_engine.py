@@ -21,7 +21,7 @@ from __future__ import annotations
 
 import torch
 
-from ..attention import AttentionMetadata, build_prefill_rows
+from ..attention import AttentionMetadata, build_prefill_rows, to_device
 from ..kernels import argmax_rows, argmax_workspace_bytes
 from .batch_state import DecodeBatchState
 from .block_ledger import BlockLedger, covering_bucket, cut_portions, row_buckets
@@ -104,7 +104,7 @@ class PagedDecodeEngine:
             prefill_context_lens=contexts, prefill_block_tables=tables, status=st.status, prefill_rows=rows,
             token_rows=token_rows, token_edges=edges, row_tables=st.block_tables)
         self._finish_prefill_meta(meta)
-        input_ids = torch.tensor(ids, dtype=torch.int64).to(dev)
+        input_ids = to_device(ids, torch.int64, dev)
         return self.model.forward_paged(input_ids, positions, self.cache.layers, meta)
 
     @torch.no_grad()
@@ -128,21 +128,21 @@ class PagedDecodeEngine:
                 if hi == len(prompts[i]):
                     ends.append(at - 1)
             if ends:
-                last = torch.tensor(ends, dtype=torch.int64, device=self.device)
+                last = to_device(ends, torch.int64, self.device)
                 first.append(self.model.compute_logits(hidden, last).argmax(dim=-1))
         self.resume(rows, torch.cat(first))
         return rows
 
     def resume(self, rows: list[int], tokens: torch.Tensor) -> None:
         """Let held rows take part in decode steps; ``tokens`` (int64 ``[len(rows)]``) are what they are fed next."""
-        self.state.resume(torch.tensor(rows, dtype=torch.int64, device=self.device), tokens.to(self.device))
+        self.state.resume(to_device(rows, torch.int64, self.device), tokens.to(self.device))
         self.ledger.held.difference_update(rows)
 
     def hold(self, rows: list[int]) -> None:
         """Let rows that hold a sequence sit out the next decode steps."""
         rows = [r for r in rows if r not in self.ledger.held]
         if rows:
-            self.state.hold(torch.tensor(rows, dtype=torch.int64, device=self.device))
+            self.state.hold(to_device(rows, torch.int64, self.device))
             self.ledger.held.update(rows)
 
     @torch.no_grad()
@@ -157,9 +157,9 @@ class PagedDecodeEngine:
         why = self.ledger.extend_error([(r, 1) for r in rows])
         if why is not None:
             raise RuntimeError(f"cannot decode: {why}")
-        self.resume(rows, torch.tensor([tokens[r] for r in rows], dtype=torch.int64))
+        self.resume(rows, to_device([tokens[r] for r in rows], torch.int64, self.device))
         self.decode_step()
-        return self.step_logits[torch.tensor(rows, dtype=torch.int64, device=self.device)]
+        return self.step_logits[to_device(rows, torch.int64, self.device)]
 
     def release(self, row: int) -> None:
         if row in self.ledger.seq_lens:
