@@ -92,10 +92,11 @@ qk_prepare_vec_kernel(const spk_qk_prepare_args a) {
     spk_grid_release();
     constexpr int LK = DIM / 8;  // lanes per head: 8 or 16, so a warp holds whole heads
     const int lanes_t = (a.heads + 2 * a.kv_heads) * LK;
-    const int64_t item = static_cast<int64_t>(blockIdx.x) * kThreads + threadIdx.x;
-    const int64_t t = item / lanes_t;
+    // 32-bit indices (checked on the host): 64-bit divisions were a large part of this kernel's instructions
+    const uint32_t item = blockIdx.x * kThreads + threadIdx.x, row = item / static_cast<uint32_t>(lanes_t);
+    const int64_t t = row;
     const bool in = t < a.n;
-    const int l = static_cast<int>(item % lanes_t);
+    const int l = static_cast<int>(item - row * lanes_t);
     const int qk_lanes = (a.heads + a.kv_heads) * LK;
     const bool is_v = l >= qk_lanes;
     const int s = (is_v ? l - qk_lanes : l) / LK;  // head slot (q heads, then k heads) or v head
@@ -158,21 +159,20 @@ qk_prepare_vec_kernel(const spk_qk_prepare_args a) {
         return;
     }
     const int64_t slot = a.slot_mapping[t];
-    const int64_t block = slot / a.block_size;
-    if (slot < 0 || block >= a.num_blocks) {
+    const uint32_t block = static_cast<uint32_t>(slot) / static_cast<uint32_t>(a.block_size);
+    if (slot < 0 || slot > 0x7fffffff || block >= a.num_blocks) {
         spk_flag(a.status, SPK_STATUS_BAD_SLOT);
         return;
     }
     const SpkPageLayout lay{a.kv_heads, a.block_size, DIM, 1};
     __nv_bfloat16* page = static_cast<__nv_bfloat16*>(is_v ? a.v_pool : a.k_pool) + spk_page_base(lay, block, is_v ? s : s - a.heads);
-    *reinterpret_cast<uint4*>(page + spk_page_channel(lay, static_cast<int>(slot % a.block_size), sub * 8)) = r;
+    *reinterpret_cast<uint4*>(page + spk_page_channel(lay, static_cast<int>(static_cast<uint32_t>(slot) - block * a.block_size), sub * 8)) = r;
 }
 
 template <int DIM>
 int launch_prepare_vec(const spk_qk_prepare_args& a, cudaStream_t s) {
     const int64_t items = a.n * (a.heads + 2 * static_cast<int64_t>(a.kv_heads)) * (DIM / 8);
     const int64_t grid = (items + kThreads - 1) / kThreads;
-    if (grid > 0x7fffffffLL) return SPK_ERR_TOO_LARGE;
     qk_prepare_vec_kernel<DIM><<<static_cast<unsigned>(grid), kThreads, 0, s>>>(a);
     SPK_CHECK_LAUNCH();
     return SPK_OK;
@@ -305,7 +305,8 @@ extern "C" int spk_qk_prepare(const spk_qk_prepare_args* a, void* stream) {
         a->slot_mapping == nullptr)
         return SPK_ERR_NULL_POINTER;
     auto at16 = [](const void* p) { return reinterpret_cast<uintptr_t>(p) % 16 == 0; };
-    if (a->dtype == SPK_BF16 && a->k_tiled && a->v_tiled && a->dim == a->vdim && (a->dim == 64 || a->dim == 128) && a->k_pad == a->dim &&
+    const int64_t lanes = a->n * (a->heads + 2 * static_cast<int64_t>(a->kv_heads)) * (a->dim / 8);
+    if (lanes < 0x7fffff00LL && a->num_blocks <= 0x7fffffffLL / a->block_size && a->dtype == SPK_BF16 && a->k_tiled && a->v_tiled && a->dim == a->vdim && (a->dim == 64 || a->dim == 128) && a->k_pad == a->dim &&
         a->v_pad == a->vdim && a->ld % 8 == 0 && (a->rot_table == nullptr || (a->rot_dims % 16 == 0 && at16(a->rot_table))) && at16(a->q) &&
         at16(a->k) && at16(a->v) && at16(a->q_out) && at16(a->k_pool) && at16(a->v_pool))
         return a->dim == 64 ? launch_prepare_vec<64>(*a, spk_stream(stream)) : launch_prepare_vec<128>(*a, spk_stream(stream));
