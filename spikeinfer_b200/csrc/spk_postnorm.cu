@@ -157,6 +157,128 @@ residual_norm_kernel(const ResidualNormParams p, T* __restrict__ out) {
     }
 }
 
+// The same for many rows of up to 128 G elements (a multiple of four): a warp per row, its elements in registers, no barrier but the one that
+// hands rows on.  A CTA takes two times eight rows; with a token shift each warp leaves its x' in shared memory for the warp of the next
+// row, so only a CTA's first predecessor is computed twice.  A CTA per row (or per four) was bound by CTAs started and barriers waited for, at
+// 12 to 30 % of the memory's rate: 8192 x 896, 110 MB, 32.7 -> 22.0 us with the shift and 27.8 -> 19.0 us without.
+constexpr int kRowWarps = 8, kRowSteps = 2;  // each step has its buffer in shared memory: one barrier per step is enough
+
+template <typename TD, int G>
+__device__ __forceinline__ void warp_new_row(const ResidualNormParams& p, int64_t t, int64_t commit_row, float4 (&y)[G], const int lane) {
+    const float* xr = p.x + t * p.width;
+    const TD* dr = static_cast<const TD*>(p.delta) + t * p.width;
+    float4 d[G];
+#pragma unroll
+    for (int g = 0; g < G; ++g) {
+        const int c = 4 * (lane + 32 * g);
+        y[g] = spk_load4<float, true>(xr + c, p.width - c);
+        d[g] = spk_load4<TD, true>(dr + c, p.width - c);
+    }
+    if (commit_row >= 0) {
+#pragma unroll
+        for (int g = 0; g < G; ++g) {
+            const int c = 4 * (lane + 32 * g);
+            spk_store4<float, true>(p.commit + commit_row * p.state_stride + c, y[g], p.width - c);
+        }
+    }
+#pragma unroll
+    for (int g = 0; g < G; ++g) y[g] = f4_axpy(p.alpha, y[g], d[g]);
+}
+
+template <int G>
+__device__ __forceinline__ void warp_layer_norm(float4 (&y)[G], const float* __restrict__ w, int width, float eps, const int lane) {
+    float s = 0.0f, q = 0.0f;
+#pragma unroll
+    for (int g = 0; g < G; ++g) s += (y[g].x + y[g].y) + (y[g].z + y[g].w);
+    const float mean = spk_warp_sum(s) / static_cast<float>(width);
+#pragma unroll
+    for (int g = 0; g < G; ++g) {
+        const bool in = 4 * (lane + 32 * g) < width;
+        y[g] = in ? make_float4(y[g].x - mean, y[g].y - mean, y[g].z - mean, y[g].w - mean) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        q += (y[g].x * y[g].x + y[g].y * y[g].y) + (y[g].z * y[g].z + y[g].w * y[g].w);
+    }
+    const float inv = 1.0f / sqrtf(spk_warp_sum(q) / static_cast<float>(width) + eps);
+#pragma unroll
+    for (int g = 0; g < G; ++g) {
+        const int c = 4 * (lane + 32 * g);
+        const float4 wv = spk_load4<float, true>(w + c, width - c);
+        y[g] = make_float4(y[g].x * inv * wv.x, y[g].y * inv * wv.y, y[g].z * inv * wv.z, y[g].w * inv * wv.w);
+    }
+}
+
+template <typename T, typename TD, int G, bool MIX>
+__global__ void __launch_bounds__(32 * kRowWarps, 2)
+residual_norm_rows_kernel(const ResidualNormParams p, T* __restrict__ out) {
+    extern __shared__ float4 rows_s[];  // MIX: [kRowSteps][kRowWarps][32 * G]
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int64_t t0 = static_cast<int64_t>(blockIdx.x) * p.per_cta;
+    const int64_t t1 = t0 + p.per_cta < p.n ? t0 + p.per_cta : p.n;
+    for (int step = 0; step < kRowSteps && t0 + step * kRowWarps < t1; ++step) {
+        const int64_t t = t0 + step * kRowWarps + warp;
+        const bool live = t < t1;
+        float4 y[G];
+        int32_t edge = 3;
+        int64_t row = -1;
+        if (live) {
+            edge = p.token_edges != nullptr ? p.token_edges[t] : 3;
+            row = p.token_rows != nullptr ? p.token_rows[t] : t;
+            if (p.active != nullptr && p.token_rows == nullptr && p.active[t] != 1) row = -1;
+            if (row >= p.state_rows && (MIX || p.commit != nullptr)) {
+                if (lane == 0) spk_flag(p.status, SPK_STATUS_BAD_SLOT);
+                row = -1;
+            }
+            warp_new_row<TD, G>(p, t, p.commit != nullptr && (edge & 2) ? row : -1, y, lane);
+            warp_layer_norm<G>(y, p.w, p.width, p.eps, lane);
+            if (p.x_out != nullptr) {
+#pragma unroll
+                for (int g = 0; g < G; ++g) {
+                    const int c = 4 * (lane + 32 * g);
+                    spk_store4<float, true>(p.x_out + t * p.width + c, y[g], p.width - c);
+                }
+            }
+            if (MIX) {
+#pragma unroll
+                for (int g = 0; g < G; ++g) rows_s[(step * kRowWarps + warp) * 32 * G + lane + 32 * g] = y[g];
+            } else if (p.w2 != nullptr) {
+                warp_layer_norm<G>(y, p.w2, p.width, p.eps, lane);
+            }
+        }
+        if (MIX) {
+            __syncthreads();
+            float4 before[G];
+            if (live && !(edge & 1) && t == t0) {
+                warp_new_row<TD, G>(p, t - 1, -1, before, lane);
+                warp_layer_norm<G>(before, p.w, p.width, p.eps, lane);
+            } else if (live) {
+                const bool stored = row >= 0 && (edge & 1) && p.positions[t] > 0;
+                const int from = edge & 1 ? 0 : step * kRowWarps + warp - 1;
+                const float* s = p.prev + (stored ? row : 0) * p.state_stride;
+#pragma unroll
+                for (int g = 0; g < G; ++g) {
+                    const int c = 4 * (lane + 32 * g);
+                    before[g] = edge & 1 ? spk_load4<float, true>(s + c, stored ? p.width - c : 0) : rows_s[from * 32 * G + lane + 32 * g];
+                }
+            }
+            if (live) {
+#pragma unroll
+                for (int g = 0; g < G; ++g) {
+                    const int c = 4 * (lane + 32 * g);
+                    const float4 m = spk_load4<float, true>(p.mix + c, p.width - c), a = y[g], b = before[g];
+                    y[g] = make_float4(a.x + (b.x - a.x) * m.x, a.y + (b.y - a.y) * m.y, a.z + (b.z - a.z) * m.z, a.w + (b.w - a.w) * m.w);
+                }
+            }
+        }
+        if (live) {
+            T* o = out + t * p.width;
+#pragma unroll
+            for (int g = 0; g < G; ++g) {
+                const int c = 4 * (lane + 32 * g);
+                spk_store4<T, true>(o + c, y[g], p.width - c);
+            }
+        }
+    }
+}
+
 template <typename T, int V, bool VEC>
 __global__ void __launch_bounds__(1024)
 poly_norm_kernel(const T* __restrict__ z, const float* __restrict__ coef, float eps, T* __restrict__ out, int width) {
@@ -262,8 +384,36 @@ int launch_poly_packed(const void* z, const float* coef, float eps, void* out, i
     return SPK_OK;
 }
 
+template <typename T, typename TD, int G>
+int launch_residual_rows(ResidualNormParams p, T* out, cudaStream_t s) {
+    p.per_cta = kRowSteps * kRowWarps;
+    const unsigned grid = static_cast<unsigned>((p.n + p.per_cta - 1) / p.per_cta);
+    if (p.mix == nullptr) {
+        residual_norm_rows_kernel<T, TD, G, false><<<grid, 32 * kRowWarps, 0, s>>>(p, out);
+    } else {
+        constexpr int bytes = kRowSteps * kRowWarps * 32 * G * 16;
+        const cudaError_t e = cudaFuncSetAttribute(residual_norm_rows_kernel<T, TD, G, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+        if (e != cudaSuccess) return spk_set_cuda_error(e);
+        residual_norm_rows_kernel<T, TD, G, true><<<grid, 32 * kRowWarps, bytes, s>>>(p, out);
+    }
+    SPK_CHECK_LAUNCH();
+    return SPK_OK;
+}
+
 template <typename T, typename TD>
 int launch_residual(const ResidualNormParams& p, void* out, cudaStream_t s) {
+    // A warp per row from eight rows per SM on: 1184 rows of 896 with the shift 11.1 -> 7.1 us, without 5.5 -> 5.9; 1536 rows 11.7 -> 7.1 and 7.4 -> 6.3;
+    // below that (512 rows) a CTA per row has more loads in flight.  Wider rows don't fit a warp's registers.
+    if (p.ids == nullptr && p.width % 4 == 0 && p.width <= 1024 && p.n >= (p.mix != nullptr ? 8 : 10) * 148) {
+        T* o = static_cast<T*>(out);
+        switch ((p.width + 127) / 128) {
+            case 1: case 2: return launch_residual_rows<T, TD, 2>(p, o, s);
+            case 3: case 4: return launch_residual_rows<T, TD, 4>(p, o, s);
+            case 5: case 6: return launch_residual_rows<T, TD, 6>(p, o, s);
+            case 7: return launch_residual_rows<T, TD, 7>(p, o, s);
+            default: return launch_residual_rows<T, TD, 8>(p, o, s);
+        }
+    }
     int v = 1;
     const int threads = spk_row_shape(p.width, &v);
     if (threads == 0) return SPK_ERR_TOO_LARGE;

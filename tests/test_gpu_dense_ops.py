@@ -87,6 +87,57 @@ def test_residual_norm_portions(dev, dtype, width):
 
 
 @pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("n", [8 * 148 - 1, 8 * 148, 10 * 148 + 9])
+@pytest.mark.parametrize("width", [4, 128, 260, 516, 896, 1000, 1024, 1028])
+def test_residual_norm_of_many_rows(dev, dtype, n, width):
+    """Around the sizes from which a warp takes a row: portions that start and end at, before and behind a CTA's eight and sixteen rows."""
+    g = gen(n + width)
+    cuts = [0, 1, 8, 15, 16, 17, 33, 48, n - 1, n]
+    x, delta = torch.randn(n, width, generator=g), torch.randn(n, width, generator=g).to(dtype)
+    w, w2, mix = (1 + 0.3 * torch.randn(width, generator=g) for _ in range(3))
+    prev = torch.randn(len(cuts), width, generator=g)
+    trow, edge, pos = (torch.zeros(n, dtype=d) for d in (torch.int32, torch.int32, torch.int64))
+    y = mo.layer_norm(2.5 * x.double() + delta.double(), w.double(), 1e-3)
+    before = torch.cat([y[:1], y[:-1]])
+    for i, (lo, hi) in enumerate(zip(cuts, cuts[1:])):
+        start = 5 * (i % 2)  # every other portion starts a sequence
+        trow[lo:hi], pos[lo:hi] = i, torch.arange(start, start + hi - lo)
+        edge[lo] |= 1
+        edge[hi - 1] |= 2
+        before[lo] = prev[i] if start else 0.0
+        if not start:
+            prev[i] = float("nan")
+    out, x_out = torch.empty(n, width, dtype=dtype, device=dev), torch.empty(n, width, device=dev)
+    commit = torch.full_like(prev, 7.0, device=dev)
+    status = torch.zeros(1, dtype=torch.int32, device=dev)
+    args = dict(x=x.to(dev), delta=delta.to(dev), weight=w.to(dev), alpha=2.5, x_out=x_out, eps=1e-3, positions=pos.to(dev), token_rows=trow.to(dev),
+                token_edges=edge.to(dev), status=status)
+    dense.residual_norm(out, mix=mix.to(dev), prev=prev.to(dev), commit=commit, **args)
+    assert rel(x_out, y) < 3e-6 and rel(out, y + (before - y) * mix.double()) < TOL[dtype]
+    assert torch.equal(commit.cpu()[:-1], x[[c - 1 for c in cuts[1:]]]) and (commit[-1] == 7.0).all()
+    dense.residual_norm(out, second_weight=w2.to(dev), **args)
+    assert rel(out, mo.layer_norm(y, w2.double(), 1e-3)) < TOL[dtype]
+    dense.residual_norm(out, **args)
+    assert rel(out, y) < TOL[dtype] and status.item() == 0
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("n", [8 * 148 - 1, 8 * 148, 8 * 148 + 5])
+@pytest.mark.parametrize("width", [4, 260, 516, 896, 1024, 1028])
+def test_gated_norm_of_many_rows(dev, dtype, n, width):
+    g = gen(n + width)
+    x, w = torch.randn(n, width, generator=g), 1 + 0.3 * torch.randn(width, generator=g)
+    z = (3 * torch.randn(n, 2 * width, generator=g)).to(dtype)
+    z[0, width:], z[1, width:] = 200.0, -200.0
+    active = torch.ones(n, dtype=torch.int32)
+    active[[2, n - 1]] = 0
+    out = torch.full((n, 4 + width), 7.0, dtype=dtype, device=dev)
+    dense.gated_norm(x.to(dev), w.to(dev), z.to(dev)[:, width:], out, 4, eps=1e-3, scale=0.5, active=active.to(dev))
+    want = 0.5 * x.double() / (x.double().pow(2).mean(1, keepdim=True) + 1e-3).sqrt() * w.double() * torch.sigmoid(z[:, width:].double()) * active[:, None]
+    assert rel(out[:, 4:], want) < TOL[dtype] and (out[:, :4] == 7.0).all() and (out[[2, n - 1], 4:] == 0).all()
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
 def test_residual_norm_embedding_and_decode_rows(dev, dtype):
     g = gen(5)
     vocab, width, n = 50, 40, 6
