@@ -675,7 +675,7 @@ typedef struct spk_experts_args {
     int32_t experts, k, out_features;
     int32_t gated;
     int32_t dtype;
-    int32_t _pad;
+    int32_t overlap;            /* the call directly follows the one that writes x, and every earlier launch was complete when that began */
     uint32_t* status;
 } spk_experts_args;
 int spk_experts(const spk_experts_args* args, void* stream);

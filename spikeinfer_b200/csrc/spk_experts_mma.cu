@@ -7,6 +7,11 @@
 //  * gated: the two tiles are gate and up rows of the same 128 features; the epilogue multiplies silu(gate) by up and writes the operand
 //    tiles of the next product.
 //  * plain: 256 consecutive output features, 32-bit rows.
+//
+// Few tokens (TN = 32): the time is that of streaming the weights.  The plain product's are on their way before the gated one is done
+// (16 experts of 896 x 1216, one row beside the mixer: whole step 4204 -> 4107 us; 64 rows 6791 -> 6732).  Where few blocks are streamed, a
+// cluster of S CTAs shares a block, each over its own part of k; the partial sums meet in shared memory and are added in the order
+// of the CTAs, so results don't depend on timing.
 // Warp 0 copies, warp 1 issues MMAs, warps 2-5 write the results.
 #include "spk_experts.cuh"
 #include "spk_tensor.cuh"
@@ -15,7 +20,6 @@ namespace {
 
 using namespace spk_tc;
 
-constexpr int kThreads = 192;
 constexpr int kTileW = 128 * 128;  // bytes of a 128-row, 64-column weight tile
 
 template <int TN>
@@ -24,6 +28,8 @@ struct Shape {
     static constexpr int NS = TN >= 256 ? 3 : TN >= 128 ? 4 : TN >= 64 ? 5 : 3;  // the narrow form leaves room for a second CTA
     static constexpr int kBytes = NS * kStage + 1024 + 256;
     static constexpr int kColumns = 2 * TN < 32 ? 32 : 2 * TN;
+    static constexpr int kWriters = 4;  // warps that write results
+    static constexpr int kThreads = 64 + 32 * kWriters;
 };
 
 struct Bars {
@@ -32,19 +38,67 @@ struct Bars {
     uint32_t tmem;
 };
 
-template <int TN, bool GATED>
-__global__ void __launch_bounds__(kThreads, TN <= 32 ? 2 : 1)
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+// What CTA `rank` of the cluster has where this CTA has `addr`.
+__device__ __forceinline__ float cluster_load(uint32_t addr, uint32_t rank) {
+    float v;
+    asm volatile("{\n\t.reg .b32 r;\n\tmapa.shared::cluster.u32 r, %1, %2;\n\tld.shared::cluster.f32 %0, [r];\n\t}\n" : "=f"(v) : "r"(addr), "r"(rank) : "memory");
+    return v;
+}
+
+// Gated results of a warp's 32 features (this lane's is f) for J tokens from `slot` on, of which n exist.  Pairs of lanes trade a token's
+// value, so that a store carries two features.
+template <int J>
+__device__ __forceinline__ void store_gated(const spk_experts_args& a, int64_t slot, int n, int f, int lane, const float (&p)[J], const float (&q)[J]) {
+    __nv_bfloat16* out = static_cast<__nv_bfloat16*>(a.out);
+    const bool odd = lane & 1;
+    const int fe = f & ~1;
+    const bool in = fe < spk_operand_columns(a.out_features);
+#pragma unroll
+    for (int j = 0; j < J; j += 2) {
+        const float y0 = p[j] * rcp(1.0f + ex2(-1.4426950408889634f * p[j])) * q[j];
+        const float y1 = p[j + 1] * rcp(1.0f + ex2(-1.4426950408889634f * p[j + 1])) * q[j + 1];
+        const float got = __shfl_xor_sync(~0u, odd ? y0 : y1, 1);
+        const uint32_t v = odd ? pack_bf16(got, y1) : pack_bf16(y0, got);
+        const int jj = j + (odd ? 1 : 0);
+        if (in && jj < n) *reinterpret_cast<uint32_t*>(out + spk_operand_at(a.rows, slot + jj, fe)) = v;
+    }
+}
+
+template <int J>
+__device__ __forceinline__ void store_plain(const spk_experts_args& a, int64_t slot, int n, int f, const float (&p)[J], const float (&q)[J]) {
+    float* out = static_cast<float*>(a.out) + slot * a.out_features + f;
+#pragma unroll
+    for (int j = 0; j < J; ++j) {
+        if (j < n) {
+            if (f < a.out_features) out[static_cast<int64_t>(j) * a.out_features] = p[j];
+            if (f + 128 < a.out_features) out[static_cast<int64_t>(j) * a.out_features + 128] = q[j];
+        }
+    }
+}
+
+// S > 1: the CTAs of a cluster are the parts of k of one block.
+template <int TN, bool GATED, int S>
+__global__ void __launch_bounds__(Shape<TN>::kThreads, TN <= 32 ? 2 : 1)
 experts_kernel(const spk_experts_args a, const int blocks, const int ktiles) {
     using Sh = Shape<TN>;
     constexpr int NS = Sh::NS;
+    static_assert(S == 1 || (TN == 32 && 2 * TN * 128 * 4 <= NS * Sh::kStage), "partial sums take the stages' place");
     int e, rows;
     int64_t row0;
-    // uniform over the CTA: nothing has been set up yet
-    if (!spk_find_tile<TN>(a.segs, a.experts, blockIdx.y, e, row0, rows)) return;
-    if (row0 + TN > a.rows) {
-        if (threadIdx.x == 0) spk_flag(a.status, SPK_STATUS_BAD_SLOT);
+    // uniform over the cluster: nothing has been set up yet
+    if (!spk_find_tile<TN>(a.segs, a.experts, blockIdx.y, e, row0, rows)) {
+        spk_grid_wait();
         return;
     }
+    if (row0 + TN > a.rows) {
+        if (threadIdx.x == 0) spk_flag(a.status, SPK_STATUS_BAD_SLOT);
+        spk_grid_wait();
+        return;
+    }
+    const int part = S > 1 ? static_cast<int>(blockIdx.x) % S : 0;
+    const int kb = ktiles * part / S, kn = ktiles * (part + 1) / S - kb;  // this CTA's k tiles, at least one
     extern __shared__ uint8_t raw[];
     uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(raw) + 1023) & ~uintptr_t(1023));
     Bars* bars = reinterpret_cast<Bars*>(base + NS * Sh::kStage);
@@ -64,19 +118,30 @@ experts_kernel(const spk_experts_args a, const int blocks, const int ktiles) {
     tc_fence_after();
     const uint32_t tmem = bars->tmem;
     volatile int* abort = &bars->abort;
-    const int b = blockIdx.x;
+    spk_grid_release();  // this CTA has its columns of TMEM: one of the next launch cannot take them first
+    const int b = blockIdx.x / S;
     if (warp == 0) {
         if (lane == 0) {
-            const uint8_t* w = static_cast<const uint8_t*>(a.w) + (static_cast<int64_t>(e) * blocks + b) * ktiles * (2 * kTileW);
-            const uint8_t* x = static_cast<const uint8_t*>(a.x) + row0 * 128;
-            int issued = 0;
-            for (int k = 0; k < ktiles; ++k) {
+            const uint8_t* w = static_cast<const uint8_t*>(a.w) + ((static_cast<int64_t>(e) * blocks + b) * ktiles + kb) * (2 * kTileW);
+            const uint8_t* x = static_cast<const uint8_t*>(a.x) + row0 * 128 + static_cast<int64_t>(kb) * a.rows * 128;
+            auto weights = [&](int k) {
                 const int s = k % NS;
-                if (k >= NS && !mbar_wait(smem_u32(&bars->free[s]), ((k / NS) - 1) & 1, abort)) break;
-                const uint32_t bar = smem_u32(&bars->full[s]), dst = smem_u32(base + s * Sh::kStage);
+                const uint32_t bar = smem_u32(&bars->full[s]);
                 mbar_expect(bar, Sh::kStage);
-                bulk_load(dst, w + static_cast<int64_t>(k) * (2 * kTileW), 2 * kTileW, bar);
-                bulk_load(dst + 2 * kTileW, x + static_cast<int64_t>(k) * a.rows * 128, TN * 128, bar);
+                bulk_load(smem_u32(base + s * Sh::kStage), w + static_cast<int64_t>(k) * (2 * kTileW), 2 * kTileW, bar);
+            };
+            // the weights of the first stages don't wait for the launch that writes x
+            const int early = kn < NS ? kn : NS;
+            for (int k = 0; k < early; ++k) weights(k);
+            spk_grid_wait();
+            int issued = 0;
+            for (int k = 0; k < kn; ++k) {
+                const int s = k % NS;
+                if (k >= NS) {
+                    if (!mbar_wait(smem_u32(&bars->free[s]), ((k / NS) - 1) & 1, abort)) break;
+                    weights(k);
+                }
+                bulk_load(smem_u32(base + s * Sh::kStage) + 2 * kTileW, x + static_cast<int64_t>(k) * a.rows * 128, TN * 128, smem_u32(&bars->full[s]));
                 issued = k + 1;
             }
             if (*abort != 0)  // copies in flight land before the CTA's shared memory is given up
@@ -85,7 +150,7 @@ experts_kernel(const spk_experts_args a, const int blocks, const int ktiles) {
     } else if (warp == 1) {
         if (lane == 0) {
             constexpr uint32_t idesc = idesc_bf16(128, TN, false, false);
-            for (int k = 0; k < ktiles; ++k) {
+            for (int k = 0; k < kn; ++k) {
                 const int s = k % NS;
                 if (!mbar_wait(smem_u32(&bars->full[s]), (k / NS) & 1, abort)) break;
                 tc_fence_after();
@@ -108,39 +173,62 @@ experts_kernel(const spk_experts_args a, const int blocks, const int ktiles) {
         tc_fence_after();
         const int f = b * (GATED ? 128 : 256) + quad * 32 + lane;  // this lane's feature (and f + 128)
 #pragma unroll 1
-        for (int j0 = 0; j0 < TN && j0 < rows; j0 += 32) {
+        for (int j0 = (warp - 2) / 4 * 32; j0 < TN && j0 < rows; j0 += 8 * Sh::kWriters) {
             uint32_t p[32], q[32];
             tmem_ld32(tmem + lanes + j0, p);
             tmem_ld32(tmem + lanes + TN + j0, q);
             tmem_wait_ld(p);
             tmem_wait_ld(q);
-            const int n = ok ? min(32, rows - j0) : 0;
-            if (GATED) {
-                __nv_bfloat16* out = static_cast<__nv_bfloat16*>(a.out);
-                // pairs of lanes trade a token's value, so that a store carries two features
-                const bool odd = lane & 1;
-                const int fe = f & ~1;
-                const bool in = fe < spk_operand_columns(a.out_features);
+            float x[32], y[32];
 #pragma unroll
-                for (int j = 0; j < 32; j += 2) {
-                    const float y0 = __uint_as_float(p[j]) * rcp(1.0f + ex2(-1.4426950408889634f * __uint_as_float(p[j]))) * __uint_as_float(q[j]);
-                    const float y1 = __uint_as_float(p[j + 1]) * rcp(1.0f + ex2(-1.4426950408889634f * __uint_as_float(p[j + 1]))) * __uint_as_float(q[j + 1]);
-                    const float got = __shfl_xor_sync(~0u, odd ? y0 : y1, 1);
-                    const uint32_t v = odd ? pack_bf16(got, y1) : pack_bf16(y0, got);
-                    const int jj = j + (odd ? 1 : 0);
-                    if (in && jj < n) *reinterpret_cast<uint32_t*>(out + spk_operand_at(a.rows, row0 + j0 + jj, fe)) = v;
-                }
-            } else {
-                float* out = static_cast<float*>(a.out) + (row0 + j0) * a.out_features + f;
+            for (int j = 0; j < 32; ++j) {
+                x[j] = __uint_as_float(p[j]);
+                y[j] = __uint_as_float(q[j]);
+            }
+            if (S == 1) {
+                const int n = ok ? min(32, rows - j0) : 0;
+                if (GATED) store_gated<32>(a, row0 + j0, n, f, lane, x, y);
+                else store_plain<32>(a, row0 + j0, n, f, x, y);
+            } else {  // [gate and up, or the two feature halves][token][128 features]
+                float* sums = reinterpret_cast<float*>(base) + quad * 32 + lane;
 #pragma unroll
                 for (int j = 0; j < 32; ++j) {
-                    if (j < n) {
-                        if (f < a.out_features) out[static_cast<int64_t>(j) * a.out_features] = __uint_as_float(p[j]);
-                        if (f + 128 < a.out_features) out[static_cast<int64_t>(j) * a.out_features + 128] = __uint_as_float(q[j]);
+                    if (j < rows) {
+                        sums[j * 128] = ok ? x[j] : 0.0f;
+                        sums[(TN + j) * 128] = ok ? y[j] : 0.0f;
                     }
                 }
             }
         }
+    }
+    if (S > 1) {
+        __syncwarp();
+        cluster_arrive();
+        cluster_wait();
+        if (warp >= 2) {  // every CTA adds and writes its own tokens
+            constexpr int J = 32 / S;
+            const int quad = warp & 3, j0 = part * J, n = min(J, rows - j0);
+            const uint32_t own = smem_u32(base) + 4 * (j0 * 128 + quad * 32 + lane);
+            float x[J] = {}, y[J] = {};
+            if (n > 0) {
+#pragma unroll
+                for (int r = 0; r < S; ++r) {
+#pragma unroll
+                    for (int j = 0; j < J; ++j) {
+                        if (j < n) {
+                            x[j] += cluster_load(own + j * 512, r);
+                            y[j] += cluster_load(own + (TN + j) * 512, r);
+                        }
+                    }
+                }
+                const int f = b * (GATED ? 128 : 256) + quad * 32 + lane;
+                if (GATED) store_gated<J>(a, row0 + j0, n, f, lane, x, y);
+                else store_plain<J>(a, row0 + j0, n, f, x, y);
+            }
+        }
+        __syncwarp();
+        cluster_arrive();
+        cluster_wait();  // no CTA leaves while its sums are being read
     }
     __syncwarp();
     tc_fence_before();
@@ -150,16 +238,35 @@ experts_kernel(const spk_experts_args a, const int blocks, const int ktiles) {
     if (warp == 0) tmem_dealloc(tmem, Sh::kColumns);
 }
 
-template <int TN, bool GATED>
+template <int TN, bool GATED, int S>
 int launch(const spk_experts_args& a, int blocks, int ktiles, cudaStream_t s) {
     constexpr int bytes = Shape<TN>::kBytes;
     static_assert(sizeof(Bars) <= 256 && bytes <= 227 * 1024, "shared memory");
     const int64_t tiles = spk_most_tiles(a.pairs, a.experts, TN);
     if (tiles > 65535) return SPK_ERR_TOO_LARGE;
-    const cudaError_t e = cudaFuncSetAttribute(experts_kernel<TN, GATED>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    auto kernel = experts_kernel<TN, GATED, S>;
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
     if (e != cudaSuccess) return spk_set_cuda_error(e);
-    experts_kernel<TN, GATED><<<dim3(blocks, static_cast<unsigned>(tiles)), kThreads, bytes, s>>>(a, blocks, ktiles);
-    SPK_CHECK_LAUNCH();
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr[2] = {};
+    cfg.gridDim = dim3(blocks * S, static_cast<unsigned>(tiles));
+    cfg.blockDim = dim3(Shape<TN>::kThreads);
+    cfg.dynamicSmemBytes = bytes;
+    cfg.stream = s;
+    cfg.attrs = attr;
+    if (S > 1) {
+        attr[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
+        attr[cfg.numAttrs].val.clusterDim = {S, 1, 1};
+        ++cfg.numAttrs;
+    }
+    if (TN == 32 && a.overlap) {
+        attr[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[cfg.numAttrs].val.programmaticStreamSerializationAllowed = 1;
+        ++cfg.numAttrs;
+    }
+    e = cudaLaunchKernelEx(&cfg, kernel, a, blocks, ktiles);
+    if (e != cudaSuccess) return spk_set_cuda_error(e);
+    spk_count_launch();
     return SPK_OK;
 }
 
@@ -168,10 +275,17 @@ int dispatch(const spk_experts_args& a, cudaStream_t s) {
     const int per = GATED ? 128 : 256;
     const int blocks = (a.out_features + per - 1) / per, ktiles = (a.k + 63) / 64;
     const int64_t mean = (a.pairs + a.experts - 1) / a.experts;
-    if (mean > 96) return launch<256, GATED>(a, blocks, ktiles, s);
-    if (mean > 40) return launch<128, GATED>(a, blocks, ktiles, s);
-    if (mean > 16) return launch<64, GATED>(a, blocks, ktiles, s);
-    return launch<32, GATED>(a, blocks, ktiles, s);
+    if (mean > 96) return launch<256, GATED, 1>(a, blocks, ktiles, s);
+    if (mean > 40) return launch<128, GATED, 1>(a, blocks, ktiles, s);
+    if (mean > 16) return launch<64, GATED, 1>(a, blocks, ktiles, s);
+    // Blocks streamed by the second product: with fewer than 17 (a step of one user with two experts has 8) two CTAs share each.  One row of 16 experts
+    // of 896 x 1216 beside the mixer's launches: whole step 4107 us without, 3834 with two parts of the second product, 4103 with two of both, 4260
+    // with four of both: more CTAs take SMs from the mixer, although the two launches alone go on falling (20.8, 17.1, 15.1, 11.1 us).  With
+    // 8 and 64 rows (64 blocks) parts gain nothing: 5058 -> 5185 us, 6732 -> 6959.
+    if constexpr (!GATED) {
+        if (blocks * (a.pairs < a.experts ? a.pairs : a.experts) <= 16 && ktiles >= 2) return launch<32, GATED, 2>(a, blocks, ktiles, s);
+    }
+    return launch<32, GATED, 1>(a, blocks, ktiles, s);
 }
 
 }  // namespace

@@ -126,5 +126,5 @@ def experts_forward(x: torch.Tensor, w: ExpertWeights, route: LayerRoute, status
     _call("spk_experts", _lib.ExpertsArgs(x=x.data_ptr(), w=w.w_in.data_ptr(), out=hidden.data_ptr(), k=w.width, out_features=w.ff, gated=1, **common),
           x.device)
     _call("spk_experts", _lib.ExpertsArgs(x=hidden.data_ptr(), w=w.w_out.data_ptr(), out=out.data_ptr(), k=w.ff, out_features=w.width, gated=0,
-                                          **common), x.device)
+                                          overlap=1, **common), x.device)
     return out

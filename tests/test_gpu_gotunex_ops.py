@@ -133,6 +133,19 @@ def test_experts(dev, status, n, width, experts, top, ff, dtype):
     assert rel(got, want) < (3e-6 if dtype == F32 else 8e-3)
 
 
+@pytest.mark.parametrize("n,width,experts,top,ff", [(1, 896, 16, 2, 1216), (2, 72, 16, 2, 65), (3, 300, 4, 2, 129), (16, 200, 2, 2, 1000), (32, 264, 2, 1, 130)])
+def test_experts_of_few_tokens(dev, status, n, width, experts, top, ff):
+    """The forms that share a block of the second product between two CTAs: two to nineteen k tiles, one to 32 rows per expert; twice the same bits."""
+    w, weights, ids, x, cfg = expert_case(dev, BF, n, width, experts, top, ff, n + ff)
+    x = go.rms(x.double(), 0.0)
+    route, out = run_experts(dev, status, weights, ids, x)
+    slots = route.slots.long()
+    want = go.table_experts(x, ids.tolist(), go.as_float(w), "", cfg)
+    assert rel(out[slots].mean(1), want) < 8e-3 and status.item() == 0
+    again, out2 = run_experts(dev, status, weights, ids, x)  # routing may order an expert's rows otherwise
+    assert torch.equal(out2[again.slots.long()], out[slots])
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 def test_every_token_at_the_same_experts_and_rows_that_sit_out(dev, status, dtype):
     n = 150
