@@ -10,6 +10,7 @@
 // state is written by the launch that ends the sublayer (it still reads the old x), so no launch reads and
 // writes one state row from two CTAs.
 #include "spk_dense.cuh"
+#include "spk_tensor.cuh"
 
 namespace {
 
@@ -326,35 +327,39 @@ poly_norm_packed_kernel(const __nv_bfloat16* __restrict__ z, const float* __rest
         const int i = threadIdx.x + v * blockDim.x;
         raw[v] = i < groups ? zr[i] : make_uint4(0u, 0u, 0u, 0u);
     }
-    float s[3] = {0.0f, 0.0f, 0.0f};
-    auto moments = [&](float x) {
-        const float q = x * x;
-        s[0] += q;
-        s[1] = fmaf(q, q, s[1]);
-        s[2] = fmaf(q * q, q, s[2]);
-    };
+    using namespace spk_tc;
+    // two channels per instruction: the kernel is bound by issue (8192 rows of 4864: 38.1 -> 33.4 us, 4096 of 18944: 66.0 -> 53.4)
+    uint64_t m1 = f2_pack(0.0f, 0.0f), m2 = m1, m3 = m1;
 #pragma unroll
     for (int v = 0; v < G; ++v) {
         const uint32_t w[4] = {raw[v].x, raw[v].y, raw[v].z, raw[v].w};
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
-            moments(__uint_as_float(w[k] << 16));
-            moments(__uint_as_float(w[k] & 0xffff0000u));
+            const uint64_t x = f2_pack(__uint_as_float(w[k] << 16), __uint_as_float(w[k] & 0xffff0000u)), q = f2_mul(x, x), qq = f2_mul(q, q);
+            m1 = f2_add(m1, q);
+            m2 = f2_add(m2, qq);
+            m3 = f2_fma(qq, q, m3);
         }
     }
+    float s[3], y;
+    f2_unpack(m1, s[0], y); s[0] += y;
+    f2_unpack(m2, s[1], y); s[1] += y;
+    f2_unpack(m3, s[2], y); s[2] += y;
     spk_block_sum<3>(s, part);
     const float n = static_cast<float>(width);
     const float k1 = coef[0] / sqrtf(s[0] / n + eps), k2 = coef[1] / sqrtf(s[1] / n + eps);
     const float k3 = coef[2] / sqrtf(s[2] / n + eps), k0 = coef[3];
-    auto f = [&](float x) { return fmaf(x, fmaf(x, fmaf(x, k3, k2), k1), k0); };
+    const uint64_t c0 = f2_pack(k0, k0), c1 = f2_pack(k1, k1), c2 = f2_pack(k2, k2), c3 = f2_pack(k3, k3);
 #pragma unroll
     for (int v = 0; v < G; ++v) {
         const int i = threadIdx.x + v * blockDim.x;
         uint32_t w[4] = {raw[v].x, raw[v].y, raw[v].z, raw[v].w};
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
-            const __nv_bfloat162 b = __floats2bfloat162_rn(f(__uint_as_float(w[k] << 16)), f(__uint_as_float(w[k] & 0xffff0000u)));
-            w[k] = *reinterpret_cast<const uint32_t*>(&b);
+            const uint64_t x = f2_pack(__uint_as_float(w[k] << 16), __uint_as_float(w[k] & 0xffff0000u));
+            float lo, hi;
+            f2_unpack(f2_fma(x, f2_fma(x, f2_fma(x, c3, c2), c1), c0), lo, hi);
+            w[k] = pack_bf16(lo, hi);
         }
         if (i < groups) o[i] = make_uint4(w[0], w[1], w[2], w[3]);
     }
