@@ -1,13 +1,15 @@
 // Prefill attention with sigmoid key weights on the fifth-generation tensor cores (tcgen05), bf16, head sizes up to 128.
 //
-// CTA = (128 query tokens of one portion, query head).  Twenty warps:
-//  * warps 16 and 19 copy K and V: a page of the pool is stored as the swizzled operand tile it becomes, so a 128-key tile is a
+// CTA = (128 query tokens of one portion, query head).  Warps, W of them for the weights (8 with heads of up to 64 channels, else 16):
+//  * warps W and W + 3 copy K and V: a page of the pool is stored as the swizzled operand tile it becomes, so a 128-key tile is a
 //    handful of plain bulk copies (cp.async.bulk), no tensor map, whatever pages the block table names; one copy per lane, the
 //    next tile's block-table entries are read ahead;
-//  * warp 17 (one thread) issues S = Q K^T into one of two TMEM buffers, warp 18 (one thread) O += P V with P read from TMEM,
+//  * warp W + 1 (one thread) issues S = Q K^T into a TMEM buffer, warp W + 2 (one thread) O += P V with P read from TMEM,
 //    so that neither kind of MMA waits behind the other's operands;
-//  * warps 0-15 turn scores into weights: warpgroups 0 and 2 the two column halves of the even tiles, 1 and 3 those of the odd
-//    ones, one thread per query row and half.  The work is latency-bound, hence many warps of few registers.
+//  * the others turn scores into weights, one thread per query row and half of the columns.  Sixteen warps take even and odd tiles in two
+//    score buffers.  With heads of 64 one buffer and eight warps fit two CTAs into an SM: one's start and end, a large part of the
+//    time of short prompts, hide behind the other's tiles.  14 heads of 64: 16 x 512 tokens 66.8 -> 50.4 us, 1 x 4096 94.7 -> 93.2, 3 x 600 to 1200
+//    33.3 -> 31.0, 2 x 60 to 100 8.1 -> 7.8.  Values of 128 channels leave no room for a second CTA's accumulator.
 // A weight is sigmoid(score) of its own key: no running maximum, no rescaling of O, no denominator.  Weights are computed in
 // 32 bits and enter the product as a bf16 pair (hi + lo: 16 significant bits), so O is a 32-bit sum of them to 2^-17.
 // Visible keys are those up to the query's own position; the last tile's rows of V beyond the portion's end are cleared in
@@ -21,29 +23,30 @@ using namespace spk_tc;
 
 constexpr int kTile = 128;            // query rows, and keys per step
 constexpr int kColTile = kTile * 128; // bytes of a 64-channel column tile
-constexpr int kSigmoidThreads = 512;
-constexpr int kThreads = kSigmoidThreads + 128;
-constexpr uint32_t kTmemS = 0, kTmemLo = 256, kTmemO = 384;  // S/P-hi buffers 2 x 128, P-lo 2 x 64, O up to 128
 constexpr float kLog2e = 1.4426950408889634f;
 
 template <int CK, int CV>
 struct Shape {
-    static constexpr int NS = CK + CV <= 2 ? 4 : 2;  // stages of K and of V
+    static constexpr int NB = CK + CV <= 2 ? 1 : 2;  // score buffers (and parities of tiles); one lets two CTAs share an SM
+    static constexpr int NS = 2;                     // stages of K and of V
+    static constexpr int kSigmoidWarps = 8 * NB, kSigmoidThreads = 32 * kSigmoidWarps, kThreads = kSigmoidThreads + 128;
+    static constexpr uint32_t kTmemS = 0, kTmemLo = NB * 128, kTmemO = NB * 192, kColumns = NB * 256;  // S/P-hi, P-lo, O
     static constexpr int kK = CK * kColTile, kV = CV * kColTile;
     static constexpr int kBytes = kK + NS * (kK + kV) + 1024 + 256;
 };
 
 struct Bars {
-    uint64_t k_full[4], k_free[4], v_full[4], v_free[4], s_full[2], p_full[2], p_free[2], o_full, q_full, s_done;
+    uint64_t k_full[2], k_free[2], v_full[2], v_free[2], s_full[2], p_full[2], p_free[2], o_full, q_full, s_done;
     int abort;
     uint32_t tmem;
 };
 
 template <int CK, int CV>
-__global__ void __launch_bounds__(kThreads, 1)
+__global__ void __launch_bounds__(Shape<CK, CV>::kThreads, 3 - Shape<CK, CV>::NB)
 sigmoid_prefill_kernel(const spk_sigmoid_attn_args a) {
     using Sh = Shape<CK, CV>;
-    constexpr int NS = Sh::NS;
+    constexpr int NS = Sh::NS, NB = Sh::NB, W = Sh::kSigmoidWarps, kThreads = Sh::kThreads, kSigmoidThreads = Sh::kSigmoidThreads;
+    constexpr uint32_t kTmemS = Sh::kTmemS, kTmemLo = Sh::kTmemLo, kTmemO = Sh::kTmemO;
     extern __shared__ uint8_t raw[];
     uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(raw) + 1023) & ~uintptr_t(1023));
     uint8_t* q_s = base;
@@ -76,7 +79,7 @@ sigmoid_prefill_kernel(const spk_sigmoid_attn_args a) {
             mbar_init(smem_u32(&bars->v_full[i]), 1);
             mbar_init(smem_u32(&bars->v_free[i]), 1);
         }
-        for (int i = 0; i < 2; ++i) {
+        for (int i = 0; i < NB; ++i) {
             mbar_init(smem_u32(&bars->s_full[i]), 1);
             mbar_init(smem_u32(&bars->p_full[i]), 256);
             mbar_init(smem_u32(&bars->p_free[i]), 1);
@@ -86,7 +89,7 @@ sigmoid_prefill_kernel(const spk_sigmoid_attn_args a) {
         mbar_init(smem_u32(&bars->q_full), kSigmoidThreads);
         bars->abort = 0;
     }
-    if (warp == 0) tmem_alloc(smem_u32(&bars->tmem), 512);
+    if (warp == 0) tmem_alloc(smem_u32(&bars->tmem), Sh::kColumns);
     fence_async_shared();
     tc_fence_before();
     __syncthreads();
@@ -94,8 +97,8 @@ sigmoid_prefill_kernel(const spk_sigmoid_attn_args a) {
     const uint32_t tmem = bars->tmem;
     volatile int* abort = &bars->abort;
 
-    if (warp == 16 || warp == 19) {  // ---- K or V copies
-        const bool is_k = warp == 16;
+    if (warp == W || warp == W + 3) {  // ---- K or V copies
+        const bool is_k = warp == W;
         const int cols = is_k ? CK : CV;
         const int gran = a.block_size < kTile ? a.block_size : kTile;  // rows per copy
         const int per = kTile / gran;                                  // copies per column tile, at most 8
@@ -138,14 +141,14 @@ sigmoid_prefill_kernel(const spk_sigmoid_attn_args a) {
         }
         if (*abort != 0)  // copies in flight land before the CTA's shared memory is given up
             for (int t = issued > NS ? issued - NS : 0; t < issued; ++t) mbar_wait(smem_u32(full + t % NS), (t / NS) & 1);
-    } else if (warp == 17) {  // ---- scores
+    } else if (warp == W + 1) {  // ---- scores
         if (lane == 0) {
             constexpr uint32_t idesc = idesc_bf16(kTile, kTile, false, false);
             bool ok = mbar_wait(smem_u32(&bars->q_full), 0, abort);
             for (int t = 0; ok && t < tiles; ++t) {
-                const int stage = t % NS;
-                // the buffer's previous weights (tile t - 2) have been multiplied
-                ok = (t < 2 || mbar_wait(smem_u32(&bars->p_free[t & 1]), ((t >> 1) - 1) & 1, abort)) &&
+                const int stage = t % NS, buf = t % NB;
+                // the buffer's previous weights (tile t - NB) have been multiplied
+                ok = (t < NB || mbar_wait(smem_u32(&bars->p_free[buf]), ((t / NB) - 1) & 1, abort)) &&
                      mbar_wait(smem_u32(&bars->k_full[stage]), (t / NS) & 1, abort);
                 if (!ok) break;
                 tc_fence_after();
@@ -153,21 +156,21 @@ sigmoid_prefill_kernel(const spk_sigmoid_attn_args a) {
 #pragma unroll
                 for (int s = 0; s < CK * 4; ++s) {
                     const uint32_t off = (s >> 2) * kColTile + (s & 3) * 32;
-                    mma_ss(tmem + kTmemS + (t & 1) * 128, desc_sw128(qa + off, 16, 1024), desc_sw128(kb + off, 16, 1024), idesc, s > 0);
+                    mma_ss(tmem + kTmemS + buf * 128, desc_sw128(qa + off, 16, 1024), desc_sw128(kb + off, 16, 1024), idesc, s > 0);
                 }
                 mma_commit(smem_u32(&bars->k_free[stage]));
-                mma_commit(smem_u32(&bars->s_full[t & 1]));
+                mma_commit(smem_u32(&bars->s_full[buf]));
             }
             mma_commit(smem_u32(&bars->s_done));
             mbar_wait(smem_u32(&bars->s_done), 0);  // nothing this thread issued is in the tensor pipe any more
         }
-    } else if (warp == 18) {  // ---- weighted sums
+    } else if (warp == W + 2) {  // ---- weighted sums
         if (lane == 0) {
             constexpr uint32_t idesc = idesc_bf16(kTile, CV * 64, false, true);
             for (int t = 0; t < tiles; ++t) {
-                const int stage = t % NS, buf = t & 1;
+                const int stage = t % NS, buf = t % NB;
                 if (!mbar_wait(smem_u32(&bars->v_full[stage]), (t / NS) & 1, abort) ||
-                    !mbar_wait(smem_u32(&bars->p_full[buf]), (t >> 1) & 1, abort))
+                    !mbar_wait(smem_u32(&bars->p_full[buf]), (t / NB) & 1, abort))
                     break;
                 tc_fence_after();
                 const uint32_t vb = smem_u32(v_s + stage * Sh::kV);
@@ -196,14 +199,14 @@ sigmoid_prefill_kernel(const spk_sigmoid_attn_args a) {
         }
         fence_async_shared();
         mbar_arrive(smem_u32(&bars->q_full));
-        const int wg = (warp >> 2) & 1, half = warp >> 3;  // tile parity, column half
+        const int wg = NB == 2 ? (warp >> 2) & 1 : 0, half = NB == 2 ? warp >> 3 : warp >> 2;  // tile parity, column half
         const int r = (warp & 3) * 32 + lane;
         const uint32_t lanes = static_cast<uint32_t>((warp & 3) * 32) << 16;
         const uint64_t c1 = f2_pack(-a.scale * kLog2e, -a.scale * kLog2e), c0 = f2_pack(-a.head_bias[h] * kLog2e, -a.head_bias[h] * kLog2e);
         bool ok = true;
-        for (int t = wg; t < tiles; t += 2) {
+        for (int t = wg; t < tiles; t += NB) {
             const int stage = t % NS;
-            ok = __all_sync(~0u, mbar_wait(smem_u32(&bars->s_full[wg]), (t >> 1) & 1, abort));
+            ok = __all_sync(~0u, mbar_wait(smem_u32(&bars->s_full[wg]), (t / NB) & 1, abort));
             if (!ok) break;
             tc_fence_after();
             const int last = pos0 + r - t * kTile;  // last visible column of this row
@@ -281,7 +284,7 @@ sigmoid_prefill_kernel(const spk_sigmoid_attn_args a) {
     __syncthreads();
     tc_fence_after();
     if (threadIdx.x == 0 && *abort != 0) spk_flag(a.status, SPK_STATUS_DEVICE_WAIT_EXPIRED);
-    if (warp == 0) tmem_dealloc(tmem, 512);
+    if (warp == 0) tmem_dealloc(tmem, Sh::kColumns);
 }
 
 template <int CK, int CV>
@@ -290,7 +293,7 @@ int launch(const spk_sigmoid_attn_args& a, cudaStream_t s) {
     static_assert(sizeof(Bars) <= 256 && bytes <= 227 * 1024, "shared memory");
     const cudaError_t e = cudaFuncSetAttribute(sigmoid_prefill_kernel<CK, CV>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
     if (e != cudaSuccess) return spk_set_cuda_error(e);
-    sigmoid_prefill_kernel<CK, CV><<<dim3(a.heads, a.n_tiles), kThreads, bytes, s>>>(a);
+    sigmoid_prefill_kernel<CK, CV><<<dim3(a.heads, a.n_tiles), Shape<CK, CV>::kThreads, bytes, s>>>(a);
     SPK_CHECK_LAUNCH();
     return SPK_OK;
 }
