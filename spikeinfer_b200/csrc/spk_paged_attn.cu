@@ -85,44 +85,36 @@ qk_prepare_kernel(const spk_qk_prepare_args a) {
 }
 
 // The same for bf16 heads of DIM = 64 or 128 channels (q, k and v alike) in tiled pools, eight channels (16 bytes) per lane: a
-// rotated pair's channels sit in two lanes of the head.  rot_dims is a multiple of 16.
-template <int DIM>
+// rotated pair's channels sit in two lanes of the head.  rot_dims is a multiple of 16.  A lane takes H heads of its token: their loads are in flight
+// together and share the rotation's factors, four times as many bytes as the channels
+// (8192 tokens, 14/2 heads of 64: 14.9 -> 13.4 us; 4096 tokens, 28/4 of 128: 33.4 -> 25.3).
+template <int DIM, int H>
 __global__ void __launch_bounds__(kThreads)
 qk_prepare_vec_kernel(const spk_qk_prepare_args a) {
     spk_grid_release();
     constexpr int LK = DIM / 8;  // lanes per head: 8 or 16, so a warp holds whole heads
-    const int lanes_t = (a.heads + 2 * a.kv_heads) * LK;
+    const int qk_heads = a.heads + a.kv_heads, slots = qk_heads + a.kv_heads;  // q heads, then k heads, then v heads
+    const uint32_t lanes_t = (slots + H - 1) / H * LK;
     // 32-bit indices (checked on the host): 64-bit divisions were a large part of this kernel's instructions
-    const uint32_t item = blockIdx.x * kThreads + threadIdx.x, row = item / static_cast<uint32_t>(lanes_t);
+    const uint32_t item = blockIdx.x * kThreads + threadIdx.x, row = item / lanes_t;
     const int64_t t = row;
     const bool in = t < a.n;
-    const int l = static_cast<int>(item - row * lanes_t);
-    const int qk_lanes = (a.heads + a.kv_heads) * LK;
-    const bool is_v = l >= qk_lanes;
-    const int s = (is_v ? l - qk_lanes : l) / LK;  // head slot (q heads, then k heads) or v head
-    const int sub = l % LK;
-    const bool is_q = !is_v && s < a.heads;
-    const __nv_bfloat16* src = is_v ? static_cast<const __nv_bfloat16*>(a.v) + t * a.ld + s * DIM + sub * 8
-                             : is_q ? static_cast<const __nv_bfloat16*>(a.q) + t * a.ld + s * DIM + sub * 8
-                                    : static_cast<const __nv_bfloat16*>(a.k) + t * a.ld + (s - a.heads) * DIM + sub * 8;
-    const uint4 u = in ? *reinterpret_cast<const uint4*>(src) : make_uint4(0u, 0u, 0u, 0u);
-    float x[8];
-    {
-        const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+    const int l = static_cast<int>(item - row * lanes_t), s0 = l / LK * H, sub = l % LK;
+    uint4 u[H];
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            x[2 * k] = __uint_as_float(w[k] << 16);
-            x[2 * k + 1] = __uint_as_float(w[k] & 0xffff0000u);
-        }
+    for (int i = 0; i < H; ++i) {
+        const int s = s0 + i;
+        const __nv_bfloat16* src = s >= qk_heads ? static_cast<const __nv_bfloat16*>(a.v) + (s - qk_heads) * DIM
+                                 : s >= a.heads ? static_cast<const __nv_bfloat16*>(a.k) + (s - a.heads) * DIM
+                                                : static_cast<const __nv_bfloat16*>(a.q) + s * DIM;
+        u[i] = in && s < slots ? *reinterpret_cast<const uint4*>(src + t * a.ld + sub * 8) : make_uint4(0u, 0u, 0u, 0u);
     }
     const int half = a.rot_table != nullptr ? a.rot_dims / 2 : 0;
     const int hl = half / 8;  // lanes of each half of the rotated channels
-    const bool low = sub < hl, turn = !is_v && sub < 2 * hl;
-    float y[8];
-    const int partner = (threadIdx.x & 31) + (turn ? (low ? hl : -hl) : 0);
-#pragma unroll
-    for (int k = 0; k < 8; ++k) y[k] = __shfl_sync(~0u, x[k], partner);
-    if (turn && in) {
+    const bool low = sub < hl, rotates = sub < 2 * hl;
+    const int partner = (threadIdx.x & 31) + (rotates ? (low ? hl : -hl) : 0);
+    float4 f[4];  // (cos, sin) of two pairs each
+    if (rotates && in && s0 < qk_heads) {
         int64_t pos = a.positions[t];
         if (pos < 0 || pos >= a.rot_positions) {
             spk_flag(a.status, SPK_STATUS_BAD_SEQ_LEN);
@@ -130,50 +122,67 @@ qk_prepare_vec_kernel(const spk_qk_prepare_args a) {
         }
         const float4* cs = reinterpret_cast<const float4*>(reinterpret_cast<const float2*>(a.rot_table) + pos * half + (low ? sub : sub - hl) * 8);
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            const float4 f = cs[k];  // (cos, sin) of two pairs
-            const float s0 = low ? -f.y : f.y, s1 = low ? -f.w : f.w;
-            x[2 * k] = x[2 * k] * f.x + y[2 * k] * s0;
-            x[2 * k + 1] = x[2 * k + 1] * f.z + y[2 * k + 1] * s1;
-        }
+        for (int k = 0; k < 4; ++k) f[k] = cs[k];
     }
-    float ss = 0.0f;
-#pragma unroll
-    for (int k = 0; k < 8; ++k) ss = fmaf(x[k], x[k], ss);
-#pragma unroll
-    for (int o = LK / 2; o >= 1; o >>= 1) ss += __shfl_xor_sync(~0u, ss, o);
-    if (!in) return;
-    const float inv = a.unit_norm ? 1.0f / sqrtf(ss / static_cast<float>(DIM) + a.eps) : 1.0f;
-    uint4 r = u;
-    if (!is_v) {
-        uint32_t w[4];
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            const __nv_bfloat162 b = __floats2bfloat162_rn(x[2 * k] * inv, x[2 * k + 1] * inv);
-            w[k] = *reinterpret_cast<const uint32_t*>(&b);
-        }
-        r = make_uint4(w[0], w[1], w[2], w[3]);
-    }
-    if (is_q) {
-        *reinterpret_cast<uint4*>(static_cast<__nv_bfloat16*>(a.q_out) + (t * a.heads + s) * DIM + sub * 8) = r;
-        return;
-    }
-    const int64_t slot = a.slot_mapping[t];
+    int64_t slot = -1;
+    if (in && s0 + H > a.heads) slot = a.slot_mapping[t];
     const uint32_t block = static_cast<uint32_t>(slot) / static_cast<uint32_t>(a.block_size);
-    if (slot < 0 || slot > 0x7fffffff || block >= a.num_blocks) {
-        spk_flag(a.status, SPK_STATUS_BAD_SLOT);
-        return;
-    }
+    const int r = static_cast<int>(static_cast<uint32_t>(slot) - block * a.block_size);
+    const bool slot_ok = slot >= 0 && slot <= 0x7fffffff && block < a.num_blocks;
     const SpkPageLayout lay{a.kv_heads, a.block_size, DIM, 1};
-    __nv_bfloat16* page = static_cast<__nv_bfloat16*>(is_v ? a.v_pool : a.k_pool) + spk_page_base(lay, block, is_v ? s : s - a.heads);
-    *reinterpret_cast<uint4*>(page + spk_page_channel(lay, static_cast<int>(static_cast<uint32_t>(slot) - block * a.block_size), sub * 8)) = r;
+#pragma unroll
+    for (int i = 0; i < H; ++i) {
+        const int s = s0 + i;
+        const bool is_v = s >= qk_heads;
+        uint32_t w[4] = {u[i].x, u[i].y, u[i].z, u[i].w};
+        float x[8], y[8];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const uint32_t o = __shfl_sync(~0u, w[k], partner);
+            x[2 * k] = __uint_as_float(w[k] << 16);
+            x[2 * k + 1] = __uint_as_float(w[k] & 0xffff0000u);
+            y[2 * k] = __uint_as_float(o << 16);
+            y[2 * k + 1] = __uint_as_float(o & 0xffff0000u);
+        }
+        if (rotates && in && !is_v) {
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const float sin0 = low ? -f[k].y : f[k].y, sin1 = low ? -f[k].w : f[k].w;
+                x[2 * k] = x[2 * k] * f[k].x + y[2 * k] * sin0;
+                x[2 * k + 1] = x[2 * k + 1] * f[k].z + y[2 * k + 1] * sin1;
+            }
+        }
+        float ss = 0.0f;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) ss = fmaf(x[k], x[k], ss);
+#pragma unroll
+        for (int o = LK / 2; o >= 1; o >>= 1) ss += __shfl_xor_sync(~0u, ss, o);
+        if (!in || s >= slots) continue;
+        if (!is_v) {
+            const float inv = a.unit_norm ? 1.0f / sqrtf(ss / static_cast<float>(DIM) + a.eps) : 1.0f;
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const __nv_bfloat162 b = __floats2bfloat162_rn(x[2 * k] * inv, x[2 * k + 1] * inv);
+                w[k] = *reinterpret_cast<const uint32_t*>(&b);
+            }
+        }
+        const uint4 v = make_uint4(w[0], w[1], w[2], w[3]);
+        if (s < a.heads) {
+            *reinterpret_cast<uint4*>(static_cast<__nv_bfloat16*>(a.q_out) + (t * a.heads + s) * DIM + sub * 8) = v;
+        } else if (!slot_ok) {
+            spk_flag(a.status, SPK_STATUS_BAD_SLOT);
+        } else {
+            __nv_bfloat16* page = static_cast<__nv_bfloat16*>(is_v ? a.v_pool : a.k_pool) + spk_page_base(lay, block, is_v ? s - qk_heads : s - a.heads);
+            *reinterpret_cast<uint4*>(page + spk_page_channel(lay, r, sub * 8)) = v;
+        }
+    }
 }
 
-template <int DIM>
+template <int DIM, int H>
 int launch_prepare_vec(const spk_qk_prepare_args& a, cudaStream_t s) {
-    const int64_t items = a.n * (a.heads + 2 * static_cast<int64_t>(a.kv_heads)) * (DIM / 8);
+    const int64_t items = a.n * ((a.heads + 2 * static_cast<int64_t>(a.kv_heads) + H - 1) / H) * (DIM / 8);
     const int64_t grid = (items + kThreads - 1) / kThreads;
-    qk_prepare_vec_kernel<DIM><<<static_cast<unsigned>(grid), kThreads, 0, s>>>(a);
+    qk_prepare_vec_kernel<DIM, H><<<static_cast<unsigned>(grid), kThreads, 0, s>>>(a);
     SPK_CHECK_LAUNCH();
     return SPK_OK;
 }
@@ -308,8 +317,14 @@ extern "C" int spk_qk_prepare(const spk_qk_prepare_args* a, void* stream) {
     const int64_t lanes = a->n * (a->heads + 2 * static_cast<int64_t>(a->kv_heads)) * (a->dim / 8);
     if (lanes < 0x7fffff00LL && a->num_blocks <= 0x7fffffffLL / a->block_size && a->dtype == SPK_BF16 && a->k_tiled && a->v_tiled && a->dim == a->vdim && (a->dim == 64 || a->dim == 128) && a->k_pad == a->dim &&
         a->v_pad == a->vdim && a->ld % 8 == 0 && (a->rot_table == nullptr || (a->rot_dims % 16 == 0 && at16(a->rot_table))) && at16(a->q) &&
-        at16(a->k) && at16(a->v) && at16(a->q_out) && at16(a->k_pool) && at16(a->v_pool))
-        return a->dim == 64 ? launch_prepare_vec<64>(*a, spk_stream(stream)) : launch_prepare_vec<128>(*a, spk_stream(stream));
+        at16(a->k) && at16(a->v) && at16(a->q_out) && at16(a->k_pool) && at16(a->v_pool)) {
+        // four heads per lane once that still leaves 512 lanes per SM: 1024 tokens of 28/4 heads of 128 (590 k lanes) 9.7 -> 8.6 us, 4096 of 14/2 of 64 8.6 -> 8.3;
+        // below, a head per lane starts more loads at once (64 tokens 2.8 -> 2.6 us, by exchanging packed pairs)
+        cudaStream_t s = spk_stream(stream);
+        const bool many = lanes >= 148LL * 2048;
+        if (a->dim == 64) return many ? launch_prepare_vec<64, 4>(*a, s) : launch_prepare_vec<64, 1>(*a, s);
+        return many ? launch_prepare_vec<128, 4>(*a, s) : launch_prepare_vec<128, 1>(*a, s);
+    }
     const int64_t items = a->n * (a->heads + 2 * static_cast<int64_t>(a->kv_heads));
     const int64_t grid = (items + kWarps - 1) / kWarps;
     const size_t bytes = sizeof(float) * kWarps * a->dim;
