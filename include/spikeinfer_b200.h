@@ -822,7 +822,7 @@ typedef struct spk_latent_prefill_args {
     int32_t vec_q, vec_out;     /* set by the call */
     int32_t dtype;
     float scale;
-    float _pad;
+    int32_t vec_rot;            /* set by the call */
     uint32_t* status;
 } spk_latent_prefill_args;
 int spk_latent_prefill(const spk_latent_prefill_args* args, void* stream);

@@ -190,7 +190,7 @@ class LatentPrefillArgs(Structure):
     """Mirror of ``spk_latent_prefill_args``."""
 
     _fields_ = _fields("p q kv kr tiles sink gate out rot_table; l rot_positions n n_ctx gate_stride out_stride; "
-                       "i n_tiles heads dim rot_dim vdim dim_pad vdim_pad vec_q vec_out dtype; f scale _pad; p status")
+                       "i n_tiles heads dim rot_dim vdim dim_pad vdim_pad vec_q vec_out dtype; f scale; i vec_rot; p status")
 
 
 class DeltaArgs(Structure):
