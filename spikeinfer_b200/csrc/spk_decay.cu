@@ -169,10 +169,8 @@ decay_chunk_sum_kernel(const spk_decay_attn_args a) {
     }
 }
 
-// Element (seq, head, d, e): replaces every chunk's own sum by the state the chunk starts from and, with FINAL, leaves the sequence's
-// final state in its slot.  Without, a sequence's last chunk has no sum (its outputs' launch carries the state to the end), and sequences
-// of one chunk are left out.
-template <bool FINAL>
+// Element (seq, head, d, e): replaces every chunk's own sum by the state the chunk starts from, leaves the sequence's
+// final state in its slot.
 __global__ void __launch_bounds__(kThreads)
 decay_scan_kernel(const spk_decay_attn_args a) {
     const int64_t per_head = static_cast<int64_t>(a.dim) * a.vdim;
@@ -180,12 +178,10 @@ decay_scan_kernel(const spk_decay_attn_args a) {
     const int64_t i = static_cast<int64_t>(blockIdx.x) * kThreads + threadIdx.x;
     if (i >= per_chunk) return;
     const int4 sq = reinterpret_cast<const int4*>(a.seqs)[blockIdx.y];  // first chunk, chunks, state row, context
-    if (!FINAL && sq.y == 1) return;
     if (sq.z < 0 || sq.z >= a.state_rows) {
         if (i == 0) spk_flag(a.status, SPK_STATUS_BAD_SLOT);
         return;
     }
-    const int sums = FINAL ? sq.y : sq.y - 1;
     const float* pw = a.decay_pow + (i / per_head) * kPow;
     float* slot = a.state + sq.z * a.state_stride + i;
     float S = sq.w > 0 ? *slot : 0.0f;
@@ -195,7 +191,7 @@ decay_scan_kernel(const spk_decay_attn_args a) {
         float own[U], p[U];
 #pragma unroll
         for (int u = 0; u < U; ++u) {
-            const bool in = c0 + u < sums;
+            const bool in = c0 + u < sq.y;
             own[u] = in ? w[(c0 + u) * per_chunk] : 0.0f;
             p[u] = in ? pw[a.chunks[4 * (sq.x + c0 + u) + 1]] : 1.0f;
         }
@@ -205,7 +201,7 @@ decay_scan_kernel(const spk_decay_attn_args a) {
             S = fmaf(p[u], S, own[u]);
         }
     }
-    if (FINAL) *slot = S;
+    *slot = S;
 }
 
 template <typename T>
@@ -467,10 +463,9 @@ int launch_step(const spk_decay_attn_args& a, cudaStream_t s) {
     return spk_launch(vec ? decay_step_kernel<T, 4> : decay_step_kernel<T, 1>, grid, kThreads, bytes, s, a.overlap != 0, a);
 }
 
-template <bool FINAL>
 int launch_scan(const spk_decay_attn_args& a, cudaStream_t s) {
     const int64_t per = static_cast<int64_t>(a.heads) * a.dim * a.vdim;
-    decay_scan_kernel<FINAL><<<dim3(static_cast<unsigned>((per + kThreads - 1) / kThreads), a.n_seqs), kThreads, 0, s>>>(a);
+    decay_scan_kernel<<<dim3(static_cast<unsigned>((per + kThreads - 1) / kThreads), a.n_seqs), kThreads, 0, s>>>(a);
     SPK_CHECK_LAUNCH();
     return SPK_OK;
 }
@@ -484,7 +479,7 @@ int launch_chunks(const spk_decay_attn_args& a, cudaStream_t s) {
     const dim3 grid(a.n_chunks, a.heads);
     decay_chunk_sum_kernel<T><<<grid, kThreads, b1, s>>>(a);
     SPK_CHECK_LAUNCH();
-    if (const int rc = launch_scan<true>(a, s)) return rc;
+    if (const int rc = launch_scan(a, s)) return rc;
     decay_chunk_out_kernel<T><<<grid, kThreads, b3, s>>>(a);
     SPK_CHECK_LAUNCH();
     return SPK_OK;
@@ -537,10 +532,8 @@ extern "C" int spk_decay_attn_chunks(const spk_decay_attn_args* a, void* stream)
         return SPK_ERR_WORKSPACE_TOO_SMALL;
     cudaStream_t s = spk_stream(stream);
     if (spk_decay_tensor_form(a->dtype, a->dim, a->vdim)) {
-        if (a->n_chunks > a->n_seqs) {  // a portion of several spans
-            if (const int e = spk_decay_mma_sums(*a, s)) return e;
-            if (const int e = launch_scan<false>(*a, s)) return e;
-        }
+        if (const int e = spk_decay_mma_sums(*a, s)) return e;
+        if (const int e = launch_scan(*a, s)) return e;
         return spk_decay_mma_outputs(*a, s);
     }
     return a->dtype == SPK_F32 ? launch_chunks<float>(*a, s) : launch_chunks<__nv_bfloat16>(*a, s);

@@ -2,12 +2,10 @@
 //
 // A stored state every `span` tokens (64 .. 512, chosen by the host for the call's size) keeps the traffic of the
 // states small; inside a span a CTA walks 64-token chunks with the running state in its registers:
-//  * decay_span_sum_kernel:  U = sum_j decay^(L-1-j) k_j v_j^T of a span of L tokens, for all but a portion's last span;
+//  * decay_span_sum_kernel:  U = sum_j decay^(L-1-j) k_j v_j^T of a span of L tokens;
 //  * (the scan of spk_decay.cu turns the U of every span into the state the span starts from);
 //  * decay_span_out_kernel:  per chunk o_i = decay^(i+1) S^T q_i + sum_{j<=i} decay^(i-j) (q_i.k_j) v_j, then
-//    S <- decay^len S + sum_j decay^(len-1-j) k_j v_j^T; a portion's last span ends at the portion's state.
-// A portion of one span needs the last launch alone: 16 portions of 512 tokens, 14 heads of 64, took 44.5 us there and 26 + 14 us in the sums and
-// the scan before it.
+//    S <- decay^len S + sum_j decay^(len-1-j) k_j v_j^T.
 // q, k and v are bf16 after their activation; everything the recurrence adds to them (decayed keys, decayed scores, states)
 // is 32-bit and enters a product as a bf16 pair (hi + lo, 16 significant bits), accumulated in 32 bits.
 #include "spk_decay.cuh"
@@ -126,7 +124,6 @@ decay_span_sum_kernel(const spk_decay_attn_args a, const bool vec_k, const bool 
     __nv_bfloat16* vb = kb + 2 * C * SK;
     const int h = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const SpkChunk ci = spk_chunk(a, blockIdx.x);
-    if (ci.index == reinterpret_cast<const int4*>(a.seqs)[ci.seq].y - 1) return;  // nothing starts from a portion's last span
     const float* pw = a.decay_pow + static_cast<int64_t>(h) * (kDecayMaxSpan + 1);
     const __nv_bfloat16* ks = static_cast<const __nv_bfloat16*>(a.k) + ci.start * a.ld + static_cast<int64_t>(h) * a.dim;
     const __nv_bfloat16* vs = static_cast<const __nv_bfloat16*>(a.v) + ci.start * a.ld + static_cast<int64_t>(h) * a.vdim;
@@ -180,18 +177,14 @@ decay_span_out_kernel(const spk_decay_attn_args a, const bool vec_k, const bool 
     const __nv_bfloat16* qs = static_cast<const __nv_bfloat16*>(a.q) + ci.start * a.ld + static_cast<int64_t>(h) * a.dim;
     const __nv_bfloat16* ks = static_cast<const __nv_bfloat16*>(a.k) + ci.start * a.ld + static_cast<int64_t>(h) * a.dim;
     const __nv_bfloat16* vs = static_cast<const __nv_bfloat16*>(a.v) + ci.start * a.ld + static_cast<int64_t>(h) * a.vdim;
-    const int4 sq = reinterpret_cast<const int4*>(a.seqs)[ci.seq];  // first span, spans, state row, tokens before
-    const bool last = ci.index == sq.y - 1, row_ok = sq.z >= 0 && sq.z < a.state_rows;
-    if (last && !row_ok && threadIdx.x == 0) spk_flag(a.status, SPK_STATUS_BAD_SLOT);
-    float* slot = a.state + (row_ok ? sq.z : 0) * a.state_stride + static_cast<int64_t>(h) * a.dim * a.vdim;
-    const float* S0 = sq.y > 1 ? a.workspace + (static_cast<int64_t>(blockIdx.x) * a.heads + h) * a.dim * a.vdim : row_ok && sq.w > 0 ? slot : nullptr;
+    const float* S0 = a.workspace + (static_cast<int64_t>(blockIdx.x) * a.heads + h) * a.dim * a.vdim;
     float S[T::NT][4];
 #pragma unroll
     for (int n = 0; n < T::NT; ++n)
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
             const int d = T::row0(warp) + gid + (i >> 1) * 8, e = T::col0(warp) + n * 8 + tig * 2 + (i & 1);
-            S[n][i] = S0 != nullptr && d < a.dim && e < a.vdim ? S0[static_cast<int64_t>(d) * a.vdim + e] : 0.0f;
+            S[n][i] = d < a.dim && e < a.vdim ? S0[static_cast<int64_t>(d) * a.vdim + e] : 0.0f;
         }
     const int i0 = (warp & 3) * 16;                 // this warp's 16 tokens
     constexpr int OC = T::V / (NW / 4), ON = OC / 8;  // and its share of the output columns
@@ -211,7 +204,7 @@ decay_span_out_kernel(const spk_decay_attn_args a, const bool vec_k, const bool 
         cp_async_wait_all();
         __syncthreads();  // the previous chunk's reads are done (and pw is there)
         activate<T::D, T::THREADS, true>(q, len, a.silu, nullptr, nullptr, pw, 0);
-        activate<T::D, T::THREADS, true>(k, len, a.silu, more || last ? hi : nullptr, lo, pw, len - 1);
+        activate<T::D, T::THREADS, true>(k, len, a.silu, more ? hi : nullptr, lo, pw, len - 1);
         activate<T::V, T::THREADS, true>(v, len, a.silu, nullptr, nullptr, pw, 0);
         if (more) fetch_chunk(c0 + C, buf ^ 1);
 #pragma unroll
@@ -302,8 +295,8 @@ decay_span_out_kernel(const spk_decay_attn_args a, const bool vec_k, const bool 
                 }
             }
         }
-        if (more || last) {
-            const float w = pw[len];
+        if (more) {  // a whole chunk: len == C
+            const float w = pw[C];
 #pragma unroll
             for (int n = 0; n < T::NT; ++n)
 #pragma unroll
@@ -311,14 +304,6 @@ decay_span_out_kernel(const spk_decay_attn_args a, const bool vec_k, const bool 
             add_outer<CD, CV, NW>(S, hi, lo, v, warp, lane);
         }
     }
-    if (!last || !row_ok) return;
-#pragma unroll
-    for (int n = 0; n < T::NT; ++n)
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const int d = T::row0(warp) + gid + (i >> 1) * 8, e = T::col0(warp) + n * 8 + tig * 2 + (i & 1);
-            if (d < a.dim && e < a.vdim) slot[static_cast<int64_t>(d) * a.vdim + e] = S[n][i];
-        }
 }
 
 template <typename F>

@@ -457,31 +457,6 @@ def test_decay_attention_portions_and_steps(dev, shape, dtype):
     assert rel(state[2], S_x) < tol and torch.equal(state[0], kept) and torch.isnan(state[1]).all() and status.item() == 0
 
 
-@pytest.mark.parametrize("dim", [64, 128])
-@pytest.mark.parametrize("lens", [[1, 64, 65, 63], [200, 1, 64, 300], [512, 513]])
-def test_decay_portions_of_one_and_of_several_spans(dev, lens, dim):
-    """States and outputs where portions of one span, whose launch ends at the state, lie beside portions of several; every other one continues."""
-    heads, n, decay = 2, sum(lens), [0.9, 0.998]
-    g = gen(dim + n)
-    x = torch.randn(n, 3 * heads * dim, generator=g).to(torch.bfloat16)
-    first = torch.randn(len(lens) + 1, heads, dim, dim, generator=g)
-    state = first.to(dev)
-    starts, before = [sum(lens[:i]) for i in range(len(lens))], [7 * (i % 2) for i in range(len(lens))]
-    status = torch.zeros(1, dtype=torch.int32, device=dev)
-    plan = PrefillPlan(starts, lens, before, list(range(len(lens))), dev)
-    o = dense.decay_attention(*x.to(dev).split(heads * dim, dim=1), state, dense.decay_powers(decay, dev), plan=plan, status=status)
-    q, k, v = (mo.silu(p.double()).view(n, heads, dim) for p in x.split(heads * dim, dim=1))
-    a = torch.tensor(decay, dtype=torch.float64)[:, None, None]
-    for i, (at, m) in enumerate(zip(starts, lens)):
-        S = first[i].double() if before[i] else torch.zeros(heads, dim, dim, dtype=torch.float64)
-        want = []
-        for t in range(at, at + m):
-            S = a * S + k[t][:, :, None] * v[t][:, None, :]
-            want.append(torch.einsum("hd,hde->he", q[t], S).flatten())
-        assert rel(o[at: at + m], torch.stack(want)) < TOL[torch.bfloat16] and rel(state[i], S) < TOL[torch.bfloat16], (i, m)
-    assert torch.equal(state[-1].cpu(), first[-1]) and status.item() == 0
-
-
 def test_decay_of_a_long_prompt_keeps_the_first_token(dev):
     """A decay next to one, keys that are zero except the first: the first token's value must still be there at the end."""
     for dtype in DTYPES:
