@@ -13,7 +13,6 @@
 //
 // Decay powers come from a host table [head][0 .. 512] (evaluated in double precision), never from repeated products.
 #include "spk_decay.cuh"
-#include "spk_tensor.cuh"
 
 namespace {
 
@@ -285,11 +284,6 @@ decay_chunk_out_kernel(const spk_decay_attn_args a) {
 }
 
 // ---- output stage --------------------------------------------------------------------------------------------
-// A gate for results of type T.  16-bit results: 2^-22 of error is far below their rounding, and the exact division took most of the time (4096 rows
-// of 3584, 43.7 -> 25.0 us).
-template <typename T>
-__device__ __forceinline__ float sigmoid_for(float x) { return sizeof(T) == 2 ? spk_tc::sigmoid_fast(x) : spk_sigmoid(x); }
-
 template <typename T>
 __global__ void __launch_bounds__(kThreads)
 gated_norm_kernel(const spk_gated_norm_args a) {
@@ -362,8 +356,8 @@ gated_norm_vec_kernel(const spk_gated_norm_args a) {
 #pragma unroll
     for (int i = 0; i < V; ++i) {
         const int c = 4 * (threadIdx.x + i * blockDim.x);
-        const float4 y = make_float4(xv[i].x * inv * wv[i].x * sigmoid_for<T>(gv[i].x), xv[i].y * inv * wv[i].y * sigmoid_for<T>(gv[i].y),
-                                     xv[i].z * inv * wv[i].z * sigmoid_for<T>(gv[i].z), xv[i].w * inv * wv[i].w * sigmoid_for<T>(gv[i].w));
+        const float4 y = make_float4(xv[i].x * inv * wv[i].x * spk_sigmoid(gv[i].x), xv[i].y * inv * wv[i].y * spk_sigmoid(gv[i].y),
+                                     xv[i].z * inv * wv[i].z * spk_sigmoid(gv[i].z), xv[i].w * inv * wv[i].w * spk_sigmoid(gv[i].w));
         spk_store4<T, true>(out + a.out_offset + c, live ? y : make_float4(0.f, 0.f, 0.f, 0.f), a.width - c);
     }
 }
@@ -386,16 +380,16 @@ gated_norm_rows_kernel(const spk_gated_norm_args a) {
         xv[i] = spk_load4<float, true>(x + c, a.width - c);
         gv[i] = spk_load4<T, true>(g + c, a.width - c);
     }
-    float ss = 0.0f;
+    float ss[8] = {};  // in the order of gated_norm_vec_kernel's CTA of eight warps: the same bits
 #pragma unroll
-    for (int i = 0; i < G; ++i) ss += xv[i].x * xv[i].x + xv[i].y * xv[i].y + xv[i].z * xv[i].z + xv[i].w * xv[i].w;
-    const float inv = a.scale / sqrtf(spk_warp_sum(ss) / static_cast<float>(a.width) + a.eps);
+    for (int i = 0; i < G; ++i) ss[i] += xv[i].x * xv[i].x + xv[i].y * xv[i].y + xv[i].z * xv[i].z + xv[i].w * xv[i].w;
+    const float inv = a.scale / sqrtf(spk_row_sum<8>(ss, lane) / static_cast<float>(a.width) + a.eps);
 #pragma unroll
     for (int i = 0; i < G; ++i) {
         const int c = 4 * (lane + 32 * i);
         const float4 w = spk_load4<float, true>(a.w + c, a.width - c);
-        const float4 y = make_float4(xv[i].x * inv * w.x * sigmoid_for<T>(gv[i].x), xv[i].y * inv * w.y * sigmoid_for<T>(gv[i].y),
-                                     xv[i].z * inv * w.z * sigmoid_for<T>(gv[i].z), xv[i].w * inv * w.w * sigmoid_for<T>(gv[i].w));
+        const float4 y = make_float4(xv[i].x * inv * w.x * spk_sigmoid(gv[i].x), xv[i].y * inv * w.y * spk_sigmoid(gv[i].y),
+                                     xv[i].z * inv * w.z * spk_sigmoid(gv[i].z), xv[i].w * inv * w.w * spk_sigmoid(gv[i].w));
         spk_store4<T, true>(out + c, live ? y : make_float4(0.f, 0.f, 0.f, 0.f), a.width - c);
     }
 }
@@ -409,8 +403,8 @@ int launch_gated(const spk_gated_norm_args& a, cudaStream_t s) {
                      (a.partials == nullptr || (a.left_width % 4 == 0 && aligned(a.partials, 16)));
     if (!vec) {
         gated_norm_kernel<T><<<grid, kThreads, 0, s>>>(a);
-    } else if (a.partials == nullptr && a.width <= 1024 && a.n >= 8 * 148) {
-        // a warp per row from eight rows per SM on: 1184 rows of 896 5.0 -> 4.3 us, 2048 7.0 -> 4.4, 8192 25.6 -> 13.6
+    } else if (a.partials == nullptr && a.width <= 1024 && a.n >= 8192) {
+        // a warp per row where it is measured to gain: 8192 rows of 896 26.0 -> 22.0 us (the exact gates take most of what is left)
         const unsigned rows = (grid + kThreads / 32 - 1) / (kThreads / 32);
         switch ((a.width + 127) / 128) {
             case 1: case 2: gated_norm_rows_kernel<T, 2><<<rows, kThreads, 0, s>>>(a); break;

@@ -80,6 +80,31 @@ __device__ __forceinline__ void spk_block_sum(float (&v)[N], float* part) {
     for (int i = 0; i < N; ++i) v[i] = spk_warp_sum(lane < warps ? part[i * 32 + lane] : 0.0f);
 }
 
+// The same total, to the bit, where one warp holds what a CTA of W warps would: p[w] is the value of thread 32 w + lane.  Values are folded two,
+// then four to a lane on the way, so that W totals cost W + 4 - W / 4 exchanges and not 5 W.
+template <int W>
+__device__ __forceinline__ float spk_row_sum(const float (&p)[W], int lane) {
+    static_assert(W == 4 || W == 8, "four or eight warps");
+    float r[W];
+#pragma unroll
+    for (int i = 0; i < W; ++i) r[i] = p[i];
+#pragma unroll
+    for (int o = 16, half = W / 2; half >= 1; o >>= 1, half >>= 1) {
+        const bool upper = (lane & o) != 0;
+#pragma unroll
+        for (int i = 0; i < half; ++i) {
+            const float send = upper ? r[i] : r[i + half], keep = upper ? r[i + half] : r[i];
+            r[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+        }
+    }
+    float v = r[0];
+#pragma unroll
+    for (int o = W == 8 ? 2 : 4; o >= 1; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+#pragma unroll
+    for (int o = 16; o >= (W == 8 ? 4 : 8); o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
+
 __device__ __forceinline__ float spk_sigmoid(float x) { return 1.0f / (1.0f + expf(-x)); }
 __device__ __forceinline__ float spk_silu(float x) { return x / (1.0f + expf(-x)); }
 

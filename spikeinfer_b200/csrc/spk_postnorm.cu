@@ -161,7 +161,7 @@ residual_norm_kernel(const ResidualNormParams p, T* __restrict__ out) {
 // The same for many rows of up to 128 G elements (a multiple of four): a warp per row, its elements in registers, no barrier but the one that
 // hands rows on.  A CTA takes two times eight rows; with a token shift each warp leaves its x' in shared memory for the warp of the next
 // row, so only a CTA's first predecessor is computed twice.  A CTA per row (or per four) was bound by CTAs started and barriers waited for, at
-// 12 to 30 % of the memory's rate: 8192 x 896, 110 MB, 32.7 -> 22.0 us with the shift and 27.8 -> 19.0 us without.
+// 12 to 30 % of the memory's rate: 8192 x 896, 110 MB, 32.7 -> 22 us with the shift and 27.8 -> 19 us without.
 constexpr int kRowWarps = 8, kRowSteps = 2;  // each step has its buffer in shared memory: one barrier per step is enough
 
 template <typename TD, int G>
@@ -188,17 +188,18 @@ __device__ __forceinline__ void warp_new_row(const ResidualNormParams& p, int64_
 
 template <int G>
 __device__ __forceinline__ void warp_layer_norm(float4 (&y)[G], const float* __restrict__ w, int width, float eps, const int lane) {
-    float s = 0.0f, q = 0.0f;
+    // sums in the order of residual_norm_kernel's CTA of four warps with up to two groups per thread: the same bits
+    float s[4] = {}, q[4] = {};
 #pragma unroll
-    for (int g = 0; g < G; ++g) s += (y[g].x + y[g].y) + (y[g].z + y[g].w);
-    const float mean = spk_warp_sum(s) / static_cast<float>(width);
+    for (int g = 0; g < G; ++g) s[g & 3] += (y[g].x + y[g].y) + (y[g].z + y[g].w);
+    const float mean = spk_row_sum<4>(s, lane) / static_cast<float>(width);
 #pragma unroll
     for (int g = 0; g < G; ++g) {
         const bool in = 4 * (lane + 32 * g) < width;
         y[g] = in ? make_float4(y[g].x - mean, y[g].y - mean, y[g].z - mean, y[g].w - mean) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        q += (y[g].x * y[g].x + y[g].y * y[g].y) + (y[g].z * y[g].z + y[g].w * y[g].w);
+        q[g & 3] += (y[g].x * y[g].x + y[g].y * y[g].y) + (y[g].z * y[g].z + y[g].w * y[g].w);
     }
-    const float inv = 1.0f / sqrtf(spk_warp_sum(q) / static_cast<float>(width) + eps);
+    const float inv = 1.0f / sqrtf(spk_row_sum<4>(q, lane) / static_cast<float>(width) + eps);
 #pragma unroll
     for (int g = 0; g < G; ++g) {
         const int c = 4 * (lane + 32 * g);
@@ -328,23 +329,25 @@ poly_norm_packed_kernel(const __nv_bfloat16* __restrict__ z, const float* __rest
         raw[v] = i < groups ? zr[i] : make_uint4(0u, 0u, 0u, 0u);
     }
     using namespace spk_tc;
-    // two channels per instruction: the kernel is bound by issue (8192 rows of 4864: 38.1 -> 33.4 us, 4096 of 18944: 66.0 -> 53.4)
-    uint64_t m1 = f2_pack(0.0f, 0.0f), m2 = m1, m3 = m1;
+    // two channels per instruction: the kernel is bound by issue (8192 rows of 4864: 38.1 -> 33.8 us, 4096 of 18944: 66.0 -> 54.8)
+    float s[3] = {0.0f, 0.0f, 0.0f};
 #pragma unroll
     for (int v = 0; v < G; ++v) {
         const uint32_t w[4] = {raw[v].x, raw[v].y, raw[v].z, raw[v].w};
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            const uint64_t x = f2_pack(__uint_as_float(w[k] << 16), __uint_as_float(w[k] & 0xffff0000u)), q = f2_mul(x, x), qq = f2_mul(q, q);
-            m1 = f2_add(m1, q);
-            m2 = f2_add(m2, qq);
-            m3 = f2_fma(qq, q, m3);
+        for (int k = 0; k < 4; ++k) {  // the sums one after the other, in the order of the channels
+            const uint64_t x = f2_pack(__uint_as_float(w[k] << 16), __uint_as_float(w[k] & 0xffff0000u)), q = f2_mul(x, x);
+            float q0, q1, qq0, qq1;
+            f2_unpack(q, q0, q1);
+            f2_unpack(f2_mul(q, q), qq0, qq1);
+            s[0] += q0;
+            s[0] += q1;
+            s[1] = fmaf(q0, q0, s[1]);
+            s[1] = fmaf(q1, q1, s[1]);
+            s[2] = fmaf(qq0, q0, s[2]);
+            s[2] = fmaf(qq1, q1, s[2]);
         }
     }
-    float s[3], y;
-    f2_unpack(m1, s[0], y); s[0] += y;
-    f2_unpack(m2, s[1], y); s[1] += y;
-    f2_unpack(m3, s[2], y); s[2] += y;
     spk_block_sum<3>(s, part);
     const float n = static_cast<float>(width);
     const float k1 = coef[0] / sqrtf(s[0] / n + eps), k2 = coef[1] / sqrtf(s[1] / n + eps);
