@@ -14,8 +14,8 @@
 // What bounds it: the special-function pipe, one exponential per (query, key) pair, 1024 cycles per 128 x 128 pairs; S and O take about 400 at
 // 64 channels.  Why 64 keys per step: S is double-buffered beside O of up to 128 channels within 256 TMEM columns, so that two CTAs fit an
 // SM and one's set-up and drain hide behind the other's steps.
-// Measured, whole fused_qkv_attention calls against SDPA on spikes unpacked to bf16: 16 x 512 tokens, 14/2 heads of 64, 608 -> 152 us; three
-// portions of 766 to 1531 tokens behind 700 cached, 28/4 heads of 128, 4922 -> 375 us; error against 64 bits 1.8e-3 -> 1.6e-3.
+// Measured, whole fused_qkv_attention calls against SDPA on spikes unpacked to bf16: 16 x 512 tokens, 14/2 heads of 64, 608 -> 129 us; three
+// portions of 766 to 1531 tokens behind 700 cached, 28/4 heads of 128, 4922 -> 338 us; error against 64 bits 1.8e-3 -> 1.6e-3.
 #include <algorithm>
 
 #include "spk_tensor.cuh"
@@ -207,8 +207,10 @@ spike_prefill_kernel(const __grid_constant__ Launch l) {
         bool ok = __all_sync(~0u, mbar_wait(smem_u32(&bars->q_full), 0, abort)) && __all_sync(~0u, scores(0));
         for (int t = 0; ok && t < steps; ++t) {
             const int stage = t % kStages, buf = t & 1;
-            // MMAs of one thread run in order: the buffer's previous weights (step t - 1) have been read before S overwrites them
-            if (t + 1 < steps) ok = __all_sync(~0u, scores(t + 1));
+            // S of step t + 1 overwrites the weights of step t - 1: their product has to be complete.  Issue order does not say so, it holds
+            // among MMAs of one shape and accumulator only; the commit that frees the product's stage does.
+            if (t + 1 < steps)
+                ok = __all_sync(~0u, (t == 0 || mbar_wait(smem_u32(&bars->kv_free[(t - 1) % kStages]), ((t - 1) / kStages) & 1, abort)) && scores(t + 1));
             ok = ok && __all_sync(~0u, mbar_wait(smem_u32(&bars->p_full[buf]), (t >> 1) & 1, abort));
             if (!ok) break;
             tc_fence_after();

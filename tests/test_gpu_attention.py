@@ -463,6 +463,37 @@ def test_prefill_attention_on_the_tensor_cores(dev, portions, heads, kv_heads, d
         assert bool(((got - want).abs() <= ulp * want.abs() + 2.0 ** -11).all())
 
 
+@pytest.mark.parametrize("heads, kv_heads, dim", [(4, 2, 64), (2, 1, 128)])
+def test_prefill_attention_over_many_steps(dev, heads, kv_heads, dim):
+    """Sixty steps of 64 keys and more per query tile, several CTAs on every SM: a score buffer is taken again for the scores of two steps
+    later while the other one's weights are multiplied.  Against float64, and twice the same bits."""
+    T, n, page = 4, 1500, 16
+    contexts = [4000, 2500, 3801]
+    g = torch.Generator(device=dev).manual_seed(dim)
+    need = [-(-(n + c) // page) for c in contexts]
+    word = lambda *s: torch.randint(-2 ** 31, 2 ** 31, s, generator=g, device=dev, dtype=torch.int32)
+    # half of a page's keys hold few spikes: weights of neighbouring steps differ by orders of magnitude
+    pool = lambda: word(T, kv_heads, sum(need) * page, dim // 32) & torch.where(torch.rand(1, 1, sum(need) * page, 1, generator=g, device=dev) < 0.5, -1, 0x01010101).to(torch.int32)
+    k, v, q = pool(), pool(), word(T, 3 * n, heads, dim // 32)
+    tables = list(torch.randperm(sum(need), generator=g, device=dev).to(torch.int32).split(need))
+    run = lambda: kernels.paged_spike_attn_prefill(q, k, v, tables, [0, n, 2 * n], [n] * 3, contexts, torch.empty(T, 3 * n, heads, dim, dtype=torch.float16, device=dev),
+                                                   head_dim=dim, block_size=page, num_q_heads=heads, num_kv_heads=kv_heads)
+    out = run()
+    for _ in range(3):
+        assert torch.equal(run(), out)
+    at = torch.arange(32, device=dev)
+    bits = lambda w: ((w[..., None] >> at) & 1).flatten(-2).to(torch.float64)
+    for i, (c, table) in enumerate(zip(contexts, tables)):
+        pos = torch.arange(c + n, device=dev)
+        rows = table[pos // page].long() * page + pos % page
+        kk, vv = (bits(p[:, :, rows]).repeat_interleave(heads // kv_heads, dim=1) for p in (k, v))
+        score = bits(q[:, i * n: (i + 1) * n]).transpose(1, 2) @ kk.mT * dim ** -0.5
+        score.masked_fill_(torch.ones(n, n + c, dtype=torch.bool, device=dev).triu(c + 1), float("-inf"))
+        want = (score.softmax(-1) @ vv).transpose(1, 2)
+        # as above: one rounding to halves, weights of 11 bits
+        assert bool(((out[:, i * n: (i + 1) * n].to(torch.float64) - want).abs() <= 2.0 ** -11 * want.abs() + 2.0 ** -11).all())
+
+
 def test_prefill_attention_flags_blocks_outside_the_pool(dev):
     q = torch.zeros(1, 20, 2, 2, dtype=torch.int32, device=dev)
     pool = torch.full((1, 1, 32, 2), -1, dtype=torch.int32, device=dev)
