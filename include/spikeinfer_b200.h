@@ -424,7 +424,8 @@ int spk_meta_release(int32_t row, int32_t* free_list, int32_t* free_count, int32
  *   otherwise y.
  * commit != NULL: for the last token of a portion commit[row] <- x[t] (the OLD x), so that the launch that ends a sublayer
  * saves what the next portion's first token needs.  In the prefill form with mix, x_out must not alias x.
- * prev and commit are [state_rows, width] contiguous. */
+ * prev and commit are [state_rows, width] contiguous; they may be one buffer where every portion is a single token (a row's prev is read
+ * before its commit), else not: the token that reads a row's prev and the one that writes it may run side by side. */
 typedef struct spk_residual_norm_args {
     const float* x;
     float* x_out;

@@ -122,6 +122,28 @@ def test_residual_norm_of_many_rows(dev, dtype, n, width):
 
 
 @pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("portions", [False, True])
+@pytest.mark.parametrize("n, width", [(6, 40), (8 * 148 - 1, 896), (8 * 148, 896), (8 * 148, 130), (4150, 128), (2500, 1024)])
+def test_residual_norm_with_one_state_buffer(dev, dtype, portions, n, width):
+    """Rows of one token each, as batch rows or as portions: the state is read before the old x takes its place, at every size."""
+    g = gen(n + width)
+    x, delta, prev = (torch.randn(n, width, generator=g).to(dev) for _ in range(3))
+    args = dict(x=x, delta=delta.to(dtype), weight=(1 + 0.3 * torch.randn(width, generator=g)).to(dev), alpha=2.5, eps=1e-3, mix=torch.rand(width, generator=g).to(dev),
+                positions=(torch.arange(n) % 3).to(dev), status=torch.zeros(1, dtype=torch.int32, device=dev))
+    if portions:
+        rows = torch.randperm(n, generator=g).to(torch.int32).to(dev)
+        args.update(token_rows=rows, token_edges=torch.full((n,), 3, dtype=torch.int32, device=dev))
+    want, commit = torch.empty(n, width, dtype=dtype, device=dev), torch.zeros_like(prev)
+    dense.residual_norm(want, prev=prev, commit=commit, **args)
+    out, state = torch.empty_like(want), prev.clone()
+    dense.residual_norm(out, prev=state, commit=state, **args)
+    assert torch.equal(out, want) and torch.equal(state, commit) and int(args["status"]) == 0
+    y = mo.layer_norm(2.5 * x.double() + args["delta"].double(), args["weight"].double(), 1e-3)
+    before = prev.double()[args["token_rows"].long() if portions else slice(None)] * (args["positions"] > 0)[:, None]
+    assert rel(out, y + (before - y) * args["mix"].double()) < TOL[dtype]
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("n", [8191, 8192, 8197])
 @pytest.mark.parametrize("width", [4, 260, 516, 896, 1024, 1028])
 def test_gated_norm_of_many_rows(dev, dtype, n, width):
