@@ -300,12 +300,13 @@ def fused_qkv_attention(qkv: torch.Tensor, lif_q, lif_k, lif_v, k_cache, v_cache
     q_packed = torch.empty((T, n_tok, hq, W), dtype=torch.int32, device=device)
     q_dense = None
     packed_prefill = meta.num_prefills and meta.prefill_row_tables is not None
-    # 16-bit outputs attend on the tensor cores from the packed pools; fp32 keeps 32-bit probabilities (SDPA on unpacked spikes)
-    tensor_prefill = meta.num_prefills and not packed_prefill and spike_prefill_form(d, dtype)
-    if meta.num_prefills and not packed_prefill and not tensor_prefill:
-        q_dense = torch.empty((T, hq, n_tok, d), dtype=dtype, device=device)
     kc, vc = _flat_pool(k_cache), _flat_pool(v_cache)
     num_slots = kc.shape[2]
+    # 16-bit outputs attend on the tensor cores from the packed pools; fp32 keeps 32-bit probabilities (SDPA on unpacked spikes), and pools of
+    # other timesteps or heads than the call's stay there too: it takes or refuses them by its own rules
+    tensor_prefill = (meta.num_prefills and not packed_prefill and spike_prefill_form(d, dtype) and kc.shape[:2] == (T, hkv) and vc.shape[:2] == (T, hkv))
+    if meta.num_prefills and not packed_prefill and not tensor_prefill:
+        q_dense = torch.empty((T, hq, n_tok, d), dtype=dtype, device=device)
     cos, sin = rope if rope is not None else (None, None)
     lif_pack_scatter([
         LifSiteSpec(x=xq, beta=lif_q[0], threshold=lif_q[1], packed=q_packed, rope_cos=cos, rope_sin=sin,

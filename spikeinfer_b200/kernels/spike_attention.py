@@ -194,6 +194,9 @@ def paged_spike_attn_prefill(q_packed: torch.Tensor, k_cache: torch.Tensor, v_ca
     dev = q_packed.device
     if q_packed.stride(3) != 1 or out.stride(3) != 1 or out.shape != (T, n_tok, n_heads, head_dim):
         raise ValueError("q_packed and out must have a contiguous last axis, out [T, n_tok, H_q, head_dim]")
+    for cache in (k_cache, v_cache):
+        if cache.dtype != torch.int32 or cache.shape[:2] != (T, num_kv_heads) or cache.shape[-1] < words:
+            raise ValueError(f"a pool must be int32 [{T}, {num_kv_heads}, .., {words} words or more], got {cache.dtype} {list(cache.shape)}")
     if not len(block_tables) == len(starts) == len(lens) == len(contexts):
         raise ValueError("one table, start, length and context per portion")
     if T == 0 or not lens:

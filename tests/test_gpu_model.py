@@ -363,3 +363,24 @@ def test_packed_prefill_equals_sdpa_prefill_with_cached_context(dev):
     assert torch.equal(sdpa[:, :2], packed[:, :2])
     err = ((sdpa - packed).abs().max() / sdpa.abs().max()).item()
     assert err < 1e-5, f"{err:.2e}"
+
+
+@pytest.mark.parametrize("timesteps, pool_heads", [(8, 2), (4, 3)])
+def test_16_bit_prefill_refuses_pools_of_other_shapes(dev, timesteps, pool_heads):
+    """Pools with more timesteps than the call, or with heads that its query heads are no multiple of: no prefill path may read a part of them."""
+    from spikeinfer_b200 import kernels
+    from spikeinfer_b200.attention import fused_qkv_attention
+    T, hq, hkv, d, bs, n = 4, 4, 2, 64, 16, 20
+    pool = torch.zeros(timesteps, pool_heads, 3 * bs, d // 32, dtype=torch.int32, device=dev)
+    tables = [torch.tensor([0, 1], dtype=torch.int32, device=dev)]
+    meta = AttentionMetadata(slot_mapping=torch.arange(n, device=dev), block_size=bs, prefill_query_starts=[0], prefill_query_lens=[n],
+                             prefill_context_lens=[0], prefill_block_tables=tables)
+    lif = (torch.full((d,), 0.9, device=dev), torch.full((d,), 0.8, device=dev))
+    qkv = torch.randn(T, n, (hq + 2 * hkv) * d, device=dev).to(torch.bfloat16)
+    with pytest.raises(Exception):
+        fused_qkv_attention(qkv, lif, lif, lif, pool, pool.clone(), meta, hq, hkv, d)
+    q, out = torch.zeros(T, n, hq, 2, dtype=torch.int32, device=dev), torch.empty(T, n, hq, d, dtype=torch.bfloat16, device=dev)
+    good = torch.zeros(T, hkv, 3 * bs, 2, dtype=torch.int32, device=dev)
+    for bad in (pool, good.to(torch.int64), good[..., :1]):
+        with pytest.raises(ValueError):
+            kernels.paged_spike_attn_prefill(q, good, bad, tables, [0], [n], [0], out, head_dim=d, block_size=bs, num_q_heads=hq, num_kv_heads=hkv)
