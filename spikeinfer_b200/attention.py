@@ -21,9 +21,13 @@ from .kernels.packing import packed_width
 
 def to_device(values: list, dtype: torch.dtype, device: torch.device) -> torch.Tensor:
     """A small host table on the device.  It goes through pinned memory: a copy from pageable memory makes the host wait for all work in flight
-    on the stream, and the device then waits for the host's next launches (about 1 ms of a prompt batch's pass over 24 layers)."""
-    cuda = device.type == "cuda"
-    return torch.tensor(values, dtype=dtype, pin_memory=cuda).to(device, non_blocking=cuda)
+    on the stream, and the device then waits for the host's next launches (about 1 ms of a prompt batch's pass over 24 layers).  During
+    a capture the copy is a pageable one, which torch refuses: a graph would repeat the copy of a table that is made anew for every batch."""
+    if device.type != "cuda":
+        return torch.tensor(values, dtype=dtype, device=device)
+    with torch.cuda.device(device):
+        pinned = not torch.cuda.is_current_stream_capturing()
+    return torch.tensor(values, dtype=dtype, pin_memory=pinned).to(device, non_blocking=pinned)
 
 
 @dataclass

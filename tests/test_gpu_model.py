@@ -384,3 +384,19 @@ def test_16_bit_prefill_refuses_pools_of_other_shapes(dev, timesteps, pool_heads
     for bad in (pool, good.to(torch.int64), good[..., :1]):
         with pytest.raises(ValueError):
             kernels.paged_spike_attn_prefill(q, good, bad, tables, [0], [n], [0], out, head_dim=d, block_size=bs, num_q_heads=hq, num_kv_heads=hkv)
+
+
+def test_host_tables_are_not_captured(dev):
+    """A table of one batch must not become part of a graph; the capture itself goes on."""
+    from spikeinfer_b200.attention import PrefillPlan, to_device
+    assert to_device([], torch.int64, dev).shape == (0,) and to_device([3, 4], torch.int32, dev).tolist() == [3, 4]
+    plan = PrefillPlan([0], [5], [0], [0], dev)
+    x, graph = torch.zeros(2, device=dev), torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        x += 1
+        with pytest.raises(RuntimeError):
+            to_device([1, 2], torch.int64, dev)
+        with pytest.raises(RuntimeError):
+            plan.tiles(128)
+    graph.replay()
+    assert x.tolist() == [1.0, 1.0] and plan.tiles(128).tolist() == [[0, 5, 0, 0]]
