@@ -523,6 +523,7 @@ typedef struct spk_sigmoid_attn_args {
     float scale;
     float out_scale;
     int32_t overlap;            /* partial form only: see below */
+    int32_t paired;             /* prefill form: two CTAs per SM, as spk_sigmoid_attn_paired advises (heads of 64; ignored by the others) */
     uint32_t* status;
 } spk_sigmoid_attn_args;
 int spk_sigmoid_attn_tile_tokens(int dtype, int k_pad, int v_pad, int k_tiled, int v_tiled, int block_size);
@@ -530,6 +531,9 @@ int spk_sigmoid_attn_tile_tokens(int dtype, int k_pad, int v_pad, int k_tiled, i
  * sizes. */
 int spk_sigmoid_attn_splits(int dtype, int k_pad, int v_pad, int k_tiled, int v_tiled, int block_size, int64_t n, int heads,
                             int kv_heads, int64_t max_keys);
+/* Whether the prefill form should run two CTAs per SM: `key_tiles` is the sum over the query tiles of the tiles of spk_sigmoid_attn_tile_tokens
+ * keys that each sees, `most` the largest of them.  The result is the same either way. */
+int spk_sigmoid_attn_paired(int k_pad, int v_pad, int heads, int64_t n_tiles, int64_t key_tiles, int64_t most);
 int spk_sigmoid_attn(const spk_sigmoid_attn_args* args, void* stream);
 
 /* S_t = decay_h S_{t-1} + k_t v_t^T, out_t = S_t^T q_t, with silu applied to q, k and v first when silu != 0.

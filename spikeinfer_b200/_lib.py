@@ -116,7 +116,7 @@ class SigmoidAttnArgs(Structure):
 
     _fields_ = _fields("p q k_pool v_pool tables seq_lens active tiles head_bias out; l out_stride table_stride table_rows "
                        "max_blocks n num_blocks; p partials; i n_tiles splits heads kv_heads dim vdim k_pad v_pad k_tiled v_tiled block_size dtype; "
-                       "f scale out_scale; i overlap; p status")
+                       "f scale out_scale; i overlap paired; p status")
 
 
 class DecayAttnArgs(Structure):
@@ -278,6 +278,7 @@ SIGNATURES = {
     "spk_qk_prepare": (c_int, [POINTER(QkPrepareArgs), c_void_p]),
     "spk_sigmoid_attn_tile_tokens": (c_int, [c_int] * 6),
     "spk_sigmoid_attn_splits": (c_int, [c_int] * 6 + [c_int64, c_int, c_int, c_int64]),
+    "spk_sigmoid_attn_paired": (c_int, [c_int] * 3 + [c_int64] * 3),
     "spk_sigmoid_attn": (c_int, [POINTER(SigmoidAttnArgs), c_void_p]),
     "spk_decay_powers": (c_int, []),
     "spk_decay_chunk_tokens": (c_int, [c_int, c_int, c_int, c_int64, c_int]),

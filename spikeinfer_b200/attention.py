@@ -109,6 +109,7 @@ class PrefillPlan:
             raise ValueError("every prefill portion needs its batch row")
         self.device = device
         self._tiles: dict[int, torch.Tensor] = {}
+        self._key_tiles: dict[int, tuple[int, int, int]] = {}
         self._chunks: dict[int, tuple[torch.Tensor, torch.Tensor]] = {}
         self._portions: torch.Tensor | None = None
         self._contexts: tuple[list[int], int, torch.Tensor] | None = None
@@ -158,6 +159,13 @@ class PrefillPlan:
             out.sort(key=lambda e: -e[3])  # the tiles that see the most keys start first
             self._tiles[tokens] = self._table(out)
         return self._tiles[tokens]
+
+    def key_tiles(self, tokens: int) -> tuple[int, int, int]:
+        """Entries of :meth:`tiles`, the tiles of ``tokens`` keys that all of them see together, and the most that one sees."""
+        if tokens not in self._key_tiles:
+            seen = [-(-(ctx + min(n, lo + tokens)) // tokens) for n, ctx in zip(self.lens, self.contexts_before) for lo in range(0, n, tokens)]
+            self._key_tiles[tokens] = (len(seen), sum(seen), max(seen, default=0))
+        return self._key_tiles[tokens]
 
     def chunks(self, tokens: int) -> tuple[torch.Tensor, torch.Tensor]:
         """``(chunks, seqs)``: int32 ``[n, 4]`` (first token, tokens, portion, index in the portion) and ``[portions, 4]``

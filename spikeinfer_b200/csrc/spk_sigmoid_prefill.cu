@@ -1,15 +1,16 @@
 // Prefill attention with sigmoid key weights on the fifth-generation tensor cores (tcgen05), bf16, head sizes up to 128.
 //
-// CTA = (128 query tokens of one portion, query head).  Warps, W of them for the weights (8 with heads of up to 64 channels, else 16):
+// CTA = (128 query tokens of one portion, query head).  Warps, W of them for the weights (16, or 8 in the paired form):
 //  * warps W and W + 3 copy K and V: a page of the pool is stored as the swizzled operand tile it becomes, so a 128-key tile is a
 //    handful of plain bulk copies (cp.async.bulk), no tensor map, whatever pages the block table names; one copy per lane, the
 //    next tile's block-table entries are read ahead;
 //  * warp W + 1 (one thread) issues S = Q K^T into a TMEM buffer, warp W + 2 (one thread) O += P V with P read from TMEM,
 //    so that neither kind of MMA waits behind the other's operands;
 //  * the others turn scores into weights, one thread per query row and half of the columns.  Sixteen warps take even and odd tiles in two
-//    score buffers.  With heads of 64 one buffer and eight warps fit two CTAs into an SM: one's start and end, a large part of the
-//    time of short prompts, hide behind the other's tiles.  14 heads of 64: 16 x 512 tokens 66.8 -> 50.4 us, 1 x 4096 94.7 -> 93.2, 3 x 600 to 1200
-//    33.3 -> 31.0, 2 x 60 to 100 8.1 -> 7.8.  Values of 128 channels leave no room for a second CTA's accumulator.
+//    score buffers: 1.4 us per tile of keys.  The paired form, for heads of up to 64 channels (values of 128 leave no room for a second
+//    accumulator), has one buffer and eight warps, so that two CTAs fit an SM: a tile takes 2.4 us alone and 2.8 beside another CTA, but one
+//    CTA's start and end hide behind the other's tiles.  14 heads of 64, sixteen warps / paired: 16 x 512 tokens 60.8 / 42.9 us, 2048 tokens of
+//    one prompt 29.5 / 45.4, 512 tokens behind 4096 56.2 / 91.4.  spk_sigmoid_attn_paired draws the line.  Both give the same bits.
 // A weight is sigmoid(score) of its own key: no running maximum, no rescaling of O, no denominator.  Weights are computed in
 // 32 bits and enter the product as a bf16 pair (hi + lo: 16 significant bits), so O is a 32-bit sum of them to 2^-17.
 // Visible keys are those up to the query's own position; the last tile's rows of V beyond the portion's end are cleared in
@@ -25,10 +26,10 @@ constexpr int kTile = 128;            // query rows, and keys per step
 constexpr int kColTile = kTile * 128; // bytes of a 64-channel column tile
 constexpr float kLog2e = 1.4426950408889634f;
 
-template <int CK, int CV>
+// NB: score buffers, and parities of tiles.
+template <int CK, int CV, int NB>
 struct Shape {
-    static constexpr int NB = CK + CV <= 2 ? 1 : 2;  // score buffers (and parities of tiles); one lets two CTAs share an SM
-    static constexpr int NS = 2;                     // stages of K and of V
+    static constexpr int NS = NB == 2 && CK + CV <= 2 ? 4 : 2;  // stages of K and of V
     static constexpr int kSigmoidWarps = 8 * NB, kSigmoidThreads = 32 * kSigmoidWarps, kThreads = kSigmoidThreads + 128;
     static constexpr uint32_t kTmemS = 0, kTmemLo = NB * 128, kTmemO = NB * 192, kColumns = NB * 256;  // S/P-hi, P-lo, O
     static constexpr int kK = CK * kColTile, kV = CV * kColTile;
@@ -36,16 +37,16 @@ struct Shape {
 };
 
 struct Bars {
-    uint64_t k_full[2], k_free[2], v_full[2], v_free[2], s_full[2], p_full[2], p_free[2], o_full, q_full, s_done;
+    uint64_t k_full[4], k_free[4], v_full[4], v_free[4], s_full[2], p_full[2], p_free[2], o_full, q_full, s_done;
     int abort;
     uint32_t tmem;
 };
 
-template <int CK, int CV>
-__global__ void __launch_bounds__(Shape<CK, CV>::kThreads, 3 - Shape<CK, CV>::NB)
+template <int CK, int CV, int NB>
+__global__ void __launch_bounds__(Shape<CK, CV, NB>::kThreads, 3 - NB)
 sigmoid_prefill_kernel(const spk_sigmoid_attn_args a) {
-    using Sh = Shape<CK, CV>;
-    constexpr int NS = Sh::NS, NB = Sh::NB, W = Sh::kSigmoidWarps, kThreads = Sh::kThreads, kSigmoidThreads = Sh::kSigmoidThreads;
+    using Sh = Shape<CK, CV, NB>;
+    constexpr int NS = Sh::NS, W = Sh::kSigmoidWarps, kThreads = Sh::kThreads, kSigmoidThreads = Sh::kSigmoidThreads;
     constexpr uint32_t kTmemS = Sh::kTmemS, kTmemLo = Sh::kTmemLo, kTmemO = Sh::kTmemO;
     extern __shared__ uint8_t raw[];
     uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(raw) + 1023) & ~uintptr_t(1023));
@@ -287,24 +288,47 @@ sigmoid_prefill_kernel(const spk_sigmoid_attn_args a) {
     if (warp == 0) tmem_dealloc(tmem, Sh::kColumns);
 }
 
-template <int CK, int CV>
+template <int CK, int CV, int NB>
 int launch(const spk_sigmoid_attn_args& a, cudaStream_t s) {
-    constexpr int bytes = Shape<CK, CV>::kBytes;
-    static_assert(sizeof(Bars) <= 256 && bytes <= 227 * 1024, "shared memory");
-    const cudaError_t e = cudaFuncSetAttribute(sigmoid_prefill_kernel<CK, CV>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    constexpr int bytes = Shape<CK, CV, NB>::kBytes;
+    static_assert(sizeof(Bars) <= 256 && (3 - NB) * bytes <= 227 * 1024, "shared memory");
+    const cudaError_t e = cudaFuncSetAttribute(sigmoid_prefill_kernel<CK, CV, NB>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
     if (e != cudaSuccess) return spk_set_cuda_error(e);
-    sigmoid_prefill_kernel<CK, CV><<<dim3(a.heads, a.n_tiles), Shape<CK, CV>::kThreads, bytes, s>>>(a);
+    sigmoid_prefill_kernel<CK, CV, NB><<<dim3(a.heads, a.n_tiles), Shape<CK, CV, NB>::kThreads, bytes, s>>>(a);
     SPK_CHECK_LAUNCH();
     return SPK_OK;
 }
 
 }  // namespace
 
+// Both forms take about 1.4 us of an SM per tile; the paired one saves most of a CTA's start and end (about 5 us), and loses where an SM has one CTA
+// alone or the longest CTA sets the time.  Gain of the paired form, measured over heads of 64 (4, 14 and 28 of them, one prompt of 256 to 8192
+// tokens, equal and ragged batches of 2 to 16, 0 to 4096 keys before them):
+//  * at most an SM's worth of CTAs: 0.57 to 1.03;
+//  * up to 6 key tiles: 1.04 to 1.7 once an SM's share of all tiles is 0.85 of the longest CTA's, 0.72 to 1.04 below;
+//  * equal CTAs of 7 to 20 tiles: 1.03 to 1.16 where they make an even number of rounds over the SMs, 0.88 to 0.99 in three (pairs take two, each as
+//    long as two), 1.06 and 1.01 in five of 8 and 12 tiles, 0.98 and 0.96 of 16 and 20;
+//  * CTAs of a mean length between two thirds and nine tenths of the longest, as behind long contexts: 0.85 to 1.03;
+//  * prompts of their own (mean about half of the longest): up to 12 tiles 1.06 to 1.4 from 297 CTAs and a share of 1.05 on, 0.85 to 0.92 below;
+//    up to 48 tiles 1.02 to 1.18 from a share of 1.4 on, 0.8 to 0.98 below; beyond, 0.95 to 1.04.
+extern "C" int spk_sigmoid_attn_paired(int k_pad, int v_pad, int heads, int64_t n_tiles, int64_t key_tiles, int64_t most) {
+    if (k_pad != 64 || v_pad != 64 || heads < 1 || heads > 65535 || n_tiles < 1 || n_tiles > 65535 || most < 1 || most > (1 << 24) || key_tiles < 1 || key_tiles > n_tiles * most)
+        return 0;
+    constexpr int64_t sms = 148;
+    const int64_t ctas = heads * n_tiles, work = heads * key_tiles;
+    if (ctas <= sms) return 0;
+    if (most <= 6) return 20 * work >= 17 * sms * most;
+    const int64_t rounds = (ctas + sms - 1) / sms;
+    if (10 * key_tiles >= 9 * n_tiles * most) return most <= 20 && (rounds % 2 == 0 || (most <= 12 && rounds >= 5));
+    if (3 * key_tiles > 2 * n_tiles * most) return 0;
+    return most <= 12 ? ctas > 2 * sms && 20 * work >= 21 * sms * most : most <= 48 && 5 * work >= 7 * sms * most;
+}
+
 int spk_sigmoid_prefill_launch(const spk_sigmoid_attn_args& a, cudaStream_t s) {
     if (a.n_tiles > 65535) return SPK_ERR_TOO_LARGE;
     const int ck = a.k_pad / 64, cv = a.v_pad / 64;
-    if (ck == 1 && cv == 1) return launch<1, 1>(a, s);
-    if (ck == 1 && cv == 2) return launch<1, 2>(a, s);
-    if (ck == 2 && cv == 1) return launch<2, 1>(a, s);
-    return launch<2, 2>(a, s);
+    if (ck == 1 && cv == 1) return a.paired ? launch<1, 1, 1>(a, s) : launch<1, 1, 2>(a, s);
+    if (ck == 1 && cv == 2) return launch<1, 2, 2>(a, s);
+    if (ck == 2 && cv == 1) return launch<2, 1, 2>(a, s);
+    return launch<2, 2, 2>(a, s);
 }

@@ -125,7 +125,10 @@ def sigmoid_attention(q: torch.Tensor, k_pool, v_pool, tables: torch.Tensor, hea
         raise ValueError("out must be [n, heads * vdim] in the dtype of q with unit column stride")
     lib = _lib.load()
     form = (_lib.dtype_code(q.dtype), k_pool.pad, v_pool.pad, int(k_pool.tiled), int(v_pool.tiled), k_pool.block_size)
-    tiles = None if plan is None else plan.tiles(int(lib.spk_sigmoid_attn_tile_tokens(*form)))
+    tiles, paired = None, 0
+    if plan is not None:
+        tokens = int(lib.spk_sigmoid_attn_tile_tokens(*form))
+        tiles, paired = plan.tiles(tokens), int(lib.spk_sigmoid_attn_paired(k_pool.pad, v_pool.pad, heads, *plan.key_tiles(tokens)))
     partials, splits = None, 0
     if partial_sums and plan is None:
         splits = int(lib.spk_sigmoid_attn_splits(*form, n, heads, kv_heads, tables.shape[1] * k_pool.block_size))
@@ -138,7 +141,7 @@ def sigmoid_attention(q: torch.Tensor, k_pool, v_pool, tables: torch.Tensor, hea
         num_blocks=k_pool.data.shape[0], partials=_ptr(partials), n_tiles=0 if tiles is None else tiles.shape[0], splits=splits,
         heads=heads, kv_heads=kv_heads, dim=dim, vdim=vdim, k_pad=k_pool.pad, v_pad=v_pool.pad, k_tiled=int(k_pool.tiled),
         v_tiled=int(v_pool.tiled), block_size=k_pool.block_size, dtype=form[0], scale=scale, out_scale=out_scale,
-        overlap=int(overlap_previous and partials is not None), status=_ptr(status))
+        overlap=int(overlap_previous and partials is not None), paired=paired, status=_ptr(status))
     _call("spk_sigmoid_attn", a, q.device)
     return partials
 

@@ -325,6 +325,37 @@ def test_sigmoid_attention_portions(dev, shape, dtype):
     assert (full[:, heads * vdim:] == 9.0).all() and status.item() == 0
 
 
+@pytest.mark.parametrize("heads, kv_heads, dim, page", [(4, 2, 64, 16), (3, 1, 48, 128), (7, 7, 64, 8)])
+def test_sigmoid_attention_portions_with_two_ctas_per_sm(dev, heads, kv_heads, dim, page):
+    """The two forms for heads of up to 64 channels give the same bits: one to nine tiles of keys, full and partial, one CTA per SM and more."""
+    new, ctx = [1, 127, 128, 129, 600, 3, 256] * 4, [0, 5, 1000, 0, 300, 128, 127] * 4
+    g = torch.Generator(device=dev).manual_seed(heads)
+    need = [-(-(a + b) // page) for a, b in zip(new, ctx)]
+    kp, vp = (PagedKVPool(sum(need) + 1, kv_heads, page, dim, torch.bfloat16, dev) for _ in range(2))
+    for p in (kp, vp):
+        p.data.copy_(torch.randn(p.data.shape, generator=g, device=dev))
+    tables = torch.zeros(len(new), max(need), dtype=torch.int32, device=dev)
+    for i, blocks in enumerate(torch.randperm(sum(need), generator=g, device=dev).to(torch.int32).split(need)):
+        tables[i, : need[i]] = blocks
+    n = sum(new)
+    q = torch.randn(n, heads, kp.pad, generator=g, device=dev).to(torch.bfloat16)
+    q[..., dim:] = 0
+    bias, status = torch.randn(heads, generator=g, device=dev) - 2, torch.zeros(1, dtype=torch.int32, device=dev)
+
+    def run(tiles):
+        plan = PrefillPlan([sum(new[:i]) for i in range(len(new))], new, ctx, list(range(len(new))), dev)
+        plan.key_tiles = lambda tokens: tiles  # what the choice is made from
+        out = torch.full((n, heads * dim), float("nan"), dtype=torch.bfloat16, device=dev)
+        dense.sigmoid_attention(q, kp, vp, tables, bias, out, heads=heads, kv_heads=kv_heads, dim=dim, vdim=dim, scale=0.15, out_scale=0.6, plan=plan, status=status)
+        return out
+    lib = _lib.load()
+    assert lib.spk_sigmoid_attn_paired(kp.pad, vp.pad, heads, 148, 148, 1) and not lib.spk_sigmoid_attn_paired(kp.pad, vp.pad, heads, 1, 1, 1)
+    want = run((1, 1, 1))
+    for _ in range(3):
+        assert torch.equal(run((148, 148, 1)), want)
+    assert torch.isfinite(want).all() and status.item() == 0
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("shape", sorted(ATTN_SHAPES))
 def test_sigmoid_attention_decode_rows(dev, shape, dtype):

@@ -123,6 +123,26 @@ def test_host_argument_checks(lib):
     assert lib.spk_meta_extend(0, 0, *([1] * 11), 4, 4, 0, 16, None, None) == -2
 
 
+def test_when_sigmoid_prefill_runs_two_ctas_per_sm(lib):
+    """The plan's count of key tiles, and the rule that reads it, on both sides of its lines."""
+    plan = PrefillPlan([0, 300, 300], [300, 0, 129], [100, 7, 0], [0, 1, 2], torch.device("cpu"))
+    assert plan.key_tiles(128) == (5, 2 + 3 + 4 + 1 + 2, 4) == (plan.tiles(128).shape[0], 12, 4)
+    assert plan.key_tiles(16) == (19 + 9, sum(-(-(100 + min(300, lo + 16)) // 16) for lo in range(0, 300, 16)) + sum(range(1, 10)), 25)
+
+    def paired(heads, lens, contexts, pad=64):
+        p = PrefillPlan([0] * len(lens), lens, contexts, [0] * len(lens), torch.device("cpu"))
+        return bool(lib.spk_sigmoid_attn_paired(pad, pad, heads, *p.key_tiles(128)))
+    assert paired(14, [512] * 16, [0] * 16) and not paired(14, [512] * 16, [0] * 16, pad=128)
+    assert not paired(14, [2048], [0]) and not paired(14, [512], [4096]) and paired(28, [2048], [0])
+    assert not paired(2, [128] * 74, [0] * 74) and paired(2, [128] * 75, [0] * 75)            # more CTAs than SMs
+    assert paired(2, [100] * 148, [900] * 148) and not paired(2, [100] * 149, [900] * 149) and paired(2, [100] * 223, [900] * 223)
+    assert paired(2, [100] * 310, [900] * 310) and not paired(2, [100] * 310, [1600] * 310)   # five rounds, of eight and fourteen tiles
+    assert paired(2, [100] * 223, [2400] * 223) and not paired(2, [100] * 223, [2500] * 223)  # equal CTAs of twenty and 21 tiles
+    assert not paired(28, [1536], [2048]) and paired(28, [1536], [512])                       # mean length 0.8 and 0.66 of the longest
+    assert not paired(14, [8192], [0]) and paired(14, [6000], [0])                            # beyond 48 tiles
+    assert not lib.spk_sigmoid_attn_paired(64, 64, 0, 5, 5, 1) and not lib.spk_sigmoid_attn_paired(64, 64, 4, 0, 0, 0)
+
+
 def test_portions_and_ledger():
     assert cut_portions([5, 3], None) == [[(0, 0, 5), (1, 0, 3)]]
     calls = cut_portions([5, 3, 9], 4)
