@@ -309,7 +309,7 @@ int launch(const spk_sigmoid_attn_args& a, cudaStream_t s) {
 //  * equal CTAs of 7 to 20 tiles: 1.03 to 1.16 where they make an even number of rounds over the SMs, 0.88 to 0.99 in three (pairs take two, each as
 //    long as two), 1.06 and 1.01 in five of 8 and 12 tiles, 0.98 and 0.96 of 16 and 20;
 //  * CTAs of a mean length between two thirds and nine tenths of the longest, as behind long contexts: 0.85 to 1.03;
-//  * prompts of their own (mean about half of the longest): up to 12 tiles 1.06 to 1.4 from 297 CTAs and a share of 1.05 on, 0.85 to 0.92 below;
+//  * prompts of their own (mean about half of the longest): up to 12 tiles 1.06 to 1.4 from 297 CTAs and a share of 1 on, 0.85 to 0.92 below;
 //    up to 48 tiles 1.02 to 1.18 from a share of 1.4 on, 0.8 to 0.98 below; beyond, 0.95 to 1.04.
 extern "C" int spk_sigmoid_attn_paired(int k_pad, int v_pad, int heads, int64_t n_tiles, int64_t key_tiles, int64_t most) {
     if (k_pad != 64 || v_pad != 64 || heads < 1 || heads > 65535 || n_tiles < 1 || n_tiles > 65535 || most < 1 || most > (1 << 24) || key_tiles < 1 || key_tiles > n_tiles * most)
@@ -321,7 +321,7 @@ extern "C" int spk_sigmoid_attn_paired(int k_pad, int v_pad, int heads, int64_t 
     const int64_t rounds = (ctas + sms - 1) / sms;
     if (10 * key_tiles >= 9 * n_tiles * most) return most <= 20 && (rounds % 2 == 0 || (most <= 12 && rounds >= 5));
     if (3 * key_tiles > 2 * n_tiles * most) return 0;
-    return most <= 12 ? ctas > 2 * sms && 20 * work >= 21 * sms * most : most <= 48 && 5 * work >= 7 * sms * most;
+    return most <= 12 ? ctas > 2 * sms && work >= sms * most : most <= 48 && 5 * work >= 7 * sms * most;
 }
 
 int spk_sigmoid_prefill_launch(const spk_sigmoid_attn_args& a, cudaStream_t s) {
