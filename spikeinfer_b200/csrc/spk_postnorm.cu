@@ -209,7 +209,7 @@ __device__ __forceinline__ void warp_layer_norm(float4 (&y)[G], const float* __r
 }
 
 template <typename T, typename TD, int G, bool MIX>
-__global__ void __launch_bounds__(32 * kRowWarps, G <= 4 ? 3 : 2)
+__global__ void __launch_bounds__(32 * kRowWarps, 2)
 residual_norm_rows_kernel(const ResidualNormParams p, T* __restrict__ out) {
     extern __shared__ float4 rows_s[];  // MIX: [kRowSteps][kRowWarps][32 * G]
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -218,7 +218,7 @@ residual_norm_rows_kernel(const ResidualNormParams p, T* __restrict__ out) {
     for (int step = 0; step < kRowSteps && t0 + step * kRowWarps < t1; ++step) {
         const int64_t t = t0 + step * kRowWarps + warp;
         const bool live = t < t1;
-        float4 y[G], before[G];
+        float4 y[G];
         int32_t edge = 3;
         int64_t row = -1;
         if (live) {
@@ -228,15 +228,6 @@ residual_norm_rows_kernel(const ResidualNormParams p, T* __restrict__ out) {
             if (row >= p.state_rows && (MIX || p.commit != nullptr)) {
                 if (lane == 0) spk_flag(p.status, SPK_STATUS_BAD_SLOT);
                 row = -1;
-            }
-            if (MIX && (edge & 1)) {  // ahead of the commit: with portions of one token, prev and commit may be one buffer
-                const bool stored = row >= 0 && p.positions[t] > 0;
-                const float* s = p.prev + (stored ? row : 0) * p.state_stride;
-#pragma unroll
-                for (int g = 0; g < G; ++g) {
-                    const int c = 4 * (lane + 32 * g);
-                    before[g] = spk_load4<float, true>(s + c, stored ? p.width - c : 0);
-                }
             }
             warp_new_row<TD, G>(p, t, p.commit != nullptr && (edge & 2) ? row : -1, y, lane);
             warp_layer_norm<G>(y, p.w, p.width, p.eps, lane);
@@ -256,12 +247,19 @@ residual_norm_rows_kernel(const ResidualNormParams p, T* __restrict__ out) {
         }
         if (MIX) {
             __syncthreads();
+            float4 before[G];
             if (live && !(edge & 1) && t == t0) {
                 warp_new_row<TD, G>(p, t - 1, -1, before, lane);
                 warp_layer_norm<G>(before, p.w, p.width, p.eps, lane);
-            } else if (live && !(edge & 1)) {
+            } else if (live) {
+                const bool stored = row >= 0 && (edge & 1) && p.positions[t] > 0;
+                const int from = edge & 1 ? 0 : step * kRowWarps + warp - 1;
+                const float* s = p.prev + (stored ? row : 0) * p.state_stride;
 #pragma unroll
-                for (int g = 0; g < G; ++g) before[g] = rows_s[(step * kRowWarps + warp - 1) * 32 * G + lane + 32 * g];
+                for (int g = 0; g < G; ++g) {
+                    const int c = 4 * (lane + 32 * g);
+                    before[g] = edge & 1 ? spk_load4<float, true>(s + c, stored ? p.width - c : 0) : rows_s[from * 32 * G + lane + 32 * g];
+                }
             }
             if (live) {
 #pragma unroll
@@ -413,8 +411,9 @@ int launch_residual_rows(ResidualNormParams p, T* out, cudaStream_t s) {
 template <typename T, typename TD>
 int launch_residual(const ResidualNormParams& p, void* out, cudaStream_t s) {
     // A warp per row from eight rows per SM on: 1184 rows of 896 with the shift 11.1 -> 7.1 us, without 5.5 -> 5.9; 1536 rows 11.7 -> 7.1 and 7.4 -> 6.3;
-    // below that (512 rows) a CTA per row has more loads in flight.  Wider rows don't fit a warp's registers.
-    if (p.ids == nullptr && p.width % 4 == 0 && p.width <= 1024 && p.n >= (p.mix != nullptr ? 8 : 10) * 148) {
+    // below that (512 rows) a CTA per row has more loads in flight.  Wider rows don't fit a warp's registers.  One buffer as prev and commit: this
+    // form stores a row's commit before it reads its prev (the other order, in registers or through shared memory, takes 4 to 13 %).
+    if (p.ids == nullptr && !(p.mix != nullptr && p.prev == p.commit) && p.width % 4 == 0 && p.width <= 1024 && p.n >= (p.mix != nullptr ? 8 : 10) * 148) {
         T* o = static_cast<T*>(out);
         switch ((p.width + 127) / 128) {
             case 1: case 2: return launch_residual_rows<T, TD, 2>(p, o, s);
