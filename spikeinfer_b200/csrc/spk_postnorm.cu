@@ -408,15 +408,31 @@ int launch_residual_rows(ResidualNormParams p, T* out, cudaStream_t s) {
     return SPK_OK;
 }
 
+// Whether a warp takes a row; below these lines a CTA per row has more loads in flight.  CTA / warp per row, us, bf16 where nothing else is said:
+//  * portions with the token shift, from 8 rows per SM on (the other form computes the predecessor of every CTA's first row again): 1184 rows of 128
+//    6.7 / 4.0, of 896 10.4 / 6.5; 8192 of 896 28.0 / 16.7.  Rows of up to 256 only up to 200 per SM: fp32, 20000 of 256 18.5 / 17.3, 32768 28.6 / 32.9;
+//  * without it, rows of more than 512 from 12 per SM on (1480 of 896 5.4 / 5.4, 1776 6.6 / 5.4; fp32 of 1024 6.8 / 6.6), of more than 256 from 13
+//    (1776 of 512 4.4 / 4.4, 2072 4.8 / 4.5), of more than 128 from 24 (2960 of 256 4.2 / 4.3, 3552 4.5 / 4.3), others from 16 (2072 of 128
+//    3.4 / 3.5, 2368 3.5 / 3.4);
+//  * batch rows with the shift read their predecessors from the state: rows of more than 512 from 14 per SM on (1480 of 896 6.1 / 7.2, 2072 8.9 / 7.2),
+//    others from 24 (2072 of 512 5.3 / 5.6, 4096 8.6 / 7.0; 4096 of 128 5.0 / 4.5), but for those of 129 to 256 (8192 of 256 8.8 / 9.5).
+// Rows of more than 1024 don't fit a warp's registers.  One buffer as prev and commit: the warp form stores a row's commit before it reads its prev
+// (the other order, in registers or through shared memory, takes 4 to 13 %).
+inline bool row_per_warp(const ResidualNormParams& p) {
+    if (p.ids != nullptr || p.width % 4 != 0 || p.width > 1024 || (p.mix != nullptr && p.prev == p.commit)) return false;
+    const int64_t per_sm = p.n / 148;
+    if (p.mix == nullptr) return per_sm >= (p.width > 512 ? 12 : p.width > 256 ? 13 : p.width > 128 ? 24 : 16);
+    if (p.token_rows == nullptr) return per_sm >= (p.width > 512 ? 14 : 24) && (p.width > 256 || p.width <= 128);
+    return per_sm >= 8 && (p.width > 256 || per_sm < 200);
+}
+
 template <typename T, typename TD>
 int launch_residual(const ResidualNormParams& p, void* out, cudaStream_t s) {
-    // A warp per row from eight rows per SM on: 1184 rows of 896 with the shift 11.1 -> 7.1 us, without 5.5 -> 5.9; 1536 rows 11.7 -> 7.1 and 7.4 -> 6.3;
-    // below that (512 rows) a CTA per row has more loads in flight.  Wider rows don't fit a warp's registers.  One buffer as prev and commit: this
-    // form stores a row's commit before it reads its prev (the other order, in registers or through shared memory, takes 4 to 13 %).
-    if (p.ids == nullptr && !(p.mix != nullptr && p.prev == p.commit) && p.width % 4 == 0 && p.width <= 1024 && p.n >= (p.mix != nullptr ? 8 : 10) * 148) {
+    if (row_per_warp(p)) {
         T* o = static_cast<T*>(out);
         switch ((p.width + 127) / 128) {
-            case 1: case 2: return launch_residual_rows<T, TD, 2>(p, o, s);
+            case 1: return launch_residual_rows<T, TD, 1>(p, o, s);
+            case 2: return launch_residual_rows<T, TD, 2>(p, o, s);
             case 3: case 4: return launch_residual_rows<T, TD, 4>(p, o, s);
             case 5: case 6: return launch_residual_rows<T, TD, 6>(p, o, s);
             case 7: return launch_residual_rows<T, TD, 7>(p, o, s);

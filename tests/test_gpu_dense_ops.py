@@ -144,6 +144,35 @@ def test_residual_norm_with_one_state_buffer(dev, dtype, portions, n, width):
 
 
 @pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("n, width", [(8 * 148, 128), (8 * 148, 512), (12 * 148, 516), (12 * 148, 1024), (13 * 148, 260), (14 * 148, 896), (16 * 148, 4),
+                                      (16 * 148 + 5, 100), (24 * 148, 128), (24 * 148, 132), (24 * 148, 256), (24 * 148, 384), (24 * 148, 512), (200 * 148 - 1, 256)])
+def test_residual_norm_of_many_rows_gives_the_bits_of_few(dev, dtype, n, width):
+    """From some number of rows on a warp takes a row; slices of the batch below it go to a CTA per row.  The same bits, with and without the
+    shift, as portions and as batch rows."""
+    g = gen(n + width)
+    x, delta, prev = (torch.randn(n, width, generator=g).to(dev) for _ in range(3))
+    w, w2, mix = (1 + 0.3 * torch.randn(width, generator=g).to(dev) for _ in range(3))
+    delta, pos = delta.to(dtype), torch.arange(n, device=dev)
+    edges = torch.zeros(n, dtype=torch.int32, device=dev)
+    edges[0::37] |= 1
+    edges[36::37] |= 2
+    rows = torch.arange(n, dtype=torch.int32, device=dev) // 37
+
+    def run(lo, hi, portions, **kw):
+        at = dict(token_rows=rows[lo:hi], token_edges=edges[lo:hi]) if portions else {}
+        state = {} if "mix" not in kw else dict(prev=prev if portions else prev[lo:hi])
+        out, x_out = torch.empty(hi - lo, width, dtype=dtype, device=dev), torch.empty(hi - lo, width, device=dev)
+        dense.residual_norm(out, x=x[lo:hi], delta=delta[lo:hi], weight=w, alpha=2.5, eps=1e-3, x_out=x_out, positions=pos[lo:hi], **at, **state, **kw)
+        return out, x_out
+    for portions in (True, False):
+        for kw in ({}, dict(second_weight=w2), dict(mix=mix)):
+            whole = run(0, n, portions, **kw)
+            parts = [run(lo, min(n, lo + 37 * 8), portions, **kw) for lo in range(0, n, 37 * 8)]
+            for got, want in zip(whole, zip(*parts)):
+                assert torch.equal(got, torch.cat(want)), (portions, kw.keys())
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("n", [8191, 8192, 8197])
 @pytest.mark.parametrize("width", [4, 260, 516, 896, 1024, 1028])
 def test_gated_norm_of_many_rows(dev, dtype, n, width):
