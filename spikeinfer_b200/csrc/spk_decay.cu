@@ -403,11 +403,15 @@ int launch_gated(const spk_gated_norm_args& a, cudaStream_t s) {
                      (a.partials == nullptr || (a.left_width % 4 == 0 && aligned(a.partials, 16)));
     if (!vec) {
         gated_norm_kernel<T><<<grid, kThreads, 0, s>>>(a);
-    } else if (a.partials == nullptr && a.width <= 1024 && a.n >= 8192) {
-        // a warp per row where it is measured to gain: 8192 rows of 896 26.0 -> 22.0 us (the exact gates take most of what is left)
+    } else if (a.partials == nullptr && a.width <= 1024 && a.n / 148 >= (a.width <= 256 ? 10 : a.width <= 768 ? 14 : 40)) {
+        // A warp per row where that leaves enough warps per SM: the wider the row, the fewer of them its registers allow and the longer the last
+        // round.  CTA / warp per row, bf16, us (fp32 within 6 %): 256 columns 1184 rows 2.8 / 2.8, 1480 3.5 / 2.8; 512 1776 3.9 / 4.0, 2072 4.2 / 4.0, 8192
+        // 10.5 / 7.4; 768 1480 5.0 / 5.1, 2072 6.3 / 5.3, 8192 19.7 / 12.0; 896 2960 8.3 / 9.0, 4144 10.9 / 9.3, 5920 14.8 / 12.6, 8192 20.0 / 16.2; 1024
+        // 3552 9.7 / 10.3, 5328 13.6 / 13.9, 5920 14.9 / 14.1, 8192 20.2 / 18.1.
         const unsigned rows = (grid + kThreads / 32 - 1) / (kThreads / 32);
         switch ((a.width + 127) / 128) {
-            case 1: case 2: gated_norm_rows_kernel<T, 2><<<rows, kThreads, 0, s>>>(a); break;
+            case 1: gated_norm_rows_kernel<T, 1><<<rows, kThreads, 0, s>>>(a); break;
+            case 2: gated_norm_rows_kernel<T, 2><<<rows, kThreads, 0, s>>>(a); break;
             case 3: case 4: gated_norm_rows_kernel<T, 4><<<rows, kThreads, 0, s>>>(a); break;
             case 5: case 6: gated_norm_rows_kernel<T, 6><<<rows, kThreads, 0, s>>>(a); break;
             case 7: gated_norm_rows_kernel<T, 7><<<rows, kThreads, 0, s>>>(a); break;

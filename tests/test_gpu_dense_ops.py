@@ -189,6 +189,28 @@ def test_gated_norm_of_many_rows(dev, dtype, n, width):
 
 
 @pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("n, width", [(10 * 148, 4), (10 * 148, 128), (10 * 148 + 7, 132), (10 * 148, 256), (14 * 148, 260), (14 * 148, 512), (14 * 148 + 3, 768),
+                                      (40 * 148, 772), (40 * 148, 896), (40 * 148 + 1, 1024)])
+def test_gated_norm_of_many_rows_gives_the_bits_of_few(dev, dtype, n, width):
+    """From some number of rows on a warp takes a row; slices below it go to a CTA per row.  The same bits, and rows that sit out are zero in both."""
+    g = gen(n + width)
+    x, w = torch.randn(n, width, generator=g).to(dev), (1 + 0.3 * torch.randn(width, generator=g)).to(dev)
+    z = (3 * torch.randn(n, 2 * width, generator=g)).to(dtype).to(dev)
+    active = torch.ones(n, dtype=torch.int32, device=dev)
+    active[[3, n - 1]] = 0
+
+    def run(lo, hi):
+        out = torch.full((hi - lo, 4 + width), 7.0, dtype=dtype, device=dev)
+        dense.gated_norm(x[lo:hi], w, z[lo:hi, width:], out, 4, eps=1e-3, scale=0.5, active=active[lo:hi])
+        return out
+    got = run(0, n)
+    assert torch.equal(got, torch.cat([run(lo, min(n, lo + 1024)) for lo in range(0, n, 1024)]))
+    assert (got[[3, n - 1], 4:] == 0).all() and (got[:, :4] == 7.0).all()
+    # the largest size below the line has the other form: one row less, the same rows
+    assert torch.equal(run(0, n // 148 * 148 - 1), got[: n // 148 * 148 - 1])
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
 def test_residual_norm_embedding_and_decode_rows(dev, dtype):
     g = gen(5)
     vocab, width, n = 50, 40, 6
