@@ -290,6 +290,14 @@ def paged_attention(q_spk, k_spk, v_spk, k_cache, v_cache, meta: AttentionMetada
     return out.view(T, 1, n_tok, num_q_heads * head_dim)
 
 
+def _one_token_far_behind(meta: AttentionMetadata, channels: int) -> bool:
+    """A prefill of one token behind many keys, of few key channels (over all timesteps).  The tensor-core kernel walks all keys in one CTA per head
+    and timestep, 11 us per thousand; reading them back and SDPA of a single query split the keys over the chip.  14/2 heads of 64, SDPA / tensor
+    cores, whole calls: 12000 keys 170 / 147 us, 16000 173 / 188, 64000 459 / 688; 7/1 of 128: 167 / 156, 172 / 201, 447 / 741.  Twice the key
+    channels or portions (28/4 of 128, 64000 keys: 1638 / 742; two portions of 14/2 of 64: 890 / 688) or a second token (3867 / 691) turn that."""
+    return meta.num_prefills == 1 and meta.prefill_query_lens[0] == 1 and meta.prefill_context_lens[0] >= 14000 and channels <= 512
+
+
 def fused_qkv_attention(qkv: torch.Tensor, lif_q, lif_k, lif_v, k_cache, v_cache, meta: AttentionMetadata,
                         num_q_heads: int, num_kv_heads: int, head_dim: int, reset_mode: int = 0,
                         rope: tuple[torch.Tensor, torch.Tensor] | None = None) -> torch.Tensor:
@@ -316,7 +324,8 @@ def fused_qkv_attention(qkv: torch.Tensor, lif_q, lif_k, lif_v, k_cache, v_cache
     num_slots = kc.shape[2]
     # 16-bit outputs attend on the tensor cores from the packed pools; fp32 keeps 32-bit probabilities (SDPA on unpacked spikes), and pools of
     # other timesteps or heads than the call's stay there too: it takes or refuses them by its own rules
-    tensor_prefill = (meta.num_prefills and not packed_prefill and spike_prefill_form(d, dtype) and kc.shape[:2] == (T, hkv) and vc.shape[:2] == (T, hkv))
+    tensor_prefill = (meta.num_prefills and not packed_prefill and spike_prefill_form(d, dtype) and kc.shape[:2] == (T, hkv) and vc.shape[:2] == (T, hkv)
+                      and not _one_token_far_behind(meta, T * hkv * d))
     if meta.num_prefills and not packed_prefill and not tensor_prefill:
         q_dense = torch.empty((T, hq, n_tok, d), dtype=dtype, device=device)
     cos, sin = rope if rope is not None else (None, None)

@@ -400,3 +400,36 @@ def test_host_tables_are_not_captured(dev):
             plan.tiles(128)
     graph.replay()
     assert x.tolist() == [1.0, 1.0] and plan.tiles(128).tolist() == [[0, 5, 0, 0]]
+
+
+@pytest.mark.parametrize("context", [13999, 14000, 20001])
+def test_16_bit_prefill_of_one_token_far_behind(dev, context, monkeypatch):
+    """One token behind many keys goes through SDPA from 14000 of them on; with more tokens, portions or key channels it does not."""
+    from spikeinfer_b200 import attention
+    T, hq, hkv, d, bs = 4, 4, 2, 64, 16
+    g = torch.Generator(device=dev).manual_seed(context)
+    blocks = context // bs + 1
+    pool = lambda: (torch.rand(T, hkv, blocks * bs, d, generator=g, device=dev) < 0.3)
+    bits = [pool(), pool()]
+    pack = lambda b: ((b.view(T, hkv, -1, 2, 32).long() << torch.arange(32, device=dev)).sum(-1)).to(torch.int32)
+    table = torch.randperm(blocks, generator=g, device=dev).to(torch.int32)
+    slot = int(table[context // bs]) * bs + context % bs
+    calls = []
+    monkeypatch.setattr(attention, "paged_spike_attn_prefill", lambda *a, _f=attention.paged_spike_attn_prefill, **k: (calls.append(1), _f(*a, **k))[1])
+    lif = (torch.full((d,), 0.9, device=dev), torch.full((d,), 0.8, device=dev))
+    qkv = torch.randn(T, 1, (hq + 2 * hkv) * d, generator=g, device=dev).to(torch.bfloat16)
+    meta = AttentionMetadata(slot_mapping=torch.tensor([slot], device=dev), block_size=bs, prefill_query_starts=[0], prefill_query_lens=[1],
+                             prefill_context_lens=[context], prefill_block_tables=[table])
+    kc, vc = map(pack, bits)
+    out = attention.fused_qkv_attention(qkv, lif, lif, lif, kc, vc, meta, hq, hkv, d)
+    assert bool(calls) == (context < 14000)
+    # the same through the batched popcount path, whose weights have 32 bits
+    attention.build_prefill_rows(meta)
+    want = attention.fused_qkv_attention(qkv, lif, lif, lif, kc.clone(), vc.clone(), meta, hq, hkv, d)
+    # values of at most one, weights of 8 bits and more that sum to one, one rounding of the result
+    assert bool(((out.double() - want.double()).abs() <= 2.0 ** -7).all())
+    few = dict(meta=AttentionMetadata(slot_mapping=meta.slot_mapping, block_size=bs, prefill_query_lens=[1], prefill_context_lens=[20000]))
+    assert attention._one_token_far_behind(**few, channels=512) and not attention._one_token_far_behind(**few, channels=513)
+    for lens, contexts in (([2], [20000]), ([1, 1], [20000, 20000]), ([1], [13999]), ([], [])):
+        few["meta"].prefill_query_lens, few["meta"].prefill_context_lens = lens, contexts
+        assert not attention._one_token_far_behind(**few, channels=512)
