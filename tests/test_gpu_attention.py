@@ -494,6 +494,63 @@ def test_prefill_attention_over_many_steps(dev, heads, kv_heads, dim):
         assert bool(((out[:, i * n: (i + 1) * n].to(torch.float64) - want).abs() <= 2.0 ** -11 * want.abs() + 2.0 ** -11).all())
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("heads, kv_heads, dim", [(6, 2, 64), (3, 1, 128)])
+def test_prefill_attention_over_strides_and_gaps(dev, heads, kv_heads, dim, dtype):
+    """Portions that start behind other tokens and leave gaps, rows of the output that allow no wide stores, queries of a wider buffer, pools of
+    other layouts: the bits of the plain call, and nothing else is written."""
+    T, page, W = 3, 16, dim // 32
+    starts, lens, contexts, n_tok = [5, 140, 150], [130, 3, 70], [20, 0, 64], 223
+    g = torch.Generator(device=dev).manual_seed(dim)
+    word = lambda *s: torch.randint(-2 ** 31, 2 ** 31, s, generator=g, device=dev, dtype=torch.int32)
+    blocks = 30
+    k, v, q = word(T, kv_heads, blocks * page, W), word(T, kv_heads, blocks * page, W), word(T, n_tok, heads, W)
+    need = [-(-(a + b) // page) for a, b in zip(lens, contexts)]
+    tables = list(torch.randperm(blocks, generator=g, device=dev)[: sum(need)].to(torch.int32).split(need))
+    run = lambda q, k, v, out, tables=tables: kernels.paged_spike_attn_prefill(q, k, v, tables, starts, lens, contexts, out, head_dim=dim, block_size=page,
+                                                                                num_q_heads=heads, num_kv_heads=kv_heads)
+    want = run(q, k, v, torch.full((T, n_tok, heads, dim), 7.0, dtype=dtype, device=dev))
+    used = torch.zeros(n_tok, dtype=torch.bool, device=dev)
+    for s, m in zip(starts, lens):
+        used[s: s + m] = True
+    assert bool((want[:, ~used] == 7.0).all()) and bool((want[:, used] <= 1.0).all())
+    odd = torch.full((T, n_tok, heads, dim + 1), 7.0, dtype=dtype, device=dev)
+    run(q, k, v, odd[..., :dim])
+    assert torch.equal(odd[..., :dim], want) and bool((odd[..., dim] == 7.0).all())
+    shifted = torch.full((want.numel() + 1,), 7.0, dtype=dtype, device=dev)
+    assert torch.equal(run(q, k, v, shifted[1:].view_as(want)), want) and float(shifted[0]) == 7.0
+    wide = word(T, n_tok + 4, heads + 3, W + 1)
+    wide[:, 2: 2 + n_tok, 1: 1 + heads, :W] = q
+    slot_major = lambda p: p.permute(2, 0, 1, 3).contiguous().permute(1, 2, 0, 3)                       # [slots, T, heads, words] in memory
+    page_major = lambda p: p.unflatten(2, (blocks, page)).permute(2, 0, 1, 3, 4).contiguous().permute(1, 2, 0, 3, 4)
+    for pools in ((slot_major(k), slot_major(v)), (page_major(k), page_major(v)), (slot_major(k), page_major(v))):
+        got = run(wide[:, 2: 2 + n_tok, 1: 1 + heads, :W], *pools, torch.full_like(want, 7.0), [t.to(torch.int64).repeat_interleave(2)[::2] for t in tables])
+        assert torch.equal(got, want)
+
+
+def test_prefill_attention_of_more_tiles_than_a_launch_holds(dev):
+    """A portion that is cut by the end of a launch's list of 512 query tiles goes on in the next, behind a full list of portions too."""
+    page, dim = 64, 64
+    g = torch.Generator(device=dev).manual_seed(2)
+    word = lambda *s: torch.randint(-2 ** 31, 2 ** 31, s, generator=g, device=dev, dtype=torch.int32)
+    lens, contexts = [3] * 47 + [66000, 200, 1], [5] * 47 + [0, 77, 9]
+    need = [-(-(a + b) // page) for a, b in zip(lens, contexts)]
+    k, v, q = word(1, 1, sum(need) * page, 2), word(1, 1, sum(need) * page, 2), word(1, sum(lens), 1, 2)
+    tables = list(torch.randperm(sum(need), generator=g, device=dev).to(torch.int32).split(need))
+    starts = [sum(lens[:i]) for i in range(len(lens))]
+    run = lambda at, out: kernels.paged_spike_attn_prefill(q, k, v, [tables[i] for i in at], [starts[i] for i in at], [lens[i] for i in at], [contexts[i] for i in at],
+                                                           out, head_dim=dim, block_size=page, num_q_heads=1, num_kv_heads=1)
+    got, want = (torch.full((1, sum(lens), 1, dim), 7.0, dtype=torch.bfloat16, device=dev) for _ in range(2))
+    run(range(len(lens)), got)
+    run(range(47), want)
+    run([48, 49], want)
+    # the long portion as two, the second behind the first's keys: 256 and 260 tiles
+    cut = 256 * 128
+    for start, m, c in ((starts[47], cut, 0), (starts[47] + cut, 66000 - cut, cut)):
+        kernels.paged_spike_attn_prefill(q, k, v, [tables[47]], [start], [m], [c], want, head_dim=dim, block_size=page, num_q_heads=1, num_kv_heads=1)
+    assert torch.equal(got, want) and bool((got <= 1.0).all())
+
+
 def test_prefill_attention_flags_blocks_outside_the_pool(dev):
     q = torch.zeros(1, 20, 2, 2, dtype=torch.int32, device=dev)
     pool = torch.full((1, 1, 32, 2), -1, dtype=torch.int32, device=dev)

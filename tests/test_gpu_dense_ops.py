@@ -288,6 +288,34 @@ def test_qk_prepare(dev, dtype, heads, kv_heads, dim, vdim, rot, block_size):
     assert status.item() == _lib.STATUS_BAD_SLOT
 
 
+@pytest.mark.parametrize("heads, kv_heads, dim, rot", [(14, 2, 64, (64, 1e4, 1.0)), (3, 1, 64, (32, 1e4, 4.0)), (6, 3, 64, None), (5, 5, 128, (128, 1e5, 8.0)),
+                                                       (3, 1, 128, None), (14, 2, 128, (48, 1e3, 2.0))])
+def test_qk_prepare_of_many_tokens_gives_the_bits_of_few(dev, heads, kv_heads, dim, rot):
+    """From 2048 lanes of sixteen bytes per SM on a lane takes four heads: groups that straddle q, k and v, and a short last one.  Slices of the batch go a
+    head per lane; one token's slot lies outside the pool."""
+    from spikeinfer_b200.modeling_manirax import RotaryConfig
+    n = -(-148 * 2048 // ((heads + 2 * kv_heads) * dim // 8)) + 1
+    blocks = n // 16 + 2
+    g = gen(heads * dim)
+    x = torch.randn(n, (heads + 2 * kv_heads) * dim, generator=g).to(torch.bfloat16).to(dev)
+    q, k, v = x.split([heads * dim, kv_heads * dim, kv_heads * dim], dim=1)
+    pos, slots = torch.randint(0, 4001, (n,), generator=g).to(dev), torch.randperm(blocks * 16, generator=g)[:n].to(dev)
+    slots[n // 2] = blocks * 16
+    table = None if rot is None else RotaryConfig(*rot).table(4001, dev)
+
+    def run(step):
+        pools = [PagedKVPool(blocks, kv_heads, 16, dim, torch.bfloat16, dev) for _ in range(2)]
+        status = torch.zeros(1, dtype=torch.int32, device=dev)
+        out = [dense.qk_prepare(q[at: at + step], k[at: at + step], v[at: at + step], *pools, slots[at: at + step], heads=heads, kv_heads=kv_heads, dim=dim, vdim=dim,
+                                eps=1e-3, rot_table=table, positions=pos[at: at + step], status=status) for at in range(0, n, step)]
+        assert status.item() == _lib.STATUS_BAD_SLOT
+        return torch.cat(out), pools[0].data, pools[1].data
+    whole, below, few = run(n), run(n - 2), run(999)
+    for a, b, c in zip(whole, below, few):
+        assert torch.equal(a, b) and torch.equal(a, c)
+    assert torch.isfinite(whole[0]).all() and bool((whole[1] != 0).any()) and bool((whole[2] != 0).any())
+
+
 # ---- attention -----------------------------------------------------------------------------------------------------
 def fill_pool(pool, values, slots):
     """Write ``values [n, heads, dim]`` at flat ``slots`` (pages in the pool's own order)."""

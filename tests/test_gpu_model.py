@@ -402,6 +402,73 @@ def test_host_tables_are_not_captured(dev):
     assert x.tolist() == [1.0, 1.0] and plan.tiles(128).tolist() == [[0, 5, 0, 0]]
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("hq, hkv, d", [(4, 2, 64), (7, 1, 128)])
+@pytest.mark.parametrize("layout", ["layer", "slots"])
+def test_16_bit_prefill_of_a_mixed_batch(dev, dtype, hq, hkv, d, layout):
+    """Two decode rows, then three portions, two of them behind cached keys, through fused_qkv_attention with the rotary embedding, over pools that are a
+    layer of a larger one or slot-major: the tensor-core path against float64 and the batched popcount path.  Both write the same pools and decode rows."""
+    from oracle import torch_oracle as orc
+    from spikeinfer_b200.attention import build_prefill_rows, fused_qkv_attention
+    T, bs, num_blocks, W = 4, 16, 40, d // 32
+    g = torch.Generator().manual_seed(d + hq)
+    seqs = [(19, 1), (36, 1), (0, 140), (19, 33), (64, 1)]  # (cached, new)
+    order = torch.randperm(num_blocks - 1, generator=g).tolist()
+    tables = []
+    for c, n in seqs:
+        tables.append([order.pop() for _ in range(-(-(c + n) // bs))])
+    slots = [t[p // bs] * bs + p % bs for t, (c, n) in zip(tables, seqs) for p in range(c, c + n)]
+    positions = torch.tensor([p for c, n in seqs for p in range(c, c + n)])
+    n_tok = len(slots)
+    pool = lambda: orc.pack_spikes((torch.rand(T, hkv, num_blocks * bs, d, generator=g) < 0.3).float())
+    k0, v0 = pool(), pool()
+
+    def placed(p):
+        if layout == "slots":
+            return p.permute(2, 0, 1, 3).contiguous().to(dev).permute(1, 2, 0, 3)
+        whole = torch.zeros(3, *p.shape, dtype=torch.int32, device=dev)
+        whole[1] = p.to(dev)
+        return whole[1]
+    bt = torch.full((2, 4), num_blocks - 1, dtype=torch.int32)
+    for i in range(2):
+        bt[i, : len(tables[i])] = torch.tensor(tables[i])
+    ints = lambda x: torch.tensor(x, dtype=torch.int32, device=dev)
+    starts = [2, 142, 175]
+
+    def meta():
+        return AttentionMetadata(
+            slot_mapping=torch.tensor(slots, device=dev), block_size=bs, num_decode_tokens=2, block_tables=bt.to(dev), seq_lens=ints([20, 37]),
+            prefill_query_starts=starts, prefill_query_lens=[140, 33, 1], prefill_context_lens=[0, 19, 64],
+            prefill_block_tables=[ints(t) for t in tables[2:]], status=torch.zeros(1, dtype=torch.int32, device=dev))
+    qkv = (1.5 * torch.randn(T, n_tok, (hq + 2 * hkv) * d, generator=g)).to(dtype)
+    angle = positions[:, None].float() / 1e4 ** (torch.arange(0, d, 2).float() / d)[None, :]
+    cos, sin = (f(torch.cat((angle, angle), dim=-1)).to(dtype) for f in (torch.cos, torch.sin))
+    lif = [(0.7 + 0.25 * torch.rand(d, generator=g), 0.6 + 0.6 * torch.rand(d, generator=g)) for _ in range(3)]
+    on = lambda pair: tuple(t.to(dev) for t in pair)
+    outs = []
+    for packed in (False, True):
+        kc, vc, m = placed(k0), placed(v0), meta()
+        if packed:
+            build_prefill_rows(m, pad_block=num_blocks - 1)
+        out = fused_qkv_attention(qkv.to(dev), *map(on, lif), kc, vc, m, hq, hkv, d, rope=(cos.to(dev), sin.to(dev)))
+        assert int(m.status) == 0 and out.dtype == dtype
+        outs.append((out.view(T, n_tok, hq, d).cpu(), kc.cpu(), vc.cpu()))
+    (got, kc, vc), (ref, kr, vr) = outs
+    assert torch.equal(kc, kr) and torch.equal(vc, vr) and torch.equal(got[:, :2], ref[:, :2])
+    q = qkv[..., : hq * d].unflatten(-1, (hq, d))
+    q = (q * cos[None, :, None, :]) + (torch.cat((-q[..., d // 2:], q[..., : d // 2]), dim=-1) * sin[None, :, None, :])
+    q = orc.lif_multistep(q, *lif[0], out_dtype=torch.uint8)[0].to(torch.float64)
+    # one rounding to the output's type, and weights of 11 bits whose sum is one against values of at most one
+    ulp = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11
+    for start, (c, n), table in zip(starts, seqs[2:], tables[2:]):
+        kk, vv = (orc.gather_kv_unpacked(p, torch.tensor(table, dtype=torch.int32), c + n, d, bs, torch.float64).repeat_interleave(hq // hkv, dim=1) for p in (kc, vc))
+        score = q[:, start: start + n].transpose(1, 2) @ kk.mT * d ** -0.5
+        score.masked_fill_(torch.ones(n, c + n, dtype=torch.bool).triu(c + 1), float("-inf"))
+        want = (score.softmax(-1) @ vv).transpose(1, 2)
+        for out in (got, ref):
+            assert bool(((out[:, start: start + n].double() - want).abs() <= ulp * want.abs() + 2.0 ** -11).all())
+
+
 @pytest.mark.parametrize("context", [13999, 14000, 20001])
 def test_16_bit_prefill_of_one_token_far_behind(dev, context, monkeypatch):
     """One token behind many keys goes through SDPA from 14000 of them on; with more tokens, portions or key channels it does not."""
