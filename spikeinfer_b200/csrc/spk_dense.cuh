@@ -81,7 +81,7 @@ __device__ __forceinline__ void spk_block_sum(float (&v)[N], float* part) {
 }
 
 // The same total, to the bit, where one warp holds what a CTA of W warps would: p[w] is the value of thread 32 w + lane.  Values are folded two,
-// then four to a lane on the way, so that W totals cost W + 4 - W / 4 exchanges and not 5 W.
+// then four to a lane on the way, so that W totals cost W + 4 exchanges and not 5 W.
 template <int W>
 __device__ __forceinline__ float spk_row_sum(const float (&p)[W], int lane) {
     static_assert(W == 4 || W == 8, "four or eight warps");

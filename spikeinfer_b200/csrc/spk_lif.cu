@@ -305,7 +305,8 @@ __device__ __forceinline__ float round_to<__half>(float v) { return __half2float
 // Rotary embedding of a segment: x * cos + p * sin, every operation rounded to the model dtype as the eager expression
 // (x * cos) + (rotate_half(x) * sin) does; `p` is the partner segment, negated when `negate`.  The 16-bit forms work on pairs: a product of
 // two of their values is exact in 32 bits and a sum of two rounds the same directly or through 32 bits (24 >= 2 * 11 + 2 bits), so
-// one packed operation gives the bits of the 32-bit operation rounded afterwards, in 3 instead of about 20 instructions per pair.
+// one packed operation gives the bits of the 32-bit operation rounded afterwards, in 3 instead of about 20 instructions per pair.  (Products of
+// bf16 below 2^-126 are not exact in 32 bits; they can differ by bf16's smallest step there, 2^-133.)
 __device__ __forceinline__ void rotate8(Raw8<float>& x, const Raw8<float>& p, const Raw8<float>& c, const Raw8<float>& s, bool negate) {
     const float sign = negate ? -1.0f : 1.0f;
     auto turn = [&](float& xv, float pv, float cv, float sv) { xv = __fadd_rn(__fmul_rn(xv, cv), __fmul_rn(sign * pv, sv)); };
@@ -716,7 +717,7 @@ __device__ __forceinline__ void fused_site_vec(const spk_lif_site& s, uint32_t u
     }
 }
 
-// The streaming plain form on its own (T = 4, no rotary embedding, no initial membrane, dense spikes or gated
+// The streaming plain form on its own (T = 4; no initial membrane, dense spikes or gated
 // product): the same copies, arithmetic and stores as fused_site_vec<.., ASYNC, PLAIN> would issue, with the
 // per-token bookkeeping reduced to running pointers and 32-bit counters.  At 11 instructions per element-step that
 // bookkeeping was 40 % of the issue slots of an issue-bound kernel.
