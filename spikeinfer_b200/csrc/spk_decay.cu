@@ -405,7 +405,7 @@ int launch_gated(const spk_gated_norm_args& a, cudaStream_t s) {
         gated_norm_kernel<T><<<grid, kThreads, 0, s>>>(a);
     } else if (a.partials == nullptr && a.width <= 1024 && a.n / 148 >= (a.width <= 256 ? 10 : a.width <= 768 ? 14 : 40)) {
         // A warp per row where that leaves enough warps per SM: the wider the row, the fewer of them its registers allow and the longer the last
-        // round.  CTA / warp per row, bf16, us (fp32 within 6 %): 256 columns 1184 rows 2.8 / 2.8, 1480 3.5 / 2.8; 512 1776 3.9 / 4.0, 2072 4.2 / 4.0, 8192
+        // round.  CTA / warp per row, bf16, us of repeated calls (fp32 within 6 %): 256 columns 1184 rows 2.8 / 2.8, 1480 3.5 / 2.8; 512 1776 3.9 / 4.0, 2072 4.2 / 4.0, 8192
         // 10.5 / 7.4; 768 1480 5.0 / 5.1, 2072 6.3 / 5.3, 8192 19.7 / 12.0; 896 2960 8.3 / 9.0, 4144 10.9 / 9.3, 5920 14.8 / 12.6, 8192 20.0 / 16.2; 1024
         // 3552 9.7 / 10.3, 5328 13.6 / 13.9, 5920 14.9 / 14.1, 8192 20.2 / 18.1.
         const unsigned rows = (grid + kThreads / 32 - 1) / (kThreads / 32);

@@ -408,7 +408,7 @@ int launch_residual_rows(ResidualNormParams p, T* out, cudaStream_t s) {
     return SPK_OK;
 }
 
-// Whether a warp takes a row; below these lines a CTA per row has more loads in flight.  CTA / warp per row, us, bf16 where nothing else is said:
+// Whether a warp takes a row; below these lines a CTA per row has more loads in flight.  CTA / warp per row, us of repeated calls, bf16 where nothing else is said:
 //  * portions with the token shift, from 8 rows per SM on (the other form computes the predecessor of every CTA's first row again): 1184 rows of 128
 //    6.7 / 4.0, of 896 10.4 / 6.5; 8192 of 896 28.0 / 16.7.  Rows of up to 256 only up to 200 per SM: fp32, 20000 of 256 18.5 / 17.3, 32768 28.6 / 32.9;
 //  * without it, rows of more than 512 from 12 per SM on (1480 of 896 5.4 / 5.4, 1776 6.6 / 5.4; fp32 of 1024 6.8 / 6.6), of more than 256 from 13
