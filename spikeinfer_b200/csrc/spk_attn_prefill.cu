@@ -7,7 +7,11 @@
 //    TMEM).  S of step t + 1 goes out before the wait for the weights of step t, so scores are ready when a step's weights are done;
 //  * warps 0-3, a thread per query row, turn scores into weights exp((score - popc(q)) * scale) * 2^14 in halves.  popc(q) bounds every
 //    score of the row: no running maximum, no rescaling of O, and 2^14 keeps the smallest possible weight a normal half.  Their 32-bit
-//    sum, also times 2^14, divides the row at the end.
+//    sum, also times 2^14, divides the row at the end.  For fp16 outputs, whose rounding is as fine as the weights', the sum takes the weights as
+//    they are rounded: keys of one score share their rounding, which then cancels (error against 64 bits, three portions of up to
+//    300 tokens behind 200, heads of 64 and 128: 2.32e-4 and 2.30e-4 with the sum of the unrounded ones, 2.15e-4 and 2.14e-4 so, 2.20e-4 and 2.29e-4 by
+//    SDPA in fp16).  That takes 6 % of the long portions' time below, 358 -> 380 us of single calls; bf16 results, whose rounding is 8 times coarser,
+//    sum the unrounded ones.
 // Bits expand in an order that is cheapest for the bit tricks (byte b of word j: bit j + 8 b; half h: bit j + 16 h), the same for Q and K;
 // V's column order is undone when a row is stored.
 //
@@ -17,6 +21,7 @@
 // Measured, whole fused_qkv_attention calls against SDPA on spikes unpacked to bf16: 16 x 512 tokens, 14/2 heads of 64, 608 -> 129 us; three
 // portions of 766 to 1531 tokens behind 700 cached, 28/4 heads of 128, 4922 -> 338 us; error against 64 bits 1.8e-3 -> 1.6e-3.
 #include <algorithm>
+#include <type_traits>
 
 #include "spk_tensor.cuh"
 
@@ -270,8 +275,13 @@ spike_prefill_kernel(const __grid_constant__ Launch l) {
                         x = 2 * i <= seen ? x : 0.0f;
                         y = 2 * i + 1 <= seen ? y : 0.0f;
                     }
-                    sums = f2_add(sums, f2_pack(x, y));
                     p[i] = pack_pair<__half>(x, y);
+                    if (std::is_same<TO, __half>::value) {  // the weights as they enter the product
+                        const float2 r = __half22float2(*reinterpret_cast<const __half2*>(&p[i]));
+                        x = r.x;
+                        y = r.y;
+                    }
+                    sums = f2_add(sums, f2_pack(x, y));
                 }
                 tmem_st16(at + c * 16, p);  // over columns of this half that have been read
             }
