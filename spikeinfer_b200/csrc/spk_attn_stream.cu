@@ -10,9 +10,10 @@
 //    holds four equally sized pieces of work whatever the mix of row lengths.
 //  * K and V pages go from global to shared memory with 16-byte cp.async copies, four 32-key tiles in
 //    flight per warp; the unit's block-table entries are staged once.  No register staging, no selects.
-//  * Scores: popc(q & k) per (head, key) on the integer pipes, thread = (head, key quad).  A score is an
-//    integer in [0, popc(q)], so the softmax weight exp((s - popc(q)) * scale) comes from one table shared by
-//    all heads, and partial sums of different units combine by plain addition.
+//  * Scores: popc(q & k) as mma.sync.m16n8k32 of unsigned bytes (exact): sixteen keys x eight heads, the K words masked in place
+//    as the left operand.  A score is an integer in [0, popc(q)], so the softmax weight exp((s - popc(q)) * scale) comes from one table
+//    shared by all heads, and partial sums of different units combine by plain addition.  The weights, 16 bits each, reach the
+//    layout of the weighted sum's right operand by a transposing move between the lanes.
 //  * Weighted sum on the tensor cores, transposed: out^T[channel][head] += V^T[channel][key] * P^T[key][head]
 //    as mma.sync.m16n8k16 (fp16 in, fp32 accumulate).  Sixteen channels fill the sixteen rows, eight heads
 //    the eight columns: nothing of the tile is padding.  The left operand is the V bits IN PLACE: the rows
@@ -24,8 +25,12 @@
 //  * The weight totals (softmax denominators) come from one more MMA per 16 keys whose left operand is all ones.
 //  * 16-bit outputs use one fp16 weight (2^-11 relative, the same rounded weight in numerator and denominator);
 //    fp32 output uses a {hi, lo} fp16 pair (22 bits) as a second block of columns.
-// Per 32-key tile at head_dim 64: 16 popc, 10 MMAs and about 130 instructions per warp; the integer pipe that
-// executes popc (a quarter-rate unit) and the issue slots are the two limits.
+// Per 32-key tile at head_dim 64: 14 MMAs (8 cycles of a sub-partition's tensor pipe each), 48 masks and about 130 instructions per warp; the
+// integer pipe of the masks (a half-rate unit, 58 % busy) and the tensor pipe (44 %) are the two limits, and warps per SM decide how well they
+// overlap.  Scores by popc (a unit of an eighth of the rate, one per head and word) took the K rows through shared memory
+// to every thread (16 wavefronts per tile against 4): 256 rows x 4096 keys 75.1 -> 68.6 us, with a CTA more per SM 67; 256 rows
+// of 1024 to 32768 keys at head_dim 128 248 -> 221 us.  The e4m3 form of the scores is no MMA of its own on sm_100 but conversions and fp16
+// MMAs: 105 us; heads as the left operand's rows (no transposition, half of the tile empty): 74.6.
 #include "spk_attn.cuh"
 
 #include <atomic>
@@ -98,41 +103,79 @@ __device__ __forceinline__ int clamp_len(int len, int max_keys) {
     return len < 1 ? 0 : (len > max_keys ? max_keys : len);
 }
 
-// 32 keys.  kst: their K rows [key][W]; xb: their V rows regrouped by key pair and BYTE: word g of pair p holds
+// c = a (16x32 u8, row major) * b (32x8 u8, column major) + c, 32-bit integers.  Thread (gid, tig) holds a0 = A[gid][4tig..+3],
+// a1 = A[gid+8][4tig..+3], a2 = A[gid][16+4tig..+3], a3 = A[gid+8][16+4tig..+3]; b0 = B[4tig..+3][gid], b1 = B[16+4tig..+3][gid];
+// c[0], c[1] = C[gid][2tig, 2tig+1], c[2], c[3] = C[gid+8][2tig, 2tig+1].
+__device__ __forceinline__ void mma16832(int (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+    asm("mma.sync.aligned.m16n8k32.row.col.s32.u8.u8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+        : "+r"(c[0]), "+r"(c[1]), "+r"(c[2]), "+r"(c[3])
+        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+
+// The transpose of the 8x8 matrix of 16-bit elements whose row gid, columns 2tig and 2tig+1 thread (gid, tig) holds.
+__device__ __forceinline__ uint32_t transposed(uint32_t x) {
+    uint32_t y;
+    asm("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(y) : "r"(x));
+    return y;
+}
+
+// A word of the weight table, which does not change after set-up (so the load may move freely).
+__device__ __forceinline__ uint32_t table_word(uint32_t addr) {
+    uint32_t v;
+    asm("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(addr));
+    return v;
+}
+
+// Scores on the tensor cores.  A K word is the left operand IN PLACE: masked with 0x01010101 << e, e = 0..3, its four bytes are 0 or 2^e,
+// and the query's operand holds 2^(3 - e) where its bit is set, so every matching bit adds 8, the distance of two entries of the weight
+// table.  Thread tig supplies the channels of (word tig / 2, half nibbles tig % 2) at head_dim 64 and of word
+// tig at 128: 2 W masked registers per key.
+
+// This thread's registers of the query operand for its head's words.
+template <int W>
+__device__ __forceinline__ void score_query(const uint32_t (&qw)[W], int tig, uint32_t (&qa)[2 * W]) {
+    uint32_t w = qw[0];
+#pragma unroll
+    for (int i = 1; i < W; ++i)
+        if ((W == 2 ? tig >> 1 : tig) == i) w = qw[i];
+    if (W == 2) w >>= 4 * (tig & 1);
+#pragma unroll
+    for (int r = 0; r < 2 * W; ++r) qa[r] = ((w >> r) & 0x01010101u) << (3 - (r & 3));
+}
+
+// 32 keys.  kw0: this thread's word of key gid (key gid of the tile's rows [key][W]); xb: their V rows regrouped by key
+// pair and BYTE: word g of pair p holds
 // byte g of key 2p's row in bits 0..7 and byte g of key 2p+1's row in bits 16..23 (the other two bytes are
 // don't-care) and sits at xb[(g / 4) * kXGroup + 4 p + g % 4].  Thread gid supplies the channels of byte gid (and, at head_dim 128, of byte
 // gid + 8): in channel block j its two rows are bits 2j and 2j+1 of that byte, so one word per key pair feeds
 // all blocks, and a masked bit is always an fp16 subnormal 2^(e - 24), e = 0..7.
-// rlut: the weight table positioned so that rlut[score] is this head's weight.
+// lut0, lut1: the shared addresses of the weights of heads 2tig and 2tig + 1 for score 0.
 // ALL: every key is live; otherwise keys at or beyond `nlive` get weight zero.
 template <int W, int NB, bool ALL>
-__device__ __forceinline__ void tile_compute(const uint32_t* kst, const uint32_t* xb, const uint32_t (&qw)[W],
-                                             const uint32_t* rlut, int nlive, const uint32_t (&ones)[4], int gid,
+__device__ __forceinline__ void tile_compute(const uint32_t* kw0, const uint32_t* xb, const uint32_t (&qa)[2 * W], int sh,
+                                             uint32_t lut0, uint32_t lut1, int nlive, const uint32_t (&ones)[4], int gid,
                                              int tig, float (&acc)[NB][2 * W + 1][4]) {
     constexpr int MB = 2 * W;  // blocks of 16 channels
     const uint32_t* xt = xb + (gid >> 2) * kXGroup + (gid & 3);  // this thread's byte of pair 0
 #pragma unroll
     for (int ks = 0; ks < 2; ++ks) {
-        // weights of (this thread's head, keys kp, kp+1) for the two key pairs of the 16-key step
+        // weights of keys gid and gid + 8 of the 16-key step for heads 2tig and 2tig + 1, then transposed to keys 2tig, 2tig + 1 (and + 8) of
+        // head gid, the right operand of the weighted sum
+        int c[4] = {0, 0, 0, 0};
+        const uint32_t w0 = kw0[16 * ks * W] >> (W == 2 ? sh : 0), w1 = kw0[(16 * ks + 8) * W] >> (W == 2 ? sh : 0);
+#pragma unroll
+        for (int r = 0; r < 2 * W; r += 2) {
+            const uint32_t s0 = r < 4 ? w0 : w0 >> 4, s1 = r < 4 ? w1 : w1 >> 4, m0 = 0x01010101u << (r & 3), m1 = m0 << 1;
+            const uint32_t a[4] = {s0 & m0, s1 & m0, s0 & m1, s1 & m1};
+            mma16832(c, a, qa[r], qa[r + 1]);
+        }
         uint32_t bh[2], bl[2];
 #pragma unroll
         for (int pr = 0; pr < 2; ++pr) {
-            const int kp = 16 * ks + 8 * pr + 2 * tig;
-            uint32_t kw[2 * W];
-            load_words<2 * W>(kst + kp * W, kw);
-            int s0 = 0, s1 = 0;
-#pragma unroll
-            for (int w = 0; w < W; ++w) {
-                s0 += __popc(qw[w] & kw[w]);
-                s1 += __popc(qw[w] & kw[W + w]);
-            }
-            uint32_t e0 = rlut[s0], e1 = rlut[s1];
-            if (!ALL) {
-                if (kp >= nlive) e0 = 0u;
-                if (kp + 1 >= nlive) e1 = 0u;
-            }
-            bh[pr] = prmt(e0, e1, 0x5410);
-            if (NB == 2) bl[pr] = prmt(e0, e1, 0x7632);
+            uint32_t e0 = table_word(lut0 + c[2 * pr]), e1 = table_word(lut1 + c[2 * pr + 1]);
+            if (!ALL && 16 * ks + 8 * pr + gid >= nlive) e0 = e1 = 0u;
+            bh[pr] = transposed(prmt(e0, e1, 0x5410));
+            if (NB == 2) bl[pr] = transposed(prmt(e0, e1, 0x7632));
         }
 #pragma unroll
         for (int hb = 0; hb < W / 2; ++hb) {  // byte gid (and byte gid + 8 at head_dim 128)
@@ -181,13 +224,11 @@ __device__ __forceinline__ void store_channels(TO* dst, const float* src, float 
     }
 }
 
-#ifndef SPK_STREAM_MINB
-#define SPK_STREAM_MINB 4
-#endif
-
-#ifndef SPK_STREAM_MINB4
-#define SPK_STREAM_MINB4 3
-#endif
+// CTAs per SM that a form is built for.  Range form, 16-bit outputs (64 rows of 128 to 4096 keys, 8 layers with their LIF launches; 256 long rows at 128
+// channels): 3 / 4 / 5 of head_dim 64 200 / 168 / 164 us, 2 / 3 / 4 of head_dim 128 325 / 225 / 221.  Where a warp has one short row alone (the unit form) registers
+// beat residency: 144 us against 140 for 8 rows of 96 to 224 keys, 24 layers.
+template <int W, int NB, bool DENSE>
+struct StreamResident { static constexpr int N = W == 2 ? (NB == 1 && DENSE ? 5 : 4) : (NB == 1 && DENSE ? 4 : 3); };
 
 #ifndef SPK_SHORT_STEPS
 #define SPK_SHORT_STEPS 8
@@ -214,7 +255,7 @@ struct StreamSmem {
 template <int W, int NB>
 __device__ __forceinline__ void stream_piece(const AttnParams& p, const StreamParams& sp, int row, int gt, int key0,
                                              int kend, bool whole, float* rec, uint32_t* ring, uint32_t* xb,
-                                             int32_t* tbl, const uint32_t* rlut, int lane) {
+                                             int32_t* tbl, const uint2* rlut, int lane) {
     using S = StreamSmem<W>;
     constexpr int D = S::D, MB = 2 * W, STAGES = S::STAGES, HALF_WORDS = S::HALF_WORDS, TILE_WORDS = S::TILE_WORDS;
     constexpr int TILE_BYTES = TILE_WORDS * 4, ES = S::ES;
@@ -250,19 +291,14 @@ __device__ __forceinline__ void stream_piece(const AttnParams& p, const StreamPa
         for (int w = 0; w < W; ++w)
             qw[w] = gid < nh ? __ldg(p.q + t * p.sq_t + row * p.sq_n + (h0 + gid) * p.sq_h + w) : 0u;
     };
-    if (!p.overlap) load_q();  // in flight together with the table entries
     __syncwarp();  // every lane is done with the previous piece's entries
     stage_tables(key0, min(kend, key0 + span));
-    if (p.overlap) {
-        // Everything above read lengths and block tables only.  q and the newest K/V rows come from the kernel
-        // launched just before this one, which this launch overlaps (programmatic dependent launch): wait for it.
-        asm volatile("griddepcontrol.wait;" ::: "memory");
-        load_q();
-    }
-    int cmax = 0;
-#pragma unroll
-    for (int w = 0; w < W; ++w) cmax += __popc(qw[w]);
-    const uint32_t* my_rlut = rlut + (D - cmax);
+    // Everything above read lengths and block tables only.  q and the newest K/V rows come from the kernel launched just before this one,
+    // which this launch may overlap (programmatic dependent launch): wait for it.
+    if (p.overlap) asm volatile("griddepcontrol.wait;" ::: "memory");
+    load_q();  // used behind the first copies of K and V, so that both are in flight together
+    uint32_t lut0 = 0, lut1 = 0, qa[2 * W];
+    const int sh = 4 * (tig & 1);
     uint32_t ones[4];  // fp16 {1, 1}: the left operand of the weight totals (kept in registers, opaque to the compiler)
 #pragma unroll
     for (int i = 0; i < 4; ++i) asm volatile("mov.b32 %0, 0x3C003C00;" : "=r"(ones[i]));
@@ -311,7 +347,17 @@ __device__ __forceinline__ void stream_piece(const AttnParams& p, const StreamPa
             if (s < ntiles) issue();
             cp_async_commit();
         }
+        if (c0 == key0) {
+            int cmax = 0;  // the popcount of this thread's head: the softmax bound
+#pragma unroll
+            for (int w = 0; w < W; ++w) cmax += __popc(qw[w]);
+            const uint32_t lut = static_cast<uint32_t>(__cvta_generic_to_shared(rlut + (D - cmax)));
+            lut0 = __shfl_sync(0xffffffffu, lut, 8 * tig);
+            lut1 = __shfl_sync(0xffffffffu, lut, 8 * tig + 4) + 4;
+            score_query<W>(qw, tig, qa);
+        }
         const uint32_t* kst = ring;
+        const int kw_at = gid * W + (W == 2 ? tig >> 1 : tig);  // this thread's word of a tile's key gid
         int nlive = nkeys;
         for (int tile = 0; tile < ntiles; ++tile) {
             cp_async_wait<STAGES - 2>();  // this tile has landed (the newer STAGES - 2 groups may be in flight)
@@ -336,13 +382,14 @@ __device__ __forceinline__ void stream_piece(const AttnParams& p, const StreamPa
                     *reinterpret_cast<uint4*>(xb + q * kXGroup + lane * 4) = make_uint4(x[4 * q], x[4 * q + 1], x[4 * q + 2], x[4 * q + 3]);
             }
             __syncwarp();
+            const uint32_t* kw0 = kst + kw_at;
             if (nlive >= kTileKeys) {
-                tile_compute<W, NB, true>(kst, xb, qw, my_rlut, 32, ones, gid, tig, acc);
-                tile_compute<W, NB, true>(kst + 32 * W, xb + 64, qw, my_rlut, 32, ones, gid, tig, acc);
+                tile_compute<W, NB, true>(kw0, xb, qa, sh, lut0, lut1, 32, ones, gid, tig, acc);
+                tile_compute<W, NB, true>(kw0 + 32 * W, xb + 64, qa, sh, lut0, lut1, 32, ones, gid, tig, acc);
             } else {
-                tile_compute<W, NB, false>(kst, xb, qw, my_rlut, nlive, ones, gid, tig, acc);
+                tile_compute<W, NB, false>(kw0, xb, qa, sh, lut0, lut1, nlive, ones, gid, tig, acc);
                 if (nlive > 32)
-                    tile_compute<W, NB, false>(kst + 32 * W, xb + 64, qw, my_rlut, nlive - 32, ones, gid, tig, acc);
+                    tile_compute<W, NB, false>(kw0 + 32 * W, xb + 64, qa, sh, lut0, lut1, nlive - 32, ones, gid, tig, acc);
             }
             nlive -= kTileKeys;
             kst = (tile % STAGES == STAGES - 1) ? ring : kst + TILE_WORDS;
@@ -448,14 +495,14 @@ __device__ __forceinline__ int64_t range_of(const RangeSplit& r, int64_t x) {
 // after it (slot 1).
 // Otherwise: one warp per (unit of unit_keys keys, gt), units enumerated as row * max_units + unit.
 template <int W, int NB, bool DENSE>
-__global__ void __launch_bounds__(kThreads, (W == 2 ? (NB == 1 ? SPK_STREAM_MINB : 4) : (NB == 1 ? SPK_STREAM_MINB4 : 3)))
+__global__ void __launch_bounds__(kThreads, StreamResident<W, NB, DENSE>::N)
 attn_stream_kernel(const AttnParams p, const StreamParams sp) {
     using S = StreamSmem<W>;
     constexpr int D = S::D;
     __shared__ __align__(16) uint32_t ring_all[kWarps][S::STAGES][S::TILE_WORDS];
     __shared__ __align__(16) uint32_t x_all[kWarps][W * kXGroup];
     __shared__ int32_t tbl_all[kWarps][kTblMax];
-    __shared__ uint32_t rlut[D + 1];  // rlut[i] = {hi, lo} fp16 of 2^14 exp(-(D - i) scale)
+    __shared__ uint2 rlut[D + 1];  // rlut[i]: twice (for even and odd heads, in banks of their own) {hi, lo} fp16 of 2^14 exp(-(D - i) scale)
     __shared__ int prefix[DENSE ? kDenseRows + 1 : 1];
     __shared__ int lens_s[DENSE ? kDenseRows : 1];
     __shared__ int warp_sums[kWarps];
@@ -491,7 +538,8 @@ attn_stream_kernel(const AttnParams p, const StreamParams sp) {
             const float wv = ldexpf(expf(-static_cast<float>(D - i) * p.scale), kScaleLog2);
             const __half hi = __float2half_rn(wv);
             const __half lo = __float2half_rn((wv - __half2float(hi)) * 2048.0f);
-            rlut[i] = static_cast<uint32_t>(__half_as_ushort(hi)) | (static_cast<uint32_t>(__half_as_ushort(lo)) << 16);
+            const uint32_t both = static_cast<uint32_t>(__half_as_ushort(hi)) | (static_cast<uint32_t>(__half_as_ushort(lo)) << 16);
+            rlut[i] = make_uint2(both, both);
         }
         __syncthreads();
         int run = incl - local;
@@ -509,7 +557,8 @@ attn_stream_kernel(const AttnParams p, const StreamParams sp) {
             const float wv = ldexpf(expf(-static_cast<float>(D - i) * p.scale), kScaleLog2);
             const __half hi = __float2half_rn(wv);
             const __half lo = __float2half_rn((wv - __half2float(hi)) * 2048.0f);
-            rlut[i] = static_cast<uint32_t>(__half_as_ushort(hi)) | (static_cast<uint32_t>(__half_as_ushort(lo)) << 16);
+            const uint32_t both = static_cast<uint32_t>(__half_as_ushort(hi)) | (static_cast<uint32_t>(__half_as_ushort(lo)) << 16);
+            rlut[i] = make_uint2(both, both);
         }
     }
     __syncthreads();
@@ -1115,8 +1164,8 @@ int spk_attn_selected_form() { return g_attn_form.load(std::memory_order_relaxed
 
 // CTAs per SM the main kernel is built for (its __launch_bounds__), by rows of words and weight blocks.
 static int stream_ctas_per_sm(int head_dim, bool wide) {
-    if (head_dim == 64) return wide ? 4 : SPK_STREAM_MINB;
-    return wide ? 3 : SPK_STREAM_MINB4;
+    if (head_dim == 64) return wide ? StreamResident<2, 2, true>::N : StreamResident<2, 1, true>::N;
+    return wide ? StreamResident<4, 2, true>::N : StreamResident<4, 1, true>::N;
 }
 
 StreamPlan spk_attn_stream_plan(int T, int64_t n_seqs, int Hq, int Hkv, int head_dim, int block_size,

@@ -353,6 +353,33 @@ def tcgen05_form(lib):
     assert lib.spk_attn_select_form(_lib.ATTN_FORM_AUTO) == 0
 
 
+@pytest.mark.parametrize("dim", [64, 128])
+@pytest.mark.parametrize("heads, kv_heads", [(1, 1), (5, 1), (16, 2), (22, 2)])
+def test_every_channel_of_a_score(heads, kv_heads, dim, dev):
+    """One-bit queries against one-bit keys of every channel (a wrong mask or position shows as a wrong weight), full words against
+    full words (the table's far end), lengths at the edges of the 8-, 16-, 32- and 64-key steps, whole rows and rows cut between warps."""
+    for max_blocks in (16, 128):
+        lens = [1, 7, 8, 9, 15, 16, 17, 31, 33, 63, 64, 65, dim, dim + 1, 250]
+        case = cases.attention_case(lens, head_dim=dim, num_q_heads=heads, num_kv_heads=kv_heads, max_blocks=max_blocks, seed=dim + heads)
+        one = torch.eye(dim, dtype=torch.float32)
+        q = torch.stack([one[(7 * i + 3 * torch.arange(heads) + 5 * t) % dim] for t in range(4) for i in range(len(lens))])
+        case["q_packed"] = orc.pack_spikes(q.view(4, len(lens), heads, dim))
+        case["q_packed"][1, :, heads // 2] = -1  # every bit
+        for i, n in enumerate(lens):
+            pos = torch.arange(n)
+            slots = case["block_tables"][i, pos // 16].long() * 16 + pos % 16
+            case["k_cache"][:, :, slots] = orc.pack_spikes(one[(pos * 11 + i) % dim])
+            case["k_cache"][1, :, slots[::3]] = -1
+        got, want = run(case, dev).cpu(), orc.paged_spike_attn_decode(**case)
+        others = [0, 2, 3]
+        assert rel_err(got[others], want[others]) < REL_TOL
+        # Full queries meet keys whose weights are 2^11 (64 channels) or 2^16 apart.  A V bit enters its product as a subnormal half of down to
+        # one significant bit out of eleven, so beside the largest weight a term keeps the 24 bits of a sum less those ten: 2^-14.
+        assert rel_err(got[1], want[1]) < 2.0 ** -14
+        out = torch.empty_like(want, dtype=torch.bfloat16, device=dev)
+        assert within_bf16_bar(run(case, dev, out=out).cpu(), want)
+
+
 @pytest.mark.parametrize("name", ["single_token", "ragged", "bs64", "gqa_4_2", "gqa_28_2", "T1", "T8", "long_split", "wide_table"])
 def test_tcgen05_form_matches_oracle(name, dev, tcgen05_form):
     """The tcgen05 form (int8 MMAs out of shared memory, int32 sums in tensor memory) on the cases it applies to
