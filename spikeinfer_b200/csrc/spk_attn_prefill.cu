@@ -1,25 +1,28 @@
 // Prefill attention over the packed spike pools on the fifth-generation tensor cores (tcgen05), 16-bit outputs, head_dim 64 or 128.
 //
-// CTA = (128 query tokens of one portion, timestep, query head), two CTAs per SM.  Nine warps:
-//  * warps 4-7 read the packed K and V rows of 64 keys through the block table and expand their bits: K to bytes (e4m3 0 or 1), V to
-//    halves (0 or 1), in the swizzled operand layouts; a stage ahead of the MMAs, the next stage's words already in registers;
-//  * warp 8 issues S = Q K^T (kind::f8f6f4, exact: scores are counts) into one of two TMEM buffers and O += P V (kind::f16, P read from
-//    TMEM).  S of step t + 1 goes out before the wait for the weights of step t, so scores are ready when a step's weights are done;
-//  * warps 0-3, a thread per query row, turn scores into weights exp((score - popc(q)) * scale) * 2^14 in halves.  popc(q) bounds every
-//    score of the row: no running maximum, no rescaling of O, and 2^14 keeps the smallest possible weight a normal half.  Their 32-bit
-//    sum, also times 2^14, divides the row at the end.  For fp16 outputs, whose rounding is as fine as the weights', the sum takes the weights as
-//    they are rounded: keys of one score share their rounding, which then cancels (error against 64 bits, three portions of up to
+// CTA = (128 query tokens of one portion, timestep, query head), two CTAs per SM.  Thirteen warps:
+//  * warps 8-11 read the packed K and V rows of 64 keys through the block table and turn their bits into operands: K e4m3 bytes, V halves, each
+//    a masked word as it is, in the swizzled operand layouts; a stage ahead of the MMAs, the next stage's words already in registers;
+//  * warp 12 issues S = Q K^T (kind::f8f6f4, exact: scores are counts) and O += P V (kind::f16, P read from TMEM).  S of step t + 1 goes out as
+//    soon as S of step t has been read, ahead of the wait for the weights of step t;
+//  * warps 0-7, two threads per query row (32 keys of a step each), turn scores into weights exp((score - popc(q)) * scale) * 2^14 in halves.
+//    popc(q) bounds every score of the row: no running maximum, no rescaling of O, and 2^14 keeps the smallest possible weight a normal half.
+//    Their 32-bit sum, also times 2^14, divides the row at the end.  For fp16 outputs, whose rounding is as fine as the weights', the sum takes the
+//    weights as they are rounded: keys of one score share their rounding, which then cancels (error against 64 bits, three portions of up to
 //    300 tokens behind 200, heads of 64 and 128: 2.32e-4 and 2.30e-4 with the sum of the unrounded ones, 2.15e-4 and 2.14e-4 so, 2.20e-4 and 2.29e-4 by
-//    SDPA in fp16).  That takes 6 % of the long portions' time below, 358 -> 380 us of single calls; bf16 results, whose rounding is 8 times coarser,
-//    sum the unrounded ones.
+//    SDPA in fp16); bf16 results, whose rounding is 8 times coarser, sum the unrounded ones.
 // Bits expand in an order that is cheapest for the bit tricks (byte b of word j: bit j + 8 b; half h: bit j + 16 h), the same for Q and K;
 // V's column order is undone when a row is stored.
 //
-// What bounds it: the special-function pipe, one exponential per (query, key) pair, 1024 cycles per 128 x 128 pairs; S and O take about 400 at
-// 64 channels.  Why 64 keys per step: S is double-buffered beside O of up to 128 channels within 256 TMEM columns, so that two CTAs fit an
-// SM and one's set-up and drain hide behind the other's steps.
-// Measured, whole fused_qkv_attention calls against SDPA on spikes unpacked to bf16: 16 x 512 tokens, 14/2 heads of 64, 608 -> 129 us; three
-// portions of 766 to 1531 tokens behind 700 cached, 28/4 heads of 128, 4922 -> 338 us; error against 64 bits 1.8e-3 -> 1.6e-3.
+// What bounds it: shared memory (the operands written, 24 KB a step at 128 channels, and read by the MMAs, 40 KB: about four fifths of its
+// cycles), then the special-function pipe (one exponential per (query, key) pair, half of its cycles) and, for prompts of a few hundred tokens,
+// a CTA's set-up and drain.  Why 64 keys per step: scores, two buffers of weights and O of up to 128 channels are 256 TMEM columns, so
+// that two CTAs fit an SM and one's set-up and drain hide behind the other's steps.
+// Measured, whole fused_qkv_attention calls: three portions of 766 to 1531 tokens behind 700 cached, 28/4 heads of 128, 338 -> 294 us; four of 875
+// to 2000 behind 300, 7/1 heads of 128, 137 -> 118; 16 x 512 tokens, 14/2 heads of 64, 130 as before.  What came before: comparisons with the
+// diagonal in every step and shifts and products per operand register (190 M instructions, 131 M without them), a warp per 32 rows on
+// scores (its waits and its exponentials took turns), S behind the weights' product of two steps before.  With 64 keys per
+// warpgroup and step (even and odd steps): 307 us; one warpgroup that reads all 64 scores ahead: 324.
 #include <algorithm>
 #include <type_traits>
 
@@ -32,11 +35,11 @@ using namespace spk_tc;
 constexpr int kRows = 128;                  // query tokens per CTA
 constexpr int kKeys = 64;                   // keys per step
 constexpr int kStages = 3;
-constexpr int kThreads = 288;
+constexpr int kThreads = 416;              // two warpgroups on scores, one on operands, one warp on MMAs
 constexpr int kQBytes = kRows * 128;        // rows of 128 bytes; 64 channels use the first half
 constexpr int kKBytes = kKeys * 128;
 constexpr int kVColTile = kKeys * 128;      // 64 channels
-constexpr uint32_t kTmemS = 0, kTmemO = 128;
+constexpr uint32_t kTmemS = 0, kTmemP = kKeys, kTmemO = 128;  // scores, two buffers of weights (32 columns each), weighted sum
 constexpr int kMaxPortions = 48, kMaxTiles = 512;
 constexpr float kLog2e = 1.4426950408889634f;
 
@@ -48,7 +51,7 @@ struct Launch {
 };
 
 struct Bars {
-    uint64_t kv_full[kStages], kv_free[kStages], s_full[2], p_full[2], q_full, o_full;
+    uint64_t kv_full[kStages], kv_free[kStages], s_full, s_read, p_full[2], q_full, o_full;
     int abort;
     uint32_t tmem;
 };
@@ -64,27 +67,46 @@ __device__ __forceinline__ void mma_ts_by(uint32_t who, uint32_t d, uint32_t a, 
                  ::"r"(d), "r"(a), "l"(b), "r"(idesc), "r"(acc ? 1 : 0), "r"(who) : "memory");
 }
 
-// One word's 32 channels as e4m3 bytes (0x38 is 1.0) at 16-byte groups 2 w and 2 w + 1 of a 128-byte row.
-__device__ __forceinline__ void expand_bytes(uint8_t* row, int r, int w, uint32_t bits) {
+__device__ __forceinline__ void st_shared16(uint32_t addr, const uint32_t (&v)[4]) {
+    asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]) : "memory");
+}
+
+// Operands are the packed bits IN PLACE, one logic operation per register: what a masked bit stands for depends on its position alone, a power of
+// two that the other operand, or the store of the result, takes out again.
+//
+// One word's 32 channels as e4m3 bytes at 16-byte groups 2 w and 2 w + 1 of a 128-byte row; row: shared address of the row plus (row & 7) << 4, the
+// swizzle.  Register j holds bits j + 8 b; bit e = j % 4 of a byte reads as 2^(e - 9), so a query's register holds 2^(3 - e) where its bit is set
+// and every matching bit adds 2^-6 to a score.
+constexpr float kScoreUnit = 64.0f;
+template <bool QUERY>
+__device__ __forceinline__ void expand_bytes(uint32_t row, int w, uint32_t bits) {
 #pragma unroll
     for (int g = 0; g < 2; ++g) {
-        uint4 v;
-        uint32_t* p = reinterpret_cast<uint32_t*>(&v);
+        const uint32_t from = g == 0 ? bits : bits >> 4;
+        uint32_t v[4];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) p[j] = ((bits >> (4 * g + j)) & 0x01010101u) * 0x38u;
-        *reinterpret_cast<uint4*>(row + (((2 * w + g) ^ (r & 7)) << 4)) = v;
+        for (int e = 0; e < 4; ++e) v[e] = QUERY ? ((from >> e) & 0x01010101u) * ((10u - e) << 3) : from & (0x01010101u << e);
+        st_shared16(row ^ ((2 * w + g) << 4), v);
     }
 }
-// The same as halves (0x3c00 is 1.0), four groups of a 64-channel column tile.
-__device__ __forceinline__ void expand_halves(uint8_t* row, int r, int w, uint32_t bits) {
+// One word's 32 channels as halves, four groups of a 64-channel column tile.  Register j holds bits j and j + 16, moved by 4, 8 or 12 (bit 15: by -1) to
+// one of positions 11 to 14 of a half: 2^-13, 2^-11, 2^-7 or 2, a normal number each (in a subnormal one a product would lose bits beside
+// larger ones of the sum); channel_unit(j) is what takes that out of a column's sum.
+__device__ __forceinline__ void expand_halves(uint32_t row, int w, uint32_t bits) {
+    const uint32_t moved[5] = {bits << 12, bits << 8, bits << 4, bits, bits >> 1};
 #pragma unroll
     for (int g = 0; g < 4; ++g) {
-        uint4 v;
-        uint32_t* p = reinterpret_cast<uint32_t*>(&v);
+        uint32_t v[4];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) p[j] = ((bits >> (4 * g + j)) & 0x00010001u) * 0x3c00u;
-        *reinterpret_cast<uint4*>(row + (((4 * (w & 1) + g) ^ (r & 7)) << 4)) = v;
+        for (int i = 0; i < 4; ++i) {
+            const int j = 4 * g + i, m = j == 15 ? 4 : (j + 1) / 4;
+            v[i] = moved[m] & (0x00010001u << (m == 4 ? 14 : j + 12 - 4 * m));
+        }
+        st_shared16(row ^ ((4 * (w & 1) + g) << 4), v);
     }
+}
+__device__ __forceinline__ constexpr float channel_unit(int j) {
+    return j == 15 || j % 4 == 2 ? 0.5f : j % 4 == 3 ? 8192.0f : j % 4 == 0 ? 2048.0f : 128.0f;
 }
 
 template <typename TO>
@@ -121,20 +143,37 @@ spike_prefill_kernel(const __grid_constant__ Launch l) {
     const int keys = pos0 + nq;
     const int steps = (keys + kKeys - 1) / kKeys;
 
+    // what the first copies wait for is on its way before the set-up below: the table entries of the first two steps' keys, the query's words
+    const int e = threadIdx.x & 127, key = e & (kKeys - 1), half = e >> 6;
+    const int bs_log2 = 31 - __clz(a.block_size), bs_mask = a.block_size - 1;
+    auto entry = [&](int t) {
+        const int j = t * kKeys + key;
+        return j < keys ? por.table[j >> bs_log2] : -1;
+    };
+    const int64_t token = por.start + first + e;
+    int block0 = -1, block = -1;
+    uint32_t qw[W];
+    if (warp >= 8 && warp < 12) {
+        block0 = entry(0);
+        block = entry(1);
+    } else if (warp < 8) {
+        const uint32_t* q = static_cast<const uint32_t*>(a.q_packed) + ts * a.sq_t + token * a.sq_tok + h * a.sq_h;
+#pragma unroll
+        for (int w = 0; w < W; ++w) qw[w] = e < nq ? q[w] : 0u;
+    }
     if (threadIdx.x == 0) {
         for (int i = 0; i < kStages; ++i) {
             mbar_init(smem_u32(&bars->kv_full[i]), 128);
             mbar_init(smem_u32(&bars->kv_free[i]), 1);
         }
-        for (int i = 0; i < 2; ++i) {
-            mbar_init(smem_u32(&bars->s_full[i]), 1);
-            mbar_init(smem_u32(&bars->p_full[i]), 128);
-        }
+        mbar_init(smem_u32(&bars->s_full), 1);
+        mbar_init(smem_u32(&bars->s_read), 256);
+        for (int i = 0; i < 2; ++i) mbar_init(smem_u32(&bars->p_full[i]), 256);
         mbar_init(smem_u32(&bars->q_full), 128);
         mbar_init(smem_u32(&bars->o_full), 1);
         bars->abort = 0;
     }
-    if (warp == 8) tmem_alloc(smem_u32(&bars->tmem), 256);
+    if (warp == 12) tmem_alloc(smem_u32(&bars->tmem), 256);
     fence_async_shared();
     tc_fence_before();
     __syncthreads();
@@ -142,15 +181,9 @@ spike_prefill_kernel(const __grid_constant__ Launch l) {
     const uint32_t tmem = bars->tmem;
     volatile int* abort = &bars->abort;
 
-    if (warp >= 4 && warp < 8) {  // ---- K and V bits to operands: thread = (key, half of the words)
-        const int e = threadIdx.x - 128, key = e & (kKeys - 1), half = e >> 6;
-        const int bs_log2 = 31 - __clz(a.block_size), bs_mask = a.block_size - 1;
+    if (warp >= 8 && warp < 12) {  // ---- K and V bits to operands: thread = (key, half of the words)
         const uint32_t* kp = static_cast<const uint32_t*>(a.k_pool) + ts * a.sk_t + g * a.sk_h + half * (W / 2);
         const uint32_t* vp = static_cast<const uint32_t*>(a.v_pool) + ts * a.sv_t + g * a.sv_h + half * (W / 2);
-        auto entry = [&](int t) {
-            const int j = t * kKeys + key;
-            return j < keys ? por.table[j >> bs_log2] : -1;
-        };
         uint32_t kw[W / 2], vw[W / 2];
         auto fetch = [&](int t, int block) {
             const int j = t * kKeys + key;
@@ -168,8 +201,7 @@ spike_prefill_kernel(const __grid_constant__ Launch l) {
                 vw[i] = vp[vo + i];
             }
         };
-        int block = entry(1);
-        fetch(0, entry(0));
+        fetch(0, block0);
         for (int t = 0; t < steps; ++t) {
             const int stage = t % kStages;
             uint32_t kb[W / 2], vb[W / 2];
@@ -183,18 +215,17 @@ spike_prefill_kernel(const __grid_constant__ Launch l) {
                 block = entry(t + 2);
             }
             if (t >= kStages && !__all_sync(~0u, mbar_wait(smem_u32(&bars->kv_free[stage]), ((t / kStages) - 1) & 1, abort))) break;
-            uint8_t* kr = k_s + stage * kKBytes + key * 128;
-            uint8_t* vr = v_s + stage * kVBytes + key * 128;
+            const uint32_t at = key * 128 + ((key & 7) << 4), kr = smem_u32(k_s) + stage * kKBytes + at, vr = smem_u32(v_s) + stage * kVBytes + at;
 #pragma unroll
             for (int i = 0; i < W / 2; ++i) {
                 const int w = half * (W / 2) + i;
-                expand_bytes(kr, key, w, kb[i]);
-                expand_halves(vr + (w >> 1) * kVColTile, key, w, vb[i]);
+                expand_bytes<false>(kr, w, kb[i]);
+                expand_halves(vr + (w >> 1) * kVColTile, w, vb[i]);
             }
             fence_async_shared();
             mbar_arrive(smem_u32(&bars->kv_full[stage]));
         }
-    } else if (warp == 8) {  // ---- MMAs
+    } else if (warp == 12) {  // ---- MMAs
         constexpr uint32_t s_desc = (1u << 4) | (static_cast<uint32_t>(kKeys >> 3) << 17) | (static_cast<uint32_t>(kRows >> 4) << 24);
         constexpr uint32_t o_desc = (1u << 4) | (1u << 16) | (static_cast<uint32_t>(W * 32 >> 3) << 17) | (static_cast<uint32_t>(kRows >> 4) << 24);
         const uint32_t who = elect_one();
@@ -205,99 +236,106 @@ spike_prefill_kernel(const __grid_constant__ Launch l) {
             const uint64_t qd = desc_sw128(smem_u32(q_s), 16, 1024), kd = desc_sw128(smem_u32(k_s + stage * kKBytes), 16, 1024);
 #pragma unroll
             for (int s = 0; s < W; ++s)  // 32 channels (32 bytes of a row) per MMA
-                mma_f8_by(who, tmem + kTmemS + (t & 1) * kKeys, qd + 2 * s, kd + 2 * s, s_desc, s > 0);
-            if (who) mma_commit(smem_u32(&bars->s_full[t & 1]));
+                mma_f8_by(who, tmem + kTmemS, qd + 2 * s, kd + 2 * s, s_desc, s > 0);
+            if (who) mma_commit(smem_u32(&bars->s_full));
             return true;
         };
         bool ok = __all_sync(~0u, mbar_wait(smem_u32(&bars->q_full), 0, abort)) && __all_sync(~0u, scores(0));
         for (int t = 0; ok && t < steps; ++t) {
-            const int stage = t % kStages, buf = t & 1;
-            // S of step t + 1 overwrites the weights of step t - 1: their product has to be complete.  Issue order does not say so, it holds
-            // among MMAs of one shape and accumulator only; the commit that frees the product's stage does.
-            if (t + 1 < steps)
-                ok = __all_sync(~0u, (t == 0 || mbar_wait(smem_u32(&bars->kv_free[(t - 1) % kStages]), ((t - 1) / kStages) & 1, abort)) && scores(t + 1));
-            ok = ok && __all_sync(~0u, mbar_wait(smem_u32(&bars->p_full[buf]), (t >> 1) & 1, abort));
+            const int stage = t % kStages;
+            // S of step t + 1 as soon as that of step t is in registers, ahead of the wait for the weights
+            if (t + 1 < steps) ok = __all_sync(~0u, mbar_wait(smem_u32(&bars->s_read), t & 1, abort) && scores(t + 1));
+            ok = ok && __all_sync(~0u, mbar_wait(smem_u32(&bars->p_full[t & 1]), (t >> 1) & 1, abort));
             if (!ok) break;
             tc_fence_after();
             const uint64_t vd = desc_sw128(smem_u32(v_s + stage * kVBytes), kVColTile, 1024);
 #pragma unroll
             for (int s = 0; s < kKeys / 16; ++s)
-                mma_ts_by(who, tmem + kTmemO, tmem + kTmemS + buf * kKeys + s * 8, vd + s * (2048 >> 4), o_desc, t > 0 || s > 0);
+                mma_ts_by(who, tmem + kTmemO, tmem + kTmemP + (t & 1) * (kKeys / 2) + s * 8, vd + s * (2048 >> 4), o_desc, t > 0 || s > 0);
             if (who) mma_commit(smem_u32(&bars->kv_free[stage]));
             __syncwarp();
         }
         if (who) mma_commit(smem_u32(&bars->o_full));
         mbar_wait(smem_u32(&bars->o_full), 0);
-    } else {  // ---- scores to weights: thread = query row
-        const int r = threadIdx.x;
-        const int64_t token = por.start + first + r;
-        float sum = 0.0f;
+    } else {  // ---- scores to weights: thread = query row, warps 0-3 the first 32 keys of a step, 4-7 the others
+        const int r = e, wg = warp >> 2;
         uint64_t c1, c0;
         {
-            const uint32_t* q = static_cast<const uint32_t*>(a.q_packed) + ts * a.sq_t + token * a.sq_tok + h * a.sq_h;
             int ones = 0;
 #pragma unroll
             for (int w = 0; w < W; ++w) {
-                const uint32_t bits = r < nq ? q[w] : 0u;
-                ones += __popc(bits);
-                expand_bytes(q_s + r * 128, r, w, bits);
+                ones += __popc(qw[w]);
+                if (wg == 0) expand_bytes<true>(smem_u32(q_s) + r * 128 + ((r & 7) << 4), w, qw[w]);
             }
-            fence_async_shared();
-            mbar_arrive(smem_u32(&bars->q_full));
+            if (wg == 0) {
+                fence_async_shared();
+                mbar_arrive(smem_u32(&bars->q_full));
+            }
             const float c = a.scale * kLog2e, b = 14.0f - ones * c;
-            c1 = f2_pack(c, c);
+            c1 = f2_pack(c * kScoreUnit, c * kScoreUnit);
             c0 = f2_pack(b, b);
         }
-        const uint32_t lanes = static_cast<uint32_t>(warp * 32) << 16;
+        const uint32_t lanes = static_cast<uint32_t>((warp & 3) * 32) << 16;
         uint64_t sums = f2_pack(0.0f, 0.0f);
         bool ok = true;
         for (int t = 0; t < steps; ++t) {
-            ok = __all_sync(~0u, mbar_wait(smem_u32(&bars->s_full[t & 1]), (t >> 1) & 1, abort));
+            // also says that the product of step t - 2, issued before these scores, is complete: its weights lay where step t's go
+            ok = __all_sync(~0u, mbar_wait(smem_u32(&bars->s_full), t & 1, abort));
             if (!ok) break;
             tc_fence_after();
-            const uint32_t at = tmem + lanes + kTmemS + (t & 1) * kKeys;
-            const int last = pos0 + r - t * kKeys;  // last visible column of this row
-#pragma unroll 1
-            for (int c = 0; c < 2; ++c) {
-                uint32_t sc[32];
-                tmem_ld32(at + c * 32, sc);
-                tmem_wait_ld(sc);
-                const int seen = last - c * 32;
-                const bool whole = __all_sync(~0u, seen >= 31);
-                uint32_t p[16];
+            uint32_t sc[32], p[16];
+            tmem_ld32(tmem + lanes + kTmemS + wg * 32, sc);
+            tmem_wait_ld(sc);
+            tc_fence_before();
+            mbar_arrive(smem_u32(&bars->s_read));
+            const int seen = pos0 + r - t * kKeys - wg * 32;  // last visible column of this row
+            auto weights = [&](auto masked) {  // the two forms are code of their own: only the steps on the diagonal compare columns
 #pragma unroll
                 for (int i = 0; i < 16; ++i) {
                     float x, y;
                     f2_unpack(f2_fma(f2_pack(__uint_as_float(sc[2 * i]), __uint_as_float(sc[2 * i + 1])), c1, c0), x, y);
                     x = ex2(x);
                     y = ex2(y);
-                    if (!whole) {
+                    if (decltype(masked)::value) {
                         x = 2 * i <= seen ? x : 0.0f;
                         y = 2 * i + 1 <= seen ? y : 0.0f;
                     }
                     p[i] = pack_pair<__half>(x, y);
                     if (std::is_same<TO, __half>::value) {  // the weights as they enter the product
-                        const float2 r = __half22float2(*reinterpret_cast<const __half2*>(&p[i]));
-                        x = r.x;
-                        y = r.y;
+                        const float2 v = __half22float2(*reinterpret_cast<const __half2*>(&p[i]));
+                        x = v.x;
+                        y = v.y;
                     }
                     sums = f2_add(sums, f2_pack(x, y));
                 }
-                tmem_st16(at + c * 16, p);  // over columns of this half that have been read
+            };
+            if (__all_sync(~0u, seen >= 31)) {
+                weights(std::false_type{});
+            } else if (__all_sync(~0u, seen < 0)) {
+#pragma unroll
+                for (int i = 0; i < 16; ++i) p[i] = 0u;
+            } else {
+                weights(std::true_type{});
             }
+            tmem_st16(tmem + lanes + kTmemP + (t & 1) * (kKeys / 2) + wg * 16, p);
             tmem_wait_st();
             tc_fence_before();
-            mbar_arrive(smem_u32(&bars->p_full[t & 1]));
+            mbar_arrive(smem_u32(&bars->p_full[t & 1]));  // one per parity: a fast warp may be a step ahead of a slow one, not two
         }
         float x, y;
         f2_unpack(sums, x, y);
-        sum = x + y;
         ok = __all_sync(~0u, ok && mbar_wait(smem_u32(&bars->o_full), 0, abort) && *abort == 0);
         tc_fence_after();
+        // both warpgroups' sums of a row, through the query's operand (every MMA is complete); each stores half of the words
+        float* parts = reinterpret_cast<float*>(q_s);
+        parts[wg * kRows + r] = x + y;
+        asm volatile("bar.sync 1, 256;" ::: "memory");
+        const float sum = parts[r] + parts[kRows + r];
         const float inv = ok && r < nq ? 1.0f / sum : 0.0f;
         TO* out = static_cast<TO*>(a.out) + ts * a.so_t + token * a.so_tok + h * a.so_h;
 #pragma unroll
-        for (int w = 0; w < W; ++w) {
+        for (int i = 0; i < W / 2; ++i) {
+            const int w = wg * (W / 2) + i;
             uint32_t o[32];
             tmem_ld32(tmem + lanes + kTmemO + w * 32, o);
             tmem_wait_ld(o);
@@ -309,7 +347,8 @@ spike_prefill_kernel(const __grid_constant__ Launch l) {
 #pragma unroll
                     for (int k = 0; k < 4; ++k) {
                         const int j = (m & 1) * 8 + 2 * k;
-                        const float lo = __uint_as_float(o[2 * j + (m >> 1)]) * inv, hi = __uint_as_float(o[2 * j + 2 + (m >> 1)]) * inv;
+                        const float lo = __uint_as_float(o[2 * j + (m >> 1)]) * (inv * channel_unit(j));
+                        const float hi = __uint_as_float(o[2 * j + 2 + (m >> 1)]) * (inv * channel_unit(j + 1));
                         v[k] = ok ? pack_pair<TO>(lo, hi) : 0u;
                     }
                     TO* dst = out + w * 32 + m * 8;
@@ -332,7 +371,7 @@ spike_prefill_kernel(const __grid_constant__ Launch l) {
     __syncthreads();
     tc_fence_after();
     if (threadIdx.x == 0 && *abort != 0) spk_flag(a.status, SPK_STATUS_DEVICE_WAIT_EXPIRED);
-    if (warp == 8) tmem_dealloc(tmem, 256);
+    if (warp == 12) tmem_dealloc(tmem, 256);
 }
 
 template <int W, typename TO>

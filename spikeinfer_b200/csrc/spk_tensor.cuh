@@ -24,11 +24,12 @@ __device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
                  : "=r"(done) : "r"(bar), "r"(parity) : "memory");
     return done != 0;
 }
-// Waits for a phase; false (and *abort set) after kWaitLimit polls, or as soon as another waiter of the CTA gave up.
+// Waits for a phase; false (and *abort set) after kWaitLimit polls, or soon after another waiter of the CTA gave up (looked at every
+// sixteenth poll: a load between two polls delays what the wait is for).
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort) {
     for (int i = 0; i < kWaitLimit; ++i) {
         if (mbar_try(bar, parity)) return true;
-        if (*abort != 0) return false;
+        if ((i & 15) == 15 && *abort != 0) return false;
     }
     *abort = 1;
     return false;
