@@ -28,9 +28,8 @@
 // Per 32-key tile at head_dim 64: 14 MMAs (8 cycles of a sub-partition's tensor pipe each), 48 masks and about 130 instructions per warp; the
 // integer pipe of the masks (a half-rate unit, 58 % busy) and the tensor pipe (44 %) are the two limits, and warps per SM decide how well they
 // overlap.  Scores by popc (a unit of an eighth of the rate, one per head and word) took the K rows through shared memory
-// to every thread (16 wavefronts per tile against 4): 256 rows x 4096 keys 75.1 -> 68.6 us, with a CTA more per SM 67; 256 rows
-// of 1024 to 32768 keys at head_dim 128 248 -> 221 us.  The e4m3 form of the scores is no MMA of its own on sm_100 but conversions and fp16
-// MMAs: 105 us; heads as the left operand's rows (no transposition, half of the tile empty): 74.6.
+// to every thread (16 wavefronts per tile against 4): 256 rows x 4096 keys 75.1 -> 68.6 us; 256 rows of 1024 to 32768 keys at head_dim 128
+// 248 -> 221 us.  The e4m3 form of the scores is no MMA of its own on sm_100 but conversions and fp16 MMAs: 105 us; heads as the left operand's rows (no transposition, half of the tile empty): 74.6.
 #include "spk_attn.cuh"
 
 #include <atomic>
@@ -83,6 +82,13 @@ __device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, int by
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+
+// A word that the launch ahead may have written: a load of the read-only path could be moved ahead of the wait for that launch.
+__device__ __forceinline__ uint32_t ordered_word(const uint32_t* p) {
+    uint32_t v;
+    asm volatile("ld.global.b32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    return v;
+}
 
 // N consecutive words of shared memory, 16-byte aligned (N = 4 or 8).
 template <int N>
@@ -224,11 +230,11 @@ __device__ __forceinline__ void store_channels(TO* dst, const float* src, float 
     }
 }
 
-// CTAs per SM that a form is built for.  Range form, 16-bit outputs (64 rows of 128 to 4096 keys, 8 layers with their LIF launches; 256 long rows at 128
-// channels): 3 / 4 / 5 of head_dim 64 200 / 168 / 164 us, 2 / 3 / 4 of head_dim 128 325 / 225 / 221.  Where a warp has one short row alone (the unit form) registers
-// beat residency: 144 us against 140 for 8 rows of 96 to 224 keys, 24 layers.
+// CTAs per SM that a form is built for.  256 rows of 1024 to 32768 keys at 128 channels, 16-bit outputs: 2 / 3 / 4 of them 325 / 225 / 221 us (124
+// registers of the range form fit four; the unit form's 129 do not).  64 channels: 3 / 4 / 5 of them 200 / 168 / 164 us for 64 rows of 128 to 4096 keys,
+// 8 layers with their LIF launches; five would take a quarter more workspace (two records a warp) and stay at four.
 template <int W, int NB, bool DENSE>
-struct StreamResident { static constexpr int N = W == 2 ? (NB == 1 && DENSE ? 5 : 4) : (NB == 1 && DENSE ? 4 : 3); };
+struct StreamResident { static constexpr int N = W == 2 || (NB == 1 && DENSE) ? 4 : 3; };
 
 #ifndef SPK_SHORT_STEPS
 #define SPK_SHORT_STEPS 8
@@ -289,7 +295,7 @@ __device__ __forceinline__ void stream_piece(const AttnParams& p, const StreamPa
     auto load_q = [&]() {
 #pragma unroll
         for (int w = 0; w < W; ++w)
-            qw[w] = gid < nh ? __ldg(p.q + t * p.sq_t + row * p.sq_n + (h0 + gid) * p.sq_h + w) : 0u;
+            qw[w] = gid < nh ? ordered_word(p.q + t * p.sq_t + row * p.sq_n + (h0 + gid) * p.sq_h + w) : 0u;
     };
     __syncwarp();  // every lane is done with the previous piece's entries
     stage_tables(key0, min(kend, key0 + span));
