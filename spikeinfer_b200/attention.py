@@ -16,6 +16,7 @@ import torch.nn.functional as F
 
 from .kernels import (LifSiteSpec, gather_kv_unpacked, gather_kv_unpacked_batch, lif_pack_scatter, pack_spikes,
                       paged_spike_attn_decode, paged_spike_attn_prefill, spike_prefill_form)
+from .kernels.lif import qkv_lif_scatter
 from .kernels.packing import packed_width
 
 
@@ -298,6 +299,26 @@ def _one_token_far_behind(meta: AttentionMetadata, channels: int) -> bool:
     return meta.num_prefills == 1 and meta.prefill_query_lens[0] == 1 and meta.prefill_context_lens[0] >= 14000 and channels <= 512
 
 
+def _qkv_sites(qkv, lif_q, lif_k, lif_v, q_packed, q_dense, kc, vc, meta, hq, hkv, d, rope, reset_mode) -> None:
+    """The q, k and v sites of any ``qkv``, with dense spikes of q where they are asked for."""
+    n_tok, W = qkv.shape[1], packed_width(d)
+    xq = qkv[..., : hq * d].unflatten(-1, (hq, d))
+    xk = qkv[..., hq * d:(hq + hkv) * d].unflatten(-1, (hkv, d))
+    xv = qkv[..., (hq + hkv) * d:].unflatten(-1, (hkv, d))
+    cos, sin = rope if rope is not None else (None, None)
+    lif_pack_scatter([
+        LifSiteSpec(x=xq, beta=lif_q[0], threshold=lif_q[1], packed=q_packed, rope_cos=cos, rope_sin=sin,
+                    packed_strides=(n_tok * hq * W, hq * W, W), dense=q_dense,
+                    dense_strides=None if q_dense is None else (q_dense.stride(0), q_dense.stride(2), q_dense.stride(1))),
+        LifSiteSpec(x=xk, beta=lif_k[0], threshold=lif_k[1], packed=kc, rope_cos=cos, rope_sin=sin,
+                    packed_strides=(kc.stride(0), kc.stride(2), kc.stride(1)),
+                    slot_mapping=meta.slot_mapping, num_rows=kc.shape[2]),
+        LifSiteSpec(x=xv, beta=lif_v[0], threshold=lif_v[1], packed=vc,
+                    packed_strides=(vc.stride(0), vc.stride(2), vc.stride(1)),
+                    slot_mapping=meta.slot_mapping, num_rows=min(kc.shape[2], vc.shape[2])),
+    ], reset_mode=reset_mode, status=meta.status)
+
+
 def fused_qkv_attention(qkv: torch.Tensor, lif_q, lif_k, lif_v, k_cache, v_cache, meta: AttentionMetadata,
                         num_q_heads: int, num_kv_heads: int, head_dim: int, reset_mode: int = 0,
                         rope: tuple[torch.Tensor, torch.Tensor] | None = None) -> torch.Tensor:
@@ -310,36 +331,24 @@ def fused_qkv_attention(qkv: torch.Tensor, lif_q, lif_k, lif_v, k_cache, v_cache
     rotary embedding to the q and k currents inside the same launch; without it ``qkv`` must already be
     rotated.  Returns ``[T, n_tok, H_q * head_dim]`` in ``qkv.dtype``.
     """
-    T, n_tok, _ = qkv.shape
+    T, n_tok, width = qkv.shape
     dtype, device = qkv.dtype, qkv.device
     hq, hkv, d = num_q_heads, num_kv_heads, head_dim
     W = packed_width(d)
-    xq = qkv[..., : hq * d].unflatten(-1, (hq, d))
-    xk = qkv[..., hq * d:(hq + hkv) * d].unflatten(-1, (hkv, d))
-    xv = qkv[..., (hq + hkv) * d:].unflatten(-1, (hkv, d))
     q_packed = torch.empty((T, n_tok, hq, W), dtype=torch.int32, device=device)
     q_dense = None
     packed_prefill = meta.num_prefills and meta.prefill_row_tables is not None
     kc, vc = _flat_pool(k_cache), _flat_pool(v_cache)
-    num_slots = kc.shape[2]
     # 16-bit outputs attend on the tensor cores from the packed pools; fp32 keeps 32-bit probabilities (SDPA on unpacked spikes), and pools of
     # other timesteps or heads than the call's stay there too: it takes or refuses them by its own rules
     tensor_prefill = (meta.num_prefills and not packed_prefill and spike_prefill_form(d, dtype) and kc.shape[:2] == (T, hkv) and vc.shape[:2] == (T, hkv)
                       and not _one_token_far_behind(meta, T * hkv * d))
     if meta.num_prefills and not packed_prefill and not tensor_prefill:
         q_dense = torch.empty((T, hq, n_tok, d), dtype=dtype, device=device)
-    cos, sin = rope if rope is not None else (None, None)
-    lif_pack_scatter([
-        LifSiteSpec(x=xq, beta=lif_q[0], threshold=lif_q[1], packed=q_packed, rope_cos=cos, rope_sin=sin,
-                    packed_strides=(n_tok * hq * W, hq * W, W), dense=q_dense,
-                    dense_strides=None if q_dense is None else (q_dense.stride(0), q_dense.stride(2), q_dense.stride(1))),
-        LifSiteSpec(x=xk, beta=lif_k[0], threshold=lif_k[1], packed=kc, rope_cos=cos, rope_sin=sin,
-                    packed_strides=(kc.stride(0), kc.stride(2), kc.stride(1)),
-                    slot_mapping=meta.slot_mapping, num_rows=num_slots),
-        LifSiteSpec(x=xv, beta=lif_v[0], threshold=lif_v[1], packed=vc,
-                    packed_strides=(vc.stride(0), vc.stride(2), vc.stride(1)),
-                    slot_mapping=meta.slot_mapping, num_rows=num_slots),
-    ], reset_mode=reset_mode, status=meta.status)
+    if q_dense is None and width == (hq + 2 * hkv) * d and qkv.stride(2) == 1:
+        qkv_lif_scatter(qkv, lif_q, lif_k, lif_v, q_packed, kc, vc, meta.slot_mapping, hq, hkv, d, rope, reset_mode, meta.status)
+    else:
+        _qkv_sites(qkv, lif_q, lif_k, lif_v, q_packed, q_dense, kc, vc, meta, hq, hkv, d, rope, reset_mode)
     out = torch.empty((T, n_tok, hq, d), device=device, dtype=dtype)
     n_dec = meta.num_decode_tokens
     if n_dec:

@@ -8,6 +8,7 @@ slot-mapped write into the paged pool in one launch for up to four neuron sites.
 from __future__ import annotations
 
 import ctypes
+import struct
 from dataclasses import dataclass
 
 import torch
@@ -20,9 +21,8 @@ HARD_ZERO = _lib.RESET_HARD_ZERO
 
 
 def _param(p: torch.Tensor, device: torch.device) -> torch.Tensor:
-    p = p.detach()
     if p.dtype != torch.float32 or p.device != device or not p.is_contiguous():
-        p = p.to(device=device, dtype=torch.float32).contiguous()
+        p = p.detach().to(device=device, dtype=torch.float32).contiguous()
     return p
 
 
@@ -67,12 +67,10 @@ def lif_multistep(x, beta, threshold, mem0=None, out_dtype=None, return_membrane
         u_in = mem0.reshape(M, N).to(device=dev, dtype=torch.float32).contiguous()
     if spikes.numel() or (return_membrane and M * N):
         lib = _lib.load()
-        with torch.cuda.device(dev):
-            rc = lib.spk_lif(x.data_ptr(), _lib.dtype_code(x.dtype), T, x.stride(0) if T > 0 else 0,
-                             len(sizes), _lib.i64_array(sizes), _lib.i64_array(strides), N,
-                             beta.data_ptr(), threshold.data_ptr(), _lib.ptr(u_in), spikes.data_ptr(),
-                             _lib.dtype_code(out_dtype), _lib.ptr(u_out), reset_mode,
-                             _lib.current_stream(dev))
+        rc = _lib.on_device(dev, lib.spk_lif, x.data_ptr(), _lib.dtype_code(x.dtype), T, x.stride(0) if T > 0 else 0,
+                            len(sizes), _lib.i64_array(sizes), _lib.i64_array(strides), N,
+                            beta.data_ptr(), threshold.data_ptr(), _lib.ptr(u_in), spikes.data_ptr(),
+                            _lib.dtype_code(out_dtype), _lib.ptr(u_out), reset_mode)
         _lib.check(rc, "spk_lif")
     if return_membrane:
         return spikes, u_out
@@ -186,10 +184,62 @@ def lif_pack_scatter(sites: list[LifSiteSpec], reset_mode: int = SUBTRACT_DELAYE
     if n_tok == 0 or T == 0:
         return
     lib = _lib.load()
-    with torch.cuda.device(dev):
-        rc = lib.spk_lif_pack_scatter(arr, len(sites), T, n_tok, reset_mode, _lib.ptr(status),
-                                      _lib.current_stream(dev))
+    rc = _lib.on_device(dev, lib.spk_lif_pack_scatter, arr, len(sites), T, n_tok, reset_mode, _lib.ptr(status))
     _lib.check(rc, "spk_lif_pack_scatter")
+
+
+def qkv_lif_scatter(qkv: torch.Tensor, lif_q, lif_k, lif_v, q_packed: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor,
+                    slot_mapping: torch.Tensor, heads: int, kv_heads: int, dim: int, rope=None, reset_mode: int = SUBTRACT_DELAYED,
+                    status: torch.Tensor | None = None) -> None:
+    """:func:`lif_pack_scatter` of the three sites of ``qkv [T, n_tok, (heads + 2 kv_heads) * dim]`` (contiguous channels): q to ``q_packed``
+    (contiguous ``[T, n_tok, heads, W]``), k and v at ``slot_mapping`` of pools ``[T, kv_heads, slots, W]``.
+
+    The same launch and the same errors without a view and a description per site: those were half of the 95 us that the host spends on a
+    small prefill's :func:`~spikeinfer_b200.attention.fused_qkv_attention`, more than the GPU does."""
+    _lib.require_cuda(qkv, "lif_pack_scatter input")
+    (T, n_tok, _), (s_t, s_tok, _), dev, x = qkv.shape, qkv.stride(), qkv.device, qkv.data_ptr()
+    code, size = _lib.dtype_code(qkv.dtype), qkv.element_size()
+    if slot_mapping.dtype != torch.int64 or slot_mapping.numel() < n_tok:
+        raise ValueError("site 1: slot_mapping must be int64 [n_tok]")
+    slots = slot_mapping.data_ptr()
+    cos_p = sin_p = s_rope = 0
+    if rope is not None:
+        cos, sin = rope
+        if cos.dtype != qkv.dtype or sin.dtype != qkv.dtype or cos.shape != (n_tok, dim) or sin.shape != (n_tok, dim):
+            raise ValueError("site 0: rope cos/sin must be [n_tok, N] in the dtype of x")
+        (s_rope, one), other = cos.stride(), sin.stride()
+        if one != 1 or other != (s_rope, 1):
+            raise ValueError("site 0: rope cos/sin must share a row stride and have contiguous rows")
+        cos_p, sin_p = cos.data_ptr(), sin.data_ptr()
+    words = packed_width(dim)
+    keep, fields, first = [], [], 0
+    for i, (lif, h, dst) in enumerate(((lif_q, heads, q_packed), (lif_k, kv_heads, k_pool), (lif_v, kv_heads, v_pool))):
+        beta, threshold = lif
+        if beta.numel() != dim or threshold.numel() != dim:
+            raise ValueError(f"site {i}: beta/threshold must have N={dim} elements")
+        beta, threshold = _param(beta, dev), _param(threshold, dev)
+        keep += [beta, threshold]  # converted copies live until the launch
+        if dst.dtype != torch.int32:
+            raise TypeError(f"site {i}: packed destination must be int32")
+        if i == 0:
+            to = (n_tok * h * words, h * words, words, 0, 0)
+        else:
+            so = dst.stride()
+            to = (so[0], so[2], so[1], slots, min(k_pool.shape[2], dst.shape[2]))
+        fields += (x + first * size, code, h, dim, s_t, s_tok, dim, beta.data_ptr(), threshold.data_ptr(), 0, 0, dst.data_ptr(), *to, 0, 0, 0, 0, 0, 0)
+        fields += (cos_p, sin_p, s_rope, *_NO_PRODUCT) if i < 2 else (0, 0, 0, *_NO_PRODUCT)
+        first += h * dim
+    if n_tok == 0 or T == 0:
+        return
+    rc = _lib.on_device(dev, _lib.load().spk_lif_pack_scatter, _QkvSites.from_buffer_copy(_QKV_FIELDS.pack(*fields)), 3, T, n_tok, reset_mode, _lib.ptr(status))
+    _lib.check(rc, "spk_lif_pack_scatter")
+
+
+# three LifSite, packed at once: a ctypes structure set field by field takes 10 us
+_NO_PRODUCT = (0,) * 8
+_QKV_FIELDS = struct.Struct("@" + "P2i4q2P2PP3qPqP2i3q2PqP3qP3q" * 3)
+_QkvSites = _lib.LifSite * 3
+assert _QKV_FIELDS.size == ctypes.sizeof(_QkvSites)
 
 
 def lif_pack(x: torch.Tensor, beta: torch.Tensor, threshold: torch.Tensor, *, dense_dtype=None,

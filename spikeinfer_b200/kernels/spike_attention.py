@@ -6,8 +6,10 @@ is :224-244.  ``qk_scores`` exposes the exact integer scores for checking.
 """
 from __future__ import annotations
 
+import functools
 import math
-from ctypes import byref
+import struct
+from ctypes import byref, sizeof
 
 import torch
 
@@ -18,16 +20,17 @@ from .packing import packed_width
 def _pool_strides(cache: torch.Tensor, block_size: int):
     """(s_t, s_h, s_blk, s_slot) of a pool given as ``[T, H_kv, num_slots, W]`` (the reference
     layout, any strides) or as ``[T, H_kv, num_blocks, block_size, W]`` (explicit block axis)."""
-    if cache.ndim == 4:
-        if cache.stride(3) != 1 and cache.shape[3] > 1:
+    shape, s = cache.shape, cache.stride()
+    if len(shape) == 4:
+        if s[3] != 1 and shape[3] > 1:
             raise ValueError("the word axis of a spike cache must be contiguous")
-        return cache.stride(0), cache.stride(1), cache.stride(2) * block_size, cache.stride(2), cache.shape[2] // block_size
-    if cache.ndim == 5:
-        if cache.stride(4) != 1 and cache.shape[4] > 1:
+        return s[0], s[1], s[2] * block_size, s[2], shape[2] // block_size
+    if len(shape) == 5:
+        if s[4] != 1 and shape[4] > 1:
             raise ValueError("the word axis of a spike cache must be contiguous")
-        if cache.shape[3] != block_size:
-            raise ValueError(f"cache block axis holds {cache.shape[3]} slots, expected {block_size}")
-        return cache.stride(0), cache.stride(1), cache.stride(2), cache.stride(3), cache.shape[2]
+        if shape[3] != block_size:
+            raise ValueError(f"cache block axis holds {shape[3]} slots, expected {block_size}")
+        return s[0], s[1], s[2], s[3], shape[2]
     raise ValueError(f"spike cache must be 4-D or 5-D, got {cache.ndim}-D")
 
 
@@ -83,18 +86,16 @@ def paged_spike_attn_decode(
     ws_bytes = lib.spk_attn_decode_workspace_bytes(T, n_seqs, num_q_heads, num_kv_heads, head_dim,
                                                    block_size, max_blocks)
     ws = torch.empty(ws_bytes, dtype=torch.uint8, device=dev) if ws_bytes > 0 else None
-    with torch.cuda.device(dev):
-        if overlap_previous:
-            lib.spk_attn_overlap_next_call()
-        rc = lib.spk_attn_decode(
-            q_packed.data_ptr(), q_packed.stride(0), q_packed.stride(1), q_packed.stride(2),
-            k_cache.data_ptr(), sk[0], sk[1], sk[2], sk[3],
-            v_cache.data_ptr(), sv[0], sv[1], sv[2], sv[3],
-            block_tables.data_ptr(), block_tables.stride(0), seq_lens.data_ptr(),
-            out.data_ptr(), _lib.dtype_code(out.dtype), out.stride(0), out.stride(1), out.stride(2),
-            T, n_seqs, num_q_heads, num_kv_heads, head_dim, block_size, max_blocks, min(sk[4], sv[4]),
-            1.0 / math.sqrt(head_dim), _lib.ptr(ws), ws_bytes, _lib.ptr(status),
-            _lib.current_stream(dev))
+    if overlap_previous:
+        lib.spk_attn_overlap_next_call()
+    rc = _lib.on_device(
+        dev, lib.spk_attn_decode, q_packed.data_ptr(), *q_packed.stride()[:3],
+        k_cache.data_ptr(), sk[0], sk[1], sk[2], sk[3],
+        v_cache.data_ptr(), sv[0], sv[1], sv[2], sv[3],
+        block_tables.data_ptr(), block_tables.stride(0), seq_lens.data_ptr(),
+        out.data_ptr(), _lib.dtype_code(out.dtype), *out.stride()[:3],
+        T, n_seqs, num_q_heads, num_kv_heads, head_dim, block_size, max_blocks, min(sk[4], sv[4]),
+        1.0 / math.sqrt(head_dim), _lib.ptr(ws), ws_bytes, _lib.ptr(status))
     _lib.check(rc, "spk_attn_decode")
     return out
 
@@ -175,6 +176,7 @@ def gather_kv_unpacked_batch(cache: torch.Tensor, block_tables: torch.Tensor, se
     return out
 
 
+@functools.cache
 def spike_prefill_form(head_dim: int, dtype: torch.dtype) -> bool:
     """Whether :func:`paged_spike_attn_prefill` covers this head size and output type."""
     return dtype in (torch.bfloat16, torch.float16) and bool(_lib.load().spk_spike_prefill_form(head_dim, _lib.dtype_code(dtype)))
@@ -192,10 +194,12 @@ def paged_spike_attn_prefill(q_packed: torch.Tensor, k_cache: torch.Tensor, v_ca
         raise ValueError(f"q has {n_heads} heads of {words} words, expected {num_q_heads} of {packed_width(head_dim)}")
     _lib.require_cuda(q_packed, "paged_spike_attn_prefill q_packed")
     dev = q_packed.device
-    if q_packed.stride(3) != 1 or out.stride(3) != 1 or out.shape != (T, n_tok, n_heads, head_dim):
+    sq, so = q_packed.stride(), out.stride()
+    if sq[3] != 1 or so[3] != 1 or out.shape != (T, n_tok, n_heads, head_dim):
         raise ValueError("q_packed and out must have a contiguous last axis, out [T, n_tok, H_q, head_dim]")
     for cache in (k_cache, v_cache):
-        if cache.dtype != torch.int32 or cache.shape[:2] != (T, num_kv_heads) or cache.shape[-1] < words:
+        shape = cache.shape
+        if cache.dtype != torch.int32 or shape[0] != T or shape[1] != num_kv_heads or shape[-1] < words:
             raise ValueError(f"a pool must be int32 [{T}, {num_kv_heads}, .., {words} words or more], got {cache.dtype} {list(cache.shape)}")
     if not len(block_tables) == len(starts) == len(lens) == len(contexts):
         raise ValueError("one table, start, length and context per portion")
@@ -203,17 +207,22 @@ def paged_spike_attn_prefill(q_packed: torch.Tensor, k_cache: torch.Tensor, v_ca
         return out
     tables = [t if t.dtype == torch.int32 and t.device == dev and t.is_contiguous() else t.to(device=dev, dtype=torch.int32).contiguous()
               for t in block_tables]
-    portions = (_lib.SpikePortion * len(lens))(*[(t.data_ptr(), int(s), int(n), int(c), t.numel()) for t, s, n, c in zip(tables, starts, lens, contexts)])
+    fields = []
+    for t, s, n, c in zip(tables, starts, lens, contexts):
+        fields += (t.data_ptr(), int(s), int(n), int(c), t.numel())
+    portions = (_lib.SpikePortion * len(lens)).from_buffer_copy(struct.pack("@" + "P4i" * len(lens), *fields))
     sk, sv = _pool_strides(k_cache, block_size), _pool_strides(v_cache, block_size)
-    a = _lib.SpikePrefillArgs(q_packed.data_ptr(), q_packed.stride(0), q_packed.stride(1), q_packed.stride(2), k_cache.data_ptr(), *sk[:4],
-                              v_cache.data_ptr(), *sv[:4], out.data_ptr(), out.stride(0), out.stride(1), out.stride(2), n_tok, min(sk[4], sv[4]),
-                              T, num_q_heads, num_kv_heads, head_dim, block_size, _lib.dtype_code(out.dtype), 1.0 / math.sqrt(head_dim), 0.0,
-                              _lib.ptr(status))
-    lib = _lib.load()
-    with torch.cuda.device(dev):
-        rc = lib.spk_spike_prefill(byref(a), portions, len(lens), _lib.current_stream(dev))
+    a = _PREFILL_FIELDS.pack(q_packed.data_ptr(), *sq[:3], k_cache.data_ptr(), *sk[:4], v_cache.data_ptr(), *sv[:4], out.data_ptr(), *so[:3], n_tok,
+                             min(sk[4], sv[4]), T, num_q_heads, num_kv_heads, head_dim, block_size, _lib.dtype_code(out.dtype),
+                             1.0 / math.sqrt(head_dim), 0.0, _lib.ptr(status) or 0)
+    rc = _lib.on_device(dev, _lib.load().spk_spike_prefill, byref(_lib.SpikePrefillArgs.from_buffer_copy(a)), portions, len(lens))
     _lib.check(rc, "spk_spike_prefill")
     return out
+
+
+# one SpikePrefillArgs
+_PREFILL_FIELDS = struct.Struct("@P3qP4qP4qP5q6i2fP")
+assert _PREFILL_FIELDS.size == sizeof(_lib.SpikePrefillArgs)
 
 
 def paged_spike_attn_decode_noalloc(q_packed, k_cache, v_cache, block_tables, seq_lens, head_dim: int,

@@ -159,3 +159,79 @@ def test_row_buckets_and_the_covering_bucket():
     assert covering_bucket([48], [0]) == 48             # buckets switched off
     with pytest.raises(ValueError):
         row_buckets(0)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("T, tokens, heads, kv_heads, dim", [(4, 3, 14, 2, 64), (1, 1, 1, 1, 32), (5, 7, 7, 1, 128), (4, 2, 3, 3, 40), (4, 0, 4, 2, 64)])
+@pytest.mark.parametrize("form", ["plain", "rope", "strided", "half params"])
+def test_qkv_sites_are_described_as_three_sites(monkeypatch, dtype, T, tokens, heads, kv_heads, dim, form):
+    """:func:`qkv_lif_scatter` hands the library the structures that the general description of its sites does, field by field."""
+    from spikeinfer_b200.attention import AttentionMetadata, _qkv_sites
+    from spikeinfer_b200.kernels.lif import qkv_lif_scatter
+
+    calls = []
+
+    class Library:
+        def spk_lif_pack_scatter(self, sites, count, *rest):
+            calls.append(([{n: getattr(sites[i], n) for n, *_ in _lib.LifSite._fields_} for i in range(count)], count, rest))
+            return 0
+
+    monkeypatch.setattr(_lib, "require_cuda", lambda *a: None)
+    monkeypatch.setattr(_lib, "load", lambda: Library())
+    monkeypatch.setattr(_lib, "on_device", lambda device, fn, *a: fn(*a, 0))
+    width = (heads + 2 * kv_heads) * dim
+    qkv = torch.randn(T, tokens, width).to(dtype)
+    if form == "strided":  # a slice of a wider product, timesteps inside tokens
+        qkv = torch.randn(tokens, T, width + 24).to(dtype).transpose(0, 1)[..., 8: 8 + width]
+    rope = None
+    if form == "rope":
+        wide = torch.randn(tokens, 2 * dim).to(dtype)
+        rope = wide[:, :dim], wide[:, dim:]
+    params = [tuple(torch.rand(dim) for _ in range(2)) for _ in range(3)]
+    words = kernels.packed_width(dim)
+    q = torch.empty(T, tokens, heads, words, dtype=torch.int32)
+    k = torch.empty(T, kv_heads, 96, words, dtype=torch.int32)
+    v = torch.empty(T, 80, kv_heads, words, dtype=torch.int32).transpose(1, 2) if form == "strided" else torch.empty_like(k)
+    slots, status = torch.zeros(tokens, dtype=torch.int64), torch.zeros(1, dtype=torch.int32)
+    meta = AttentionMetadata(slot_mapping=slots, block_size=16, status=status)
+    if form == "half params":
+        params = [tuple(p.half() for p in ps) for ps in params]
+    qkv_lif_scatter(qkv, *params, q, k, v, slots, heads, kv_heads, dim, rope, 0, status)
+    _qkv_sites(qkv, *params, q, None, k, v, meta, heads, kv_heads, dim, rope, 0)
+    if tokens == 0:
+        assert calls == []
+        return
+    (got, n, rest), (want, m, rest2) = calls
+    if form == "half params":  # converted copies: other addresses
+        for site in (*got, *want):
+            assert site.pop("beta") and site.pop("threshold")
+    for site in (*got, *want):  # the stride of an axis of one element has no meaning
+        for axis, length in (("t", T), ("tok", tokens), ("h", site["H"])):
+            if length == 1:
+                site.pop("sx_" + axis)
+    assert n == m == 3 and rest == rest2 and got == want
+
+
+def test_qkv_sites_refuse_what_the_general_description_refuses(monkeypatch):
+    from spikeinfer_b200.attention import AttentionMetadata, _qkv_sites
+    from spikeinfer_b200.kernels.lif import qkv_lif_scatter
+
+    with pytest.raises(_lib.SpkError):  # a CPU tensor
+        qkv_lif_scatter(torch.zeros(4, 2, 256), *[(torch.ones(64),) * 2] * 3, None, None, None, torch.zeros(2, dtype=torch.int64), 2, 1, 64)
+    monkeypatch.setattr(_lib, "require_cuda", lambda *a: None)
+    good = dict(qkv=torch.zeros(4, 2, 256), lif=[(torch.ones(64), torch.ones(64))] * 3, q=torch.zeros(4, 2, 2, 2, dtype=torch.int32),
+                k=torch.zeros(4, 1, 32, 2, dtype=torch.int32), v=torch.zeros(4, 1, 32, 2, dtype=torch.int32), slots=torch.zeros(2, dtype=torch.int64),
+                rope=(torch.zeros(2, 64), torch.zeros(2, 64)))
+    bad = [dict(slots=torch.zeros(2, dtype=torch.int32)), dict(slots=torch.zeros(1, dtype=torch.int64)), dict(k=good["k"].float()),
+           dict(lif=[(torch.ones(32), torch.ones(64))] * 3), dict(rope=(torch.zeros(2, 64).bfloat16(),) * 2), dict(rope=(torch.zeros(1, 64),) * 2),
+           dict(rope=(torch.zeros(2, 64), torch.zeros(64, 2).t())), dict(qkv=torch.zeros(4, 2, 256, dtype=torch.float64))]
+    for change in bad:
+        c = {**good, **change}
+        errors = []
+        for call in (lambda: qkv_lif_scatter(c["qkv"], *c["lif"], c["q"], c["k"], c["v"], c["slots"], 2, 1, 64, c["rope"]),
+                     lambda: _qkv_sites(c["qkv"], *c["lif"], c["q"], None, c["k"], c["v"], AttentionMetadata(slot_mapping=c["slots"], block_size=16), 2, 1, 64,
+                                        c["rope"], 0)):
+            with pytest.raises((ValueError, TypeError)) as e:
+                call()
+            errors.append(type(e.value))
+        assert errors[0] is errors[1], change
