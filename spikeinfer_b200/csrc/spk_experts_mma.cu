@@ -8,10 +8,9 @@
 //    tiles of the next product.
 //  * plain: 256 consecutive output features, 32-bit rows.
 //
-// Few tokens (TN = 32): the time is that of streaming the weights.  The plain product's are on their way before the gated one is done
-// (16 experts of 896 x 1216, one row beside the mixer: whole step 4204 -> 4107 us; 64 rows 6791 -> 6732).  Where few blocks are streamed, a
-// cluster of S CTAs shares a block, each over its own part of k; the partial sums meet in shared memory and are added in the order
-// of the CTAs, so results don't depend on timing.
+// Few tokens: the time is that of streaming the weights, experts_stream_kernel.  The plain product's are on their way before the gated one is done.
+// Where few blocks are streamed, a cluster of S CTAs shares a block, each over its own part of k; the partial sums meet in shared memory and are
+// added in the order of the CTAs, so results don't depend on timing.
 // Warp 0 copies, warp 1 issues MMAs, the others write the results.  A tile of 64 tokens and more has eight of them, each with half of the tokens: a
 // CTA's results wait for its last MMA, and with four warps they took about as long as the MMAs (7500 tokens, 16 experts of 896 x 1216, two
 // per token: 91.8 -> 78.9 us gated, 45.7 -> 41.9 plain; 1200 tokens 36.1 -> 33.3, 22.8 -> 21.4).
@@ -240,6 +239,199 @@ experts_kernel(const spk_experts_args a, const int blocks, const int ktiles) {
     if (warp == 0) tmem_dealloc(tmem, Sh::kColumns);
 }
 
+// Few tokens per expert: the CTAs go over the blocks of all experts, the copies of the next block under way while the last stages of this one are
+// multiplied and its results written (two sets of accumulators).  What bounds it is HBM, shared with the mixer's launches beside it, and those
+// need whole SMs for their products: so one CTA per SM with six stages, no more of them than kStreamCtas, and the next launch's CTAs are let in
+// when the copies are all under way.  16 experts of 896 x 1216, whole decode steps of four, 64 rows: a CTA per block, two per SM (160 blocks) 6285 us;
+// 160, 80, 54 CTAs 6640, 6070, 6090; 30 rows 5590 -> 5050, 12 rows 5040 -> 4800, one row 3850 -> 3775 (with the mixer on a stream of higher priority).
+struct StreamBars {
+    uint64_t full[8], free[8], done[2], drained[2], all;
+    int abort;
+    uint32_t tmem;
+};
+constexpr int kStreamTokens = 32;
+constexpr int kStreamStages = 6;
+constexpr int kStreamStage = 2 * kTileW + kStreamTokens * 128;
+constexpr int kStreamBytes = kStreamStages * kStreamStage + 1024 + 256;
+constexpr int kStreamThreads = 192;
+constexpr int kStreamColumns = 128;
+constexpr int kStreamCtas = 96;
+
+template <bool GATED>
+__global__ void __launch_bounds__(kStreamThreads, 1)
+experts_stream_kernel(const spk_experts_args a, const int blocks, const int ktiles) {
+    constexpr int NS = kStreamStages, TN = kStreamTokens;
+    extern __shared__ uint8_t raw[];
+    uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(raw) + 1023) & ~uintptr_t(1023));
+    StreamBars* bars = reinterpret_cast<StreamBars*>(base + NS * kStreamStage);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    struct Tile {
+        int e, rows, b;
+        int64_t row0;
+    };
+    // Block i of this CTA, 1; 0 where there is none, -1 where its rows lie outside the matrix (nothing is done for it).  Called by a whole warp.
+    auto find = [&](int i, Tile& t) {
+        const int at = static_cast<int>(blockIdx.x) + i * static_cast<int>(gridDim.x);
+        t.b = at % blocks;
+        if (!spk_find_tile<TN>(a.segs, a.experts, at / blocks, t.e, t.row0, t.rows)) return 0;
+        return t.row0 + TN > a.rows ? -1 : 1;
+    };
+    Tile t;
+    int there = find(0, t);
+    if (there == 0) {  // uniform over the CTA: nothing has been set up yet
+        spk_grid_wait();
+        return;
+    }
+    if (threadIdx.x == 0) {
+        for (int i = 0; i < NS; ++i) {
+            mbar_init(smem_u32(&bars->full[i]), 1);
+            mbar_init(smem_u32(&bars->free[i]), 1);
+        }
+        for (int i = 0; i < 2; ++i) {
+            mbar_init(smem_u32(&bars->done[i]), 1);
+            mbar_init(smem_u32(&bars->drained[i]), 128);
+        }
+        mbar_init(smem_u32(&bars->all), 1);
+        bars->abort = 0;
+    }
+    if (warp == 0) tmem_alloc(smem_u32(&bars->tmem), kStreamColumns);
+    fence_async_shared();
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = bars->tmem;
+    volatile int* abort = &bars->abort;
+    if (warp == 0) {
+        int copied = 0, issued = 0;  // stages since the first block, the same count in warp 1; those whose copies are under way
+        bool go = true;
+        for (int i = 0; there != 0 && go; ++i) {
+            if (there > 0 && lane == 0) {
+                const uint8_t* w = static_cast<const uint8_t*>(a.w) + (static_cast<int64_t>(t.e) * blocks + t.b) * ktiles * (2 * kTileW);
+                const uint8_t* x = static_cast<const uint8_t*>(a.x) + t.row0 * 128;
+                auto weights = [&](int k, int c) {
+                    const uint32_t bar = smem_u32(&bars->full[c % NS]);
+                    mbar_expect(bar, kStreamStage);
+                    bulk_load(smem_u32(base + (c % NS) * kStreamStage), w + static_cast<int64_t>(k) * (2 * kTileW), 2 * kTileW, bar);
+                };
+                // launched to overlap: the weights of the first stages don't wait for the launch that writes x
+                const int early = copied > 0 || !a.overlap ? 0 : ktiles < NS ? ktiles : NS;
+                for (int k = 0; k < early; ++k) weights(k, k);
+                if (copied == 0) spk_grid_wait();
+                for (int k = 0; k < ktiles; ++k) {
+                    const int c = copied + k;
+                    if (c >= NS && !mbar_wait(smem_u32(&bars->free[c % NS]), ((c / NS) - 1) & 1, abort)) {
+                        go = false;
+                        break;
+                    }
+                    if (k >= early) weights(k, c);
+                    bulk_load(smem_u32(base + (c % NS) * kStreamStage) + 2 * kTileW, x + static_cast<int64_t>(k) * a.rows * 128, TN * 128,
+                              smem_u32(&bars->full[c % NS]));
+                    issued = c + 1;
+                }
+            }
+            go = __shfl_sync(~0u, go, 0);
+            if (there > 0) copied += ktiles;
+            there = find(i + 1, t);
+        }
+        spk_grid_release();  // the next launch's CTAs may take SMs from here on: this one's copies are all under way
+        if (lane == 0) {
+            spk_grid_wait();  // also where no block's rows were good
+            if (*abort != 0)  // copies in flight land before the CTA's shared memory is given up
+                for (int c = issued > NS ? issued - NS : 0; c < issued; ++c) mbar_wait(smem_u32(&bars->full[c % NS]), (c / NS) & 1);
+        }
+    } else if (warp == 1) {
+        constexpr uint32_t idesc = idesc_bf16(128, TN, false, false);
+        int used = 0, n = 0;
+        bool go = true;
+        for (int i = 0; there != 0 && go; ++i) {
+            if (there > 0) {
+                if (lane == 0) {
+                    const uint32_t acc = tmem + (n & 1) * 2 * TN;
+                    go = n < 2 || mbar_wait(smem_u32(&bars->drained[n & 1]), ((n / 2) - 1) & 1, abort);
+                    tc_fence_after();
+                    for (int k = 0; k < ktiles && go; ++k) {
+                        const int c = used + k;
+                        go = mbar_wait(smem_u32(&bars->full[c % NS]), (c / NS) & 1, abort);
+                        if (!go) break;
+                        tc_fence_after();
+                        const uint32_t wa = smem_u32(base + (c % NS) * kStreamStage), xa = wa + 2 * kTileW;
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) {
+                            const uint64_t xd = desc_sw128(xa + j * 32, 16, 1024);
+                            mma_ss(acc, desc_sw128(wa + j * 32, 16, 1024), xd, idesc, k > 0 || j > 0);
+                            mma_ss(acc + TN, desc_sw128(wa + kTileW + j * 32, 16, 1024), xd, idesc, k > 0 || j > 0);
+                        }
+                        mma_commit(smem_u32(&bars->free[c % NS]));
+                    }
+                    mma_commit(smem_u32(&bars->done[n & 1]));
+                }
+                go = __shfl_sync(~0u, go, 0);
+                used += ktiles;
+                ++n;
+            }
+            there = find(i + 1, t);
+        }
+        if (lane == 0) {
+            mma_commit(smem_u32(&bars->all));
+            mbar_wait(smem_u32(&bars->all), 0);  // nothing this thread issued is in the tensor pipe any more
+        }
+    } else {
+        const int quad = warp & 3;
+        const uint32_t lanes = static_cast<uint32_t>(quad * 32) << 16;
+        int n = 0;
+        bool ok = true;
+        for (int i = 0; there != 0 && ok; ++i) {
+            if (there > 0) {
+                ok = __all_sync(~0u, mbar_wait(smem_u32(&bars->done[n & 1]), (n / 2) & 1, abort)) && *abort == 0;
+                ok = __all_sync(~0u, ok);
+                tc_fence_after();
+                uint32_t p[32], q[32];
+                const uint32_t acc = tmem + lanes + (n & 1) * 2 * TN;
+                tmem_ld32(acc, p);
+                tmem_ld32(acc + TN, q);
+                tmem_wait_ld(p);
+                tmem_wait_ld(q);
+                tc_fence_before();
+                mbar_arrive(smem_u32(&bars->drained[n & 1]));
+                float x[32], y[32];
+#pragma unroll
+                for (int j = 0; j < 32; ++j) {
+                    x[j] = __uint_as_float(p[j]);
+                    y[j] = __uint_as_float(q[j]);
+                }
+                const int f = t.b * (GATED ? 128 : 256) + quad * 32 + lane;  // this lane's feature (and f + 128)
+                const int live = ok ? t.rows : 0;
+                if (GATED) store_gated<32>(a, t.row0, live, f, lane, x, y);
+                else store_plain<32>(a, t.row0, live, f, x, y);
+                ++n;
+            } else if (threadIdx.x == 64) {
+                spk_flag(a.status, SPK_STATUS_BAD_SLOT);
+            }
+            there = find(i + 1, t);
+        }
+    }
+    __syncwarp();
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    if (threadIdx.x == 0 && *abort != 0) spk_flag(a.status, SPK_STATUS_DEVICE_WAIT_EXPIRED);
+    if (warp == 0) tmem_dealloc(tmem, kStreamColumns);
+}
+
+template <bool GATED>
+int launch_stream(const spk_experts_args& a, int blocks, int ktiles, cudaStream_t s) {
+    static_assert(sizeof(StreamBars) <= 256 && kStreamBytes <= 227 * 1024, "shared memory");
+    const int64_t most = spk_most_tiles(a.pairs, a.experts, kStreamTokens) * blocks;
+    if (most > 0x3fffffff) return SPK_ERR_TOO_LARGE;
+    // as many CTAs as leave each the same number of blocks if every expert in use has one run of tokens, at most kStreamCtas
+    const int64_t expected = static_cast<int64_t>(blocks) * (a.pairs < a.experts ? a.pairs : a.experts);
+    const int64_t rounds = (expected + kStreamCtas - 1) / kStreamCtas;
+    const int64_t ctas = (expected + rounds - 1) / rounds;
+    const cudaError_t e = cudaFuncSetAttribute(experts_stream_kernel<GATED>, cudaFuncAttributeMaxDynamicSharedMemorySize, kStreamBytes);
+    if (e != cudaSuccess) return spk_set_cuda_error(e);
+    return spk_launch(experts_stream_kernel<GATED>, dim3(static_cast<unsigned>(ctas)), kStreamThreads, kStreamBytes, s, a.overlap != 0, a, blocks, ktiles);
+}
+
 template <int TN, bool GATED, int S>
 int launch(const spk_experts_args& a, int blocks, int ktiles, cudaStream_t s) {
     constexpr int bytes = Shape<TN>::kBytes;
@@ -281,13 +473,11 @@ int dispatch(const spk_experts_args& a, cudaStream_t s) {
     if (mean > 40) return launch<128, GATED, 1>(a, blocks, ktiles, s);
     if (mean > 16) return launch<64, GATED, 1>(a, blocks, ktiles, s);
     // Blocks streamed by the second product: with fewer than 17 (a step of one user with two experts has 8) two CTAs share each.  One row of 16 experts
-    // of 896 x 1216 beside the mixer's launches: whole step 4107 us without, 3834 with two parts of the second product, 4103 with two of both, 4260
-    // with four of both: more CTAs take SMs from the mixer, although the two launches alone go on falling (20.8, 17.1, 15.1, 11.1 us).  With
-    // 8 and 64 rows (64 blocks) parts gain nothing: 5058 -> 5185 us, 6732 -> 6959.
+    // of 896 x 1216 beside the mixer's launches: whole step 4107 us without, 3834 with two parts; more parts take SMs from the mixer.
     if constexpr (!GATED) {
         if (blocks * (a.pairs < a.experts ? a.pairs : a.experts) <= 16 && ktiles >= 2) return launch<32, GATED, 2>(a, blocks, ktiles, s);
     }
-    return launch<32, GATED, 1>(a, blocks, ktiles, s);
+    return launch_stream<GATED>(a, blocks, ktiles, s);
 }
 
 }  // namespace

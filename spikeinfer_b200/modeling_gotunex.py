@@ -267,9 +267,10 @@ class GotunexModel:
             layer.route_index = i
         self.router = ExpertRouter([layer.experts for layer in routed], c.vocab) if routed else None
         self._rot: dict[RotaryConfig, torch.Tensor] = {}
-        # the feed-forward reads the same x as the mixer: steps of up to this many tokens run it on a stream of its own beside it
+        # the mixer reads the same x as the feed-forward: steps of up to this many tokens run it on a stream of its own beside it, one of
+        # higher priority, since the experts' copies would keep every SM from the mixer's short launches
         self.side_tokens = 1024
-        self._side = torch.cuda.Stream(device=self.device)
+        self._side = torch.cuda.Stream(device=self.device, priority=-1)
 
     def prepare(self, max_positions: int) -> None:
         """Engine hook: positions ``0 .. max_positions - 1`` may be fed (tabulates the rotary factors)."""
@@ -328,17 +329,18 @@ class GotunexModel:
             if beside:
                 self._side.wait_stream(main)
             with torch.cuda.stream(self._side if beside else main):
-                if L.up is not None:
-                    gelu_tanh(self._matmul(hand["out2"], L.up), both[:, mixed:])
-                elif L.experts is not None:
-                    route = routes[L.route_index]
-                    added = dict(pairs=experts_forward(hand["out2"], L.experts, route, meta.status), pair_slots=route.slots, pair_scale=1.0 / L.experts.top)
-            L.mixer.forward(self, h, both[:, :mixed], positions, caches[i], meta)
-            if beside and L.up is not None:
+                L.mixer.forward(self, h, both[:, :mixed], positions, caches[i], meta)
+                if L.up is None:
+                    delta = self._matmul_f32(both, L.w_out)
+            if L.up is not None:
+                gelu_tanh(self._matmul(hand["out2"], L.up), both[:, mixed:])
+            elif L.experts is not None:
+                route = routes[L.route_index]
+                added = dict(pairs=experts_forward(hand["out2"], L.experts, route, meta.status), pair_slots=route.slots, pair_scale=1.0 / L.experts.top)
+            if beside:
                 main.wait_stream(self._side)
-            delta = self._matmul_f32(both, L.w_out)
-            if beside and L.experts is not None:
-                main.wait_stream(self._side)
+            if L.up is not None:
+                delta = self._matmul_f32(both, L.w_out)
             hand = reads(i + 1)
             rms_residual(x=x, delta=delta, **added, **hand, **common)
             if residuals is not None:

@@ -133,6 +133,19 @@ def test_experts(dev, status, n, width, experts, top, ff, dtype):
     assert rel(got, want) < (3e-6 if dtype == F32 else 8e-3)
 
 
+@pytest.mark.parametrize("n,width,experts,top,ff", [(60, 130, 40, 2, 1300), (24, 1024, 30, 4, 64), (100, 448, 8, 1, 384), (90, 64, 96, 2, 640),
+                                                    (7, 900, 12, 3, 130)])
+def test_experts_streamed_over_several_blocks_a_cta(dev, status, n, width, experts, top, ff):
+    """More blocks than the streaming kernel has CTAs (440, 120, 24, 480, 24 gated ones), a CTA's rounds unequal, fewer and more k tiles than stages, one
+    k tile, several runs of tokens per expert, experts without tokens."""
+    w, weights, ids, x, cfg = expert_case(dev, BF, n, width, experts, top, ff, n + ff)
+    x = go.rms(x.double(), 0.0)
+    for _ in range(3):
+        route, out = run_experts(dev, status, weights, ids, x)
+        got = out.cpu().double()[route.slots.cpu().long()].mean(1)
+        assert rel(got, go.table_experts(x, ids.tolist(), go.as_float(w), "", cfg)) < 8e-3
+
+
 @pytest.mark.parametrize("n,width,experts,top,ff", [(1, 896, 16, 2, 1216), (2, 72, 16, 2, 65), (3, 300, 4, 2, 129), (16, 200, 2, 2, 1000), (32, 264, 2, 1, 130)])
 def test_experts_of_few_tokens(dev, status, n, width, experts, top, ff):
     """The forms that share a block of the second product between two CTAs: two to nineteen k tiles, one to 32 rows per expert; twice the same bits."""
