@@ -15,10 +15,7 @@ _ptr = _lib.ptr
 
 
 def _call(name: str, args, device: torch.device) -> None:
-    lib = _lib.load()
-    with torch.cuda.device(device):
-        rc = getattr(lib, name)(byref(args), _lib.current_stream(device))
-    _lib.check(rc, name)
+    _lib.check(_lib.on_device(device, getattr(_lib.load(), name), byref(args)), name)
 
 
 def _f32(t: torch.Tensor | None, name: str, numel: int | None = None) -> None:
@@ -69,10 +66,8 @@ def poly_norm(z: torch.Tensor, coef: torch.Tensor, eps: float, out: torch.Tensor
     out = torch.empty_like(z) if out is None else out
     if not z.is_contiguous() or not out.is_contiguous() or out.shape != z.shape or out.dtype != z.dtype:
         raise ValueError("z and out must be contiguous, same shape and dtype")
-    lib = _lib.load()
-    with torch.cuda.device(z.device):
-        rc = lib.spk_poly_norm(z.data_ptr(), coef.data_ptr(), eps, out.data_ptr(), z.shape[0], z.shape[1],
-                               _lib.dtype_code(z.dtype), _lib.current_stream(z.device))
+    rc = _lib.on_device(z.device, _lib.load().spk_poly_norm, z.data_ptr(), coef.data_ptr(), eps, out.data_ptr(), z.shape[0], z.shape[1],
+                        _lib.dtype_code(z.dtype))
     _lib.check(rc, "spk_poly_norm")
     return out
 
@@ -256,9 +251,7 @@ def gelu_tanh(z: torch.Tensor, out: torch.Tensor) -> torch.Tensor:
     _lib.require_cuda(z, "gelu_tanh input")
     if not z.is_contiguous() or out.shape != z.shape or out.dtype != z.dtype or out.stride(1) != 1:
         raise ValueError("z must be contiguous, out of the same shape and dtype with unit column stride")
-    lib = _lib.load()
-    with torch.cuda.device(z.device):
-        rc = lib.spk_gelu_tanh(z.data_ptr(), out.data_ptr(), out.stride(0), z.shape[0], z.shape[1], _lib.dtype_code(z.dtype),
-                               _lib.current_stream(z.device))
+    rc = _lib.on_device(z.device, _lib.load().spk_gelu_tanh, z.data_ptr(), out.data_ptr(), out.stride(0), z.shape[0], z.shape[1],
+                        _lib.dtype_code(z.dtype))
     _lib.check(rc, "spk_gelu_tanh")
     return out
