@@ -33,6 +33,12 @@ delta_step_kernel(const spk_delta_args a) {
     const int64_t row = blockIdx.y;
     const int dim = a.dim, vdim = a.vdim, rep = a.heads / a.kv_heads, g = h / rep;
     T* out = static_cast<T*>(a.out) + row * a.out_stride + static_cast<int64_t>(h) * vdim;
+    // what waits for nothing is asked for first (stores to the ring would hold it back below)
+    const int64_t pos = a.positions[row];
+    const T* gate = static_cast<const T*>(a.gate) + row * a.ld2 + static_cast<int64_t>(h) * vdim;
+    const float raw_beta = spk_to_float<T>(static_cast<const T*>(a.b)[row * a.ld + h]);
+    const float gate_mine = static_cast<int>(threadIdx.x) < vdim ? spk_to_float<T>(gate[threadIdx.x]) : 0.0f;
+    const float norm_mine = static_cast<int>(threadIdx.x) < vdim ? a.w_norm[threadIdx.x] : 0.0f;
     if (a.active != nullptr && a.active[row] != 1) {
         for (int e = threadIdx.x; e < vdim; e += NT) out[e] = spk_from_float<T>(0.0f);
         return;
@@ -57,13 +63,11 @@ delta_step_kernel(const spk_delta_args a) {
     const int first = slices > 1 ? threadIdx.x % cols : threadIdx.x;
     const bool mine = slice < slices;
     const SpkDeltaShape sh = spk_delta_shape(a);
-    const int64_t pos = a.positions[row];
     const bool fresh = pos == 0;  // whatever the slot holds, a sequence starts from zeros
     float* ring = a.conv_state + row * a.taps * sh.channels;
     const int now_slot = static_cast<int>(static_cast<uint64_t>(pos) % static_cast<uint32_t>(a.taps));
     const int past = pos < a.taps - 1 ? static_cast<int>(pos) : a.taps - 1;  // earlier tokens the convolution sees
     const bool leader = h % rep == 0;
-    const T* gate = static_cast<const T*>(a.gate) + row * a.ld2 + static_cast<int64_t>(h) * vdim;
     float sums[3] = {0.0f, 0.0f, 0.0f};
     // one channel of q, k, the decays or v per thread and turn; two turns' loads are in flight together
     struct Item {
@@ -125,14 +129,11 @@ delta_step_kernel(const spk_delta_args a) {
             v[it.local] = y;
         }
     };
-    const float raw_beta = spk_to_float<T>(static_cast<const T*>(a.b)[row * a.ld + h]);
     for (int i = threadIdx.x; i < items; i += 2 * NT) {
         const Item x = fetch(i), y = fetch(i + NT);
         finish(x);
         finish(y);
     }
-    const float gate_mine = static_cast<int>(threadIdx.x) < vdim ? spk_to_float<T>(gate[threadIdx.x]) : 0.0f;
-    const float norm_mine = static_cast<int>(threadIdx.x) < vdim ? a.w_norm[threadIdx.x] : 0.0f;
     spk_block_sum<3>(sums, part);  // its barriers also publish q, k, v and the decays
     const float qi = 1.0f / (sqrtf(sums[0] + 1e-6f) * sqrtf(static_cast<float>(dim))), ki = 1.0f / sqrtf(sums[1] + 1e-6f);
     const float beta = spk_sigmoid(raw_beta);

@@ -11,12 +11,29 @@ namespace {
 
 using namespace spk_tc;
 
-template <typename T, typename TD, int V, bool VEC>
-__global__ void __launch_bounds__(1024)
+// AHEAD: everything that does not depend on the row's sums is asked for at once.  A decode step's row is a chain of round trips to L2, and the
+// norms' weights and the destinations behind the mean square, and expert rows one after the other behind their slots, were six of them: whole
+// Gotunex steps of one, four, 30 and 64 rows 3795 -> 3590, 4115 -> 3925, 5060 -> 4928, 6110 -> 5950 us (with the loads of the delta rule's step moved up in
+// the same way).  Prompt batches hide the trips behind other rows and want the registers (72 against 40): 0.6 % of a prompt pass slower with it.
+template <typename T, typename TD, int V, bool VEC, bool AHEAD>
+__global__ void __launch_bounds__(AHEAD ? 256 : 1024)  // spk_row_shape: up to two groups a thread are at most 256 threads
 rms_residual_kernel(const spk_rms_residual_args p) {
     __shared__ float part[32];
     const int64_t t = blockIdx.x;
     const int width = static_cast<int>(p.width);
+    SpkRow<V> w1, w2;
+    if (AHEAD) {
+#pragma unroll
+        for (int v = 0; v < V; ++v) {
+            const int c = 4 * (threadIdx.x + v * blockDim.x);
+            w1.g[v] = spk_load4<float, VEC>(p.w1 + c, p.w1 != nullptr ? width - c : 0);
+            w2.g[v] = spk_load4<float, VEC>(p.w2 + c, p.w2 != nullptr ? width - c : 0);
+        }
+    }
+    constexpr int kSlots = AHEAD ? 2 : 1;
+    int64_t to[kSlots];
+#pragma unroll
+    for (int j = 0; j < kSlots; ++j) to[j] = AHEAD && p.w2 != nullptr && p.out2_slots != nullptr && j < p.out2_top ? p.out2_slots[t * p.out2_top + j] : -1;
     SpkRow<V> y;
     if (p.ids != nullptr) {
         const int64_t id = p.ids[t];
@@ -49,20 +66,27 @@ rms_residual_kernel(const spk_rms_residual_args p) {
             SpkRow<V> s;
 #pragma unroll
             for (int v = 0; v < V; ++v) s.g[v] = make_float4(0.f, 0.f, 0.f, 0.f);
-            for (int j = 0; j < p.pair_top; ++j) {
-                const int64_t slot = p.pair_slots[t * p.pair_top + j];
-                if (slot < 0) continue;
-                if (slot >= p.pair_rows) {
-                    if (threadIdx.x == 0) spk_flag(p.status, SPK_STATUS_BAD_SLOT);
-                    continue;
-                }
-                const float* r = p.pairs + slot * p.width;
+            for (int j0 = 0; j0 < p.pair_top; j0 += kSlots) {
+                int64_t slot[kSlots];
+                SpkRow<V> f[kSlots];
 #pragma unroll
-                for (int v = 0; v < V; ++v) {
-                    const int c = 4 * (threadIdx.x + v * blockDim.x);
-                    const float4 f = spk_load4<float, VEC>(r + c, width - c);
-                    s.g[v] = make_float4(s.g[v].x + f.x, s.g[v].y + f.y, s.g[v].z + f.z, s.g[v].w + f.w);
+                for (int j = 0; j < kSlots; ++j) slot[j] = j0 + j < p.pair_top ? p.pair_slots[t * p.pair_top + j0 + j] : -1;
+#pragma unroll
+                for (int j = 0; j < kSlots; ++j) {
+                    const bool in = slot[j] >= 0 && slot[j] < p.pair_rows;
+                    if (slot[j] >= p.pair_rows && threadIdx.x == 0) spk_flag(p.status, SPK_STATUS_BAD_SLOT);
+                    const float* r = p.pairs + (in ? slot[j] : 0) * p.width;
+#pragma unroll
+                    for (int v = 0; v < V; ++v) {
+                        const int c = 4 * (threadIdx.x + v * blockDim.x);
+                        f[j].g[v] = spk_load4<float, VEC>(r + c, in ? width - c : 0);
+                    }
                 }
+#pragma unroll
+                for (int j = 0; j < kSlots; ++j)  // a row that is not there adds zeros
+#pragma unroll
+                    for (int v = 0; v < V; ++v)
+                        s.g[v] = make_float4(s.g[v].x + f[j].g[v].x, s.g[v].y + f[j].g[v].y, s.g[v].z + f[j].g[v].z, s.g[v].w + f[j].g[v].w);
             }
             const float m = p.pair_scale;
 #pragma unroll
@@ -79,8 +103,8 @@ rms_residual_kernel(const spk_rms_residual_args p) {
     }
     spk_block_sum<1>(q, part);
     const float inv = 1.0f / sqrtf(q[0] / static_cast<float>(width) + p.eps);
-    auto normed = [&](int v, int c, const float* w) {
-        const float4 f = spk_load4<float, VEC>(w + c, width - c);
+    auto normed = [&](int v, int c, const float* w, const SpkRow<V>& ahead) {
+        const float4 f = AHEAD ? ahead.g[v] : spk_load4<float, VEC>(w + c, width - c);
         return make_float4(y.g[v].x * inv * f.x, y.g[v].y * inv * f.y, y.g[v].z * inv * f.z, y.g[v].w * inv * f.w);
     };
     if (p.w1 != nullptr) {
@@ -88,7 +112,7 @@ rms_residual_kernel(const spk_rms_residual_args p) {
 #pragma unroll
         for (int v = 0; v < V; ++v) {
             const int c = 4 * (threadIdx.x + v * blockDim.x);
-            spk_store4<T, VEC>(o + c, normed(v, c, p.w1), width - c);
+            spk_store4<T, VEC>(o + c, normed(v, c, p.w1, w1), width - c);
         }
     }
     if (p.w2 == nullptr) return;
@@ -96,21 +120,25 @@ rms_residual_kernel(const spk_rms_residual_args p) {
 #pragma unroll
     for (int v = 0; v < V; ++v) {
         const int c = 4 * (threadIdx.x + v * blockDim.x);
-        const float4 f = normed(v, c, p.w2);
+        const float4 f = normed(v, c, p.w2, w2);
         if (p.out2_slots == nullptr) {
             spk_store4<T, VEC>(o2 + t * p.width + c, f, width - c);
             continue;
         }
-        for (int j = 0; j < p.out2_top; ++j) {
-            const int64_t slot = p.out2_slots[t * p.out2_top + j];
-            if (slot < 0) continue;
+        auto put = [&](int64_t slot) {
+            if (slot < 0) return;
             if (slot >= p.out2_rows) {
                 if (threadIdx.x == 0 && v == 0) spk_flag(p.status, SPK_STATUS_BAD_SLOT);
-                continue;
+                return;
             }
             if (!p.out2_tiled) spk_store4<T, VEC>(o2 + slot * p.width + c, f, width - c);
             else if (c < spk_operand_columns(width)) spk_store4<T, true>(o2 + spk_operand_at(p.out2_rows, slot, c), f, 4);
+        };
+        if (AHEAD) {
+#pragma unroll
+            for (int j = 0; j < kSlots; ++j) put(to[j]);
         }
+        for (int j = AHEAD ? kSlots : 0; j < p.out2_top; ++j) put(p.out2_slots[t * p.out2_top + j]);
     }
 }
 
@@ -121,15 +149,18 @@ int launch_boundary(const spk_rms_residual_args& p, cudaStream_t s) {
     if (threads == 0) return SPK_ERR_TOO_LARGE;
     const unsigned grid = static_cast<unsigned>(p.n);
     const bool vec = p.width % 4 == 0;
-#define SPK_RR(V_)                                                                      \
-    do {                                                                                \
-        if (vec) rms_residual_kernel<T, TD, V_, true><<<grid, threads, 0, s>>>(p);      \
-        else rms_residual_kernel<T, TD, V_, false><<<grid, threads, 0, s>>>(p);         \
+    const bool ahead = p.n <= 4 * 148;  // the rows of a decode batch, all of them on the chip at once
+#define SPK_RR(V_, AHEAD_)                                                                  \
+    do {                                                                                    \
+        if (vec) rms_residual_kernel<T, TD, V_, true, AHEAD_><<<grid, threads, 0, s>>>(p);  \
+        else rms_residual_kernel<T, TD, V_, false, AHEAD_><<<grid, threads, 0, s>>>(p);     \
     } while (0)
-    if (v == 1) SPK_RR(1);
-    else if (v == 2) SPK_RR(2);
-    else if (v == 4) SPK_RR(4);
-    else SPK_RR(8);
+    if (v == 1 && ahead) SPK_RR(1, true);
+    else if (v == 1) SPK_RR(1, false);
+    else if (v == 2 && ahead) SPK_RR(2, true);
+    else if (v == 2) SPK_RR(2, false);
+    else if (v == 4) SPK_RR(4, false);
+    else SPK_RR(8, false);
 #undef SPK_RR
     SPK_CHECK_LAUNCH();
     return SPK_OK;
