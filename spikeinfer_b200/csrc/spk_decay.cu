@@ -334,7 +334,8 @@ gated_norm_vec_kernel(const spk_gated_norm_args a) {
         wv[i] = spk_load4<float, true>(a.w + c, a.width - c);
     }
     if (a.partials != nullptr) {
-        const int len = live ? a.seq_lens[t] : 0;
+        const int keys = a.seq_lens[t];  // asked for beside the mark
+        const int len = live ? keys : 0;
         const int per = spk_split_keys(len, a.splits);
         const int valid = (len + per - 1) / per;
         const float* p = a.partials + t * a.splits * a.left_width;

@@ -42,7 +42,8 @@ sigmoid_decode_kernel(const spk_sigmoid_attn_args a) {
     const int g = blockIdx.y / blocks16, h0 = g * rep + (blockIdx.y % blocks16) * 16;
     const int nh = min(16, (g + 1) * rep - h0);
     const int row = blockIdx.z;
-    const int len = (a.active == nullptr || a.active[row] == 1) ? a.seq_lens[row] : 0;
+    const int keys = a.seq_lens[row];  // asked for beside the mark
+    const int len = (a.active == nullptr || a.active[row] == 1) ? keys : 0;
     if (len < 0 || len > a.max_blocks * a.block_size) {
         if (threadIdx.x == 0) spk_flag(a.status, SPK_STATUS_BAD_SEQ_LEN);
         spk_grid_wait();

@@ -144,6 +144,34 @@ def test_residual_norm_with_one_state_buffer(dev, dtype, portions, n, width):
 
 
 @pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("n, width", [(1, 896), (64, 896), (5, 45), (300, 512), (592, 896), (593, 896), (7, 1024), (6, 1028), (3, 2048)])
+def test_residual_norm_of_batch_rows_gives_the_bits_of_one_token_portions(dev, dtype, n, width):
+    """Batch rows on the chip at once take a form that reads everything ahead; portions of one token each take the general one.  The same rows, with
+    the shift (rows at position 0, rows that sit out, one buffer as prev and commit), without it, and with a second norm."""
+    g = torch.Generator(device=dev).manual_seed(n + width)
+    x, w, mix, prev0 = (torch.randn(s, generator=g, device=dev) for s in ((n, width), (width,), (width,), (n + 2, width)))
+    prev0[n:] = float("nan")
+    delta = torch.randn(n, width, generator=g, device=dev).to(dtype)
+    positions = torch.randint(0, 3, (n,), generator=g, device=dev)
+    active = (torch.rand(n, generator=g, device=dev) < 0.8).to(torch.int32)
+    prev0[:n][(positions == 0) | (active == 0)] = float("nan")  # not read
+    rows = torch.where(active == 1, torch.arange(n, device=dev), -1).to(torch.int32)
+    portions = dict(token_rows=rows, token_edges=torch.full((n,), 3, dtype=torch.int32, device=dev))
+    common = dict(eps=1e-5, delta=delta, weight=w, alpha=1.7)
+    for shift in (dict(mix=mix, positions=positions), dict(second_weight=mix), {}):
+        for same in (False, True):
+            results = []
+            for where in (dict(active=active), portions):
+                prev, xo, out = prev0.clone(), torch.empty(n, width, device=dev), torch.empty(n, width, device=dev, dtype=dtype)
+                commit = prev if same else torch.zeros_like(prev)
+                state = dict(commit=commit, **(dict(prev=prev) if "mix" in shift else {}))
+                dense.residual_norm(out, x=x, x_out=xo, **state, **shift, **where, **common)
+                results.append((out, xo, commit[active.bool().nonzero()[:, 0]]))
+            for a, b in zip(*results):
+                assert torch.equal(a, b) and torch.isfinite(a).all()
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("n, width", [(8 * 148, 128), (8 * 148, 512), (12 * 148, 516), (12 * 148, 1024), (13 * 148, 260), (14 * 148, 896), (16 * 148, 4),
                                       (16 * 148 + 5, 100), (24 * 148, 128), (24 * 148, 132), (24 * 148, 256), (24 * 148, 384), (24 * 148, 512), (200 * 148 - 1, 256)])
 def test_residual_norm_of_many_rows_gives_the_bits_of_few(dev, dtype, n, width):
