@@ -40,44 +40,59 @@ latent_prepare_kernel(const spk_latent_prepare_args a) {
     if (t >= a.n) return;
     const int part = static_cast<int>(item % parts);
     const SpkPageLayout lay = spk_latent_layout(a.block_size, a.rank_pad, a.rot_pad, a.tiled);
+    // A CTA per item (decode): the row stays in registers and is asked for, with the norm's weights, beside the slot; behind it they were three round
+    // trips to L2 one after the other (with the output's gates asked for ahead: whole Gotunex steps of one row 3590 -> 3570 us, of 64 rows 5950 -> 5925).
+    constexpr bool kHeld = WPI > 1;
+    const int width = part == 0 ? a.q_rank : a.rank;
+    const T* src = part == 0 ? static_cast<const T*>(a.cq) + t * a.ld : static_cast<const T*>(a.kv) + t * a.ld;
+    const float* w = part == 0 ? a.w_q : a.w_kv;
+    float4 x0 = make_float4(0.f, 0.f, 0.f, 0.f), m0 = x0;
+    if (kHeld && part < 2) {
+        x0 = spk_load4<T, VEC>(src + 4 * lane, width - 4 * lane);
+        m0 = spk_load4<float, VEC>(w + 4 * lane, width - 4 * lane);
+    }
+    const int64_t pos = part == 2 ? a.positions[t] : 0;
     T* page = nullptr;
     int r = 0;
     if (part > 0) {
-        const int64_t slot = a.slot_mapping[t], block = slot / a.block_size;
+        const int64_t slot = a.slot_mapping[t];
+        int64_t block;
+        if (static_cast<uint64_t>(slot) <= 0x7fffffffull) {  // a 64-bit division is a hundred instructions
+            const uint32_t b32 = static_cast<uint32_t>(slot) / static_cast<uint32_t>(a.block_size);
+            block = b32;
+            r = static_cast<int>(static_cast<uint32_t>(slot) - b32 * static_cast<uint32_t>(a.block_size));
+        } else {
+            block = slot / a.block_size;
+            r = static_cast<int>(slot % a.block_size);
+        }
         if (slot < 0 || block >= a.num_blocks) {
             if (lane == 0) spk_flag(a.status, SPK_STATUS_BAD_SLOT);
             return;
         }
-        r = static_cast<int>(slot % a.block_size);
         page = static_cast<T*>(a.pool) + spk_page_base(lay, block, 0);
     }
     if (part == 2) {
-        const T* src = static_cast<const T*>(a.kv) + t * a.ld + a.rank;
+        const T* rot = src + a.rank;
         const int half = a.rot_dim / 2;
-        const int64_t pos = a.positions[t];
         for (int i = lane; i < half; i += L) {
             const float2 f = rot_factor(a.rot_table, a.rot_positions, half, pos, i, a.status);
-            const float u = spk_to_float<T>(src[i]), v = spk_to_float<T>(src[i + half]);
+            const float u = spk_to_float<T>(rot[i]), v = spk_to_float<T>(rot[i + half]);
             page[spk_latent_channel(lay, r, a.rank_pad + i)] = spk_from_float<T>(u * f.x - v * f.y);
             page[spk_latent_channel(lay, r, a.rank_pad + i + half)] = spk_from_float<T>(v * f.x + u * f.y);
         }
         return;
     }
-    const int width = part == 0 ? a.q_rank : a.rank;
-    const T* src = part == 0 ? static_cast<const T*>(a.cq) + t * a.ld : static_cast<const T*>(a.kv) + t * a.ld;
-    const float* w = part == 0 ? a.w_q : a.w_kv;
     float ss[1] = {0.0f};
+    if (kHeld) ss[0] += (x0.x * x0.x + x0.y * x0.y) + (x0.z * x0.z + x0.w * x0.w);
 #pragma unroll 4
-    for (int c = 4 * lane; c < width; c += 4 * L) {
+    for (int c = 4 * lane + (kHeld ? 4 * L : 0); c < width; c += 4 * L) {
         const float4 x = spk_load4<T, VEC>(src + c, width - c);
         ss[0] += (x.x * x.x + x.y * x.y) + (x.z * x.z + x.w * x.w);
     }
     if (WPI == 1) ss[0] = spk_warp_sum(ss[0]);
     else spk_block_sum<1>(ss, sums);
     const float inv = 1.0f / sqrtf(ss[0] / static_cast<float>(width) + a.eps);
-#pragma unroll 4
-    for (int c = 4 * lane; c < width; c += 4 * L) {
-        const float4 x = spk_load4<T, VEC>(src + c, width - c), m = spk_load4<float, VEC>(w + c, width - c);
+    auto put = [&](int c, const float4& x, const float4& m) {
         const float4 y = make_float4(x.x * inv * m.x, x.y * inv * m.y, x.z * inv * m.z, x.w * inv * m.w);
         if (part == 0) {
             spk_store4<T, VEC>(static_cast<T*>(a.cq_out) + t * width + c, y, width - c);
@@ -89,7 +104,11 @@ latent_prepare_kernel(const spk_latent_prepare_args a) {
             for (int k = 0; k < 4; ++k)
                 if (c + k < width) page[spk_latent_channel(lay, r, c + k)] = spk_from_float<T>(e[k]);
         }
-    }
+    };
+    if (kHeld && 4 * lane < width) put(4 * lane, x0, m0);
+#pragma unroll 4
+    for (int c = 4 * lane + (kHeld ? 4 * L : 0); c < width; c += 4 * L)
+        put(c, spk_load4<T, VEC>(src + c, width - c), spk_load4<float, VEC>(w + c, width - c));
 }
 
 // ---- queries ---------------------------------------------------------------------------------------------------------
@@ -429,6 +448,17 @@ latent_out_mma_kernel(const spk_latent_out_args a, const bool vec_w) {
     };
     float4 head_sums[U];  // of the first range, on their way while the weights are made
     sums_of(head_sums, 0, 0);
+    const bool writes = kw == 0 && cw < used;
+    float gate[4][2];  // of the results this thread writes: asked for here, not behind the products
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int n = 0; n < 2; ++n) {
+            const int q = gid + 8 * (i >> 1), e = cw + n * 8 + tig * 2 + (i & 1);
+            gate[i][n] = writes && q < rows && e < live
+                             ? __bfloat162float(static_cast<const __nv_bfloat16*>(a.gate)[(t0 + q) * a.gate_stride + static_cast<int64_t>(h) * a.vdim + e0 + e])
+                             : 0.0f;
+        }
     range_weights(a, h, t0, rows, wts);
     __syncthreads();
     for (int g = 0; g < 2 * chunks; g += U) {
@@ -477,7 +507,7 @@ latent_out_mma_kernel(const spk_latent_out_args a, const bool vec_w) {
             for (int i = 0; i < 4; ++i) half[(cw + n * 8 + tig * 2 + (i & 1)) * 17 + gid + 8 * (i >> 1)] = acc[n][i];
     }
     __syncthreads();
-    if (kw > 0 || cw >= used) return;
+    if (!writes) return;
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
         const int q = gid + 8 * (i >> 1);
@@ -487,8 +517,7 @@ latent_out_mma_kernel(const spk_latent_out_args a, const bool vec_w) {
             const int e = cw + n * 8 + tig * 2 + (i & 1);
             if (e >= live) continue;
             const int64_t c = static_cast<int64_t>(h) * a.vdim + e0 + e;
-            const float g = __bfloat162float(static_cast<const __nv_bfloat16*>(a.gate)[(t0 + q) * a.gate_stride + c]);
-            static_cast<__nv_bfloat16*>(a.out)[(t0 + q) * a.out_stride + c] = __float2bfloat16_rn((acc[n][i] + half[e * 17 + q]) * sigmoid_fast(g));
+            static_cast<__nv_bfloat16*>(a.out)[(t0 + q) * a.out_stride + c] = __float2bfloat16_rn((acc[n][i] + half[e * 17 + q]) * sigmoid_fast(gate[i][n]));
         }
     }
 }
