@@ -21,7 +21,8 @@ constexpr float kLog2e = 1.4426950408889634f;
 
 template <int CK, int CV>
 struct Shape {
-    static constexpr int NS = CK + CV <= 2 ? 4 : 3;
+    static constexpr int NS = 3;  // heads of 64: 48 KB a CTA, so that four fit an SM: the key ranges of a batch are cut for 3 x 148 CTAs and more, and with
+                                  // four stages and three CTAs the 512 of 64 rows were two waves
     static constexpr int kStage = (CK + CV) * kStepTile;
     static constexpr int kRing = kWarps * NS * kStage;
     static constexpr int kBytes = kRing + 128 + kWarps * NS * 8;

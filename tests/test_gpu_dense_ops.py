@@ -617,6 +617,27 @@ def test_decay_attention_portions_and_steps(dev, shape, dtype):
     assert rel(state[2], S_x) < tol and torch.equal(state[0], kept) and torch.isnan(state[1]).all() and status.item() == 0
 
 
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("n, heads, dim, vdim", [(64, 14, 64, 64), (43, 14, 64, 64), (300, 2, 32, 128), (75, 8, 16, 64), (200, 3, 12, 256), (100, 6, 64, 32),
+                                                 (60, 10, 60, 64), (620, 1, 64, 4), (90, 7, 24, 40)])
+def test_decay_steps_of_many_rows_give_the_bits_of_few(dev, dtype, n, heads, dim, vdim):
+    """From some number of heads and rows on, small heads take a form of two slices per thread; parts of the batch below it the general one."""
+    g = torch.Generator(device=dev).manual_seed(n + dim)
+    q, k, v = torch.randn(n, heads * (2 * dim + vdim), generator=g, device=dev).to(dtype).split([heads * dim, heads * dim, heads * vdim], dim=1)
+    powers = dense.decay_powers([1 - 2.0 ** -(1 + i % 9) for i in range(heads)], dev)
+    active = (torch.rand(n, generator=g, device=dev) < 0.9).to(torch.int32)
+    state0 = torch.randn(n, heads, dim, vdim, generator=g, device=dev)
+    state0[active == 0] = float("nan")
+    whole, parts = state0.clone(), state0.clone()
+    for _ in range(2):
+        got = dense.decay_attention(q, k, v, whole, powers, active=active)
+        few = max(1, 500 // heads)
+        want = torch.cat([dense.decay_attention(q[i: i + few], k[i: i + few], v[i: i + few], parts[i: i + few], powers, active=active[i: i + few])
+                          for i in range(0, n, few)])
+        assert torch.equal(got, want) and torch.isfinite(got).all()
+        assert torch.equal(whole[active == 1], parts[active == 1]) and torch.isnan(whole[active == 0]).all()
+
+
 def test_decay_of_a_long_prompt_keeps_the_first_token(dev):
     """A decay next to one, keys that are zero except the first: the first token's value must still be there at the end."""
     for dtype in DTYPES:
