@@ -513,12 +513,15 @@ int launch_residual(const ResidualNormParams& p, void* out, cudaStream_t s) {
     const bool vec = p.width % 4 == 0;
     T* o = static_cast<T*>(out);
     // batch rows, all of them on the chip at once (prev may be commit: it is read first)
-    const bool ahead = p.ids == nullptr && p.token_rows == nullptr && p.token_edges == nullptr && p.per_cta == 1 && v <= 2 && p.n <= 4 * 148;
+    const bool ahead = p.ids == nullptr && p.token_rows == nullptr && p.token_edges == nullptr && p.per_cta == 1 && v <= 4 &&
+                       p.n <= (v <= 2 ? 4 : 2) * 148 && threads <= 256;
     if (ahead) {
         if (v == 1 && vec) residual_norm_ahead_kernel<T, TD, 1, true><<<grid, threads, 0, s>>>(p, o);
         else if (v == 1) residual_norm_ahead_kernel<T, TD, 1, false><<<grid, threads, 0, s>>>(p, o);
-        else if (vec) residual_norm_ahead_kernel<T, TD, 2, true><<<grid, threads, 0, s>>>(p, o);
-        else residual_norm_ahead_kernel<T, TD, 2, false><<<grid, threads, 0, s>>>(p, o);
+        else if (v == 2 && vec) residual_norm_ahead_kernel<T, TD, 2, true><<<grid, threads, 0, s>>>(p, o);
+        else if (v == 2) residual_norm_ahead_kernel<T, TD, 2, false><<<grid, threads, 0, s>>>(p, o);
+        else if (vec) residual_norm_ahead_kernel<T, TD, 4, true><<<grid, threads, 0, s>>>(p, o);
+        else residual_norm_ahead_kernel<T, TD, 4, false><<<grid, threads, 0, s>>>(p, o);
         SPK_CHECK_LAUNCH();
         return SPK_OK;
     }

@@ -144,7 +144,7 @@ def test_residual_norm_with_one_state_buffer(dev, dtype, portions, n, width):
 
 
 @pytest.mark.parametrize("dtype", DTYPES)
-@pytest.mark.parametrize("n, width", [(1, 896), (64, 896), (5, 45), (300, 512), (592, 896), (593, 896), (7, 1024), (6, 1028), (3, 2048)])
+@pytest.mark.parametrize("n, width", [(1, 896), (64, 896), (5, 45), (300, 512), (592, 896), (593, 896), (7, 1024), (6, 1028), (3, 2048), (40, 3584), (297, 3584), (2, 4099), (2, 8196)])
 def test_residual_norm_of_batch_rows_gives_the_bits_of_one_token_portions(dev, dtype, n, width):
     """Batch rows on the chip at once take a form that reads everything ahead; portions of one token each take the general one.  The same rows, with
     the shift (rows at position 0, rows that sit out, one buffer as prev and commit), without it, and with a second norm."""
