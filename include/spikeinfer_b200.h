@@ -639,6 +639,23 @@ typedef struct spk_rms_residual_args {
 } spk_rms_residual_args;
 int spk_rms_residual(const spk_rms_residual_args* args, void* stream);
 
+/* out[r, f] = sum_k x[r, k] w[f, k] for n <= 2 rows: bf16 x (row stride ld_x, a multiple of eight; 16-byte aligned) and w [features, k] (k a multiple of
+ * eight; 16-byte aligned), sums in 32 bits, out in out_dtype (32-bit or bf16) with row stride ld_out.  overlap != 0: the launch may be placed while the
+ * one ahead of it on the stream still runs; it reads only w before that has finished. */
+typedef struct spk_rows_linear_args {
+    const void* x;
+    const void* w;
+    void* out;
+    int64_t ld_x;
+    int64_t ld_out;
+    int64_t n;
+    int64_t k;
+    int64_t features;
+    int32_t out_dtype;
+    int32_t overlap;
+} spk_rows_linear_args;
+int spk_rows_linear(const spk_rows_linear_args* args, void* stream);
+
 /* out[t, c] = gelu(z[t, c]), the tanh form; out has row stride out_stride, z is contiguous [n, width]. */
 int spk_gelu_tanh(const void* z, void* out, int64_t out_stride, int64_t n, int64_t width, int dtype, void* stream);
 

@@ -201,6 +201,12 @@ class DeltaArgs(Structure):
                        "i n_chunks n_portions heads kv_heads dim vdim taps dtype; f eps _pad; p status")
 
 
+class RowsLinearArgs(Structure):
+    """Mirror of ``spk_rows_linear_args``."""
+
+    _fields_ = _fields("p x w out; l ld_x ld_out n k features; i out_dtype overlap")
+
+
 class SpikePortion(Structure):
     """Mirror of ``spk_spike_portion``."""
 
@@ -287,6 +293,7 @@ SIGNATURES = {
     "spk_decay_attn_chunks": (c_int, [POINTER(DecayAttnArgs), c_void_p]),
     "spk_gated_norm": (c_int, [POINTER(GatedNormArgs), c_void_p]),
     "spk_rms_residual": (c_int, [POINTER(RmsResidualArgs), c_void_p]),
+    "spk_rows_linear": (c_int, [POINTER(RowsLinearArgs), c_void_p]),
     "spk_gelu_tanh": (c_int, [c_void_p, c_void_p, c_int64, c_int64, c_int64, c_int, c_void_p]),
     "spk_expert_route": (c_int, [POINTER(ExpertRouteArgs), c_void_p]),
     "spk_expert_rows": (c_int64, [c_int64, c_int, c_int]),

@@ -29,6 +29,7 @@ delta_step_kernel(const spk_delta_args a) {
     extern __shared__ __align__(128) float sm[];
     __shared__ float part[3 * 32];
     __shared__ uint64_t arrived;
+    spk_grid_release();
     const int h = blockIdx.x;
     const int64_t row = blockIdx.y;
     const int dim = a.dim, vdim = a.vdim, rep = a.heads / a.kv_heads, g = h / rep;

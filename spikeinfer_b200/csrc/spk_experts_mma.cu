@@ -472,11 +472,11 @@ int dispatch(const spk_experts_args& a, cudaStream_t s) {
     if (mean > 96) return launch<256, GATED, 1>(a, blocks, ktiles, s);
     if (mean > 40) return launch<128, GATED, 1>(a, blocks, ktiles, s);
     if (mean > 16) return launch<64, GATED, 1>(a, blocks, ktiles, s);
-    // Blocks streamed by the second product: with fewer than 17 (a step of one user with two experts has 8) two CTAs share each.  One row of 16 experts
-    // of 896 x 1216 beside the mixer's launches: whole step 4107 us without, 3834 with two parts; more parts take SMs from the mixer.
-    if constexpr (!GATED) {
-        if (blocks * (a.pairs < a.experts ? a.pairs : a.experts) <= 16 && ktiles >= 2) return launch<32, GATED, 2>(a, blocks, ktiles, s);
-    }
+    // Up to 40 blocks (16 experts of 896 x 1216, two per token: the gated product of one or two users, the second one of up to five) four CTAs share
+    // each: a CTA streams 30 to 60 GB/s whatever its ring holds.  Whole steps, the blocks of both whole / two parts / four / eight and four: one user
+    // 3310 us (the second product in two parts already), 3195, 3078, 3090; two users 3510, 3370, 3255, 3415; four (the second product alone) 3830, 3675,
+    // 3680, 3690.  With library products in the mixer, which want whole SMs, four parts were slower than two (4260 against 4103 us).
+    if (blocks * (a.pairs < a.experts ? a.pairs : a.experts) <= 40 && ktiles >= 4) return launch<32, GATED, 4>(a, blocks, ktiles, s);
     return launch_stream<GATED>(a, blocks, ktiles, s);
 }
 

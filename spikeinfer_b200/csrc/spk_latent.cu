@@ -33,6 +33,7 @@ latent_prepare_kernel(const spk_latent_prepare_args a) {
     constexpr int L = 32 * WPI;
     static_assert(WPI == 1 || WPI == kWarps, "a warp or a CTA per item");
     __shared__ float sums[32];
+    spk_grid_release();
     const int lane = threadIdx.x % L;
     const int parts = a.kv != nullptr ? 3 : 1;
     const int64_t item = static_cast<int64_t>(blockIdx.x) * (kWarps / WPI) + threadIdx.x / L;
@@ -435,6 +436,7 @@ latent_out_mma_kernel(const spk_latent_out_args a, const bool vec_w) {
         cp_async_commit();
     };
     for (int c = 0; c < kOutStages - 1; ++c) fetch(c);
+    spk_grid_release();
     spk_grid_wait();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, gid = lane >> 2, tig = lane & 3, m = lane >> 3, mr = lane & 7;
     const int cw = (warp & 3) * 16, kw = (warp >> 2) * 64;

@@ -25,7 +25,7 @@ from . import _lib
 from .attention import AttentionMetadata
 from .engine.kv_state_cache import LatentSpec, LayerCacheSpec, PagedKVStateCache
 from .kernels.delta import delta_rule
-from .kernels.dense import gelu_tanh, rms_residual
+from .kernels.dense import gelu_tanh, rms_residual, rows_linear, takes_few_rows
 from .kernels.experts import ExpertRouter, ExpertWeights, experts_forward
 from .kernels.latent import latent_attention, latent_prefill, latent_prepare, latent_query, spelled_out_weights
 from .rotary import RotaryConfig
@@ -172,7 +172,7 @@ class _LatentAttention:
         own = {} if c.kv_from is not None else dict(kv=z[:, self.at["dkv"]], w_kv=self.kv_norm, pool=pool, rot_table=rot, positions=positions,
                                                     slot_mapping=meta.slot_mapping)
         cq = latent_prepare(z[:, self.at["dq"]], self.q_norm, eps=model.config.eps, status=meta.status, **own)
-        q, gate = model._matmul(cq, self.w_uq), z[:, self.at["g"]]
+        q, gate = model._matmul(cq, self.w_uq, behind=True), z[:, self.at["g"]]
         common = dict(vdim=c.vdim, scale=c.scale, status=meta.status)
         if meta.num_prefills:
             latent_prefill(q, pool, meta.row_tables, self.w_uk, self.w_uv, self.w_kv, self.sink, gate, out, rot_table=rot, positions=positions,
@@ -212,7 +212,7 @@ class _ChannelDelta:
     def forward(self, model: "GotunexModel", h, out, positions, cache, meta: AttentionMetadata) -> None:
         c = self.cfg
         z = model._matmul(h, self.w_in)
-        low = model._matmul(z[:, self.low], self.w_low)
+        low = model._matmul(z[:, self.low], self.w_low, behind=True)
         where = dict(plan=meta.prefill_plan()) if meta.num_prefills else dict(positions=positions, active=meta.row_active)
         delta_rule(z[:, self.at["q"]], z[:, self.at["k"]], z[:, self.at["v"]], z[:, self.at["b"]], low[:, : c.heads * c.dim], low[:, self.gate_at:],
                    conv=self.conv, a_log=self.a_log, dt_bias=self.dt_bias, norm=self.norm, state=cache.states["delta"],
@@ -283,12 +283,16 @@ class GotunexModel:
         """Engine hook: pages of latents and rotated keys, and per row the delta states and the convolutions' last inputs."""
         return PagedKVStateCache([layer.mixer.cache_spec() for layer in self.layers], num_blocks, block_size, max_rows, self.dtype, self.device)
 
-    def _matmul(self, x: torch.Tensor, w: torch.Tensor) -> torch.Tensor:
-        """``x w^T`` in the model dtype."""
+    def _matmul(self, x: torch.Tensor, w: torch.Tensor, behind: bool = False) -> torch.Tensor:
+        """``x w^T`` in the model dtype.  ``behind``: the launch ahead is one of this package's, which lets the next one be placed early."""
+        if takes_few_rows(x, w):
+            return rows_linear(x, w, x.dtype, behind)
         return F.linear(x, w)
 
-    def _matmul_f32(self, x: torch.Tensor, w: torch.Tensor) -> torch.Tensor:
+    def _matmul_f32(self, x: torch.Tensor, w: torch.Tensor, behind: bool = False) -> torch.Tensor:
         """``x w^T`` with the 32-bit sums as they are."""
+        if takes_few_rows(x, w) and w.shape[0] <= 16384:  # the head's weights take the library's time
+            return rows_linear(x, w, torch.float32, behind)
         if x.dtype == torch.float32:
             return F.linear(x, w)
         return torch.mm(x, w.t(), out_dtype=torch.float32)
@@ -331,7 +335,7 @@ class GotunexModel:
             with torch.cuda.stream(self._side if beside else main):
                 L.mixer.forward(self, h, both[:, :mixed], positions, caches[i], meta)
                 if L.up is None:
-                    delta = self._matmul_f32(both, L.w_out)
+                    delta = self._matmul_f32(both, L.w_out, behind=True)
             if L.up is not None:
                 gelu_tanh(self._matmul(hand["out2"], L.up), both[:, mixed:])
             elif L.experts is not None:

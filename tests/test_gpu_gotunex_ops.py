@@ -91,6 +91,36 @@ def test_gelu(dev, dtype):
     assert err < (2e-6 if dtype == F32 else 4e-2)
 
 
+# ---- products of a few rows ------------------------------------------------------------------------------------------
+@pytest.mark.parametrize("n", [1, 2])
+@pytest.mark.parametrize("k, features", [(8, 1), (64, 7), (264, 9), (384, 1344), (896, 2832), (1016, 64), (1024, 2369), (1032, 40), (2048, 17)])
+def test_rows_linear(dev, n, k, features):
+    """Pieces of a warp's lanes that are missing, one and two passes over the columns, one and two features a warp, features beyond the last warp; x a column
+    range of a wider matrix whose other columns are NaN; one launch directly behind the one that makes its x."""
+    g = torch.Generator(device=dev).manual_seed(n * k + features)
+    wide = torch.full((n, k + 16), float("nan"), device=dev, dtype=BF)
+    wide[:, 8: 8 + k] = torch.randn(n, k, generator=g, device=dev).to(BF)
+    x, w = wide[:, 8: 8 + k], torch.randn(features, k, generator=g, device=dev).to(BF)
+    want, size = x.double() @ w.double().T, x.double().abs() @ w.double().abs().T
+    assert kn.takes_few_rows(x, w)
+    got = kn.rows_linear(x, w, F32)
+    # products are exact in 32 bits; at most k / 32 + 5 additions in a chain (2 per packed pair at the end), each half an ulp of a partial sum
+    assert bool(((got.double() - want).abs() <= (k / 32 + 8) * 2.0 ** -24 * size).all())
+    assert torch.equal(kn.rows_linear(x, w, BF), got.to(BF))
+    if features % 8 == 0:
+        mid = kn.rows_linear(x, w, BF)[:, : min(features, 2048)]
+        w2 = torch.randn(24, mid.shape[1], generator=g, device=dev).to(BF)
+        assert torch.equal(kn.rows_linear(kn.rows_linear(x, w, BF)[:, : min(features, 2048)], w2, F32, overlap_previous=True), kn.rows_linear(mid, w2, F32))
+
+
+def test_rows_linear_refuses_what_it_does_not_take(dev):
+    w = torch.zeros(4, 64, device=dev, dtype=BF)
+    for x in (torch.zeros(3, 64, device=dev, dtype=BF), torch.zeros(2, 64, device=dev), torch.zeros(2, 128, device=dev, dtype=BF)[:, 1:65],
+              torch.zeros(2, 56, device=dev, dtype=BF)):
+        with pytest.raises(ValueError):
+            kn.rows_linear(x, w, F32)
+
+
 # ---- experts ---------------------------------------------------------------------------------------------------------
 def expert_case(dev, dtype, n, width, experts, top, ff, seed, ids=None, vocab=61):
     g = gen(seed)
@@ -131,6 +161,18 @@ def test_experts(dev, status, n, width, experts, top, ff, dtype):
     got = out.cpu().double()[slots.long()].mean(1)
     want = go.table_experts(x, ids.tolist(), go.as_float(w), "", cfg)
     assert rel(got, want) < (3e-6 if dtype == F32 else 8e-3)
+
+
+@pytest.mark.parametrize("n,width,experts,top,ff", [(2, 896, 16, 2, 1216), (5, 896, 16, 2, 1216), (1, 256, 9, 1, 200), (1, 200, 9, 1, 256), (20, 320, 1, 1, 640)])
+def test_experts_of_few_blocks_in_four_parts(dev, status, n, width, experts, top, ff):
+    """Both products, one of them, or neither in four parts of k; four tiles of k and more, unequal parts, one to 20 rows; twice the same bits."""
+    w, weights, ids, x, cfg = expert_case(dev, BF, n, width, experts, top, ff, n + ff)
+    x = go.rms(x.double(), 0.0)
+    route, out = run_experts(dev, status, weights, ids, x)
+    want = go.table_experts(x, ids.tolist(), go.as_float(w), "", cfg)
+    assert rel(out[route.slots.long()].mean(1), want) < 8e-3 and status.item() == 0
+    again, out2 = run_experts(dev, status, weights, ids, x)
+    assert torch.equal(out2[again.slots.long()], out[route.slots.long()])
 
 
 @pytest.mark.parametrize("n,width,experts,top,ff", [(60, 130, 40, 2, 1300), (24, 1024, 30, 4, 64), (100, 448, 8, 1, 384), (90, 64, 96, 2, 640),
