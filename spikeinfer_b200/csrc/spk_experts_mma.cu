@@ -477,6 +477,10 @@ int dispatch(const spk_experts_args& a, cudaStream_t s) {
     // 3310 us (the second product in two parts already), 3195, 3078, 3090; two users 3510, 3370, 3255, 3415; four (the second product alone) 3830, 3675,
     // 3680, 3690.  With library products in the mixer, which want whole SMs, four parts were slower than two (4260 against 4103 us).
     if (blocks * (a.pairs < a.experts ? a.pairs : a.experts) <= 40 && ktiles >= 4) return launch<32, GATED, 4>(a, blocks, ktiles, s);
+    // Weights of more than 256 MB outlast the mixer beside them: a CTA per block, two to an SM, takes all of HBM's rate (16 experts of 3584 x 4736, 64 rows,
+    // both products: 243 us against 291 by the streaming form's CTAs).
+    const int64_t expected = static_cast<int64_t>(blocks) * (a.pairs < a.experts ? a.pairs : a.experts);
+    if (expected * ktiles * (2 * kTileW) > (256ll << 20)) return launch<32, GATED, 1>(a, blocks, ktiles, s);
     return launch_stream<GATED>(a, blocks, ktiles, s);
 }
 
