@@ -235,3 +235,43 @@ def test_qkv_sites_refuse_what_the_general_description_refuses(monkeypatch):
                 call()
             errors.append(type(e.value))
         assert errors[0] is errors[1], change
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("pools", ["slots", "pages", "strided"])
+def test_a_prefill_call_is_described_field_by_field(monkeypatch, dtype, pools):
+    """:func:`paged_spike_attn_prefill` packs its arguments and portions by position: every field holds what its name says, no two of one type alike."""
+    calls = []
+
+    class Library:
+        def spk_spike_prefill(self, args, portions, count, stream):
+            calls.append(({n: getattr(args._obj, n) for n, *_ in _lib.SpikePrefillArgs._fields_},
+                          [{n: getattr(portions[i], n) for n, *_ in _lib.SpikePortion._fields_} for i in range(count)]))
+            return 0
+
+    monkeypatch.setattr(_lib, "require_cuda", lambda *a: None)
+    monkeypatch.setattr(_lib, "load", lambda: Library())
+    monkeypatch.setattr(_lib, "on_device", lambda device, fn, *a: fn(*a, 0))
+    T, tokens, heads, kv_heads, dim, page = 3, 40, 10, 5, 64, 16
+    word = lambda *shape: torch.zeros(shape, dtype=torch.int32)
+    if pools == "slots":
+        k, v = word(T, kv_heads, 8 * page, 2), word(T, kv_heads, 11 * page, 2)
+    elif pools == "pages":
+        k, v = word(9, T, kv_heads, page, 2).permute(1, 2, 0, 3, 4), word(7, T, kv_heads, page, 2).permute(1, 2, 0, 3, 4)
+    else:
+        k, v = word(T, kv_heads, 8 * page, 6)[..., :2], word(12 * page, T, kv_heads, 2).permute(1, 2, 0, 3)
+    q, out = word(T, tokens + 4, heads + 1, 3)[:, 2: 2 + tokens, 1:, :2], torch.zeros(T, tokens, heads, 2 * dim, dtype=dtype)[..., :dim]
+    tables, status = [word(2), word(7)[1:4]], word(1)
+    kernels.paged_spike_attn_prefill(q, k, v, tables, [0, 21], [13, 17], [19, 23], out, head_dim=dim, block_size=page, num_q_heads=heads,
+                                     num_kv_heads=kv_heads, status=status)
+    (args, portions), = calls
+    pool = lambda c: (c.stride(0), c.stride(1), *((c.stride(2) * page, c.stride(2)) if c.ndim == 4 else (c.stride(2), c.stride(3))))
+    blocks = min(c.shape[2] // (page if c.ndim == 4 else 1) for c in (k, v))
+    (sq_t, sq_tok, sq_h, _), (so_t, so_tok, so_h, _), (sk_t, sk_h, sk_blk, sk_slot), (sv_t, sv_h, sv_blk, sv_slot) = q.stride(), out.stride(), pool(k), pool(v)
+    assert args.pop("scale") == 0.125
+    assert args == dict(q_packed=q.data_ptr(), sq_t=sq_t, sq_tok=sq_tok, sq_h=sq_h, k_pool=k.data_ptr(), sk_t=sk_t, sk_h=sk_h, sk_blk=sk_blk, sk_slot=sk_slot,
+                        v_pool=v.data_ptr(), sv_t=sv_t, sv_h=sv_h, sv_blk=sv_blk, sv_slot=sv_slot, out=out.data_ptr(), so_t=so_t, so_tok=so_tok, so_h=so_h,
+                        n_tok=tokens, num_blocks=blocks, T=T, num_q_heads=heads, num_kv_heads=kv_heads, head_dim=dim, block_size=page,
+                        dtype=_lib.dtype_code(dtype), _pad=0.0, status=status.data_ptr())
+    assert portions == [dict(table=tables[0].data_ptr(), start=0, tokens=13, context=19, table_len=2),
+                        dict(table=tables[1].data_ptr(), start=21, tokens=17, context=23, table_len=3)]
