@@ -427,8 +427,9 @@ gated_norm_kernel(const spk_gated_norm_args a) {
 }
 
 // The same with four columns per access: at most 4 * kThreads * V columns, every operand aligned to four elements.
-template <typename T, int V>
-__global__ void __launch_bounds__(kThreads, V == 4 ? 4 : 1)  // 4096 rows of 3584: two / three / four CTAs per SM 44.7 / 43.5 / 37.1 us
+// MINB: CTAs per SM it is built for, 0 as the compiler likes: four with four groups a thread spill, and pay off where rows wait for HBM.
+template <typename T, int V, int MINB = 0>
+__global__ void __launch_bounds__(kThreads, MINB)
 gated_norm_vec_kernel(const spk_gated_norm_args a) {
     __shared__ float part[32];
     const int64_t t = blockIdx.x;
@@ -476,8 +477,10 @@ gated_norm_vec_kernel(const spk_gated_norm_args a) {
 }
 
 // Many rows of up to 128 G columns and no partial sums: a warp per row.
+// Four CTAs per SM: a row's loads are the time.  Without and with the bound, us of repeated calls: 4096 rows of 640 8.7 / 6.8, of 768 9.0 / 6.9; 8192 rows of 896 16.2 / 12.1,
+// of 1024 18.0 / 16.4; fp32 768 12.1 / 11.8, 896 18.0 / 14.5, 1024 22.5 / 21.6: the spills of six groups a lane and more (20 to 76 bytes) cost less than it gains.
 template <typename T, int G>
-__global__ void __launch_bounds__(kThreads, 4)  // a row's loads are the time: 8192 rows of 896, two / three / four CTAs per SM 21.7 / 19.1 / 16.5 us
+__global__ void __launch_bounds__(kThreads, 4)
 gated_norm_rows_kernel(const spk_gated_norm_args a) {
     const int lane = threadIdx.x & 31;
     const int64_t t = static_cast<int64_t>(blockIdx.x) * (kThreads / 32) + (threadIdx.x >> 5);
@@ -535,7 +538,14 @@ int launch_gated(const spk_gated_norm_args& a, cudaStream_t s) {
         const int threads = groups <= 128 && a.partials == nullptr ? 128 : kThreads;
         const int v = (groups + threads - 1) / threads;
         if (v <= 1) gated_norm_vec_kernel<T, 1><<<grid, threads, 0, s>>>(a);
+        // Two groups a thread: 78 registers (a bound of one CTA) for the loads of a batch row's partial sums, 64 otherwise.  Without / with that bound, us: 2048 columns beside eight
+        // partial sums, 64 rows 5.2 / 4.0; no partial sums, 592 rows 3.9 / 4.6, 8192 35.6 / 43.1.
+        else if (v <= 2 && a.partials != nullptr) gated_norm_vec_kernel<T, 2, 1><<<grid, threads, 0, s>>>(a);
         else if (v <= 2) gated_norm_vec_kernel<T, 2><<<grid, threads, 0, s>>>(a);
+        // Four CTAs per SM (64 registers and spills) from sixteen rows per SM on.  Without / with them, rows of 3584, us of repeated calls on one set of buffers: 64 rows
+        // 3.3 / 3.9 (beside partial sums 6.7 / 9.2), 592 6.2 / 7.1, 2048 18.1 / 19.4, 2368 21.3 / 21.4, 2800 26.6 / 25.0, 4096 42.9 / 36.2; six sets in turn: 2048 23.2 / 20.9,
+        // 2368 26.3 / 23.2, 4096 43.0 / 36.2.  fp32 2368 26.6 / 26.9, 4096 45.2 / 43.0.
+        else if (a.n >= 16 * 148) gated_norm_vec_kernel<T, 4, 4><<<grid, threads, 0, s>>>(a);
         else gated_norm_vec_kernel<T, 4><<<grid, threads, 0, s>>>(a);
     }
     SPK_CHECK_LAUNCH();

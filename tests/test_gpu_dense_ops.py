@@ -239,6 +239,27 @@ def test_gated_norm_of_many_rows_gives_the_bits_of_few(dev, dtype, n, width):
 
 
 @pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("width", [2052, 3584, 4096])
+def test_gated_norm_of_many_wide_rows_gives_the_bits_of_few(dev, dtype, width):
+    """From 16 rows per SM on, rows of more than 2048 columns take a form with more CTAs per SM."""
+    n = 16 * 148
+    g = torch.Generator(device=dev).manual_seed(width)
+    x, w = torch.randn(n, width, generator=g, device=dev), 1 + 0.3 * torch.randn(width, generator=g, device=dev)
+    z = (3 * torch.randn(n, 2 * width, generator=g, device=dev)).to(dtype)
+    parts, lens = torch.randn(n, 3, 8, generator=g, device=dev), torch.randint(1, 200, (n,), generator=g, device=dev).to(torch.int32)
+    active = (torch.rand(n, generator=g, device=dev) < 0.9).to(torch.int32)
+
+    def run(lo, hi, **partials):
+        out = torch.full((hi - lo, 8 + width), 7.0, dtype=dtype, device=dev)
+        dense.gated_norm(x[lo:hi], w, z[lo:hi, width:], out, 8, eps=1e-3, scale=0.5, active=active[lo:hi], **partials)
+        return out
+    for with_parts in (False, True):
+        more = lambda lo, hi: dict(partials=parts[lo:hi], seq_lens=lens[lo:hi], left_scale=0.7) if with_parts else {}
+        got = run(0, n, **more(0, n))
+        assert torch.equal(got[: n - 1], run(0, n - 1, **more(0, n - 1))) and torch.equal(got[n - 1:], run(n - 1, n, **more(n - 1, n)))
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
 def test_residual_norm_embedding_and_decode_rows(dev, dtype):
     g = gen(5)
     vocab, width, n = 50, 40, 6
