@@ -592,7 +592,11 @@ int launch_step(const spk_decay_attn_args& a, cudaStream_t s) {
 
 int launch_scan(const spk_decay_attn_args& a, cudaStream_t s) {
     const int64_t per = static_cast<int64_t>(a.heads) * a.dim * a.vdim;
-    if (a.dim * static_cast<int64_t>(a.vdim) % 4 == 0 && a.state_stride % 4 == 0 && reinterpret_cast<uintptr_t>(a.state) % 16 == 0 &&
+    // Four elements a thread where one would be two CTAs per SM and more, or a sequence has two chunks at most: a long chain wants its loads spread over the SMs.  One / four,
+    // us of the whole recurrence: 2 heads of 64, 1 x 4096 tokens 18.9 / 23.7; 8 heads, 1 x 4096 26.7 / 28.9, 2 x 2048 25.6 / 25.8, 3 x 1000 24.6 / 23.8; 14 heads, 1 x 1024 17.7 / 18.3,
+    // 1 x 100 12.5 / 12.1, 3 x 1000 40.3 / 37.8.
+    const bool wide = (per + kThreads - 1) / kThreads * a.n_seqs >= 2 * 148 || a.n_chunks <= 2 * a.n_seqs;
+    if (wide && a.dim * static_cast<int64_t>(a.vdim) % 4 == 0 && a.state_stride % 4 == 0 && reinterpret_cast<uintptr_t>(a.state) % 16 == 0 &&
         reinterpret_cast<uintptr_t>(a.workspace) % 16 == 0 && per < (1LL << 31)) {
         decay_scan_wide_kernel<<<dim3(static_cast<unsigned>((per / 4 + kThreads - 1) / kThreads), a.n_seqs), kThreads, 0, s>>>(a);
         SPK_CHECK_LAUNCH();
