@@ -14,7 +14,9 @@ using namespace spk_tc;
 // AHEAD: everything that does not depend on the row's sums is asked for at once.  A decode step's row is a chain of round trips to L2, and the
 // norms' weights and the destinations behind the mean square, and expert rows one after the other behind their slots, were six of them: whole
 // Gotunex steps of one, four, 30 and 64 rows 3795 -> 3590, 4115 -> 3925, 5060 -> 4928, 6110 -> 5950 us (with the loads of the delta rule's step moved up in
-// the same way).  Prompt batches hide the trips behind other rows and want the registers (72 against 40): 0.6 % of a prompt pass slower with it.
+// the same way).  Prompt batches hide the trips behind other rows and want the registers: theirs goes over the slots one by one, without a
+// branch around a slot's loads (GATHER) only where two groups a thread of a width that is no multiple of four spill less so.  Branch / none, us: 3584 columns, two experts, 2048 rows
+// 44.5 / 50.0, 8192 149 / 170; 4102 columns, 8192 rows 332 / 577; 1022 columns, 600 rows 7.0 / 6.3, 8192 56.8 / 53.1, without experts 44.3 / 40.6, 2048 13.1 / 14.3.
 template <typename T, typename TD, int V, bool VEC, bool AHEAD>
 __global__ void __launch_bounds__(AHEAD ? 256 : 1024)  // spk_row_shape: up to two groups a thread are at most 256 threads
 rms_residual_kernel(const spk_rms_residual_args p) {
@@ -31,6 +33,7 @@ rms_residual_kernel(const spk_rms_residual_args p) {
         }
     }
     constexpr int kSlots = AHEAD ? 2 : 1;
+    constexpr bool GATHER = AHEAD || (V == 2 && !VEC);
     int64_t to[kSlots];
 #pragma unroll
     for (int j = 0; j < kSlots; ++j) to[j] = AHEAD && p.w2 != nullptr && p.out2_slots != nullptr && j < p.out2_top ? p.out2_slots[t * p.out2_top + j] : -1;
@@ -66,27 +69,45 @@ rms_residual_kernel(const spk_rms_residual_args p) {
             SpkRow<V> s;
 #pragma unroll
             for (int v = 0; v < V; ++v) s.g[v] = make_float4(0.f, 0.f, 0.f, 0.f);
-            for (int j0 = 0; j0 < p.pair_top; j0 += kSlots) {
-                int64_t slot[kSlots];
-                SpkRow<V> f[kSlots];
+            if constexpr (GATHER) {
+                for (int j0 = 0; j0 < p.pair_top; j0 += kSlots) {
+                    int64_t slot[kSlots];
+                    SpkRow<V> f[kSlots];
 #pragma unroll
-                for (int j = 0; j < kSlots; ++j) slot[j] = j0 + j < p.pair_top ? p.pair_slots[t * p.pair_top + j0 + j] : -1;
+                    for (int j = 0; j < kSlots; ++j) slot[j] = j0 + j < p.pair_top ? p.pair_slots[t * p.pair_top + j0 + j] : -1;
 #pragma unroll
-                for (int j = 0; j < kSlots; ++j) {
-                    const bool in = slot[j] >= 0 && slot[j] < p.pair_rows;
-                    if (slot[j] >= p.pair_rows && threadIdx.x == 0) spk_flag(p.status, SPK_STATUS_BAD_SLOT);
-                    const float* r = p.pairs + (in ? slot[j] : 0) * p.width;
+                    for (int j = 0; j < kSlots; ++j) {
+                        const bool in = slot[j] >= 0 && slot[j] < p.pair_rows;
+                        if (slot[j] >= p.pair_rows && threadIdx.x == 0) spk_flag(p.status, SPK_STATUS_BAD_SLOT);
+                        const float* r = p.pairs + (in ? slot[j] : 0) * p.width;
+#pragma unroll
+                        for (int v = 0; v < V; ++v) {
+                            const int c = 4 * (threadIdx.x + v * blockDim.x);
+                            f[j].g[v] = spk_load4<float, VEC>(r + c, in ? width - c : 0);
+                        }
+                    }
+#pragma unroll
+                    for (int j = 0; j < kSlots; ++j)  // a row that is not there adds zeros
+#pragma unroll
+                        for (int v = 0; v < V; ++v)
+                            s.g[v] = make_float4(s.g[v].x + f[j].g[v].x, s.g[v].y + f[j].g[v].y, s.g[v].z + f[j].g[v].z, s.g[v].w + f[j].g[v].w);
+                }
+            } else {
+                for (int j = 0; j < p.pair_top; ++j) {
+                    const int64_t slot = p.pair_slots[t * p.pair_top + j];
+                    if (slot < 0) continue;
+                    if (slot >= p.pair_rows) {
+                        if (threadIdx.x == 0) spk_flag(p.status, SPK_STATUS_BAD_SLOT);
+                        continue;
+                    }
+                    const float* r = p.pairs + slot * p.width;
 #pragma unroll
                     for (int v = 0; v < V; ++v) {
                         const int c = 4 * (threadIdx.x + v * blockDim.x);
-                        f[j].g[v] = spk_load4<float, VEC>(r + c, in ? width - c : 0);
+                        const float4 f = spk_load4<float, VEC>(r + c, width - c);
+                        s.g[v] = make_float4(s.g[v].x + f.x, s.g[v].y + f.y, s.g[v].z + f.z, s.g[v].w + f.w);
                     }
                 }
-#pragma unroll
-                for (int j = 0; j < kSlots; ++j)  // a row that is not there adds zeros
-#pragma unroll
-                    for (int v = 0; v < V; ++v)
-                        s.g[v] = make_float4(s.g[v].x + f[j].g[v].x, s.g[v].y + f[j].g[v].y, s.g[v].z + f[j].g[v].z, s.g[v].w + f[j].g[v].w);
             }
             const float m = p.pair_scale;
 #pragma unroll
@@ -125,20 +146,33 @@ rms_residual_kernel(const spk_rms_residual_args p) {
             spk_store4<T, VEC>(o2 + t * p.width + c, f, width - c);
             continue;
         }
-        auto put = [&](int64_t slot) {
-            if (slot < 0) return;
-            if (slot >= p.out2_rows) {
-                if (threadIdx.x == 0 && v == 0) spk_flag(p.status, SPK_STATUS_BAD_SLOT);
-                return;
-            }
-            if (!p.out2_tiled) spk_store4<T, VEC>(o2 + slot * p.width + c, f, width - c);
-            else if (c < spk_operand_columns(width)) spk_store4<T, true>(o2 + spk_operand_at(p.out2_rows, slot, c), f, 4);
-        };
-        if (AHEAD) {
+        if constexpr (GATHER) {
+            auto put = [&](int64_t slot) {
+                if (slot < 0) return;
+                if (slot >= p.out2_rows) {
+                    if (threadIdx.x == 0 && v == 0) spk_flag(p.status, SPK_STATUS_BAD_SLOT);
+                    return;
+                }
+                if (!p.out2_tiled) spk_store4<T, VEC>(o2 + slot * p.width + c, f, width - c);
+                else if (c < spk_operand_columns(width)) spk_store4<T, true>(o2 + spk_operand_at(p.out2_rows, slot, c), f, 4);
+            };
+            if (AHEAD) {
 #pragma unroll
-            for (int j = 0; j < kSlots; ++j) put(to[j]);
+                for (int j = 0; j < kSlots; ++j) put(to[j]);
+            }
+            for (int j = AHEAD ? kSlots : 0; j < p.out2_top; ++j) put(p.out2_slots[t * p.out2_top + j]);
+        } else {
+            for (int j = 0; j < p.out2_top; ++j) {
+                const int64_t slot = p.out2_slots[t * p.out2_top + j];
+                if (slot < 0) continue;
+                if (slot >= p.out2_rows) {
+                    if (threadIdx.x == 0 && v == 0) spk_flag(p.status, SPK_STATUS_BAD_SLOT);
+                    continue;
+                }
+                if (!p.out2_tiled) spk_store4<T, VEC>(o2 + slot * p.width + c, f, width - c);
+                else if (c < spk_operand_columns(width)) spk_store4<T, true>(o2 + spk_operand_at(p.out2_rows, slot, c), f, 4);
+            }
         }
-        for (int j = AHEAD ? kSlots : 0; j < p.out2_top; ++j) put(p.out2_slots[t * p.out2_top + j]);
     }
 }
 
@@ -149,7 +183,11 @@ int launch_boundary(const spk_rms_residual_args& p, cudaStream_t s) {
     if (threads == 0) return SPK_ERR_TOO_LARGE;
     const unsigned grid = static_cast<unsigned>(p.n);
     const bool vec = p.width % 4 == 0;
-    const bool ahead = p.n <= 4 * 148;  // the rows of a decode batch, all of them on the chip at once
+    // The rows of a decode batch, all of them on the chip at once by its registers (48 with one group a thread, 72 with two), four per SM at most.  General form / this
+    // one, us, two experts a row: 896 columns (128 threads) 64 rows 4.4 / 3.0, 592 4.9 / 3.7; 2048 columns (256) 64 rows 4.7 / 3.3, 444 5.4 / 4.5, 480 5.7 / 6.0, 592
+    // 5.9 / 6.3; 1536 columns 480 5.1 / 5.7.
+    const int resident = 65536 / ((v == 1 ? 48 : 72) * threads);
+    const bool ahead = p.n <= (resident < 4 ? resident : 4) * 148;
 #define SPK_RR(V_, AHEAD_)                                                                  \
     do {                                                                                    \
         if (vec) rms_residual_kernel<T, TD, V_, true, AHEAD_><<<grid, threads, 0, s>>>(p);  \

@@ -82,6 +82,31 @@ def test_boundary(dev, status, n, width, top, dtype):
 
 
 @pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("n,width", [(593, 896), (593, 1022), (445, 1028), (445, 2046), (445, 2048), (593, 300)])
+def test_boundary_of_more_rows_than_the_chip_holds_gives_the_bits_of_few(dev, status, n, width, dtype):
+    """One row beyond those that ask for all they read at once, against parts of the batch that do; three experts a row, some of them not there."""
+    g = torch.Generator(device=dev).manual_seed(n + width)
+    rnd = lambda *s: torch.randn(*s, generator=g, device=dev)
+    x, delta, w1, w2 = rnd(n, width), rnd(n, width), rnd(width), rnd(width)
+    rows = 8 * (-(-n * 3 // 8)) + 8
+    slots = torch.randperm(rows, generator=g, device=dev)[: n * 3].view(n, 3).to(torch.int32)
+    slots[torch.rand(n, 3, generator=g, device=dev) < 0.2] = -1
+    pairs, tiled = rnd(rows, width), dtype == BF
+
+    def run(step, expert_rows):
+        xo, o1 = torch.empty_like(x), torch.empty(n, width, dtype=dtype, device=dev)
+        o2 = torch.full((-(-width // 64), rows, 64) if tiled and expert_rows else (rows, width) if expert_rows else (n, width), 7.0, dtype=dtype, device=dev)
+        for lo in range(0, n, step):
+            at = slice(lo, lo + step)
+            second = dict(pairs=pairs, pair_slots=slots[at], pair_scale=0.3, out2=o2, out2_slots=slots[at], out2_tiled=tiled) if expert_rows else dict(out2=o2[at])
+            kn.rms_residual(eps=1e-3, x=x[at], delta=delta[at], x_out=xo[at], w1=w1, out1=o1[at], w2=w2, status=status, **second)
+        return xo, o1, o2
+    for expert_rows in (True, False):
+        for got, want in zip(run(n, expert_rows), run(100, expert_rows)):
+            assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
 def test_gelu(dev, dtype):
     z = torch.linspace(-9, 9, 3 * 41).view(3, 41).to(dtype)
     out = torch.zeros(3, 60, dtype=dtype, device=dev)
