@@ -28,8 +28,9 @@
 // Per 32-key tile at head_dim 64: 14 MMAs (8 cycles of a sub-partition's tensor pipe each), 48 masks and about 130 instructions per warp; the
 // integer pipe of the masks (a half-rate unit, 58 % busy) and the tensor pipe (44 %) are the two limits, and warps per SM decide how well they
 // overlap.  Scores by popc (a unit of an eighth of the rate, one per head and word) took the K rows through shared memory
-// to every thread (16 wavefronts per tile against 4): 256 rows x 4096 keys 75.1 -> 68.6 us; 256 rows of 1024 to 32768 keys at head_dim 128
-// 248 -> 221 us.  The e4m3 form of the scores is no MMA of its own on sm_100 but conversions and fp16 MMAs: 105 us; heads as the left operand's rows (no transposition, half of the tile empty): 74.6.
+// to every thread (16 wavefronts per tile against 4): whole calls of 256 rows x 4096 keys 75.4 -> 70.6 us, of 256 rows of 1024 to 32768 keys at head_dim 128
+// 248 -> 221.  The e4m3 form of the scores is no MMA of its own on sm_100 but conversions and fp16 MMAs: the main kernel alone 105 us of 256 x 4096; heads as the left operand's
+// rows (no transposition, half of the tile empty) 74.6, this form 68.6.
 #include "spk_attn.cuh"
 
 #include <atomic>
@@ -1219,6 +1220,12 @@ StreamPlan spk_attn_stream_plan(int T, int64_t n_seqs, int Hq, int Hkv, int head
         pl.workers = workers;
         pl.short_steps = max_steps <= kUncutSteps ? static_cast<int>(max_steps) : kShortSteps;
         pl.cut = max_steps > pl.short_steps;
+        // At 128 channels either three CTAs on every SM or four: in between, some SMs hold four that share what the others' three have.  Three on every SM / in
+        // between, us, 7/1 heads: 64 rows of 512 to 2048 keys 16.0 / 17.5, 148 rows x 800 20.2 / 22.7, 120 rows of 256 to 1024 keys 1.10 times longer.  Four are shorter ranges, more of
+        // which begin with a set-up and leave a record: 0.89 to 0.98 of three where lengths start near zero, 1.05 for rows of 1/4 to all of the table's width up to 20 steps a warp,
+        // less behind; most for rows of one length that fill the table and are just about as many as the warps of three (28/4 heads, 112 x 800: 32.7 / 38.5).
+        const int64_t third = 148LL * kWarps * 3;
+        if (head_dim == 128 && pl.cut && workers > third && workers < cap) pl.workers = workers = third;
         if (!pl.cut) {
             // whole items only: a warp per item while the GPU holds them all at once
             const int64_t items = n_seqs * gt;
@@ -1315,9 +1322,12 @@ int spk_attn_stream_launch(const AttnParams& p, const StreamPlan& plan, int head
         ctas = (sp.workers + kWarps - 1) / kWarps;
         combine = plan.cut;
         if (!plan.cut && sp.workers >= p.n_seqs * sp.gt) {
-            // Nothing can be cut and the GPU holds a warp per item at once: warp w runs item w whole, whatever the
+            // Nothing can be cut and there are no more items than the range form's warps: warp w runs item w whole, whatever the
             // rows' lengths (equal step ranges would hand some warps two ragged items and others none).  That is
-            // the unit form with one unit per row, which also needs no step prefix.
+            // the unit form with one unit per row, which also needs no step prefix.  At 128 channels and 16 bits it fits three CTAs per SM where the range form fits
+            // four; up to a wave and a third it is still the better one but for rows of one length.  Unit / range, 28/4 heads, up to 700 keys, us, rows of one length, of 1/4 to
+            // all, of 0 to all: 112 rows 27.5 / 25.3, 20.5 / 22.5, 17.6 / 28.9; 128 rows 27.9 / 25.6, 21.5 / 23.4, 19.5 / 31.2; 148 rows 28.2 / 25.8, 23.8 / 23.8, 21.1 / 37.1; 300 keys,
+            // 128 rows 16.4 / 15.6, 13.7 / 14.5, 12.5 / 17.9.
             sp.dense = 0;
             sp.unit_log2 = 30;
             sp.max_units = 1;

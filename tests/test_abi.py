@@ -152,3 +152,14 @@ def test_nvtx_ranges_follow_the_environment():
             env["SPK_NVTX"] = value
         out = subprocess.run([sys.executable, "-c", code], cwd=root, env=env, capture_output=True, text=True, check=True)
         assert out.stdout.strip().splitlines()[-1] == want
+
+
+def test_warps_that_share_a_batch_of_128_channels(lib):
+    """A decode batch whose rows may be cut is shared by the warps of up to three CTAs per SM, or, with eight steps of 32 keys for each, of four; two records of 8 x 128 sums and 8
+    totals a warp."""
+    record = 4 * (8 * 128 + 8)
+    workspace = lambda n, keys: lib.spk_attn_decode_workspace_bytes(4, n, 7, 1, 128, 16, keys // 16)
+    assert workspace(40, 1024) == 2 * 640 * record  # eight steps a warp
+    assert workspace(55, 2048) == 2 * 1760 * record
+    assert workspace(56, 2048) == workspace(73, 2048) == 2 * 3 * 4 * 148 * record
+    assert workspace(74, 2048) == workspace(256, 4096) == 2 * 4 * 4 * 148 * record
