@@ -19,20 +19,19 @@ constexpr int kStep = 16;
 constexpr int kStepTile = kStep * 128;  // bytes of a 64-channel tile of a step
 constexpr float kLog2e = 1.4426950408889634f;
 
-template <int CK, int CV>
+template <int CK, int CV, int STAGES>
 struct Shape {
-    static constexpr int NS = 3;  // heads of 64: 48 KB a CTA, so that four fit an SM: the key ranges of a batch are cut for 3 x 148 CTAs and more, and with
-                                  // four stages and three CTAs the 512 of 64 rows were two waves
+    static constexpr int NS = STAGES;
     static constexpr int kStage = (CK + CV) * kStepTile;
     static constexpr int kRing = kWarps * NS * kStage;
     static constexpr int kBytes = kRing + 128 + kWarps * NS * 8;
     static_assert(kWarps * 16 * CV * 64 * 4 <= kRing, "the final fold reuses the ring");
 };
 
-template <int CK, int CV>
+template <int CK, int CV, int STAGES>
 __global__ void __launch_bounds__(kThreads)
 sigmoid_decode_kernel(const spk_sigmoid_attn_args a) {
-    using Sh = Shape<CK, CV>;
+    using Sh = Shape<CK, CV, STAGES>;
     constexpr int NS = Sh::NS;
     extern __shared__ uint8_t raw[];
     uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(raw) + 127) & ~uintptr_t(127));
@@ -201,14 +200,14 @@ sigmoid_decode_kernel(const spk_sigmoid_attn_args a) {
     spk_grid_wait();
 }
 
-template <int CK, int CV>
+template <int CK, int CV, int STAGES>
 int launch(const spk_sigmoid_attn_args& a, cudaStream_t s) {
-    constexpr int bytes = Shape<CK, CV>::kBytes;
-    const cudaError_t e = cudaFuncSetAttribute(sigmoid_decode_kernel<CK, CV>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    constexpr int bytes = Shape<CK, CV, STAGES>::kBytes;
+    const cudaError_t e = cudaFuncSetAttribute(sigmoid_decode_kernel<CK, CV, STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
     if (e != cudaSuccess) return spk_set_cuda_error(e);
     const int rep = a.heads / a.kv_heads;
     const dim3 grid(a.splits, a.kv_heads * ((rep + 15) / 16), static_cast<unsigned>(a.n));
-    return spk_launch(sigmoid_decode_kernel<CK, CV>, grid, kThreads, bytes, s, a.overlap != 0, a);
+    return spk_launch(sigmoid_decode_kernel<CK, CV, STAGES>, grid, kThreads, bytes, s, a.overlap != 0, a);
 }
 
 }  // namespace
@@ -216,8 +215,14 @@ int launch(const spk_sigmoid_attn_args& a, cudaStream_t s) {
 int spk_sigmoid_decode_launch(const spk_sigmoid_attn_args& a, cudaStream_t s) {
     if (a.n > 65535 || a.kv_heads * ((a.heads / a.kv_heads + 15) / 16) > 65535) return SPK_ERR_TOO_LARGE;
     const int ck = a.k_pad / 64, cv = a.v_pad / 64;
-    if (ck == 1 && cv == 1) return launch<1, 1>(a, s);
-    if (ck == 1 && cv == 2) return launch<1, 2>(a, s);
-    if (ck == 2 && cv == 1) return launch<2, 1>(a, s);
-    return launch<2, 2>(a, s);
+    // Heads of 64: rings of three stages (48 KB) leave four CTAs per SM, rings of four leave three, for long ranges of more CTAs than a wave of the former where full waves
+    // of the latter hold fewer CTA slots per SM.  Four / three stages, 14/2 heads, 2048 keys, us: 444 CTAs 14.5 / 14.2, 448 18.0 / 13.0, 512 18.5 / 13.5, 592 39.0 / 29.5, 600 27.5 / 24.5,
+    // 720 40.2 / 45.4; 6000 keys 444 41.4 / 40.0, 720 98.2 / 115.1; 8/8 heads 640 67.4 / 79.2, 800 70.0 / 82.1, 960 98.6 / 84.0, 1024 99.4 / 85.2; 512 keys 640 19.2 / 18.6, 720 20.8 / 19.8.
+    const int64_t ctas = static_cast<int64_t>(a.n) * a.splits * a.kv_heads * ((a.heads / a.kv_heads + 15) / 16);
+    const int64_t three = 3 * 148, four = 4 * 148;
+    const bool deep = ctas > four && ctas % four >= 32 && (ctas + three - 1) / three * 3 < (ctas + four - 1) / four * 4 && a.max_blocks * a.block_size / a.splits >= 1024;
+    if (ck == 1 && cv == 1) return deep ? launch<1, 1, 4>(a, s) : launch<1, 1, 3>(a, s);
+    if (ck == 1 && cv == 2) return launch<1, 2, 3>(a, s);
+    if (ck == 2 && cv == 1) return launch<2, 1, 3>(a, s);
+    return launch<2, 2, 3>(a, s);
 }

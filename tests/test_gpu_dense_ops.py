@@ -521,6 +521,29 @@ def test_sigmoid_attention_decode_rows(dev, shape, dtype):
     assert status.item() == 0
 
 
+@pytest.mark.parametrize("n, few, keys", [(80, 74, 1024), (78, 74, 1040)])
+def test_sigmoid_decode_with_deeper_rings_gives_the_same_bits(dev, n, few, keys):
+    """Heads of 64 have rings of four stages where long ranges make a wave of the CTAs that rings of three allow and a part of one (640 and 592 of them here)."""
+    heads = 8
+    g = torch.Generator(device=dev).manual_seed(n + keys)
+    per = -(-keys // 16)
+    kp, vp = (PagedKVPool(n * per, heads, 16, 64, torch.bfloat16, dev) for _ in range(2))
+    kp.data.normal_(generator=g)
+    vp.data.normal_(generator=g)
+    tables = torch.randperm(n * per, generator=g, device=dev).to(torch.int32).view(n, per)
+    lens = torch.randint(1, keys + 1, (n,), generator=g, device=dev).to(torch.int32)
+    q, bias = torch.randn(n, heads, 64, generator=g, device=dev).to(torch.bfloat16), torch.randn(heads, generator=g, device=dev) - 2
+
+    def run(lo, hi):
+        out = torch.empty(hi - lo, heads * 64, dtype=torch.bfloat16, device=dev)
+        parts = dense.sigmoid_attention(q[lo:hi], kp, vp, tables[lo:hi], bias, out, heads=heads, kv_heads=heads, dim=64, vdim=64, scale=0.2, seq_lens=lens[lo:hi],
+                                        partial_sums=True)
+        assert parts.shape[1] == 1
+        return parts
+    got = run(0, n)
+    assert torch.equal(got[:few], run(0, few)) and torch.isfinite(got).all()
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("shape", ["d64", "d128", "ragged", "page256", "d160"])
 def test_single_keys_stand_out(dev, shape, dtype):
