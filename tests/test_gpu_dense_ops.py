@@ -682,6 +682,22 @@ def test_decay_steps_of_many_rows_give_the_bits_of_few(dev, dtype, n, heads, dim
         assert torch.equal(whole[active == 1], parts[active == 1]) and torch.isnan(whole[active == 0]).all()
 
 
+@pytest.mark.parametrize("heads, dim, vdim", [(4, 64, 64), (5, 64, 60), (3, 8, 4)])
+def test_decay_of_many_portions_gives_the_bits_of_each(dev, heads, dim, vdim):
+    """The scan over chunks takes four elements a thread where there are many of them, or few chunks; the general form (32-bit operands) cuts every portion alike."""
+    lens, contexts, rows = [200, 100, 1, 300, 64, 129] * 4, [0, 7, 0, 50, 9, 0] * 4, torch.randperm(24, generator=torch.Generator().manual_seed(dim)).tolist()
+    g = torch.Generator(device=dev).manual_seed(heads)
+    qkv = torch.randn(sum(lens), heads * (2 * dim + vdim), generator=g, device=dev)
+    powers = dense.decay_powers([1 - 2.0 ** -(1 + i) for i in range(heads)], dev)
+    whole = torch.randn(25, heads, dim, vdim, generator=g, device=dev)
+    each = whole.clone()
+    run = lambda x, state, plan: dense.decay_attention(*x.split([heads * dim, heads * dim, heads * vdim], dim=1), state, powers, plan=plan)
+    starts = [sum(lens[:i]) for i in range(len(lens))]
+    got = run(qkv, whole, PrefillPlan(starts, lens, contexts, rows, dev))
+    want = [run(qkv[s: s + n], each, PrefillPlan([0], [n], [c], [r], dev)) for s, n, c, r in zip(starts, lens, contexts, rows)]
+    assert torch.equal(got, torch.cat(want)) and torch.equal(whole, each)
+
+
 def test_decay_of_a_long_prompt_keeps_the_first_token(dev):
     """A decay next to one, keys that are zero except the first: the first token's value must still be there at the end."""
     for dtype in DTYPES:
@@ -705,22 +721,6 @@ def test_extend_hold_and_resume(dev):
     not fit changes nothing."""
     st = DecodeBatchState(max_rows=3, max_blocks=4, num_blocks=8, block_size=4, device=dev)
     buf = lambda n: (torch.empty(n, dtype=torch.int64, device=dev), torch.empty(n, dtype=torch.int64, device=dev),
-@pytest.mark.parametrize("heads, dim, vdim", [(4, 64, 64), (5, 64, 60), (3, 8, 4)])
-def test_decay_of_many_portions_gives_the_bits_of_each(dev, heads, dim, vdim):
-    """The scan over chunks takes four elements a thread where there are many of them, or few chunks; the general form (32-bit operands) cuts every portion alike."""
-    lens, contexts, rows = [200, 100, 1, 300, 64, 129] * 4, [0, 7, 0, 50, 9, 0] * 4, torch.randperm(24, generator=torch.Generator().manual_seed(dim)).tolist()
-    g = torch.Generator(device=dev).manual_seed(heads)
-    qkv = torch.randn(sum(lens), heads * (2 * dim + vdim), generator=g, device=dev)
-    powers = dense.decay_powers([1 - 2.0 ** -(1 + i) for i in range(heads)], dev)
-    whole = torch.randn(25, heads, dim, vdim, generator=g, device=dev)
-    each = whole.clone()
-    run = lambda x, state, plan: dense.decay_attention(*x.split([heads * dim, heads * dim, heads * vdim], dim=1), state, powers, plan=plan)
-    starts = [sum(lens[:i]) for i in range(len(lens))]
-    got = run(qkv, whole, PrefillPlan(starts, lens, contexts, rows, dev))
-    want = [run(qkv[s: s + n], each, PrefillPlan([0], [n], [c], [r], dev)) for s, n, c, r in zip(starts, lens, contexts, rows)]
-    assert torch.equal(got, torch.cat(want)) and torch.equal(whole, each)
-
-
                      torch.empty(n, dtype=torch.int32, device=dev), torch.empty(n, dtype=torch.int32, device=dev))
     p, s, r, e = buf(6)
     st.extend(1, 6, p, s, r, e)
