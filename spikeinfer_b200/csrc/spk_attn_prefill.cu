@@ -1,6 +1,6 @@
 // Prefill attention over the packed spike pools on the fifth-generation tensor cores (tcgen05), 16-bit outputs, head_dim 64 or 128.
 //
-// CTA = (128 query tokens of one portion, timestep, query head), two CTAs per SM.  Thirteen warps:
+// CTA = (128 query tokens of one portion, timestep, query head), two CTAs per SM.  Thirteen warps (nine in the form of many short portions, below):
 //  * warps 8-11 read the packed K and V rows of 64 keys through the block table and turn their bits into operands: K e4m3 bytes, V halves, each
 //    a masked word as it is, in the swizzled operand layouts; a stage ahead of the MMAs, the next stage's words already in registers;
 //  * warp 12 issues S = Q K^T (kind::f8f6f4, exact: scores are counts) and O += P V (kind::f16, P read from TMEM).  S of step t + 1 goes out as
@@ -14,12 +14,13 @@
 // Bits expand in an order that is cheapest for the bit tricks (byte b of word j: bit j + 8 b; half h: bit j + 16 h), the same for Q and K;
 // V's column order is undone when a row is stored.
 //
-// What bounds it: shared memory (the operands written, 24 KB a step at 128 channels, and read by the MMAs, 40 KB: about four fifths of its
-// cycles), then the special-function pipe (one exponential per (query, key) pair, half of its cycles) and, for prompts of a few hundred tokens,
-// a CTA's set-up and drain.  Why 64 keys per step: scores, two buffers of weights and O of up to 128 channels are 256 TMEM columns, so
-// that two CTAs fit an SM and one's set-up and drain hide behind the other's steps.
+// What bounds it: no pipe by itself.  At 128 channels and 23 steps a CTA the special-function pipe (one exponential per (query, key) pair) is 50 % busy, the
+// load/store path's data pipe (operands written, scores and weights moved to and from TMEM) 46 %, TMEM 44 %, the tensor pipe 38 %, issue 50 %, and the MMAs
+// read 40 KB of operands a step from shared memory beside that; two CTAs leave some of their waits uncovered.  For prompts of a few hundred tokens a CTA's
+// set-up and drain count: 16 x 512 tokens at 64 channels keep the special-function pipe 34 % busy.  Why 64 keys per step: scores, two buffers of weights and O of up to 128
+// channels are 256 TMEM columns, so that two CTAs fit an SM and one's set-up and drain hide behind the other's steps.
 // Measured, whole fused_qkv_attention calls: three portions of 766 to 1531 tokens behind 700 cached, 28/4 heads of 128, 338 -> 294 us; four of 875
-// to 2000 behind 300, 7/1 heads of 128, 137 -> 118; 16 x 512 tokens, 14/2 heads of 64, 130 as before.  What came before: comparisons with the
+// to 2000 behind 300, 7/1 heads of 128, 137 -> 118; 16 x 512 tokens, 14/2 heads of 64, 130 -> 123 (with one warpgroup on scores).  What came before: comparisons with the
 // diagonal in every step and shifts and products per operand register (190 M instructions, 131 M without them), a warp per 32 rows on
 // scores (its waits and its exponentials took turns), S behind the weights' product of two steps before.  With 64 keys per
 // warpgroup and step (even and odd steps): 307 us; one warpgroup that reads all 64 scores ahead: 324.
@@ -35,7 +36,7 @@ using namespace spk_tc;
 constexpr int kRows = 128;                  // query tokens per CTA
 constexpr int kKeys = 64;                   // keys per step
 constexpr int kStages = 3;
-constexpr int kThreads = 416;              // two warpgroups on scores, one on operands, one warp on MMAs
+constexpr int threads_of(int wgs) { return 128 * wgs + 160; }  // WGS warpgroups on scores, one on operands, one warp on MMAs
 constexpr int kQBytes = kRows * 128;        // rows of 128 bytes; 64 channels use the first half
 constexpr int kKBytes = kKeys * 128;
 constexpr int kVColTile = kKeys * 128;      // 64 channels
@@ -122,10 +123,12 @@ __device__ __forceinline__ uint32_t pack_pair<__half>(float lo, float hi) {
 template <int W>
 constexpr int shared_bytes() { return kQBytes + kStages * (kKBytes + W / 2 * kVColTile) + 1024 + 256; }
 
-template <int W, typename TO>
-__global__ void __launch_bounds__(kThreads, 2)
+// WGS: warpgroups on scores.  Two halve the time of a step; one leaves registers for a third CTA per SM at 64 channels, which sets itself up while it
+// waits for the tensor memory of one that ends.
+template <int W, typename TO, int WGS>
+__global__ void __launch_bounds__(threads_of(WGS), WGS == 1 && W == 2 ? 3 : 2)
 spike_prefill_kernel(const __grid_constant__ Launch l) {
-    constexpr int kVBytes = W / 2 * kVColTile;
+    constexpr int kVBytes = W / 2 * kVColTile, kScoreWarps = 4 * WGS, kMmaWarp = kScoreWarps + 4;
     extern __shared__ uint8_t raw[];
     uint8_t* q_s = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(raw) + 1023) & ~uintptr_t(1023));
     uint8_t* k_s = q_s + kQBytes;
@@ -153,10 +156,10 @@ spike_prefill_kernel(const __grid_constant__ Launch l) {
     const int64_t token = por.start + first + e;
     int block0 = -1, block = -1;
     uint32_t qw[W];
-    if (warp >= 8 && warp < 12) {
+    if (warp >= kScoreWarps && warp < kMmaWarp) {
         block0 = entry(0);
         block = entry(1);
-    } else if (warp < 8) {
+    } else if (warp < kScoreWarps) {
         const uint32_t* q = static_cast<const uint32_t*>(a.q_packed) + ts * a.sq_t + token * a.sq_tok + h * a.sq_h;
 #pragma unroll
         for (int w = 0; w < W; ++w) qw[w] = e < nq ? q[w] : 0u;
@@ -167,13 +170,13 @@ spike_prefill_kernel(const __grid_constant__ Launch l) {
             mbar_init(smem_u32(&bars->kv_free[i]), 1);
         }
         mbar_init(smem_u32(&bars->s_full), 1);
-        mbar_init(smem_u32(&bars->s_read), 256);
-        for (int i = 0; i < 2; ++i) mbar_init(smem_u32(&bars->p_full[i]), 256);
+        mbar_init(smem_u32(&bars->s_read), 32 * kScoreWarps);
+        for (int i = 0; i < 2; ++i) mbar_init(smem_u32(&bars->p_full[i]), 32 * kScoreWarps);
         mbar_init(smem_u32(&bars->q_full), 128);
         mbar_init(smem_u32(&bars->o_full), 1);
         bars->abort = 0;
     }
-    if (warp == 12) tmem_alloc(smem_u32(&bars->tmem), 256);
+    if (warp == kMmaWarp) tmem_alloc(smem_u32(&bars->tmem), 256);
     fence_async_shared();
     tc_fence_before();
     __syncthreads();
@@ -181,7 +184,7 @@ spike_prefill_kernel(const __grid_constant__ Launch l) {
     const uint32_t tmem = bars->tmem;
     volatile int* abort = &bars->abort;
 
-    if (warp >= 8 && warp < 12) {  // ---- K and V bits to operands: thread = (key, half of the words)
+    if (warp >= kScoreWarps && warp < kMmaWarp) {  // ---- K and V bits to operands: thread = (key, half of the words)
         const uint32_t* kp = static_cast<const uint32_t*>(a.k_pool) + ts * a.sk_t + g * a.sk_h + half * (W / 2);
         const uint32_t* vp = static_cast<const uint32_t*>(a.v_pool) + ts * a.sv_t + g * a.sv_h + half * (W / 2);
         uint32_t kw[W / 2], vw[W / 2];
@@ -225,7 +228,7 @@ spike_prefill_kernel(const __grid_constant__ Launch l) {
             fence_async_shared();
             mbar_arrive(smem_u32(&bars->kv_full[stage]));
         }
-    } else if (warp == 12) {  // ---- MMAs
+    } else if (warp == kMmaWarp) {  // ---- MMAs
         constexpr uint32_t s_desc = (1u << 4) | (static_cast<uint32_t>(kKeys >> 3) << 17) | (static_cast<uint32_t>(kRows >> 4) << 24);
         constexpr uint32_t o_desc = (1u << 4) | (1u << 16) | (static_cast<uint32_t>(W * 32 >> 3) << 17) | (static_cast<uint32_t>(kRows >> 4) << 24);
         const uint32_t who = elect_one();
@@ -257,7 +260,7 @@ spike_prefill_kernel(const __grid_constant__ Launch l) {
         }
         if (who) mma_commit(smem_u32(&bars->o_full));
         mbar_wait(smem_u32(&bars->o_full), 0);
-    } else {  // ---- scores to weights: thread = query row, warps 0-3 the first 32 keys of a step, 4-7 the others
+    } else {  // ---- scores to weights: thread = query row; of two warpgroups the first takes the first 32 keys of a step, the second the others
         const int r = e, wg = warp >> 2;
         uint64_t c1, c0;
         {
@@ -276,48 +279,58 @@ spike_prefill_kernel(const __grid_constant__ Launch l) {
             c0 = f2_pack(b, b);
         }
         const uint32_t lanes = static_cast<uint32_t>((warp & 3) * 32) << 16;
-        uint64_t sums = f2_pack(0.0f, 0.0f);
+        uint64_t sums = f2_pack(0.0f, 0.0f), other = sums;  // of this half of a step's keys, and of the other where one warpgroup takes both
         bool ok = true;
         for (int t = 0; t < steps; ++t) {
             // also says that the product of step t - 2, issued before these scores, is complete: its weights lay where step t's go
             ok = __all_sync(~0u, mbar_wait(smem_u32(&bars->s_full), t & 1, abort));
             if (!ok) break;
             tc_fence_after();
-            uint32_t sc[32], p[16];
-            tmem_ld32(tmem + lanes + kTmemS + wg * 32, sc);
-            tmem_wait_ld(sc);
-            tc_fence_before();
-            mbar_arrive(smem_u32(&bars->s_read));
-            const int seen = pos0 + r - t * kKeys - wg * 32;  // last visible column of this row
-            auto weights = [&](auto masked) {  // the two forms are code of their own: only the steps on the diagonal compare columns
-#pragma unroll
-                for (int i = 0; i < 16; ++i) {
-                    float x, y;
-                    f2_unpack(f2_fma(f2_pack(__uint_as_float(sc[2 * i]), __uint_as_float(sc[2 * i + 1])), c1, c0), x, y);
-                    x = ex2(x);
-                    y = ex2(y);
-                    if (decltype(masked)::value) {
-                        x = 2 * i <= seen ? x : 0.0f;
-                        y = 2 * i + 1 <= seen ? y : 0.0f;
-                    }
-                    p[i] = pack_pair<__half>(x, y);
-                    if (std::is_same<TO, __half>::value) {  // the weights as they enter the product
-                        const float2 v = __half22float2(*reinterpret_cast<const __half2*>(&p[i]));
-                        x = v.x;
-                        y = v.y;
-                    }
-                    sums = f2_add(sums, f2_pack(x, y));
+#pragma unroll 1
+            for (int c = wg; c < (WGS == 2 ? wg + 1 : 2); ++c) {
+                uint32_t sc[32], p[16];
+                tmem_ld32(tmem + lanes + kTmemS + c * 32, sc);
+                tmem_wait_ld(sc);
+                if (WGS == 2 || c == 1) {
+                    tc_fence_before();
+                    mbar_arrive(smem_u32(&bars->s_read));
                 }
-            };
-            if (__all_sync(~0u, seen >= 31)) {
-                weights(std::false_type{});
-            } else if (__all_sync(~0u, seen < 0)) {
+                const int seen = pos0 + r - t * kKeys - c * 32;  // last visible column of this row
+                auto weights = [&](auto masked) {  // the two forms are code of their own: only the steps on the diagonal compare columns
 #pragma unroll
-                for (int i = 0; i < 16; ++i) p[i] = 0u;
-            } else {
-                weights(std::true_type{});
+                    for (int i = 0; i < 16; ++i) {
+                        float x, y;
+                        f2_unpack(f2_fma(f2_pack(__uint_as_float(sc[2 * i]), __uint_as_float(sc[2 * i + 1])), c1, c0), x, y);
+                        x = ex2(x);
+                        y = ex2(y);
+                        if (decltype(masked)::value) {
+                            x = 2 * i <= seen ? x : 0.0f;
+                            y = 2 * i + 1 <= seen ? y : 0.0f;
+                        }
+                        p[i] = pack_pair<__half>(x, y);
+                        if (std::is_same<TO, __half>::value) {  // the weights as they enter the product
+                            const float2 v = __half22float2(*reinterpret_cast<const __half2*>(&p[i]));
+                            x = v.x;
+                            y = v.y;
+                        }
+                        sums = f2_add(sums, f2_pack(x, y));
+                    }
+                };
+                if (__all_sync(~0u, seen >= 31)) {
+                    weights(std::false_type{});
+                } else if (__all_sync(~0u, seen < 0)) {
+#pragma unroll
+                    for (int i = 0; i < 16; ++i) p[i] = 0u;
+                } else {
+                    weights(std::true_type{});
+                }
+                tmem_st16(tmem + lanes + kTmemP + (t & 1) * (kKeys / 2) + c * 16, p);
+                if (WGS == 1) {
+                    const uint64_t mine = sums;
+                    sums = other;
+                    other = mine;
+                }
             }
-            tmem_st16(tmem + lanes + kTmemP + (t & 1) * (kKeys / 2) + wg * 16, p);
             tmem_wait_st();
             tc_fence_before();
             mbar_arrive(smem_u32(&bars->p_full[t & 1]));  // one per parity: a fast warp may be a step ahead of a slow one, not two
@@ -326,16 +339,21 @@ spike_prefill_kernel(const __grid_constant__ Launch l) {
         f2_unpack(sums, x, y);
         ok = __all_sync(~0u, ok && mbar_wait(smem_u32(&bars->o_full), 0, abort) && *abort == 0);
         tc_fence_after();
-        // both warpgroups' sums of a row, through the query's operand (every MMA is complete); each stores half of the words
-        float* parts = reinterpret_cast<float*>(q_s);
-        parts[wg * kRows + r] = x + y;
-        asm volatile("bar.sync 1, 256;" ::: "memory");
-        const float sum = parts[r] + parts[kRows + r];
+        float sum = x + y;  // the halves' sums are added up last in either form: the same bits
+        if (WGS == 2) {     // through the query's operand (every MMA is complete)
+            float* parts = reinterpret_cast<float*>(q_s);
+            parts[wg * kRows + r] = sum;
+            asm volatile("bar.sync 1, 256;" ::: "memory");
+            sum = parts[r] + parts[kRows + r];
+        } else {
+            f2_unpack(other, x, y);
+            sum += x + y;
+        }
         const float inv = ok && r < nq ? 1.0f / sum : 0.0f;
         TO* out = static_cast<TO*>(a.out) + ts * a.so_t + token * a.so_tok + h * a.so_h;
 #pragma unroll
-        for (int i = 0; i < W / 2; ++i) {
-            const int w = wg * (W / 2) + i;
+        for (int i = 0; i < W / WGS; ++i) {  // each warpgroup stores its share of the words
+            const int w = wg * (W / WGS) + i;
             uint32_t o[32];
             tmem_ld32(tmem + lanes + kTmemO + w * 32, o);
             tmem_wait_ld(o);
@@ -371,17 +389,17 @@ spike_prefill_kernel(const __grid_constant__ Launch l) {
     __syncthreads();
     tc_fence_after();
     if (threadIdx.x == 0 && *abort != 0) spk_flag(a.status, SPK_STATUS_DEVICE_WAIT_EXPIRED);
-    if (warp == 12) tmem_dealloc(tmem, 256);
+    if (warp == kMmaWarp) tmem_dealloc(tmem, 256);
 }
 
-template <int W, typename TO>
+template <int W, typename TO, int WGS>
 int launch(const Launch& l, int tiles, cudaStream_t s) {
     constexpr int bytes = shared_bytes<W>();
     static_assert(sizeof(Bars) <= 256 && 2 * bytes <= 224 * 1024, "shared memory of two CTAs");
     static_assert(sizeof(Launch) <= 4096, "kernel parameters");
-    const cudaError_t e = cudaFuncSetAttribute(spike_prefill_kernel<W, TO>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    const cudaError_t e = cudaFuncSetAttribute(spike_prefill_kernel<W, TO, WGS>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
     if (e != cudaSuccess) return spk_set_cuda_error(e);
-    spike_prefill_kernel<W, TO><<<dim3(l.a.num_q_heads * l.a.T, tiles), kThreads, bytes, s>>>(l);
+    spike_prefill_kernel<W, TO, WGS><<<dim3(l.a.num_q_heads * l.a.T, tiles), threads_of(WGS), bytes, s>>>(l);
     SPK_CHECK_LAUNCH();
     return SPK_OK;
 }
@@ -425,8 +443,14 @@ extern "C" int spk_spike_prefill(const spk_spike_prefill_args* args, const spk_s
         std::copy(order, order + tiles, l.tiles);
         const cudaStream_t s = spk_stream(stream);
         if (tiles > 0) {
-            if (a.head_dim == 64) rc = a.dtype == SPK_BF16 ? launch<2, __nv_bfloat16>(l, tiles, s) : launch<2, __half>(l, tiles, s);
-            else rc = a.dtype == SPK_BF16 ? launch<4, __nv_bfloat16>(l, tiles, s) : launch<4, __half>(l, tiles, s);
+            // One warpgroup on scores at 64 channels where a launch is many short CTAs: up to eight steps, and a wave of a CTA per SM for each of them.  Two warpgroups / one, us,
+            // 14/2 heads: 8 x 64 tokens 9.6 / 8.5, 16 x 64 16.0 / 13.8, 32 x 64 27.8 / 22.9, 16 x 128 21.5 / 20.5, 8 x 256 24.1 / 23.5, 16 x 512 98.6 / 91.4; the other way round 4 x 256
+            // 13.7 / 13.9, 4 x 512 28.1 / 29.5, 16 x 64 behind 400 33.8 / 35.0, 1 x 1000 21.1 / 24.6.
+            const int steps = (*std::max_element(keys_of, keys_of + tiles) + kKeys - 1) / kKeys;
+            const bool brief = steps <= 8 && static_cast<int64_t>(steps) * 148 <= heads * tiles;
+            if (a.head_dim == 64 && brief) rc = a.dtype == SPK_BF16 ? launch<2, __nv_bfloat16, 1>(l, tiles, s) : launch<2, __half, 1>(l, tiles, s);
+            else if (a.head_dim == 64) rc = a.dtype == SPK_BF16 ? launch<2, __nv_bfloat16, 2>(l, tiles, s) : launch<2, __half, 2>(l, tiles, s);
+            else rc = a.dtype == SPK_BF16 ? launch<4, __nv_bfloat16, 2>(l, tiles, s) : launch<4, __half, 2>(l, tiles, s);
         }
         held = tiles = 0;
     };

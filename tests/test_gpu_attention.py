@@ -584,6 +584,28 @@ def test_prefill_attention_over_strides_and_gaps(dev, heads, kv_heads, dim, dtyp
         assert torch.equal(got, want)
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_prefill_attention_of_many_short_portions_gives_the_bits_of_each(dev, dtype):
+    """Heads of 64: a launch of many short tiles has one warpgroup on scores, a portion alone two."""
+    T, heads, kv_heads, dim, page = 4, 14, 2, 64, 16
+    lens, contexts = [64, 1, 128, 130, 200, 500, 100, 63, 64, 65, 17, 256, 320, 30, 192, 129, 64, 64], [0, 200, 0, 3, 64, 12, 0, 1, 64, 0, 400, 0, 100, 60, 0, 0, 448, 5]
+    g = torch.Generator(device=dev).manual_seed(4)
+    need = [-(-(n + c) // page) for n, c in zip(lens, contexts)]
+    word = lambda *s: torch.randint(-2 ** 31, 2 ** 31, s, generator=g, device=dev, dtype=torch.int32)
+    k, v, q = word(T, kv_heads, sum(need) * page, 2), word(T, kv_heads, sum(need) * page, 2), word(T, sum(lens), heads, 2)
+    tables = list(torch.randperm(sum(need), generator=g, device=dev).to(torch.int32).split(need))
+    starts = [sum(lens[:i]) for i in range(len(lens))]
+    run = lambda at, out: kernels.paged_spike_attn_prefill(q, k, v, [tables[i] for i in at], [starts[i] for i in at], [lens[i] for i in at], [contexts[i] for i in at],
+                                                           out, head_dim=dim, block_size=page, num_q_heads=heads, num_kv_heads=kv_heads)
+    tiles = sum(-(-n // 128) for n in lens)
+    assert max(n + c for n, c in zip(lens, contexts)) <= 8 * 64 and 8 * 148 <= tiles * T * heads and 148 > T * heads  # the rule's sides; all but the longest alone
+    got, want = (torch.full((T, sum(lens), heads, dim), 7.0, dtype=dtype, device=dev) for _ in range(2))
+    run(range(len(lens)), got)
+    for i in range(len(lens)):
+        run([i], want)
+    assert torch.equal(got, want) and bool((got <= 1.0).all())
+
+
 def test_prefill_attention_of_more_tiles_than_a_launch_holds(dev):
     """A portion that is cut by the end of a launch's list of 512 query tiles goes on in the next, behind a full list of portions too."""
     page, dim = 64, 64
