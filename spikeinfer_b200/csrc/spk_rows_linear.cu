@@ -138,9 +138,9 @@ extern "C" int spk_rows_linear(const spk_rows_linear_args* args, void* stream) {
     SpkRange nvtx_range("spk_rows_linear");
     if (args == nullptr) return SPK_ERR_NULL_POINTER;
     const spk_rows_linear_args& a = *args;
-    if (a.n < 0 || a.n > 2 || a.k < 8 || a.k > (1 << 20) || a.k % 8 != 0 || a.features < 1) return SPK_ERR_BAD_SHAPE;
+    if (a.n < 0 || a.n > 2 || a.k < 8 || a.k > (1 << 20) || a.k % 8 != 0 || a.features < 0) return SPK_ERR_BAD_SHAPE;
     if (a.out_dtype != SPK_F32 && a.out_dtype != SPK_BF16) return SPK_ERR_BAD_DTYPE;
-    if (a.n == 0) return SPK_OK;
+    if (a.n == 0 || a.features == 0) return SPK_OK;
     if (a.x == nullptr || a.w == nullptr || a.out == nullptr) return SPK_ERR_NULL_POINTER;
     if (reinterpret_cast<uintptr_t>(a.x) % 16 != 0 || reinterpret_cast<uintptr_t>(a.w) % 16 != 0 || a.ld_x % 8 != 0) return SPK_ERR_BAD_STRIDE;
     return a.out_dtype == SPK_F32 ? dispatch<float>(a, spk_stream(stream)) : dispatch<__nv_bfloat16>(a, spk_stream(stream));

@@ -249,19 +249,25 @@ def rms_residual(*, eps: float, x: torch.Tensor | None = None, delta: torch.Tens
 FEW_ROWS = 2
 
 
-def takes_few_rows(x: torch.Tensor, w: torch.Tensor) -> bool:
-    """Whether :func:`rows_linear` is the form for ``x w^T``: up to two bf16 rows of at most 2048 columns (a library product of so few rows takes 3 to
-    5 us whatever its size; longer rows it reads as fast)."""
-    return (x.shape[0] <= FEW_ROWS and x.dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and x.shape[1] % 8 == 0 and x.shape[1] <= 2048
+def few_rows(x: torch.Tensor, w: torch.Tensor) -> bool:
+    """Whether :func:`rows_linear` takes ``x w^T``: two matrices of one device, up to two aligned bf16 rows of at most 2048 columns."""
+    return (x.ndim == 2 and w.ndim == 2 and x.shape[1] == w.shape[1] and x.device == w.device and x.shape[0] <= FEW_ROWS
+            and x.dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and x.shape[1] % 8 == 0 and 8 <= x.shape[1] <= 2048
             and x.stride(1) == 1 and x.stride(0) % 8 == 0 and w.is_contiguous() and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0)
 
 
+def takes_few_rows(x: torch.Tensor, w: torch.Tensor) -> bool:
+    """Whether :func:`rows_linear` is the form for ``x w^T`` (a library product of so few rows takes 3 to 5 us whatever its size; longer rows it reads as
+    fast)."""
+    return x.is_cuda and few_rows(x, w)
+
+
 def rows_linear(x: torch.Tensor, w: torch.Tensor, out_dtype: torch.dtype, overlap_previous: bool = False) -> torch.Tensor:
-    """``x w^T`` for the operands that :func:`takes_few_rows` admits, 32-bit sums, ``out_dtype`` fp32 or bf16.  ``overlap_previous``: the launch may be
+    """``x w^T`` for the operands that :func:`few_rows` admits, 32-bit sums, ``out_dtype`` fp32 or bf16.  ``overlap_previous``: the launch may be
     placed while the one ahead of it on the stream runs (it reads only ``w`` before that has finished)."""
     _lib.require_cuda(x, "rows_linear input")
-    if not takes_few_rows(x, w) or x.shape[1] != w.shape[1]:
-        raise ValueError("rows_linear takes one or two aligned bf16 rows and a contiguous [features, columns] matrix")
+    if not few_rows(x, w):
+        raise ValueError("rows_linear takes one or two aligned bf16 rows and a contiguous [features, columns] matrix of the same device")
     out = torch.empty((x.shape[0], w.shape[0]), dtype=out_dtype, device=x.device)
     a = _lib.RowsLinearArgs(x.data_ptr(), w.data_ptr(), out.data_ptr(), x.stride(0), w.shape[0], x.shape[0], w.shape[1], w.shape[0],
                             _lib.dtype_code(out_dtype), int(overlap_previous))

@@ -144,6 +144,12 @@ def test_rows_linear_refuses_what_it_does_not_take(dev):
               torch.zeros(2, 56, device=dev, dtype=BF)):
         with pytest.raises(ValueError):
             kn.rows_linear(x, w, F32)
+    x = torch.zeros(2, 64, device=dev, dtype=BF)
+    for bad in (w.cpu(), w[None], w[:, :56]):
+        assert not kn.takes_few_rows(x, bad)
+        with pytest.raises(ValueError):
+            kn.rows_linear(x, bad, F32)
+    assert kn.rows_linear(x, w[:0], F32).shape == (2, 0)
 
 
 # ---- experts ---------------------------------------------------------------------------------------------------------
