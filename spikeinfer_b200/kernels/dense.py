@@ -257,9 +257,16 @@ def few_rows(x: torch.Tensor, w: torch.Tensor) -> bool:
 
 
 def takes_few_rows(x: torch.Tensor, w: torch.Tensor) -> bool:
-    """Whether :func:`rows_linear` is the form for ``x w^T`` (a library product of so few rows takes 3 to 5 us whatever its size; longer rows it reads as
-    fast)."""
-    return x.is_cuda and few_rows(x, w)
+    """Whether :func:`rows_linear` is the form for ``x w^T``: what it takes, up to a number of features that depends on the rows and columns.  A library
+    product of so few rows takes 2.4 to 8 us whatever its size; with more features it reads the weights as fast.
+
+    Library / here, weights from HBM, us: one row, 64 columns x 8192 features 2.5 / 2.3, x 10240 2.5 / 2.8, x 16384 2.6 / 3.3; 512 x 8192 4.4 / 3.7, x 16384 5.5 / 5.1;
+    2048 x 16384 13.7 / 11.6; two rows, 64 x 6144 2.4 / 2.4, x 8192 2.4 / 3.1; 896 x 6144 4.9 / 4.6, x 8192 5.3 / 5.4; 1536 x 4096 7.0 / 5.0, x 8192 7.0 / 7.8; 2048 x 4096 7.8 / 6.0,
+    x 5120 6.5 / 6.7."""
+    if not x.is_cuda or not few_rows(x, w):
+        return False
+    most = (16384 if x.shape[1] >= 512 else 8192) if x.shape[0] <= 1 else 6144 if x.shape[1] <= 1024 else 4096
+    return w.shape[0] <= most
 
 
 def rows_linear(x: torch.Tensor, w: torch.Tensor, out_dtype: torch.dtype, overlap_previous: bool = False) -> torch.Tensor:

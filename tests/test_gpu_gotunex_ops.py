@@ -152,6 +152,16 @@ def test_rows_linear_refuses_what_it_does_not_take(dev):
     assert kn.rows_linear(x, w[:0], F32).shape == (2, 0)
 
 
+@pytest.mark.parametrize("n,k,most", [(1, 256, 8192), (1, 512, 16384), (2, 1024, 6144), (2, 1032, 4096)])
+def test_rows_linear_up_to_a_number_of_features(dev, n, k, most):
+    """The rule's lines, and the product at them."""
+    g = torch.Generator(device=dev).manual_seed(k)
+    x, w = torch.randn(n, k, generator=g, device=dev).to(BF), torch.randn(most + 1, k, generator=g, device=dev).to(BF)
+    assert kn.takes_few_rows(x, w[:most]) and not kn.takes_few_rows(x, w)
+    want, size = x.double() @ w.double().T, x.double().abs() @ w.double().abs().T
+    assert bool(((kn.rows_linear(x, w, F32).double() - want).abs() <= (k / 32 + 8) * 2.0 ** -24 * size).all())  # as above
+
+
 # ---- experts ---------------------------------------------------------------------------------------------------------
 def expert_case(dev, dtype, n, width, experts, top, ff, seed, ids=None, vocab=61):
     g = gen(seed)
