@@ -698,6 +698,8 @@ typedef struct spk_experts_args {
     int32_t gated;
     int32_t dtype;
     int32_t overlap;            /* the call directly follows the one that writes x, and every earlier launch was complete when that began */
+    int32_t beside;             /* launches of another stream run beside this one and should find SMs free: few tokens leave them some (SPK_BF16) */
+    int32_t _pad;
     uint32_t* status;
 } spk_experts_args;
 int spk_experts(const spk_experts_args* args, void* stream);

@@ -149,7 +149,7 @@ class ExpertRouteArgs(Structure):
 class ExpertsArgs(Structure):
     """Mirror of ``spk_experts_args``."""
 
-    _fields_ = _fields("p x w out segs; l rows pairs; i experts k out_features gated dtype overlap; p status")
+    _fields_ = _fields("p x w out segs; l rows pairs; i experts k out_features gated dtype overlap beside _pad; p status")
 
 
 class LatentPrepareArgs(Structure):

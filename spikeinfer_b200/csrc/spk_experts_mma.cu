@@ -8,7 +8,7 @@
 //    tiles of the next product.
 //  * plain: 256 consecutive output features, 32-bit rows.
 //
-// Few tokens: the time is that of streaming the weights, experts_stream_kernel.  The plain product's are on their way before the gated one is done.
+// Few tokens: the time is that of streaming the weights, beside other launches by experts_stream_kernel.  The plain product's are on their way before the gated one is done.
 // Where few blocks are streamed, a cluster of S CTAs shares a block, each over its own part of k; the partial sums meet in shared memory and are
 // added in the order of the CTAs, so results don't depend on timing.
 // Warp 0 copies, warp 1 issues MMAs, the others write the results.  A tile of 64 tokens and more has eight of them, each with half of the tokens: a
@@ -239,7 +239,7 @@ experts_kernel(const spk_experts_args a, const int blocks, const int ktiles) {
     if (warp == 0) tmem_dealloc(tmem, Sh::kColumns);
 }
 
-// Few tokens per expert: the CTAs go over the blocks of all experts, the copies of the next block under way while the last stages of this one are
+// Few tokens per expert, beside another stream's launches: the CTAs go over the blocks of all experts, the copies of the next block under way while the last stages of this one are
 // multiplied and its results written (two sets of accumulators).  What bounds it is HBM, shared with the mixer's launches beside it, and those
 // need whole SMs for their products: so one CTA per SM with six stages, no more of them than kStreamCtas, and the next launch's CTAs are let in
 // when the copies are all under way.  16 experts of 896 x 1216, whole decode steps of four, 64 rows: a CTA per block, two per SM (160 blocks) 6285 us;
@@ -477,10 +477,12 @@ int dispatch(const spk_experts_args& a, cudaStream_t s) {
     // 3310 us (the second product in two parts already), 3195, 3078, 3090; two users 3510, 3370, 3255, 3415; four (the second product alone) 3830, 3675,
     // 3680, 3690.  With library products in the mixer, which want whole SMs, four parts were slower than two (4260 against 4103 us).
     if (blocks * (a.pairs < a.experts ? a.pairs : a.experts) <= 40 && ktiles >= 4) return launch<32, GATED, 4>(a, blocks, ktiles, s);
-    // Weights of more than 256 MB outlast the mixer beside them: a CTA per block, two to an SM, takes all of HBM's rate (16 experts of 3584 x 4736, 64 rows,
-    // both products: 243 us against 291 by the streaming form's CTAs).
+    // Alone a CTA per block, two to an SM, takes more of HBM's rate than the streaming form, whose fewer CTAs leave SMs to what runs beside it.  Both products of 8 and 64 tokens, us, a CTA
+    // per block / streaming: 16 experts of 896 x 1216 21.1 / 29.0, 27.9 / 32.4; 64 of 1024 x 640, four per token 21.3 / 37.6, 49.2 / 66.3; 8 of 2048 x 2048 41.3 / 53.0, 44.1 / 53.8.
+    // Whole Gotunex steps of four, the same two: 0.5b (16 of 896 x 1216) four rows 4293 / 3860, 8 rows 4277 / 4500, 16 4646 / 4789, 30 4988 / 4962, 48 5470 / 5221.  Weights of more
+    // than 256 MB outlast the mixer beside them (16 of 3584 x 4736, 64 rows: 243 / 291 alone).
     const int64_t expected = static_cast<int64_t>(blocks) * (a.pairs < a.experts ? a.pairs : a.experts);
-    if (expected * ktiles * (2 * kTileW) > (256ll << 20)) return launch<32, GATED, 1>(a, blocks, ktiles, s);
+    if (!a.beside || expected * ktiles * (2 * kTileW) > (256ll << 20)) return launch<32, GATED, 1>(a, blocks, ktiles, s);
     return launch_stream<GATED>(a, blocks, ktiles, s);
 }
 

@@ -115,14 +115,16 @@ class ExpertRouter:
         return out
 
 
-def experts_forward(x: torch.Tensor, w: ExpertWeights, route: LayerRoute, status: torch.Tensor | None = None) -> torch.Tensor:
-    """Every expert's feed-forward on its rows of the sorted matrix ``x``: fp32 ``[rows, width]``, unweighted."""
+def experts_forward(x: torch.Tensor, w: ExpertWeights, route: LayerRoute, status: torch.Tensor | None = None, beside: bool = False) -> torch.Tensor:
+    """Every expert's feed-forward on its rows of the sorted matrix ``x``: fp32 ``[rows, width]``, unweighted.  ``beside``: another stream's launches run at
+    the same time and should find SMs free (the products alone take longer then)."""
     _lib.require_cuda(x, "experts_forward input")
     n = route.slots.shape[0]
     rows = w.rows(n)
     hidden = w.sorted_matrix(n, w.ff)
     out = torch.empty((rows, w.width), dtype=torch.float32, device=x.device)
-    common = dict(segs=route.segs.data_ptr(), rows=rows, pairs=n * w.top, experts=w.experts, dtype=_lib.dtype_code(w.dtype), status=_ptr(status))
+    common = dict(segs=route.segs.data_ptr(), rows=rows, pairs=n * w.top, experts=w.experts, dtype=_lib.dtype_code(w.dtype), beside=int(beside),
+                  status=_ptr(status))
     _call("spk_experts", _lib.ExpertsArgs(x=x.data_ptr(), w=w.w_in.data_ptr(), out=hidden.data_ptr(), k=w.width, out_features=w.ff, gated=1, **common),
           x.device)
     _call("spk_experts", _lib.ExpertsArgs(x=hidden.data_ptr(), w=w.w_out.data_ptr(), out=out.data_ptr(), k=w.ff, out_features=w.width, gated=0,

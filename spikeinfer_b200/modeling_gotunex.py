@@ -340,7 +340,7 @@ class GotunexModel:
                 gelu_tanh(self._matmul(hand["out2"], L.up), both[:, mixed:])
             elif L.experts is not None:
                 route = routes[L.route_index]
-                added = dict(pairs=experts_forward(hand["out2"], L.experts, route, meta.status), pair_slots=route.slots, pair_scale=1.0 / L.experts.top)
+                added = dict(pairs=experts_forward(hand["out2"], L.experts, route, meta.status, beside), pair_slots=route.slots, pair_scale=1.0 / L.experts.top)
             if beside:
                 main.wait_stream(self._side)
             if L.up is not None:

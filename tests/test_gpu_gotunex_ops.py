@@ -176,7 +176,7 @@ def expert_case(dev, dtype, n, width, experts, top, ff, seed, ids=None, vocab=61
     return w, weights, ids, torch.randn(n, width, generator=g).to(dtype), dict(router=dict(experts=experts, top=top))
 
 
-def run_experts(dev, status, weights, ids, x, active=None):
+def run_experts(dev, status, weights, ids, x, active=None, beside=False):
     vocab = weights.table.shape[0]
     route = ke.ExpertRouter([weights], vocab)(ids.to(dev), active, status)[0]
     n, width = x.shape
@@ -186,7 +186,7 @@ def run_experts(dev, status, weights, ids, x, active=None):
     # a norm of weight root-mean-square hands the rows on as they are: use rows of unit mean square
     kn.rms_residual(eps=0.0, x=x.float().to(dev), w1=ones, out1=torch.empty(n, width, dtype=weights.dtype, device=dev), w2=ones, out2=xs,
                     out2_slots=route.slots, out2_tiled=weights.tiled, status=status)
-    return route, ke.experts_forward(xs, weights, route, status)
+    return route, ke.experts_forward(xs, weights, route, status, beside)
 
 
 @pytest.mark.parametrize("dtype", DTYPES)
@@ -204,9 +204,9 @@ def test_experts(dev, status, n, width, experts, top, ff, dtype):
     assert rel(got, want) < (3e-6 if dtype == F32 else 8e-3)
 
 
-@pytest.mark.parametrize("n,width,experts,top,ff", [(2, 896, 16, 2, 1216), (5, 896, 16, 2, 1216), (1, 256, 9, 1, 200), (1, 200, 9, 1, 256), (20, 320, 1, 1, 640)])
+@pytest.mark.parametrize("n,width,experts,top,ff", [(2, 896, 16, 2, 1216), (5, 896, 16, 2, 1216), (1, 256, 9, 1, 200), (1, 200, 9, 1, 256), (16, 320, 1, 1, 640)])
 def test_experts_of_few_blocks_in_four_parts(dev, status, n, width, experts, top, ff):
-    """Both products, one of them, or neither in four parts of k; four tiles of k and more, unequal parts, one to 20 rows; twice the same bits."""
+    """Both products or one of them in four parts of k; four tiles of k and more, unequal parts, one to 16 rows; twice the same bits."""
     w, weights, ids, x, cfg = expert_case(dev, BF, n, width, experts, top, ff, n + ff)
     x = go.rms(x.double(), 0.0)
     route, out = run_experts(dev, status, weights, ids, x)
@@ -216,22 +216,25 @@ def test_experts_of_few_blocks_in_four_parts(dev, status, n, width, experts, top
     assert torch.equal(out2[again.slots.long()], out[route.slots.long()])
 
 
-@pytest.mark.parametrize("n,width,experts,top,ff", [(60, 130, 40, 2, 1300), (24, 1024, 30, 4, 64), (100, 448, 8, 1, 384), (90, 64, 96, 2, 640),
-                                                    (7, 900, 12, 3, 130)])
-def test_experts_streamed_over_several_blocks_a_cta(dev, status, n, width, experts, top, ff):
-    """More blocks than the streaming kernel has CTAs (440, 120, 24, 480, 24 gated ones), a CTA's rounds unequal, fewer and more k tiles than stages, one
-    k tile, several runs of tokens per expert, experts without tokens."""
-    w, weights, ids, x, cfg = expert_case(dev, BF, n, width, experts, top, ff, n + ff)
+@pytest.mark.parametrize("n,width,experts,top,ff,same", [(60, 130, 40, 2, 1300, False), (24, 1024, 30, 4, 64, False), (90, 64, 96, 2, 640, False),
+                                                         (7, 900, 12, 3, 130, False), (30, 896, 40, 2, 640, False), (64, 896, 16, 2, 1216, True)])
+def test_experts_streamed_over_several_blocks_a_cta(dev, status, n, width, experts, top, ff, same):
+    """Beside other launches.  Blocks of the gated and the plain product (in brackets: shared by four CTAs each instead): 440 (40), (30) 120, 480 96, (24) 48, 200 160, 160 64;
+    a CTA goes over one to five of them, with fewer and more k tiles than stages and one k tile; the second product's first stages are asked for ahead of its x and its ring wraps
+    into the next block (160 blocks of ten k tiles); every token at the same two experts (two runs of 32 rows each); experts without tokens.  The bits of a CTA per block."""
+    w, weights, ids, x, cfg = expert_case(dev, BF, n, width, experts, top, ff, n + ff, ids=torch.full((n,), 7) if same else None)
     x = go.rms(x.double(), 0.0)
+    want = go.table_experts(x, ids.tolist(), go.as_float(w), "", cfg)
+    alone, out1 = run_experts(dev, status, weights, ids, x)
     for _ in range(3):
-        route, out = run_experts(dev, status, weights, ids, x)
-        got = out.cpu().double()[route.slots.cpu().long()].mean(1)
-        assert rel(got, go.table_experts(x, ids.tolist(), go.as_float(w), "", cfg)) < 8e-3
+        route, out = run_experts(dev, status, weights, ids, x, beside=True)
+        assert rel(out.cpu().double()[route.slots.cpu().long()].mean(1), want) < 8e-3
+        assert torch.equal(out[route.slots.long()], out1[alone.slots.long()])
 
 
 @pytest.mark.parametrize("n,width,experts,top,ff", [(1, 896, 16, 2, 1216), (2, 72, 16, 2, 65), (3, 300, 4, 2, 129), (16, 200, 2, 2, 1000), (32, 264, 2, 1, 130)])
 def test_experts_of_few_tokens(dev, status, n, width, experts, top, ff):
-    """The forms that share a block of the second product between two CTAs: two to nineteen k tiles, one to 32 rows per expert; twice the same bits."""
+    """Two to nineteen k tiles, one to 32 rows per expert: blocks shared by four CTAs, a CTA per block, tiles of 64 tokens; twice the same bits."""
     w, weights, ids, x, cfg = expert_case(dev, BF, n, width, experts, top, ff, n + ff)
     x = go.rms(x.double(), 0.0)
     route, out = run_experts(dev, status, weights, ids, x)
