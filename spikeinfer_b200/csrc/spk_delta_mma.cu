@@ -454,7 +454,7 @@ delta_chain_kernel(const spk_delta_args a, const int64_t image_bytes, float* __r
             int issued = 0;
             for (int c = 0; c < sq.y; ++c) {
                 const int st = c % NS;
-                if (c >= NS && !mbar_wait(smem_u32(empty + st), ((c / NS) - 1) & 1, abort)) break;
+                if (c >= NS && !mbar_wait<1>(smem_u32(empty + st), ((c / NS) - 1) & 1, abort)) break;
                 const uint8_t* src = static_cast<const uint8_t*>(a.workspace) + (static_cast<int64_t>(sq.x + c) * a.heads + h) * image_bytes;
                 const uint32_t bar = smem_u32(full + st), dst = smem_u32(base + st * K::kStage);
                 mbar_expect(bar, K::kHead + K::kU);
@@ -484,7 +484,7 @@ delta_chain_kernel(const spk_delta_args a, const int64_t image_bytes, float* __r
         spk_grid_wait();  // and the convolutions' past has been read
         for (int c = 0; c < sq.y; ++c) {
             const int st = c % NS;
-            if (!__all_sync(~0u, mbar_wait(smem_u32(full + st), (c / NS) & 1, abort))) break;
+            if (!__all_sync(~0u, mbar_wait<1>(smem_u32(full + st), (c / NS) & 1, abort))) break;
             const uint8_t* im = base + st * K::kStage;
             const uint32_t at = smem_u32(im);
             if (live) {
