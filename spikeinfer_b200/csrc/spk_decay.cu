@@ -538,9 +538,9 @@ int launch_gated(const spk_gated_norm_args& a, cudaStream_t s) {
         const int threads = groups <= 128 && a.partials == nullptr ? 128 : kThreads;
         const int v = (groups + threads - 1) / threads;
         if (v <= 1) gated_norm_vec_kernel<T, 1><<<grid, threads, 0, s>>>(a);
-        // Two groups a thread: 78 registers (a bound of one CTA) for the loads of a batch row's partial sums, 64 otherwise.  Without / with that bound, us: 2048 columns beside eight
-        // partial sums, 64 rows 5.2 / 4.0; no partial sums, 592 rows 3.9 / 4.6, 8192 35.6 / 43.1.
-        else if (v <= 2 && a.partials != nullptr) gated_norm_vec_kernel<T, 2, 1><<<grid, threads, 0, s>>>(a);
+        // Two groups a thread: 78 registers (a bound of one CTA) for the loads of a batch row and its partial sums, 64 for more rows.  Without / with that bound, us: 2048 columns
+        // beside eight partial sums, 64 rows 5.2 / 4.0; no partial sums, 256 rows 2.95 / 2.87, 592 3.9 / 4.6, 8192 35.6 / 43.1.
+        else if (v <= 2 && (a.partials != nullptr || a.n <= 2 * 148)) gated_norm_vec_kernel<T, 2, 1><<<grid, threads, 0, s>>>(a);
         else if (v <= 2) gated_norm_vec_kernel<T, 2><<<grid, threads, 0, s>>>(a);
         // Four CTAs per SM (64 registers and spills) from sixteen rows per SM on.  Without / with them, rows of 3584, us of repeated calls on one set of buffers: 64 rows
         // 3.3 / 3.9 (beside partial sums 6.7 / 9.2), 592 6.2 / 7.1, 2048 18.1 / 19.4, 2368 21.3 / 21.4, 2800 26.6 / 25.0, 4096 42.9 / 36.2; six sets in turn: 2048 23.2 / 20.9,

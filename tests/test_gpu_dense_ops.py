@@ -239,9 +239,9 @@ def test_gated_norm_of_many_rows_gives_the_bits_of_few(dev, dtype, n, width):
 
 
 @pytest.mark.parametrize("dtype", DTYPES)
-@pytest.mark.parametrize("width", [2052, 3584, 4096])
+@pytest.mark.parametrize("width", [1028, 2048, 2052, 3584, 4096])
 def test_gated_norm_of_many_wide_rows_gives_the_bits_of_few(dev, dtype, width):
-    """From 16 rows per SM on, rows of more than 2048 columns take a form with more CTAs per SM."""
+    """From 16 rows per SM on, rows of more than 2048 columns take a form with more CTAs per SM; up to two rows per SM, those of up to 2048 one with more registers."""
     n = 16 * 148
     g = torch.Generator(device=dev).manual_seed(width)
     x, w = torch.randn(n, width, generator=g, device=dev), 1 + 0.3 * torch.randn(width, generator=g, device=dev)
