@@ -16,7 +16,6 @@ import statistics
 from pathlib import Path
 
 import torch
-import torch.nn.functional as F
 
 BF = torch.bfloat16
 FALLBACK = {"hbm_gbs": 6650.0, "bf16_tflops": 1590.0}
@@ -263,7 +262,6 @@ def spiking_kernels(shape: str, device, repeats: int, pk: dict) -> dict:
     """The spiking model's kernels in the same parts, at the same width, heads and token counts (T = 4)."""
     import bench
     from spikeinfer_b200 import kernels
-    from spikeinfer_b200.attention import _causal_offset_mask
 
     cfg = manirax_config(shape)
     L = cfg["layers"][0]["mixer"]["left"]
@@ -306,13 +304,18 @@ def spiking_kernels(shape: str, device, repeats: int, pk: dict) -> dict:
         out[f"paged_spike_attn decode {rows}x{keys}"] = {"us": t["us_per_call"], "MB": round(t["algorithmic_bytes"] / 1e6, 2),
                                                          "frac": t["frac"], "bound": "hbm"}
     for seqs, n in ((16, 512), (1, 4096)):
-        mask = _causal_offset_mask(n, n, device, BF)
+        nb = seqs * n // 16
+        tables = list(torch.randperm(nb, device=device, dtype=torch.int32).view(seqs, -1))
+        starts = [i * n for i in range(seqs)]
 
-        def mk_sdpa():
-            q, k, v = rnd(T * seqs, H, n, D), rnd(T * seqs, G, n, D), rnd(T * seqs, G, n, D)
-            return lambda: F.scaled_dot_product_attention(q, k, v, attn_mask=mask, enable_gqa=True)
-        nbytes = T * seqs * n * (2 * H + 2 * G) * D * 2
-        add(f"prefill attention (SDPA on unpacked spikes) {seqs}x{n}", mk_sdpa, nbytes, T * seqs * n * (n + 1) // 2 * H * 4 * D)
+        def mk_pre():
+            word = lambda *s: torch.randint(-2 ** 31, 2 ** 31, s, device=device, dtype=torch.int32)
+            q, k, v = word(T, seqs * n, H, D // 32), word(T, G, nb * 16, D // 32), word(T, G, nb * 16, D // 32)
+            o = torch.empty(T, seqs * n, H, D, dtype=BF, device=device)
+            return lambda: kernels.paged_spike_attn_prefill(q, k, v, tables, starts, [n] * seqs, [0] * seqs, o, head_dim=D, block_size=16, num_q_heads=H,
+                                                            num_kv_heads=G)
+        nbytes = T * seqs * n * (H * D // 8 + 2 * G * D // 8 + H * D * 2)
+        add(f"paged_spike_attn prefill {seqs}x{n}", mk_pre, nbytes, T * seqs * n * (n + 1) // 2 * H * 4 * D)
     return out
 
 

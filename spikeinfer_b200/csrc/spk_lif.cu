@@ -517,7 +517,7 @@ __device__ __forceinline__ void fused_site_vec(const spk_lif_site& s, uint32_t u
         if (has_packed && s.slot_mapping != nullptr) {
             out_row = s.slot_mapping[tok];
             row_ok = out_row >= 0 && out_row < s.num_rows;
-            // A branch on it here holds the loads of a small launch's currents back (8 decode rows: 136.6 -> 133.1 us for 24 layers); where the currents
+            // A branch on it here holds the loads of a small launch's currents back (8 decode rows, 24 layers with their attention launches: 143.2 -> 141.4 us); where the currents
             // are on their way already it is the better place (LIF of 8192 x 4864 in one pass: 138 us, 143 with a flag at the end).
             if (ASYNC && !row_ok && sg == 0) spk_flag(status, SPK_STATUS_BAD_SLOT);
         }
